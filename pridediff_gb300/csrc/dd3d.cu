@@ -12,11 +12,11 @@
 // walked line are contiguous in both branches.
 //
 // Adjoint-type operators (ProjTrans, BackProj, BackProjWeighted): one thread
-// per (x, y) voxel column, 8 slices and 2 volumes loops over the views; for
-// each view it enumerates the segments of its pixel with the detector columns
-// (dd3_pixwalk_*) and gathers the rows that meet each slice from a sinogram
-// pre-multiplied by the per-bin scale.  A per-CTA test skips views whose
-// detector cannot see the CTA's slab (most views of a spiral scan).
+// per (x, y) voxel column, 16 or 8 slices and 2 or 1 volumes loops over the
+// views; for each view it enumerates the segments of its pixel with the
+// detector columns and merges the column's rows with its slices, reading a
+// sinogram pre-multiplied by the per-bin scale.  Views whose detector cannot
+// see the CTA's slices (most views of a spiral scan) are left out of its list.
 //
 // Both directions use the same segment widths and z-walk widths, so they are
 // exact transposes of each other; no atomics, deterministic results.
@@ -38,9 +38,9 @@ void count_launches(int n);
 namespace dd3 {
 
 constexpr int kThreads = 256;
-constexpr int kNB = 2;     // volumes per thread
+constexpr int kNB = 2;     // volumes per thread (an odd last volume runs on its own)
 constexpr int kTile = 16;  // adjoint: 16 x 16 voxel columns per CTA
-constexpr int kZS = 8;     // adjoint: slices per thread
+constexpr int kZS = 8;     // adjoint: slices of a slab (a thread takes one slab or two)
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -49,7 +49,7 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // ---------------------------------------------------------------------------
 // Per-view tables are padded to 16-byte rows so that one view's row can be
 // moved by a single bulk copy: dp (C+1 column boundaries), mag (C column
-// magnifications), rowz (R x {row0z, row1z}).
+// magnifications), rowz (R x {row0z, row1z}, closed by a row at infinity).
 struct PlanLayout {
     size_t views, dp, mag, rowz, linez, lines, slabv, total;
     int nl, nch, sdp, smag, srz, nslab;
@@ -64,13 +64,14 @@ inline PlanLayout plan_layout(const dd_geom3d *g, int V) {
     L.nch = (C + DD3_CHUNK - 1) / DD3_CHUNK;
     L.sdp = pad4(C + 1);
     L.smag = pad4(C);
-    L.srz = pad4(2 * R);
+    L.srz = pad4(2 * R + 2);
     size_t o = 0;
     L.views = o; o = align_up(o + sizeof(DdView3) * (size_t)V, 256);
     L.dp = o; o = align_up(o + sizeof(float) * (size_t)V * L.sdp, 256);
     L.mag = o; o = align_up(o + sizeof(float) * (size_t)V * L.smag, 256);
     L.rowz = o; o = align_up(o + sizeof(float) * (size_t)V * L.srz, 256);
     L.linez = o; o = align_up(o + sizeof(float4) * (size_t)V * L.nl, 256);
+    // line records [view][walk block][line]: a tile's 16 lines of one block are contiguous
     L.lines = o; o = align_up(o + sizeof(DdLine) * (size_t)V * L.nl * L.nch, 256);
     L.nslab = (g->depth + kZS - 1) / kZS;   // the adjoint's slabs of kZS slices
     L.slabv = o; o = align_up(o + sizeof(int2) * (size_t)L.nslab, 256);
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(kThreads) k_views3(dd_geom3d g, const float *_
         mx = fmaxf(mx, m);
     }
     for (int r = tid; r < R; r += kThreads) dd3_row_z(GEOM, &g, &w, r, &rz[2 * r], &rz[2 * r + 1]);
+    if (tid < 2) rz[2 * R + tid] = __int_as_float(0x7f800000);   // +inf: ends the adjoint's row walks
     for (int o = 16; o > 0; o >>= 1) {
         mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -154,6 +156,7 @@ __global__ void __launch_bounds__(kThreads) k_views3(dd_geom3d g, const float *_
         dd3_row_z(GEOM, &g, &w, R - 1, &b0, &b1);
         out.rzA = a0;
         out.rzB = (R > 1) ? (b0 - a0) / (float)(R - 1) : a1 - a0;
+        out.rzI = 1.0f / out.rzB;
         reinterpret_cast<DdView3 *>(plan + P.views)[v] = out;
     }
 }
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(128) k_lines3(dd_geom3d g, char *plan, PlanLay
     if (line >= nline) return;
     const DdView3 w = views[v];
     const float *dp = reinterpret_cast<const float *>(plan + P.dp) + (size_t)v * P.sdp;
-    DdLine *L = reinterpret_cast<DdLine *>(plan + P.lines) + ((size_t)v * P.nl + line) * P.nch + cc;
+    DdLine *L = reinterpret_cast<DdLine *>(plan + P.lines) + ((size_t)v * P.nch + cc) * P.nl + line;
     float lz[4];
     dd3_line_setup(GEOM, &g, &w, dp, line, cc, lz, L);
     if (cc == 0)
@@ -201,8 +204,26 @@ __global__ void __launch_bounds__(256) k_transpose3(const float *__restrict__ in
     }
 }
 
-// ss[b][v][r][k] = in[b][v][r][k'] * scale(v, r, k) with k the sorted column:
-// the adjoint gathers pre-scaled bins (ConeFlatDisCUDA3d.cu:400-404).
+// One volume's value, or two volumes' side by side: the adjoint's gathers move
+// both with one 8-byte load.
+template <int NB> struct Vox;
+template <> struct Vox<1> {
+    using T = float;
+    static __device__ __forceinline__ T zero() { return 0.0f; }
+    static __device__ __forceinline__ T fma(float w, T x, T a) { return fmaf(w, x, a); }
+    static __device__ __forceinline__ float get(T x, int) { return x; }
+};
+template <> struct Vox<2> {
+    using T = float2;
+    static __device__ __forceinline__ T zero() { return make_float2(0.0f, 0.0f); }
+    static __device__ __forceinline__ T fma(float w, T x, T a) { return make_float2(fmaf(w, x.x, a.x), fmaf(w, x.y, a.y)); }
+    static __device__ __forceinline__ float get(T x, int b) { return b ? x.y : x.x; }
+};
+
+// ss[v][r][k][b] = in[b][v][r][k'] * scale(v, r, k) with k the sorted column:
+// the adjoint gathers pre-scaled bins (ConeFlatDisCUDA3d.cu:400-404), the
+// volumes of a group of kNB next to each other (an odd last volume forms a
+// group of its own).
 template <int GEOM, int FAMILY>
 __global__ void __launch_bounds__(128) k_sino3(dd_geom3d g, const char *__restrict__ plan, PlanLayout P,
                                                const float *__restrict__ in, float *__restrict__ ss, int B, int V) {
@@ -222,7 +243,11 @@ __global__ void __launch_bounds__(128) k_sino3(dd_geom3d g, const char *__restri
     const int ko = w.flip ? C - 1 - k : k;
     const size_t per = (size_t)V * R * C;
     const size_t row = ((size_t)v * R + r) * C;
-    for (int b = 0; b < B; b++) ss[b * per + row + k] = FMUL(in[b * per + row + ko], scale);
+    int b = 0;
+    for (; b + 1 < B; b += 2)
+        reinterpret_cast<float2 *>(ss + b * per)[row + k] =
+            make_float2(FMUL(in[b * per + row + ko], scale), FMUL(in[(b + 1) * per + row + ko], scale));
+    if (b < B) ss[b * per + row + k] = FMUL(in[b * per + row + ko], scale);
 }
 
 // ---------------------------------------------------------------------------
@@ -285,7 +310,7 @@ __global__ void __launch_bounds__(kFwdThreads3, 3) k_fwd3(const Fwd3Args a) {
     const float *__restrict__ dpv = reinterpret_cast<const float *>(a.plan + P.dp) + (size_t)v * P.sdp;
     const float *__restrict__ rz = reinterpret_cast<const float *>(a.plan + P.rowz) + (size_t)v * P.srz;
     const float4 *__restrict__ linez = reinterpret_cast<const float4 *>(a.plan + P.linez) + (size_t)v * P.nl;
-    const DdLine *__restrict__ lines = reinterpret_cast<const DdLine *>(a.plan + P.lines) + (size_t)v * P.nl * P.nch + cc;
+    const DdLine *__restrict__ lines = reinterpret_cast<const DdLine *>(a.plan + P.lines) + ((size_t)v * P.nch + cc) * P.nl;
     if (tid <= kFC) sdp[tid] = dpv[min(cg * kFC + tid, C)];
     if (tid == 0) {
         abort_flag = 0;
@@ -301,7 +326,7 @@ __global__ void __launch_bounds__(kFwdThreads3, 3) k_fwd3(const Fwd3Args a) {
     auto issue = [&](int line, int buf) {
         nissue[buf]++;
         dd_mbar_expect_tx(&bar[buf], (uint32_t)(sizeof(DdLine) + sizeof(float4)));
-        dd_bulk_g2s(&srec[buf], lines + (size_t)line * P.nch, (uint32_t)sizeof(DdLine), &bar[buf]);
+        dd_bulk_g2s(&srec[buf], lines + line, (uint32_t)sizeof(DdLine), &bar[buf]);
         dd_bulk_g2s(&slzr[buf], linez + line, (uint32_t)sizeof(float4), &bar[buf]);
     };
     // segments of line m (record buffer m & 1) into segment buffer sb; one warp
@@ -401,7 +426,7 @@ __global__ void __launch_bounds__(kFwdThreads3, 3) k_fwd3(const Fwd3Args a) {
                 }
             } else {
                 // wide column: walk the record in global memory
-                const DdLine *Lg = lines + (size_t)line * P.nch;
+                const DdLine *Lg = lines + line;
                 const float lpos = (FAMILY == 2) ? dd3_line_pos(&g, &w, line) : 0.0f;
                 DdColWalk cw;
                 if (dd3_colwalk_init(Lg, sdp, lane, kk, &cw)) {
@@ -469,18 +494,21 @@ struct Adj3Args {
     dd_geom3d g;
     const char *plan;
     PlanLayout P;
-    const float *ss;     // pre-scaled sinogram (B, V, R, C), sorted columns
+    const float *ss;     // pre-scaled sinogram, groups of (V, R, C, volumes), sorted columns
     float *out;          // (B, Dep, H, W)
     const float *base;   // optional: out = base + scale * value (may alias out)
     float scale;
     int *status;
     int B, V, ntx;
+    int b0, family;      // first volume of the launch; operator family (dd3_coef)
 };
 
-// Shared memory of the adjoint kernel: two buffers of one view's data (the
-// records of the tile's 16 lines in every walk block, the column boundary,
-// column magnification and row tables, the lines' z quantities and the view
-// record), each moved by bulk copies; all sizes are multiples of 16 bytes.
+// Shared memory of the adjoint kernel: kAdj3Bufs buffers of one (view, walk
+// block)'s data (the records of the tile's 16 lines, the block's column
+// boundary and magnification tables, the row table, the lines' z quantities
+// and the view record), each moved by bulk copies; all sizes are multiples of
+// 16 bytes.
+constexpr int kAdj3Bufs = 3;
 struct Adj3Smem {
     int rec, dp, mag, rz, lz, vw, bar, total;
     uint32_t rec_b, dp_b, mag_b, rz_b, lz_b;
@@ -488,30 +516,38 @@ struct Adj3Smem {
 
 __host__ __device__ inline Adj3Smem adj3_smem(const PlanLayout &P) {
     Adj3Smem s;
-    s.rec_b = (uint32_t)(kTile * P.nch * sizeof(DdLine));
-    s.dp_b = (uint32_t)(P.sdp * sizeof(float));
-    s.mag_b = (uint32_t)(P.smag * sizeof(float));
+    s.rec_b = (uint32_t)(kTile * sizeof(DdLine));
+    s.dp_b = (uint32_t)((DD3_CHUNK + 4) * sizeof(float));
+    s.mag_b = (uint32_t)(DD3_CHUNK * sizeof(float));
     s.rz_b = (uint32_t)(P.srz * sizeof(float));
     s.lz_b = (uint32_t)(kTile * sizeof(float4));
     int o = 0;
-    s.rec = o; o += 2 * (int)s.rec_b;
-    s.dp = o; o += 2 * (int)s.dp_b;
-    s.mag = o; o += 2 * (int)s.mag_b;
-    s.rz = o; o += 2 * (int)s.rz_b;
-    s.lz = o; o += 2 * (int)s.lz_b;
-    s.vw = o; o += 2 * (int)sizeof(DdView3);
-    s.bar = o; o += 2 * (int)sizeof(uint64_t);
+    s.rec = o; o += kAdj3Bufs * (int)s.rec_b;
+    s.dp = o; o += kAdj3Bufs * (int)s.dp_b;
+    s.mag = o; o += kAdj3Bufs * (int)s.mag_b;
+    s.rz = o; o += kAdj3Bufs * (int)s.rz_b;
+    s.lz = o; o += kAdj3Bufs * (int)s.lz_b;
+    s.vw = o; o += kAdj3Bufs * (int)sizeof(DdView3);
+    s.bar = o; o += kAdj3Bufs * (int)sizeof(uint64_t);
     s.total = (o + 127) & ~127;
     return s;
 }
 
-// Can view w see the slab of slices [s0, s0 + kZS) on the walked lines
+// The size limit of a view's tables: what two buffers of a whole view (all
+// its walk blocks) take beside 200 KB.
+inline bool view_too_wide(const PlanLayout &P, int R) {
+    const size_t one = (size_t)kTile * P.nch * sizeof(DdLine) + sizeof(float) * ((size_t)P.sdp + P.smag + pad4(2 * R)) +
+                       kTile * sizeof(float4) + sizeof(DdView3) + sizeof(uint64_t);
+    return (2 * one + 127) / 128 * 128 > 200 * 1024;
+}
+
+// Can view w see the slab of slices [s0, s0 + ns) on the walked lines
 // l0..l1 (with one slice of margin)?
 __device__ __forceinline__ bool slab_visible(const dd_geom3d &g, const DdView3 &w, int l0, int l1, int s0,
-                                             float zr0, float zr1) {
-    const float m0 = dd3_line_mag(&w, dd3_line_pos(&g, &w, l0));
-    const float m1 = dd3_line_mag(&w, dd3_line_pos(&g, &w, l1));
-    const float zsA = w.z0 + (float)(s0 - 1) * g.pix_z, zsB = w.z0 + (float)(s0 + kZS + 1) * g.pix_z;
+                                             int ns, float zr0, float zr1) {
+    const float m0 = dd3_line_mag(&w, dd3_line_pos_f(&g, &w, l0));
+    const float m1 = dd3_line_mag(&w, dd3_line_pos_f(&g, &w, l1));
+    const float zsA = w.z0 + (float)(s0 - 1) * g.pix_z, zsB = w.z0 + (float)(s0 + ns + 1) * g.pix_z;
     return dd3_slab_lit(&w, fminf(m0, m1), fmaxf(m0, m1), zsA, zsB, zr0, zr1);
 }
 
@@ -536,7 +572,7 @@ __global__ void __launch_bounds__(256) k_slab_views3(dd_geom3d g, char *plan, Pl
         const DdView3 w = views[v];
         const int nline = w.xb ? g.height : g.width;
         const float *rzv = rzt + (size_t)v * P.srz;
-        if (slab_visible(g, w, 0, nline - 1, slab * kZS, rzv[0], rzv[2 * R - 1])) {
+        if (slab_visible(g, w, 0, nline - 1, slab * kZS, kZS, rzv[0], rzv[2 * R - 1])) {
             mylo = min(mylo, v);
             myhi = max(myhi, v);
         }
@@ -548,23 +584,43 @@ __global__ void __launch_bounds__(256) k_slab_views3(dd_geom3d g, char *plan, Pl
         reinterpret_cast<int2 *>(plan + P.slabv)[slab] = hi >= lo ? make_int2(lo, hi + 1) : make_int2(0, 0);
 }
 
-// grid: (voxel-column tile, slab of kZS slices, volume group); thread = one
-// (x, y) voxel column of a 16 x 16 tile.  Views whose detector cannot see the
-// slab are skipped when their copy would be issued.
-template <int GEOM, int FAMILY>
+// grid: (voxel-column tile, ZS slices, volume group); thread = one (x, y)
+// voxel column of a 16 x 16 tile.
+//
+// The work is a list of units (view, walk block of 256 columns).  Every 32
+// views each lane of a warp looks at one of them: whether its detector sees
+// the slab, which walk blocks the tile's shadow touches (one, or two where it
+// straddles a boundary), and the column grid linearised around the tile --
+// so views that miss the tile cost nothing, and a unit's records and tables
+// are all that is staged (three buffers, one CTA barrier per unit).
+//
+// Per segment (pixel, detector column) the thread walks its slices and the
+// column's rows together, in ascending z: the row that ends a slice is the
+// first candidate of the next one, so every row is projected (dd3_rp) and
+// loaded once per segment, and a step is an overlap of the two intervals and
+// one multiply-add per volume.
+//
+// Bound by instruction issue on that walk and on finding each pixel's columns
+// and boundaries, which ZS slices share.  One 512 x 512 x 128 volume, 1140
+// spiral views: 317 ms with a row search per slice, every walk block of every
+// view staged and searched, and 8 slices a thread; 192 ms with the carried
+// row walk alone; 108 ms with the unit list, the linear column estimate and
+// 16 slices.  2 x 256^3 cone beam, 360 views: 145, 63, 49 ms.
+template <int GEOM, int NB, int ZS>
 __global__ void __launch_bounds__(kThreads, 3) k_adj3(const Adj3Args a) {
+    using VT = Vox<NB>;
+    using T = typename VT::T;
     extern __shared__ __align__(128) unsigned char sm[];
     const dd_geom3d &g = a.g;
     const int W = g.width, H = g.height, Dp = g.depth, C = g.num_col, R = g.num_row;
     const PlanLayout &P = a.P;
     const Adj3Smem S = adj3_smem(P);
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
     const int tX = blockIdx.x % a.ntx, tY = blockIdx.x / a.ntx;
     const int xlo = tX * kTile, ylo = tY * kTile;
     const int x = xlo + (tid & (kTile - 1)), y = ylo + (tid / kTile);
     const bool active = x < W && y < H;
-    const int s0 = blockIdx.y * kZS, b0 = blockIdx.z * kNB;
-    const int nb = min(kNB, a.B - b0);
+    const int s0 = blockIdx.y * ZS, b0 = a.b0 + blockIdx.z * NB;
     const DdView3 *__restrict__ views = reinterpret_cast<const DdView3 *>(a.plan + P.views);
     const float *__restrict__ dpt = reinterpret_cast<const float *>(a.plan + P.dp);
     const float *__restrict__ magt = reinterpret_cast<const float *>(a.plan + P.mag);
@@ -572,145 +628,266 @@ __global__ void __launch_bounds__(kThreads, 3) k_adj3(const Adj3Args a) {
     const float4 *__restrict__ linez = reinterpret_cast<const float4 *>(a.plan + P.linez);
     const DdLine *__restrict__ lines = reinterpret_cast<const DdLine *>(a.plan + P.lines);
     const size_t per = (size_t)a.V * R * C;
-    const float *__restrict__ ssb = a.ss + (size_t)b0 * per;
+    const T *__restrict__ ssb = reinterpret_cast<const T *>(a.ss + (size_t)b0 * per);
+    const int family = a.family;
     uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S.bar);
     __shared__ int abort_flag;
-    __shared__ int seen[2];   // per buffer: 1 if the view sees the slab (data copied)
 
     if (tid == 0) {
         abort_flag = 0;
-        dd_mbar_init(&bar[0], 1);
-        dd_mbar_init(&bar[1], 1);
+        for (int i = 0; i < kAdj3Bufs; i++) dd_mbar_init(&bar[i], 1);
         dd_fence_mbar_init();
     }
     __syncthreads();
 
-    auto issue = [&](int v, int buf) {
-        const DdView3 wv = views[v];
-        const int xbv = wv.xb;
+    // a unit's copies (one thread)
+    auto issue = [&](int v, int cc, int buf) {
+        const int xbv = views[v].xb;
         const int l0 = xbv ? ylo : xlo;
         const int n = min(kTile, (xbv ? H : W) - l0);
-        const float *rzv = rzt + (size_t)v * P.srz;
-        const bool lit = slab_visible(g, wv, l0, l0 + n - 1, s0, rzv[0], rzv[2 * R - 1]);
-        seen[buf] = lit ? 1 : 0;
-        if (!lit) {
-            dd_mbar_expect_tx(&bar[buf], 0u);   // completes the phase with no data
-            return;
-        }
-        const uint32_t rb = (uint32_t)(n * P.nch * sizeof(DdLine)), lb = (uint32_t)(n * sizeof(float4));
-        dd_mbar_expect_tx(&bar[buf], rb + S.dp_b + S.mag_b + S.rz_b + lb + (uint32_t)sizeof(DdView3));
-        dd_bulk_g2s(sm + S.rec + buf * S.rec_b, lines + ((size_t)v * P.nl + l0) * P.nch, rb, &bar[buf]);
-        dd_bulk_g2s(sm + S.dp + buf * S.dp_b, dpt + (size_t)v * P.sdp, S.dp_b, &bar[buf]);
-        dd_bulk_g2s(sm + S.mag + buf * S.mag_b, magt + (size_t)v * P.smag, S.mag_b, &bar[buf]);
-        dd_bulk_g2s(sm + S.rz + buf * S.rz_b, rzv, S.rz_b, &bar[buf]);
+        const int c0 = cc * DD3_CHUNK;
+        const uint32_t rb = (uint32_t)(n * sizeof(DdLine)), lb = (uint32_t)(n * sizeof(float4));
+        const uint32_t db = (uint32_t)(min(DD3_CHUNK + 4, P.sdp - c0) * sizeof(float));
+        const uint32_t mb = (uint32_t)(min(DD3_CHUNK, P.smag - c0) * sizeof(float));
+        dd_mbar_expect_tx(&bar[buf], rb + db + mb + S.rz_b + lb + (uint32_t)sizeof(DdView3));
+        dd_bulk_g2s(sm + S.rec + buf * S.rec_b, lines + ((size_t)v * P.nch + cc) * P.nl + l0, rb, &bar[buf]);
+        dd_bulk_g2s(sm + S.dp + buf * S.dp_b, dpt + (size_t)v * P.sdp + c0, db, &bar[buf]);
+        dd_bulk_g2s(sm + S.mag + buf * S.mag_b, magt + (size_t)v * P.smag + c0, mb, &bar[buf]);
+        dd_bulk_g2s(sm + S.rz + buf * S.rz_b, rzt + (size_t)v * P.srz, S.rz_b, &bar[buf]);
         dd_bulk_g2s(sm + S.lz + buf * S.lz_b, linez + (size_t)v * P.nl + l0, lb, &bar[buf]);
         dd_bulk_g2s(sm + S.vw + buf * (int)sizeof(DdView3), views + v, (uint32_t)sizeof(DdView3), &bar[buf]);
     };
 
-    float acc[kZS][kNB];
+    // the views that can see the CTA's slices somewhere in the image
+    int2 vr = make_int2(a.V, 0);
+    for (int q = 0; q < ZS / kZS; q++) {
+        const int slab = s0 / kZS + q;
+        if (slab >= P.nslab) break;
+        const int2 r = reinterpret_cast<const int2 *>(a.plan + P.slabv)[slab];
+        if (r.x < r.y) {
+            vr.x = min(vr.x, r.x);
+            vr.y = max(vr.y, r.y);
+        }
+    }
+    const int ns = min(ZS, Dp - s0);
+
+    // The list of units, kept by the first warp: `next` writes one more (v < 0
+    // past the last) into its slot.  The lanes' views and what is known of
+    // them wait in shared memory, so that the walk below has the registers.
+    struct Unit {
+        int v, cc;
+        float A, B;   // column of axis position u: about A u + B
+    };
+    __shared__ Unit units[4];
+    __shared__ float la_s[32], lb_s[32];
+    __shared__ int cc_s[32];   // walk blocks of the lane's view: first | last << 16
+    int vbase = vr.x - 32, ccn = 0, cce = -1;   // next and last block of the current view
+    unsigned mask = 0;
+    int cur = 0;
+    auto next = [&](Unit *u) {
+        while (ccn > cce) {
+            while (mask == 0) {
+                vbase += 32;
+                if (vbase >= vr.y) {
+                    if (lane == 0) u->v = -1;
+                    vbase = vr.y;
+                    __syncwarp();
+                    return;
+                }
+                const int v = vbase + lane;
+                bool lit = false;
+                if (v < vr.y) {
+                    const DdView3 w = views[v];
+                    const float *rzv = rzt + (size_t)v * P.srz;
+                    const int l0 = w.xb ? ylo : xlo, l1 = min(l0 + kTile, w.xb ? H : W) - 1;
+                    lit = slab_visible(g, w, l0, l1, s0, ns, rzv[0], rzv[2 * R - 1]);
+                    if (lit) {
+                        // the tile's shadow on the axis: its four corners
+                        const float *dpv = dpt + (size_t)v * P.sdp;
+                        const float X0 = ((float)xlo - 0.5f * (float)W) * g.pix_x + g.pix_xshift;
+                        const float X1 = ((float)min(xlo + kTile, W) - 0.5f * (float)W) * g.pix_x + g.pix_xshift;
+                        const float Y0 = (0.5f * (float)H - (float)ylo) * g.pix_y + g.pix_yshift;
+                        const float Y1 = (0.5f * (float)H - (float)min(ylo + kTile, H)) * g.pix_y + g.pix_yshift;
+                        const float src = w.xb ? w.srcy : w.srcx;
+                        const float d0 = (w.xb ? Y0 : X0) - src, d1 = (w.xb ? Y1 : X1) - src;
+                        float lo = 3.0e38f, hi = -3.0e38f;
 #pragma unroll
-    for (int q = 0; q < kZS; q++)
+                        for (int i = 0; i < 4; i++) {
+                            const float px = (i & 1) ? X1 : X0, py = (i & 2) ? Y1 : Y0;
+                            const float t = w.xb ? dd_map2x(w.srcx, w.srcy, px, py) : dd_map2y(w.srcx, w.srcy, px, py);
+                            lo = fminf(lo, t);
+                            hi = fmaxf(hi, t);
+                        }
+                        int ca = 0, cb = P.nch - 1;
+                        float la = 0.0f, lb = 0.0f;
+                        if (d0 * d1 > 0.0f && lo <= hi) {   // the source's line does not cross the tile
+                            const float tol = 0.0625f * (hi - lo) + 1e-4f * (fabsf(lo) + fabsf(hi));   // a pixel, and the drift
+                            while (ca < cb) {   // blocks that end below the shadow
+                                const float e = dpv[(ca + 1) * DD3_CHUNK];
+                                if (!(e >= dpv[ca * DD3_CHUNK] && e < lo - tol)) break;
+                                ca++;
+                            }
+                            while (cb > ca) {   // blocks that start above it
+                                const float b = dpv[cb * DD3_CHUNK];
+                                if (!(b > hi + tol && b <= dpv[min((cb + 1) * DD3_CHUNK, C)])) break;
+                                cb--;
+                            }
+                            const float um = 0.5f * (lo + hi);
+                            const int k = min(dd3_col_of(GEOM, &g, &w, dpv, um, 0, C), C - 1);
+                            const float b = dpv[k], e = dpv[k + 1];
+                            if (e > b) {
+                                la = __fdividef(1.0f, e - b);
+                                lb = (float)k - b * la;
+                            }
+                        }
+                        la_s[lane] = la;
+                        lb_s[lane] = lb;
+                        cc_s[lane] = ca | (cb << 16);
+                    }
+                }
+                mask = __ballot_sync(0xffffffffu, lit);
+            }
+            __syncwarp();
+            cur = __ffs(mask) - 1;
+            mask &= mask - 1;
+            ccn = cc_s[cur] & 0xFFFF;
+            cce = cc_s[cur] >> 16;
+        }
+        if (lane == 0) *u = Unit{vbase + cur, ccn, la_s[cur], lb_s[cur]};
+        ccn++;
+        __syncwarp();
+    };
+
+    T acc[ZS];
 #pragma unroll
-        for (int b = 0; b < kNB; b++) acc[q][b] = 0.0f;
+    for (int q = 0; q < ZS; q++) acc[q] = VT::zero();
 
     DdPhases ph;
-    int inflight = -1;
-    // only the views that can see this slab somewhere in the image
-    const int2 vr = reinterpret_cast<const int2 *>(a.plan + P.slabv)[blockIdx.y];
-    if (tid == 0 && vr.x < vr.y) issue(vr.x, 0);
-    for (int v = vr.x; v < vr.y; v++) {
-        const int buf = (v - vr.x) & 1;
-        if (tid == 0 && v + 1 < vr.y) issue(v + 1, buf ^ 1);
+    // unit i uses buffer i % 3; units i + 1 and i + 2 are in flight behind it
+    if (tid < 32) {
+        next(&units[0]);
+        next(&units[1]);
+        if (tid == 0) {
+            if (units[0].v >= 0) issue(units[0].v, units[0].cc, 0);
+            if (units[1].v >= 0) issue(units[1].v, units[1].cc, 1);
+        }
+    }
+    __syncthreads();
+    int buf = 0;
+    for (int i = 0; units[i & 3].v >= 0; i++, buf = buf == 2 ? 0 : buf + 1) {
+        const int buf2 = buf == 0 ? 2 : buf - 1;   // buffer of unit i + 2 (and of unit i - 1)
+        // slot i + 2 was last read before the barrier of unit i - 1
+        if (tid < 32) next(&units[(i + 2) & 3]);
         if (!dd_mbar_wait(&bar[buf], ph.parity(buf))) abort_flag = 1;
         ph.flip(buf);
+        // past this barrier every warp has finished unit i - 1
         __syncthreads();
         if (abort_flag) {
-            // view v's copies (the wait gave up on them) and view v + 1's may be in flight
-            if (tid == 0) dd_mbar_drain(&bar[buf], ph.parity(buf) ^ 1u);
-            inflight = (v + 1 < vr.y) ? (buf ^ 1) : -1;
+            // this unit's copies (the wait gave up on them) and the next one's may be in flight
+            if (tid == 0) {
+                const int b1 = buf == 2 ? 0 : buf + 1;
+                dd_mbar_drain(&bar[buf], ph.parity(buf) ^ 1u);
+                if (units[(i + 1) & 3].v >= 0) dd_mbar_drain(&bar[b1], ph.parity(b1));
+            }
             break;
         }
-        if (active && seen[buf]) {
-            const DdView3 &w = *reinterpret_cast<const DdView3 *>(sm + S.vw + buf * (int)sizeof(DdView3));
-            const float *dp = reinterpret_cast<const float *>(sm + S.dp + buf * S.dp_b);
+        if (tid == 0 && units[(i + 2) & 3].v >= 0) issue(units[(i + 2) & 3].v, units[(i + 2) & 3].cc, buf2);
+        const DdView3 &w = *reinterpret_cast<const DdView3 *>(sm + S.vw + buf * (int)sizeof(DdView3));
+        const int xb = w.xb;
+        const int rl = xb ? (y - ylo) : (x - xlo);
+        const int j = xb ? x : H - 1 - y;
+        const DdLine *L = reinterpret_cast<const DdLine *>(sm + S.rec + buf * S.rec_b) + rl;
+        const float4 lz = reinterpret_cast<const float4 *>(sm + S.lz + buf * S.lz_b)[rl];
+        const Unit u0 = units[i & 3];
+        const int c0 = u0.cc * DD3_CHUNK;
+        float PL, PH;
+        // (a line behind the source has a negative pitch and meets nothing)
+        if (active && lz.z > 0.0f && dd3_pix_bounds(L, j, &PL, &PH)) {
+            const float *dp = reinterpret_cast<const float *>(sm + S.dp + buf * S.dp_b);     // from column c0
             const float *mg = reinterpret_cast<const float *>(sm + S.mag + buf * S.mag_b);
-            const float *rz = reinterpret_cast<const float *>(sm + S.rz + buf * S.rz_b);
-            const int xb = w.xb;
-            const int rl = xb ? (y - ylo) : (x - xlo);
-            const int line = (xb ? ylo : xlo) + rl;
-            const int j = xb ? x : H - 1 - y;
-            const float4 lz = reinterpret_cast<const float4 *>(sm + S.lz + buf * S.lz_b)[rl];
-            const DdLine *lrec = reinterpret_cast<const DdLine *>(sm + S.rec + buf * S.rec_b) + rl * P.nch;
-            const float lpos = (FAMILY == 2) ? dd3_line_pos(&g, &w, line) : 0.0f;
-            float zb[kZS + 1];   // slice boundaries of the slab on this line
+            const float2 *rz = reinterpret_cast<const float2 *>(sm + S.rz + buf * S.rz_b);
+            const int klo = L->h.idet0, khi = min(DD3_CHUNK, C - c0);
+            const float lpos = (family == 2) ? dd3_line_pos_f(&g, &w, (xb ? ylo : xlo) + rl) : 0.0f;
+            const float srcz = (GEOM == DD_GEOM3_SPIRAL) ? w.srcz : 0.0f;
+            auto row_z = [&](float mag, float2 z, float *e0, float *e1) {   // dd3_rp
+                if (GEOM == DD_GEOM3_SPIRAL) {
+                    *e0 = FADD(FMUL(mag, FSUB(z.x, srcz)), srcz);
+                    *e1 = FADD(FMUL(mag, FSUB(z.y, srcz)), srcz);
+                } else {
+                    *e0 = FMUL(mag, z.x);
+                    *e1 = FMUL(mag, z.y);
+                }
+            };
+            // past the volume's top the slice boundaries coincide, so those
+            // slices meet no row
+            const float ztop = fminf(dd3_zb(lz.x, lz.z, Dp), lz.y);
+            const float zfirst = dd3_zb(lz.x, lz.z, s0);
+            const T *__restrict__ ssv = ssb + (size_t)u0.v * R * C + c0;
+            int k = klo;
+            float CL = L->h.bound0;
+            if (dp[khi] > PL) {
+                // first column that ends above the pixel's lower boundary:
+                // the linear estimate, settled on the exact boundaries
+                k = max(klo, min(khi - 1, (int)floorf(fminf(fmaxf(fmaf(PL, u0.A, u0.B), 0.0f), 1.0e6f)) - c0));
+                while (k > klo && dp[k] > PL) k--;
+                while (k < khi && dp[k + 1] <= PL) k++;
+                if (k > klo) CL = dp[k];
+            } else {
+                k = khi;
+            }
+            for (; k < khi && CL < PH; k++) {
+                const float CH = dp[k + 1];
+                const float wd = FSUB(fminf(PH, CH), fmaxf(PL, CL));
+                CL = CH;
+                const float mag = mg[k];
+                if (!(wd > 0.0f && mag > 0.0f)) continue;
+                const float coef = dd3_coef(GEOM, family, &g, &w, lpos, j, wd, lz.w);
+                // first row that reaches above the first slice's bottom: the
+                // closed-form estimate, settled on the exact boundaries
+                // (row R lies at infinity and ends the walk)
+                const float zeta = dd3_approx_div(zfirst - srcz, mag) + srcz;
+                int r = (int)floorf(fminf(fmaxf((zeta - w.rzA) * w.rzI, 0.0f), (float)(R - 1)));
+                float e0, e1;
+                row_z(mag, rz[r], &e0, &e1);
+                while (!(e1 > zfirst) && r < R) row_z(mag, rz[++r], &e0, &e1);
+                while (r > 0 && e0 > zfirst) row_z(mag, rz[--r], &e0, &e1);
+                if (r >= R) continue;
+                const T *__restrict__ p = ssv + (size_t)r * C + k;
+                T val = __ldg(p);
+                float hi = zfirst;
 #pragma unroll
-            for (int q = 0; q <= kZS; q++) zb[q] = dd3_zb(lz.x, lz.z, s0 + q);
-            const float *__restrict__ ssv = ssb + (size_t)v * R * C;
-            for (int cc = 0; cc < P.nch; cc++) {
-                DdPixWalk pw;
-                if (!dd3_pixwalk_init(GEOM, &g, &w, lrec + cc, dp, cc, j, &pw)) continue;
-                int k;
-                float wd;
-                while (dd3_pixwalk_next(dp, &pw, &k, &wd)) {
-                    const float coef = dd3_coef(GEOM, FAMILY, &g, &w, lpos, j, wd, lz.w);
-                    const float mag = mg[k];
-                    const float *__restrict__ ssk = ssv + k;
-                    // rows meeting each slice of the slab; the first row of
-                    // slice q + 1 is found from where slice q stopped
-                    int rnext = -1;
-#pragma unroll
-                    for (int q = 0; q < kZS; q++) {
-                        const int s = s0 + q;
-                        if (s < Dp) {
-                            const float zlo = zb[q], zhi = zb[q + 1];
-                            int r;
-                            if (rnext < 0) {
-                                r = dd3_row_first(GEOM, &w, rz, R, mag, zlo, 0.0f);
-                            } else {
-                                r = max(rnext - 1, 0);
-                                for (int it = 0; it < 64 && r > 0; it++) {
-                                    float e0, e1;
-                                    dd3_rp(GEOM, &w, mag, rz[2 * (r - 1)], rz[2 * (r - 1) + 1], &e0, &e1);
-                                    if (e1 > zlo) r--;
-                                    else break;
-                                }
-                            }
-                            for (; r < R; r++) {
-                                float e0, e1;
-                                dd3_rp(GEOM, &w, mag, rz[2 * r], rz[2 * r + 1], &e0, &e1);
-                                if (!(e0 < zhi)) break;
-                                const float zw = dd3_cell(fmaxf(lz.x, e0), fminf(lz.y, e1), zlo, zhi);
-                                if (zw > 0.0f) {
-                                    const float wq = FMUL(zw, coef);
-#pragma unroll
-                                    for (int b = 0; b < kNB; b++)
-                                        if (b < nb) acc[q][b] = fmaf(wq, __ldg(ssk + (size_t)b * per + (size_t)r * C), acc[q][b]);
-                                }
-                            }
-                            rnext = r;
-                        }
+                for (int q = 0; q < ZS; q++) {
+                    const float lo = hi;
+                    hi = fminf(dd3_zb(lz.x, lz.z, s0 + q + 1), ztop);
+                    T t = VT::zero();
+                    const float w0 = FSUB(fminf(e1, hi), fmaxf(e0, lo));
+                    if (w0 > 0.0f) t = VT::fma(w0, val, t);
+                    while (e1 < hi) {
+                        row_z(mag, rz[++r], &e0, &e1);
+                        p += C;
+                        if (r < R) val = __ldg(p);
+                        const float w1 = FSUB(fminf(e1, hi), e0);
+                        if (w1 > 0.0f) t = VT::fma(w1, val, t);
                     }
+                    acc[q] = VT::fma(coef, t, acc[q]);
                 }
             }
         }
-        __syncthreads();   // buffer `buf` is refilled by the next iteration's issue
     }
     if (abort_flag) {
-        if (tid == 0 && inflight >= 0) dd_mbar_drain(&bar[inflight], ph.parity(inflight));
         if (tid == 0) dd_report_timeout(a.status);
         return;
     }
     if (!active) return;
 #pragma unroll
-    for (int q = 0; q < kZS; q++) {
+    for (int q = 0; q < ZS; q++) {
         const int s = s0 + q;
         if (s >= Dp) continue;
 #pragma unroll
-        for (int b = 0; b < kNB; b++) {
-            if (b < nb) {
-                const size_t o = (((size_t)(b0 + b) * Dp + s) * H + y) * W + x;
-                a.out[o] = a.base ? fmaf(a.scale, acc[q][b], a.base[o]) : acc[q][b];
-            }
+        for (int b = 0; b < NB; b++) {
+            const size_t o = (((size_t)(b0 + b) * Dp + s) * H + y) * W + x;
+            const float val = VT::get(acc[q], b);
+            a.out[o] = a.base ? fmaf(a.scale, val, a.base[o]) : val;
         }
     }
 }
@@ -742,8 +919,7 @@ int validate(int scan, int op, const dd_geom3d *g, int B, int V) {
     if ((long long)V * g->num_row * g->num_col * B > lim) return DD_ERR_SIZE_OVERFLOW;
     if (g->width > 8192 || g->height > 8192 || V > 65535 || g->num_row > 65535 || g->num_col > 65535)
         return DD_ERR_SIZE_OVERFLOW;
-    // one view's staged data (two buffers) must fit the adjoint's shared memory
-    if (adj3_smem(plan_layout(g, V)).total > 200 * 1024) return DD_ERR_SIZE_OVERFLOW;
+    if (view_too_wide(plan_layout(g, V), g->num_row)) return DD_ERR_SIZE_OVERFLOW;
     return DD_OK;
 }
 
@@ -790,34 +966,43 @@ int launch_fwd(int family, const Fwd3Args &a, cudaStream_t st) {
     return launch_status();
 }
 
-template <int GEOM, int FAMILY>
-int launch_adj_kernel(const Adj3Args &a, const dim3 &grid, cudaStream_t st) {
+template <int GEOM, int NB, int ZS>
+int launch_adj_slabs(const Adj3Args &a, int ngroups, cudaStream_t st) {
     const int smem = adj3_smem(a.P).total;
-    if (cudaFuncSetAttribute(k_adj3<GEOM, FAMILY>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(k_adj3<GEOM, NB, ZS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
         return DD_ERR_LAUNCH;
-    k_adj3<GEOM, FAMILY><<<grid, kThreads, smem, st>>>(a);
+    const int nty = (a.g.height + kTile - 1) / kTile;
+    const dim3 grid((unsigned)(a.ntx * nty), (unsigned)((a.g.depth + ZS - 1) / ZS), (unsigned)ngroups);
+    k_adj3<GEOM, NB, ZS><<<grid, kThreads, smem, st>>>(a);
+    dd2::count_launches(1);
     return DD_OK;
 }
 
+// 16 slices per thread share a pixel's columns and boundaries; 8 where 16
+// would leave the chip's 456 resident CTAs (3 per SM) less than twice full.
+template <int GEOM, int NB>
+int launch_adj_kernel(Adj3Args a, int b0, int ngroups, cudaStream_t st) {
+    if (ngroups <= 0) return DD_OK;
+    a.b0 = b0;
+    const long long tiles = (long long)a.ntx * ((a.g.height + kTile - 1) / kTile) * ngroups;
+    if (tiles * ((a.g.depth + 2 * kZS - 1) / (2 * kZS)) >= 2 * 456) return launch_adj_slabs<GEOM, NB, 2 * kZS>(a, ngroups, st);
+    return launch_adj_slabs<GEOM, NB, kZS>(a, ngroups, st);
+}
+
 template <int GEOM>
-int launch_adj(int family, const Adj3Args &a, const float *in, float *ss, cudaStream_t st) {
+int launch_adj(const Adj3Args &a, const float *in, float *ss, cudaStream_t st) {
     const dd_geom3d &g = a.g;
     const dim3 gs((unsigned)((g.num_col + 127) / 128), (unsigned)g.num_row, (unsigned)a.V);
     dd2::ProfRec *pt = dd2::prof_begin(DD_KERNEL_TABLES, st);
-    if (family == 0) k_sino3<GEOM, 0><<<gs, 128, 0, st>>>(g, a.plan, a.P, in, ss, a.B, a.V);
+    if (a.family == 0) k_sino3<GEOM, 0><<<gs, 128, 0, st>>>(g, a.plan, a.P, in, ss, a.B, a.V);
     else k_sino3<GEOM, 1><<<gs, 128, 0, st>>>(g, a.plan, a.P, in, ss, a.B, a.V);
     dd2::prof_end(pt, st);
-    const int nty = (g.height + kTile - 1) / kTile;
-    const dim3 grid((unsigned)(a.ntx * nty), (unsigned)((g.depth + kZS - 1) / kZS), (unsigned)((a.B + kNB - 1) / kNB));
+    dd2::count_launches(1);
     dd2::ProfRec *pr = dd2::prof_begin(DD_KERNEL_ADJOINT, st);
-    int rc;
-    if (family == 0) rc = launch_adj_kernel<GEOM, 0>(a, grid, st);
-    else if (family == 1) rc = launch_adj_kernel<GEOM, 1>(a, grid, st);
-    else rc = launch_adj_kernel<GEOM, 2>(a, grid, st);
+    int rc = launch_adj_kernel<GEOM, kNB>(a, 0, a.B / kNB, st);
+    if (rc == DD_OK) rc = launch_adj_kernel<GEOM, 1>(a, a.B / kNB * kNB, a.B % kNB, st);
     dd2::prof_end(pr, st);
-    if (rc != DD_OK) return rc;
-    dd2::count_launches(2);
-    return launch_status();
+    return rc != DD_OK ? rc : launch_status();
 }
 
 int transpose(const dd_geom3d *g, const float *in, float *out, int B, cudaStream_t st) {
@@ -871,10 +1056,12 @@ int adjoint(int scan, int op, const dd_geom3d *g, const char *planb, const float
     a.B = B;
     a.V = V;
     a.ntx = (g->width + kTile - 1) / kTile;
-    const int fam = op_family(op), geom = geom_of(scan);
-    if (geom == DD_GEOM3_CONE_FLAT) return launch_adj<DD_GEOM3_CONE_FLAT>(fam, a, in, (float *)ss, st);
-    if (geom == DD_GEOM3_CONE_ARC) return launch_adj<DD_GEOM3_CONE_ARC>(fam, a, in, (float *)ss, st);
-    return launch_adj<DD_GEOM3_SPIRAL>(fam, a, in, (float *)ss, st);
+    a.b0 = 0;
+    a.family = op_family(op);
+    const int geom = geom_of(scan);
+    if (geom == DD_GEOM3_CONE_FLAT) return launch_adj<DD_GEOM3_CONE_FLAT>(a, in, (float *)ss, st);
+    if (geom == DD_GEOM3_CONE_ARC) return launch_adj<DD_GEOM3_CONE_ARC>(a, in, (float *)ss, st);
+    return launch_adj<DD_GEOM3_SPIRAL>(a, in, (float *)ss, st);
 }
 
 }   // namespace dd3

@@ -46,7 +46,8 @@ struct DdView3 {
     float z0, z1;         // volume extent in z
     float magmin, magmax; // range of the per-column row magnification
     float rzA, rzB;       // row0z(r) ~= rzA + r * rzB (row candidate search)
-    float pad[6];
+    float rzI;            // 1 / rzB
+    float pad[5];
 };
 // the view record and the line record are moved by bulk copies: sizes must be
 // multiples of 16 bytes (and arrays of them keep every element 16-byte aligned)
@@ -166,8 +167,8 @@ DD_HD void dd3_view_scalars(int geom, const dd_geom3d *g, float view, const floa
     w->z0 = (float)DADD(DMUL(-Dp / 2.0, (double)g->pix_z), pzs);
     w->z1 = (float)DADD(DMUL(Dp / 2.0, (double)g->pix_z), pzs);
     w->magmin = w->magmax = 1.0f;
-    w->rzA = w->rzB = 0.0f;
-    for (int i = 0; i < 6; i++) w->pad[i] = 0.0f;
+    w->rzA = w->rzB = w->rzI = 0.0f;
+    for (int i = 0; i < 5; i++) w->pad[i] = 0.0f;
 }
 
 // Sorted column boundary k (0..C) on the projection axis.
@@ -257,6 +258,14 @@ DD_HD float dd3_line_pos(const dd_geom3d *g, const DdView3 *w, int line) {
     return w->xb
         ? (float)DADD(DMUL(DSUB(DSUB(H / 2.0, (double)line), 0.5), (double)g->pix_y), (double)g->pix_yshift)
         : (float)DADD(DMUL(DADD(DSUB((double)line, W / 2.0), 0.5), (double)g->pix_x), (double)g->pix_xshift);
+}
+
+// The same in single precision: one FMA of the exact half-integer offset
+// rounds the exact value once, the same float unless it lies within 2^-53
+// (relative) of an FP32 rounding boundary, at the FP32 rate.
+DD_HD float dd3_line_pos_f(const dd_geom3d *g, const DdView3 *w, int line) {
+    return w->xb ? fmaf(0.5f * (float)g->height - (float)line - 0.5f, g->pix_y, g->pix_yshift)
+                 : fmaf((float)line - 0.5f * (float)g->width + 0.5f, g->pix_x, g->pix_xshift);
 }
 
 // Line magnification onto its plane.
@@ -441,7 +450,7 @@ DD_HD int dd3_pixel_of(const DdLine *L, float u, int *p) {
 // [dd3_zb(s), dd3_zb(s + 1)].  Forward and adjoint evaluate the same
 // expression, so they stay exact transposes.
 // ---------------------------------------------------------------------------
-DD_HD float dd3_zb(float p0z, float pintz, int s) { return FADD(FMUL((float)s, pintz), p0z); }
+DD_HD float dd3_zb(float p0z, float pintz, int s) { return dd3_mul_add((float)s, pintz, p0z); }
 
 DD_HD float dd3_cell(float bz0, float bz1, float zlo, float zhi) {
     const float lo = bz0 > zlo ? bz0 : zlo;
@@ -454,6 +463,24 @@ DD_HD float dd3_cell(float bz0, float bz1, float zlo, float zhi) {
 DD_HD int dd3_slice_first(float bz0, float p0z, float pintz) {
     int s = (int)floorf(dd3_approx_div(FSUB(bz0, p0z), pintz)) - 1;
     return s < 0 ? 0 : s;
+}
+
+// Boundaries [*pl, *ph] of pixel j on a walked line (the walk start replaces
+// the first lower one); false where the walk does not reach the pixel.
+DD_HD bool dd3_pix_bounds(const DdLine *L, int j, float *pl, float *ph) {
+    const DdLineHdr h = L->h;
+    if (h.npiece == 0 || j < h.i0 || j >= h.nend) return false;
+    const DdPiece P0 = L->p[0];
+    const int p = dd_piece_of_index(L, j, FADD(P0.Q, FMUL((float)(j - P0.gb), P0.dl)));
+    DdPiece P = L->p[p];
+    *ph = FADD(P.Q, FMUL((float)(j - P.gb), P.dl));
+    if (j == h.i0) {
+        *pl = h.bound0;
+    } else {   // boundary j - 1: the same piece, or the one before it
+        if (p > 0 && j - 1 <= L->p[p - 1].gb) P = L->p[p - 1];
+        *pl = FADD(P.Q, FMUL((float)(j - 1 - P.gb), P.dl));
+    }
+    return true;
 }
 
 // ---------------------------------------------------------------------------
