@@ -4,12 +4,12 @@
 // radontorch operators (RadonTorch.cpp:1395-1414).
 //
 // Forward-type operators (Proj, BackProjTrans, BackProjTransWeighted): one
-// thread per (view, column, 8 detector rows, 2 volumes) loops over the walked
-// image lines; for each line it enumerates the overlap segments of its
-// column with the drifted pixel boundaries (dd3_colwalk_*), then walks the
-// slices each of its rows meets and gathers voxels.  Volumes are read from a
-// transposed copy for views that walk image columns, so that the pixels of a
-// walked line are contiguous in both branches.
+// thread per (view, column, up to 8 detector rows, 2 or 1 volumes) loops over
+// the walked image lines.  For each line the overlap segments of the columns
+// with the drifted pixel boundaries (dd3_colwalk_*) are summed once per slice,
+// and every row then merges its interval with the slices.  Volumes are read
+// from copies in which the pixels of a walked line are contiguous in both
+// branches.
 //
 // Adjoint-type operators (ProjTrans, BackProj, BackProjWeighted): one thread
 // per (x, y) voxel column, 16 or 8 slices and 2 or 1 volumes loops over the
@@ -20,6 +20,7 @@
 //
 // Both directions use the same segment widths and z-walk widths, so they are
 // exact transposes of each other; no atomics, deterministic results.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -80,7 +81,7 @@ inline PlanLayout plan_layout(const dd_geom3d *g, int V) {
 }
 
 struct ApplyLayout {
-    size_t volT, ss, status, total;
+    size_t volx, volt, ss, status, total;
 };
 
 inline bool op_is_forward(int op) { return op == DD_OP_PROJ || op == DD_OP_BPROJ_T || op == DD_OP_BPROJ_TW; }
@@ -92,8 +93,11 @@ inline int op_family(int op) {
 inline ApplyLayout apply_layout(bool fwd, bool adj, const dd_geom3d *g, int B, int V) {
     ApplyLayout L;
     size_t o = 0;
-    L.volT = L.ss = 0;
-    if (fwd) { L.volT = o; o = align_up(o + sizeof(float) * (size_t)B * g->depth * g->width * g->height, 256); }
+    L.volx = L.volt = L.ss = 0;
+    if (fwd) {   // the volumes' rows and columns, padded to 16 bytes (k_lines_of3)
+        L.volx = o; o = align_up(o + sizeof(float) * (size_t)B * g->depth * g->height * pad4(g->width), 256);
+        L.volt = o; o = align_up(o + sizeof(float) * (size_t)B * g->depth * g->width * pad4(g->height), 256);
+    }
     if (adj) { L.ss = o; o = align_up(o + sizeof(float) * (size_t)B * V * g->num_row * g->num_col, 256); }
     L.status = o; o = align_up(o + 256, 256);
     L.total = o;
@@ -180,30 +184,6 @@ __global__ void __launch_bounds__(128) k_lines3(dd_geom3d g, char *plan, PlanLay
         reinterpret_cast<float4 *>(plan + P.linez)[(size_t)v * P.nl + line] = make_float4(lz[0], lz[1], lz[2], lz[3]);
 }
 
-// volT[b][s][x][H-1-y] = vol[b][s][y][x]: walked lines of y-branch views
-// become contiguous rows.
-__global__ void __launch_bounds__(256) k_transpose3(const float *__restrict__ in, float *__restrict__ out, int W,
-                                                    int H, int nplanes) {
-    __shared__ float t[32][33];
-    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int pl = blockIdx.z; pl < nplanes; pl += gridDim.z) {
-        const size_t plane = (size_t)pl * W * H;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int y = y0 + ty + 8 * i, x = x0 + tx;
-            if (y < H && x < W) t[ty + 8 * i][tx] = in[plane + (size_t)y * W + x];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int x = x0 + ty + 8 * i, y = y0 + tx;
-            if (x < W && y < H) out[plane + (size_t)x * H + (H - 1 - y)] = t[tx][ty + 8 * i];
-        }
-        __syncthreads();
-    }
-}
-
 // One volume's value, or two volumes' side by side: the adjoint's gathers move
 // both with one 8-byte load.
 template <int NB> struct Vox;
@@ -211,14 +191,76 @@ template <> struct Vox<1> {
     using T = float;
     static __device__ __forceinline__ T zero() { return 0.0f; }
     static __device__ __forceinline__ T fma(float w, T x, T a) { return fmaf(w, x, a); }
+    using K = float;   // a coefficient used for all the volumes of several loads
+    static __device__ __forceinline__ K coef(float w) { return w; }
+    static __device__ __forceinline__ T kmul(K w, T x) { return FMUL(w, x); }
+    static __device__ __forceinline__ T kfma(K w, T x, T a) { return fmaf(w, x, a); }
     static __device__ __forceinline__ float get(T x, int) { return x; }
 };
 template <> struct Vox<2> {
     using T = float2;
     static __device__ __forceinline__ T zero() { return make_float2(0.0f, 0.0f); }
     static __device__ __forceinline__ T fma(float w, T x, T a) { return make_float2(fmaf(w, x.x, a.x), fmaf(w, x.y, a.y)); }
+    // two products at once (the packed FP32 instructions; each rounds as the scalar one)
+    using K = unsigned long long;
+    static __device__ __forceinline__ K coef(float w) {
+        K k;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(k) : "f"(w));
+        return k;
+    }
+    static __device__ __forceinline__ T kmul(K w, T x) {
+        asm("{\n .reg .b64 t;\n mov.b64 t, {%0, %1};\n mul.rn.f32x2 t, %2, t;\n mov.b64 {%0, %1}, t;\n}"
+            : "+f"(x.x), "+f"(x.y) : "l"(w));
+        return x;
+    }
+    static __device__ __forceinline__ T kfma(K w, T x, T a) {
+        asm("{\n .reg .b64 t, u;\n mov.b64 t, {%0, %1};\n mov.b64 u, {%3, %4};\n fma.rn.f32x2 t, %2, u, t;\n"
+            " mov.b64 {%0, %1}, t;\n}"
+            : "+f"(a.x), "+f"(a.y) : "l"(w), "f"(x.x), "f"(x.y));
+        return a;
+    }
     static __device__ __forceinline__ float get(T x, int b) { return b ? x.y : x.x; }
 };
+
+// The walked lines of either kind, each line's pixels contiguous, the volumes
+// of a group of kNB next to each other (an odd last volume forms a group of
+// its own), lines padded to a multiple of 4 pixels:
+//   vx[s][y][x][b] = vol[b][s][y][x],  vt[s][x][H-1-y][b] = vol[b][s][y][x].
+template <int NB>
+__global__ void __launch_bounds__(256) k_lines_of3(const float *__restrict__ in, float *__restrict__ vx,
+                                                   float *__restrict__ vt, int W, int H, int Dp, int ngroups) {
+    using T = typename Vox<NB>::T;
+    __shared__ T t[32][33];
+    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int Wp = pad4(W), Hp = pad4(H);
+    const size_t vox = (size_t)W * H * Dp;
+    for (int pl = blockIdx.z; pl < Dp * ngroups; pl += gridDim.z) {
+        const int gr = pl / Dp, s = pl - gr * Dp;
+        const float *__restrict__ src = in + (size_t)gr * NB * vox + (size_t)s * H * W;
+        T *__restrict__ px = reinterpret_cast<T *>(vx) + ((size_t)gr * Dp + s) * H * Wp;
+        T *__restrict__ pt = reinterpret_cast<T *>(vt) + ((size_t)gr * Dp + s) * W * Hp;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int y = y0 + ty + 8 * i, x = x0 + tx;
+            if (y < H && x < W) {
+                const size_t o = (size_t)y * W + x;
+                T val;
+                if constexpr (NB == 2) val = make_float2(src[o], src[vox + o]);
+                else val = src[o];
+                t[ty + 8 * i][tx] = val;
+                px[(size_t)y * Wp + x] = val;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int x = x0 + ty + 8 * i, y = y0 + tx;
+            if (x < W && y < H) pt[(size_t)x * Hp + (H - 1 - y)] = t[tx][ty + 8 * i];
+        }
+        __syncthreads();
+    }
+}
 
 // ss[v][r][k][b] = in[b][v][r][k'] * scale(v, r, k) with k the sorted column:
 // the adjoint gathers pre-scaled bins (ConeFlatDisCUDA3d.cu:400-404), the
@@ -253,60 +295,130 @@ __global__ void __launch_bounds__(128) k_sino3(dd_geom3d g, const char *__restri
 // ---------------------------------------------------------------------------
 // Forward-type kernel: detector gathers
 // ---------------------------------------------------------------------------
-constexpr int kFC = 32;    // detector columns per CTA (the lanes of a warp)
-// Forward CTA: 8 consumer warps x 4 consecutive detector rows per thread =
-// 32 rows, plus a producer warp that turns each line's record into column
-// segments one line ahead; 3 CTAs per SM at 72 registers.
-constexpr int kFR = 4;
-constexpr int kFwdWarps3 = 8;                          // consumer warps
-constexpr int kFwdThreads3 = (kFwdWarps3 + 1) * 32;   // + the producer warp
-constexpr int kSeg = 8;    // column segments of one line held in shared memory
+constexpr int kFC = 32;      // detector columns per CTA (the lanes of a warp)
+constexpr int kCons3 = 8;    // consumer warps
+// Producer warps (taking steps in turn), stages between them and the slowest
+// consumer, and CTAs per SM.  96 spiral / 36 cone-flat views: one volume, 3
+// producers, 3 stages, 3 CTAs 3.54 / 3.07 ms; 2, 3, 3: 3.75 / 2.94; 4, 4, 2:
+// 3.58 / 3.24; two volumes (twice the tile), 2, 3, 2: 4.72 / 4.09; 3, 3, 2:
+// 4.68 / 4.51; 2, 2, 2: 5.87 / 4.91.
+template <int NB> constexpr int kProd3 = NB == 1 ? 3 : 2;
+template <int NB> constexpr int kFwdThreads3 = (kCons3 + kProd3<NB>) * 32;
+template <int NB> constexpr int kStage3 = 3;
+template <int NB> constexpr int kFwdMin3 = NB == 1 ? 3 : 2;
+// (a producer must not wait for a stage two uses ahead of the consumers)
+static_assert(kProd3<1> <= kStage3<1> && kProd3<2> <= kStage3<2>, "at least a stage per producer");
+constexpr int kSeg = 8;      // column segments of one line held in shared memory
+constexpr int kFast = 3;     // ... and held in registers by the usual path
+constexpr int kZB = 16;      // slices of one copy
+constexpr int kZW = 62;      // most slices of a line in one step
+// pixels per slice of a tile: a CTA takes the narrowest that holds what its
+// columns meet on any line (one tensor map each)
+constexpr int kNPitch = 5;
+__host__ __device__ constexpr int pitch3(int i) { return i == 0 ? 16 : i == 1 ? 24 : i == 2 ? 32 : i == 3 ? 48 : 64; }
+// bytes of a step's voxel tile: 62 slices of 64 pixels and a neighbour at either end
+template <int NB> constexpr int kTileB3 = (kZW + 2) * 64 * 4 * NB;
+
+// Tensor maps of the volumes' rows and columns (k_lines_of3): {pixel x
+// volumes, line, slice, group}, boxes of one line, pitch3(i) pixels and kZB slices.
+struct Maps3 {
+    CUtensorMap m[2][kNPitch];   // [columns, rows][pitch]
+};
 
 struct Fwd3Args {
     dd_geom3d g;
     const char *plan;
     PlanLayout P;
-    const float *vol;    // (B, Dep, H, W)
-    const float *volT;   // (B, Dep, W, H), pixel order reversed along y
+    const float *volx, *volt;   // the volumes' rows and columns (k_lines_of3), from the launch's first volume
     float *out;          // (B, V, R, C)
     const float *sub;    // optional: out = A x - sub
     int *status;
-    int B, V, nrb;
+    int V, nrb, ncg;     // views, row blocks, column groups
+    int b0, geom, family;   // first volume of the launch; geometry and operator family
 };
 
-// grid: (view, group of 32 columns inside one walk block, row block x volume
-// group).  Lane = column, consumer warp w = rows r0 + 4w .. r0 + 4w + 3, kNB
-// volumes.  The overlap segments of a line (pixel, width x operator factor)
-// depend on the column only, so they are computed once per line and column
-// -- by the producer warp, one line ahead, while the consumer warps walk the
-// current line -- into shared memory, and reused by all 32 rows.  Line
-// records arrive by bulk copies (TMA) two lines ahead.
-template <int GEOM, int FAMILY>
-__global__ void __launch_bounds__(kFwdThreads3, 3) k_fwd3(const Fwd3Args a) {
+// A step of the forward kernel: one line, or some of its slices.
+template <int NB>
+struct Step3 {
+    float4 h;                   // p0z, 1 / pintz, first slice, slices (0: nothing to do)
+    int pitch, line;            // pixels per slice of the tile (0: no tile, read global memory)
+    int fast, pad;              // tile present, no column with more than kFast segments, and the line in one step
+    int nseg[kFC], j0[kFC];     // per column: segments, first pixel in the tile
+    float c[kSeg][kFC];         // coefficients
+    float top[kZW + 2];         // entry i: top of slice first + i - 1; +inf behind the last
+};
+
+// One column's sum over the pixels of a line at slice s, from global memory:
+// where a column meets more than kSeg pixels, or the 32 columns more pixels
+// than a tile holds.
+template <int NB>
+__device__ __noinline__ typename Vox<NB>::T column_sum3(const Fwd3Args &a, const DdView3 &w, const DdLine *Lg,
+                                                        const float *sdp, int lane, int kk, float lpos, float parea,
+                                                        const typename Vox<NB>::T *row) {
+    typename Vox<NB>::T x = Vox<NB>::zero();
+    DdColWalk cw;
+    if (dd3_colwalk_init(Lg, sdp, lane, kk, &cw)) {
+        int j;
+        float wd;
+        while (dd3_colwalk_next(Lg, &cw, &j, &wd))
+            x = Vox<NB>::fma(dd3_coef(a.geom, a.family, &a.g, &w, lpos, j, wd, parea), __ldg(row + j), x);
+    }
+    return x;
+}
+
+// grid: (row block x group of 32 columns inside one walk block, view, volume
+// group).  Lane = column, consumer warp w = rows r0 + RR w .. r0 + RR (w + 1) - 1.
+//
+// A line's part of a bin is separable: the overlaps of its column with the
+// line's pixels (segments, the same for all rows) times the overlaps of its
+// row with the slices.  So each consumer thread merges its RR rows with the
+// slices in ascending z -- the slice that ends a row begins the next one --
+// and sums the column's pixels once per slice it comes to, not once per row
+// and slice; a step of the merge is an overlap of the two intervals and one
+// multiply-add per volume.
+//
+// The producer warps turn line records (bulk copies, two in flight each) into
+// segments and slice boundaries and start the tiled copies of the voxels the
+// CTA's columns and rows can meet on the line (boxes of 16 slices) into one of
+// kStage3 stages; full / empty mbarriers order them and the consumer warps,
+// which run apart by up to a stage (no CTA barrier in the loop).
+//
+// Bound by instruction issue, about 3,400 per line and CTA (63 % of the issue
+// slots; a third of them the producers').  With every row's slices walked and
+// each of its segments' voxels gathered from global memory it was about four
+// times that.  2 x 256^3 cone beam, 36 views: 12.9 -> 4.1 ms; one 512 x 512 x
+// 128 volume, 96 spiral views: 12.6 -> 3.5 ms.  On the way: the sums of all
+// (column, slice) pairs formed first, lanes along z from global memory, 8.5 /
+// 10.1 ms (7,100 instructions); per-slice bulk copies instead of boxes and the
+// segments by the record walk, 5.0 / 7.2 ms.
+template <int NB, int RR>
+__global__ void __launch_bounds__(kFwdThreads3<NB>, kFwdMin3<NB>) k_fwd3(const __grid_constant__ Fwd3Args a, const __grid_constant__ Maps3 maps) {
+    constexpr int kP = kProd3<NB>, kS = kStage3<NB>;
+    using VT = Vox<NB>;
+    using T = typename VT::T;
+    extern __shared__ __align__(128) unsigned char sm[];   // [kS] voxel tiles
     const dd_geom3d &g = a.g;
     const int W = g.width, H = g.height, Dp = g.depth, C = g.num_col, R = g.num_row;
-    const int v = blockIdx.x, cg = blockIdx.y;
-    const int rb = blockIdx.z % a.nrb, bg = blockIdx.z / a.nrb;
+    const int v = blockIdx.y, cg = blockIdx.x % a.ncg, rb = blockIdx.x / a.ncg;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cc = (cg * kFC) / DD3_CHUNK, c0 = cc * DD3_CHUNK;
     const int k = cg * kFC + lane, kk = k - c0;
     const bool active = k < C;
-    const bool prod = warp == kFwdWarps3;   // the producer warp owns no rows
-    const int r0 = rb * (kFR * kFwdWarps3) + warp * kFR, b0 = bg * kNB;
-    const int nb = min(kNB, a.B - b0);
+    const bool prod = warp >= kCons3;   // the producer warps own no rows
+    const int r0 = rb * (RR * kCons3) + warp * RR, b0 = a.b0 + blockIdx.z * NB;
     const PlanLayout &P = a.P;
 
-    __shared__ __align__(128) DdLine srec[2];
-    __shared__ __align__(16) float4 slzr[2];        // z quantities arriving with each record
-    __shared__ __align__(16) float4 slz[2];         // z quantities of the segment buffers
-    __shared__ int segj[2][kSeg][kFC];
-    __shared__ float segc[2][kSeg][kFC];
-    __shared__ int segn[2][kFC];
+    __shared__ __align__(128) DdLine srec[kP][2];
+    __shared__ __align__(16) float4 slzr[kP][2];   // z quantities arriving with each record
+    __shared__ __align__(16) Step3<NB> steps[kS];
     __shared__ float sdp[kFC + 1];
-    __shared__ __align__(8) uint64_t bar[2];
-    __shared__ int abort_flag, nissue[2], nwait[2];   // copies issued / waited per record buffer
+    __shared__ float zrange[kCons3 + 1][2];            // rows' z range per warp, and of the CTA
+    __shared__ __align__(8) uint64_t full[kS], empty[kS], rbar[kP][2];
+    __shared__ int abort_flag, armed[kS], nrec[kP][2];   // uses of the barriers so far
 
-    const DdView3 w = reinterpret_cast<const DdView3 *>(a.plan + P.views)[v];
+    __shared__ DdView3 w;
+    if (tid < (int)(sizeof(DdView3) / sizeof(int)))
+        reinterpret_cast<int *>(&w)[tid] = reinterpret_cast<const int *>(a.plan + P.views)[v * (int)(sizeof(DdView3) / sizeof(int)) + tid];
     const float *__restrict__ dpv = reinterpret_cast<const float *>(a.plan + P.dp) + (size_t)v * P.sdp;
     const float *__restrict__ rz = reinterpret_cast<const float *>(a.plan + P.rowz) + (size_t)v * P.srz;
     const float4 *__restrict__ linez = reinterpret_cast<const float4 *>(a.plan + P.linez) + (size_t)v * P.nl;
@@ -314,156 +426,316 @@ __global__ void __launch_bounds__(kFwdThreads3, 3) k_fwd3(const Fwd3Args a) {
     if (tid <= kFC) sdp[tid] = dpv[min(cg * kFC + tid, C)];
     if (tid == 0) {
         abort_flag = 0;
-        nissue[0] = nissue[1] = nwait[0] = nwait[1] = 0;
-        dd_mbar_init(&bar[0], 1);
-        dd_mbar_init(&bar[1], 1);
+        for (int i = 0; i < kS; i++) {
+            armed[i] = 0;
+            dd_mbar_init(&full[i], 1);
+            dd_mbar_init(&empty[i], kCons3);
+        }
+        for (int i = 0; i < kP; i++)
+            for (int b = 0; b < 2; b++) {
+                nrec[i][b] = 0;
+                dd_mbar_init(&rbar[i][b], 1);
+            }
         dd_fence_mbar_init();
     }
     __syncthreads();
 
     const int xb = w.xb;
-    const int nline = xb ? H : W, npix = xb ? W : H;
-    auto issue = [&](int line, int buf) {
-        nissue[buf]++;
-        dd_mbar_expect_tx(&bar[buf], (uint32_t)(sizeof(DdLine) + sizeof(float4)));
-        dd_bulk_g2s(&srec[buf], lines + line, (uint32_t)sizeof(DdLine), &bar[buf]);
-        dd_bulk_g2s(&slzr[buf], linez + line, (uint32_t)sizeof(float4), &bar[buf]);
-    };
-    // segments of line m (record buffer m & 1) into segment buffer sb; one warp
-    auto produce = [&](int m, int sb) -> bool {
-        const int rbuf = m & 1;
-        const uint32_t parity = (uint32_t)nwait[rbuf] & 1u;
-        if (!dd_mbar_wait(&bar[rbuf], parity)) return false;
-        const DdLine *L = &srec[rbuf];
-        const float4 lz = slzr[rbuf];
-        if (lane == 0) slz[sb] = lz;
-        int n = 0;
-        DdColWalk cw;
-        if (active && dd3_colwalk_init(L, sdp, lane, kk, &cw)) {
-            const float lpos = (FAMILY == 2) ? dd3_line_pos(&g, &w, m) : 0.0f;
-            int j;
-            float wd;
-            while (dd3_colwalk_next(L, &cw, &j, &wd)) {
-                if (n == kSeg) {   // more than kSeg segments: consumers walk the record themselves
-                    n = kSeg + 1;
-                    break;
-                }
-                segj[sb][n][lane] = j;
-                segc[sb][n][lane] = dd3_coef(GEOM, FAMILY, &g, &w, lpos, j, wd, lz.w);
-                n++;
-            }
-        }
-        segn[sb][lane] = n;
-        __syncwarp();
-        if (lane == 0) nwait[rbuf]++;
-        return true;
-    };
+    const int nline = xb ? H : W;
 
-    float rp0[kFR], rp1[kFR];
+    // row boundaries; rows that do not exist (or are inverted) are empty
+    // intervals where the previous row ended
+    float rp0[RR], rp1[RR];
     {
         const float mag = active ? reinterpret_cast<const float *>(a.plan + P.mag)[(size_t)v * P.smag + k] : 1.0f;
+        float zmin = 3.0e38f, zmax = -3.0e38f, last = 0.0f;
 #pragma unroll
-        for (int q = 0; q < kFR; q++) {
+        for (int q = 0; q < RR; q++) {
             const int r = r0 + q;
-            if (active && !prod && r < R) {
-                dd3_rp(GEOM, &w, mag, rz[2 * r], rz[2 * r + 1], &rp0[q], &rp1[q]);
+            float e0 = 0.0f, e1 = 0.0f;
+            if (active && !prod && r < R) dd3_rp(a.geom, &w, mag, rz[2 * r], rz[2 * r + 1], &e0, &e1);
+            if (e0 < e1) {
+                zmin = fminf(zmin, e0);
+                zmax = fmaxf(zmax, e1);
+                last = e1;
             } else {
-                rp0[q] = 3.0e38f;    // empty row: the z walk never starts
-                rp1[q] = -3.0e38f;
+                e0 = e1 = last;
             }
+            rp0[q] = e0;
+            rp1[q] = e1;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            zmin = fminf(zmin, __shfl_xor_sync(0xffffffffu, zmin, o));
+            zmax = fmaxf(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
+        }
+        if (lane == 0 && !prod) {
+            zrange[warp][0] = zmin;
+            zrange[warp][1] = zmax;
         }
     }
-    float acc[kFR][kNB];
-#pragma unroll
-    for (int q = 0; q < kFR; q++)
-#pragma unroll
-        for (int b = 0; b < kNB; b++) acc[q][b] = 0.0f;
-
-    const float *__restrict__ src = xb ? a.vol : a.volT;
-    const size_t plane = (size_t)nline * npix;
-    const size_t vstride = (size_t)Dp * plane;
-    src += (size_t)b0 * vstride;
-
-    // prologue: records 0 and 1 in flight, segments of line 0 computed
+    __syncthreads();
     if (tid == 0) {
-        issue(0, 0);
-        if (nline > 1) issue(1, 1);
+        float lo = 3.0e38f, hi = -3.0e38f;
+        for (int i = 0; i < kCons3; i++) {
+            lo = fminf(lo, zrange[i][0]);
+            hi = fmaxf(hi, zrange[i][1]);
+        }
+        zrange[kCons3][0] = lo;
+        zrange[kCons3][1] = hi;
     }
     __syncthreads();
-    if (prod && !produce(0, 0)) abort_flag = 1;
-    __syncthreads();
-    if (tid == 0 && !abort_flag && nline > 2) issue(2, 0);
-    for (int line = 0; line < nline && !abort_flag; line++) {
-        const int sb = line & 1;
-        if (line + 1 < nline && prod && !produce(line + 1, sb ^ 1)) abort_flag = 1;
-        // consume line `line`
-        const int n = segn[sb][lane];
-        if (active && !prod && n > 0) {
-            const float4 lz = slz[sb];
-            const float *__restrict__ lsrc = src + (size_t)line * npix;
-            if (n <= kSeg) {
-#pragma unroll
-                for (int q = 0; q < kFR; q++) {
-                    const float bz0 = fmaxf(lz.x, rp0[q]), bz1 = fminf(lz.y, rp1[q]);
-                    if (!(bz0 < bz1)) continue;
-                    int s = dd3_slice_first(bz0, lz.x, lz.z);
-                    float zhi = dd3_zb(lz.x, lz.z, s);
-                    for (; s < Dp; s++) {
-                        const float zlo = zhi;
-                        if (!(zlo < bz1)) break;
-                        zhi = dd3_zb(lz.x, lz.z, s + 1);
-                        const float zw = dd3_cell(bz0, bz1, zlo, zhi);
-                        if (!(zw > 0.0f)) continue;
-                        const float *__restrict__ ps = lsrc + (size_t)s * plane;
-                        for (int t = 0; t < n; t++) {
-                            const float wq = FMUL(zw, segc[sb][t][lane]);
-                            const int j = segj[sb][t][lane];
-#pragma unroll
-                            for (int b = 0; b < kNB; b++)
-                                if (b < nb) acc[q][b] = fmaf(wq, __ldg(ps + (size_t)b * vstride + j), acc[q][b]);
+
+    // Steps per line: enough for the slices the CTA's rows can meet on the
+    // line with the most of them; the tile's pitch: for the pixels its columns
+    // meet on the line whose pixels are narrowest.  Both are an end of the
+    // lines, unless the source lies between them (a negative pitch).
+    constexpr int kAl = 4 / NB;   // pixels in 16 bytes
+    int pi, zstep, nstep, nchunk;
+    {
+        const float zmin = zrange[kCons3][0], zmax = zrange[kCons3][1];
+        const float4 la = linez[0], lb = linez[nline - 1];
+        const float pm = fminf(la.z, lb.z), px = fminf(la.w / la.z, lb.w / lb.z), span = sdp[kFC] - sdp[0];
+        const float widest = (pm > 0.0f && zmin < zmax) ? fminf((zmax - zmin) / pm + 4.0f, (float)Dp) : (float)Dp;
+        const float npx = (pm > 0.0f && px > 0.0f && span >= 0.0f) ? span / px + (float)(2 + kAl) : 1.0e6f;
+        for (pi = 0; pi < kNPitch - 1 && npx > (float)pitch3(pi); pi++) {}
+        zstep = kZW;
+        nchunk = max(1, ((int)widest + zstep - 1) / zstep);
+        nstep = nline * nchunk;
+    }
+    const int tpitch = pitch3(pi);
+    const int np4 = pad4(xb ? W : H);
+    const T *__restrict__ src = reinterpret_cast<const T *>(xb ? a.volx : a.volt) + (size_t)blockIdx.z * Dp * nline * np4;
+
+    if (prod) {
+        const int p = warp - kCons3;
+        auto issue = [&](int line, int buf) {   // a line's record (one lane)
+            nrec[p][buf]++;
+            dd_mbar_expect_tx(&rbar[p][buf], (uint32_t)(sizeof(DdLine) + sizeof(float4)));
+            dd_bulk_g2s(&srec[p][buf], lines + line, (uint32_t)sizeof(DdLine), &rbar[p][buf]);
+            dd_bulk_g2s(&slzr[p][buf], linez + line, (uint32_t)sizeof(float4), &rbar[p][buf]);
+        };
+        if (lane == 0) {
+            if (p < nstep) issue(p / nchunk, 0);
+            if (p + kP < nstep) issue((p + kP) / nchunk, 1);
+        }
+        const float zmin = zrange[kCons3][0], zmax = zrange[kCons3][1];
+        const float dlo = sdp[lane], dhi = sdp[lane + 1];
+        int st = p, use = 0, line = p / nchunk, part = p - line * nchunk;
+        for (int m = p, n = 0; m < nstep; m += kP, n++) {
+            const int buf = n & 1;
+            bool ok = dd_mbar_wait(&rbar[p][buf], (uint32_t)(n >> 1) & 1u);
+            if (ok && use > 0) ok = dd_mbar_wait(&empty[st], (uint32_t)(use - 1) & 1u);
+            if (!__all_sync(0xffffffffu, ok)) {
+                abort_flag = 1;
+                break;
+            }
+            const DdLine *L = &srec[p][buf];
+            const float4 lz = slzr[p][buf];
+            Step3<NB> &S = steps[st];
+            // slices [first, first + ns) of the step (a line behind the source
+            // has a negative pitch and meets nothing)
+            int first = 0, ns = 0;
+            const float inv = 1.0f / lz.z;
+            if (lz.z > 0.0f && zmin < zmax) {
+                const float top = (float)Dp;
+                first = (int)fminf(fmaxf(floorf((zmin - lz.x) * inv) - 1.0f, 0.0f), top);
+                ns = (int)fminf(fmaxf(floorf((zmax - lz.x) * inv) + 2.0f, 0.0f), top) - first;
+                const int skip = part * zstep;
+                first += skip;
+                ns = min(max(ns - skip, 0), zstep);
+            }
+            int nseg = 0, jb = 0, pitch = 0;
+            bool fast = false;
+            if (ns > 0) {
+                for (int i = lane; i <= ns + 1; i += 32) {
+                    float t = dd3_zb(lz.x, lz.z, first + i);
+                    if (first + i == Dp) t = fminf(t, lz.y);
+                    S.top[i] = (i == ns + 1) ? __int_as_float(0x7f800000) : t;
+                }
+                __syncwarp();
+                // The column's segments: the lane's first pixel by a linear
+                // estimate (the drift is a small part of a pixel), settled on
+                // the exact boundaries; then the pixels in order.
+                int jf = 0;
+                const DdLineHdr hd = L->h;
+                const float CL = (kk == hd.idet0) ? hd.bound0 : dlo, CH = dhi;
+                if (active && hd.npiece > 0 && kk >= hd.idet0 && CL < CH) {
+                    const DdPiece P0 = L->p[0];
+                    const float t = floorf(FMUL(FSUB(CL, P0.Q), P0.invdl)) + (float)(P0.gb + 1);
+                    int j = (int)fminf(fmaxf(t, (float)hd.i0), (float)(hd.nend - 1));
+                    int pc = L->slot[dd_slot(CL)];
+                    DdPiece Pc = L->p[pc];
+                    auto bound = [&](int e) {   // boundary e >= i0; its piece is kept
+                        while (pc < hd.npiece - 1 && e > Pc.gb) Pc = L->p[++pc];
+                        while (pc > 0 && e <= L->p[pc - 1].gb) Pc = L->p[--pc];
+                        return FADD(Pc.Q, FMUL((float)(e - Pc.gb), Pc.dl));
+                    };
+                    float plo = (j > hd.i0) ? bound(j - 1) : hd.bound0;
+                    while (j > hd.i0 && plo > CL) {
+                        j--;
+                        plo = (j > hd.i0) ? bound(j - 1) : hd.bound0;
+                    }
+                    float phi = bound(j);
+                    while (phi <= CL && j < hd.nend - 1) {
+                        plo = phi;
+                        phi = bound(++j);
+                    }
+                    jf = j;
+                    plo = fmaxf(plo, CL);
+                    if (phi > CL) {
+                        const float lpos = (a.family == 2) ? dd3_line_pos_f(&g, &w, line) : 0.0f;
+#pragma unroll 1
+                        while (plo < CH) {
+                            if (nseg == kSeg) {
+                                nseg = kSeg + 1;
+                                break;
+                            }
+                            S.c[nseg++][lane] = dd3_coef(a.geom, a.family, &g, &w, lpos, j, FSUB(fminf(phi, CH), plo), lz.w);
+                            plo = phi;
+                            if (++j >= hd.nend) break;
+                            phi = bound(j);
                         }
                     }
                 }
-            } else {
-                // wide column: walk the record in global memory
-                const DdLine *Lg = lines + line;
-                const float lpos = (FAMILY == 2) ? dd3_line_pos(&g, &w, line) : 0.0f;
-                DdColWalk cw;
-                if (dd3_colwalk_init(Lg, sdp, lane, kk, &cw)) {
-                    int j;
-                    float wd;
-                    while (dd3_colwalk_next(Lg, &cw, &j, &wd)) {
-                        const float cf = dd3_coef(GEOM, FAMILY, &g, &w, lpos, j, wd, lz.w);
+                const int lo = __reduce_min_sync(0xffffffffu, nseg > 0 ? jf : 0x7fffffff);
+                const int hi = __reduce_max_sync(0xffffffffu, nseg > 0 ? jf + nseg : -1);
+                const bool wide = __any_sync(0xffffffffu, nseg > kSeg);
+                if (hi < 0) {
+                    ns = 0;   // no column meets the line
+                } else {
+                    jb = lo / kAl * kAl;
+                    pitch = (wide || hi - jb > tpitch) ? 0 : tpitch;
+                }
+                fast = __all_sync(0xffffffffu, nseg <= kFast) && pitch > 0 && nchunk == 1;
+                S.nseg[lane] = nseg;
+                S.j0[lane] = jf - jb;
+            }
+            if (lane == 0) {
+                S.h = make_float4(lz.x, inv, __int_as_float(first), __int_as_float(ns));
+                S.pitch = pitch;
+                S.line = line;
+                S.fast = fast;
+            }
+            __syncwarp();   // the record has been read, the step's arrays are written
+            if (lane == 0) {
+                // the voxels of slices first - 1 .. first + ns, in boxes of kZB
+                // slices: the outer two are zero at the volume's ends, and
+                // otherwise beyond the rows
+                const int nbox = pitch > 0 ? (ns + 2 + kZB - 1) / kZB : 0;
+                const uint32_t box_b = (uint32_t)(kZB * pitch * (int)sizeof(T));
+                armed[st] = use + 1;
+                dd_mbar_expect_tx(&full[st], box_b * (uint32_t)nbox);
+                for (int i = 0; i < nbox; i++)
+                    dd_tensor4_g2s(sm + st * kTileB3<NB> + i * box_b, &maps.m[xb][pi], jb * NB, line, first - 1 + i * kZB,
+                                   (int)blockIdx.z, &full[st]);
+                if (m + 2 * kP < nstep) issue(nchunk == 1 ? m + 2 * kP : (m + 2 * kP) / nchunk, buf);
+            }
+            st += kP;
+            if (st >= kS) {
+                st -= kS;
+                use++;
+            }
+            for (part += kP; part >= nchunk; part -= nchunk) line++;
+        }
+    }
+
+    T acc[RR];
 #pragma unroll
-                        for (int q = 0; q < kFR; q++) {
-                            const float bz0 = fmaxf(lz.x, rp0[q]), bz1 = fminf(lz.y, rp1[q]);
-                            if (!(bz0 < bz1)) continue;
-                            for (int s = dd3_slice_first(bz0, lz.x, lz.z); s < Dp; s++) {
-                                const float zlo = dd3_zb(lz.x, lz.z, s);
-                                if (!(zlo < bz1)) break;
-                                const float zw = dd3_cell(bz0, bz1, zlo, dd3_zb(lz.x, lz.z, s + 1));
-                                if (!(zw > 0.0f)) continue;
-                                const float wq = FMUL(zw, cf);
-                                const float *__restrict__ ps = lsrc + (size_t)s * plane + j;
+    for (int q = 0; q < RR; q++) acc[q] = VT::zero();
+    if (!prod) {
+        int st = 0, par = 0;
+        for (int m = 0; m < nstep; m++) {
+            const bool ok = dd_mbar_wait(&full[st], (uint32_t)par);
+            if (!__all_sync(0xffffffffu, ok)) {
+                abort_flag = 1;
+                break;
+            }
+            const Step3<NB> &S = steps[st];
+            const float4 h = S.h;
+            const int first = __float_as_int(h.z), n = __float_as_int(h.w), pitch = S.pitch;
+            const int nseg = n > 0 ? S.nseg[lane] : 0;
+            if (nseg > 0) {
+                // entry (slice first + entry - 1) of the first row's lower
+                // boundary: the closed-form estimate, settled on the exact boundaries
+                int i = (int)fminf(fmaxf(floorf((rp0[0] - h.x) * h.y) - (float)(first - 1), 0.0f), (float)(n + 1));
+                if (i > 0 && rp0[0] < S.top[i - 1]) i--;
+                else if (i <= n && !(rp0[0] < S.top[i])) i++;
+                const T *tile = reinterpret_cast<const T *>(sm + st * kTileB3<NB>) + S.j0[lane];   // entry 0
+                const float *zp = S.top + i;
+                if (S.fast) {   // uniform: the usual case, kept short
+                    using K = typename VT::K;
+                    const K k0 = VT::coef(S.c[0][lane]), k1 = VT::coef(S.c[1][lane]), k2 = VT::coef(S.c[2][lane]);   // unused past nseg
+                    const bool p1 = nseg > 1, p2 = nseg > 2;
+                    const T *r = tile + i * pitch;
+                    auto column = [&]() -> T {
+                        const T v0 = r[0], v1 = r[1], v2 = r[2];   // the tile is followed by room for these
+                        T x = VT::kmul(k0, v0);
+                        if (p1) x = VT::kfma(k1, v1, x);
+                        if (p2) x = VT::kfma(k2, v2, x);
+                        return x;
+                    };
+                    T x = column();
+                    float zhi = *zp;
 #pragma unroll
-                                for (int b = 0; b < kNB; b++)
-                                    if (b < nb) acc[q][b] = fmaf(wq, __ldg(ps + (size_t)b * vstride), acc[q][b]);
+                    for (int q = 0; q < RR; q++) {
+                        const float w0 = FSUB(fminf(rp1[q], zhi), rp0[q]);
+                        if (w0 > 0.0f) acc[q] = VT::fma(w0, x, acc[q]);
+                        while (zhi < rp1[q]) {   // so the next slice's overlap is positive
+                            const float lo = zhi;
+                            r += pitch;
+                            x = column();
+                            zhi = *++zp;
+                            acc[q] = VT::fma(FSUB(fminf(rp1[q], zhi), lo), x, acc[q]);
+                        }
+                    }
+                } else {
+                    auto column = [&](int e) -> T {
+                        T x = VT::zero();
+                        if ((unsigned)(e - 1) < (unsigned)n) {
+                            if (pitch > 0) {
+                                for (int t = 0; t < nseg; t++) x = VT::fma(S.c[t][lane], tile[e * pitch + t], x);
+                            } else {
+                                const int line = S.line;
+                                x = column_sum3<NB>(a, w, lines + line, sdp, lane, kk,
+                                                    a.family == 2 ? dd3_line_pos_f(&g, &w, line) : 0.0f, linez[line].w,
+                                                    src + ((size_t)(first + e - 1) * nline + line) * np4);
                             }
                         }
+                        return x;
+                    };
+                    T x = column(i);
+                    float zhi = *zp;
+#pragma unroll
+                    for (int q = 0; q < RR; q++) {
+                        const float w0 = FSUB(fminf(rp1[q], zhi), rp0[q]);
+                        if (w0 > 0.0f) acc[q] = VT::fma(w0, x, acc[q]);
+                        while (zhi < rp1[q]) {
+                            const float lo = fmaxf(zhi, rp0[q]);
+                            x = column(++i);
+                            zhi = S.top[i];
+                            const float w1 = FSUB(fminf(rp1[q], zhi), lo);
+                            if (w1 > 0.0f) acc[q] = VT::fma(w1, x, acc[q]);
+                        }
                     }
                 }
             }
+            __syncwarp();
+            if (lane == 0) dd_mbar_arrive(&empty[st]);
+            if (++st == kS) {
+                st = 0;
+                par ^= 1;
+            }
         }
-        __syncthreads();
-        // the record of line + 1 has been turned into segments: its buffer takes line + 3
-        if (tid == 0 && !abort_flag && line + 3 < nline) issue(line + 3, (line + 1) & 1);
     }
     __syncthreads();
     if (abort_flag) {
         // let copies still in flight land before the CTA exits
         if (tid == 0) {
-            for (int b = 0; b < 2; b++)
-                if (nissue[b] > nwait[b]) dd_mbar_drain(&bar[b], (uint32_t)nwait[b] & 1u);
+            for (int i = 0; i < kS; i++)
+                if (armed[i] > 0) dd_mbar_drain(&full[i], (uint32_t)(armed[i] - 1) & 1u);
+            for (int p = 0; p < kP; p++)
+                for (int b = 0; b < 2; b++)
+                    if (nrec[p][b] > 0) dd_mbar_drain(&rbar[p][b], (uint32_t)(nrec[p][b] - 1) & 1u);
             dd_report_timeout(a.status);
         }
         return;
@@ -471,18 +743,22 @@ __global__ void __launch_bounds__(kFwdThreads3, 3) k_fwd3(const Fwd3Args a) {
     if (!active || prod) return;
     const int ko = w.flip ? C - 1 - k : k;
 #pragma unroll
-    for (int q = 0; q < kFR; q++) {
+    for (int q = 0; q < RR; q++) {
         const int r = r0 + q;
         if (r >= R) continue;
-        const float scale = (FAMILY == 0) ? dd3_proj_scale(&g, &w, sdp[lane], sdp[lane + 1], rp0[q], rp1[q]) : w.bp_scale;
+        float scale = w.bp_scale;
+        if (a.family == 0) {
+            float e0, e1;
+            dd3_rp(a.geom, &w, reinterpret_cast<const float *>(a.plan + P.mag)[(size_t)v * P.smag + k], rz[2 * r],
+                   rz[2 * r + 1], &e0, &e1);
+            scale = dd3_proj_scale(&g, &w, sdp[lane], sdp[lane + 1], e0, e1);
+        }
 #pragma unroll
-        for (int b = 0; b < kNB; b++) {
-            if (b < nb) {
-                const size_t o = (((size_t)(b0 + b) * a.V + v) * R + r) * C + ko;
-                float val = FMUL(acc[q][b], scale);
-                if (a.sub) val = FSUB(val, a.sub[o]);
-                a.out[o] = val;
-            }
+        for (int b = 0; b < NB; b++) {
+            const size_t o = (((size_t)(b0 + b) * a.V + v) * R + r) * C + ko;
+            float val = FMUL(VT::get(acc[q], b), scale);
+            if (a.sub) val = FSUB(val, a.sub[o]);
+            a.out[o] = val;
         }
     }
 }
@@ -953,17 +1229,77 @@ int plan(int scan, const dd_geom3d *g, const float *angles, const float *sp, int
     return launch_status();
 }
 
-template <int GEOM>
-int launch_fwd(int family, const Fwd3Args &a, cudaStream_t st) {
-    const dim3 grid((unsigned)a.V, (unsigned)((a.g.num_col + kFC - 1) / kFC),
-                    (unsigned)(a.nrb * ((a.B + kNB - 1) / kNB)));
-    dd2::ProfRec *pr = dd2::prof_begin(DD_KERNEL_FORWARD, st);
-    if (family == 0) k_fwd3<GEOM, 0><<<grid, kFwdThreads3, 0, st>>>(a);
-    else if (family == 1) k_fwd3<GEOM, 1><<<grid, kFwdThreads3, 0, st>>>(a);
-    else k_fwd3<GEOM, 2><<<grid, kFwdThreads3, 0, st>>>(a);
-    dd2::prof_end(pr, st);
+// cuTensorMapEncodeTiled, from the driver the runtime has loaded
+using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encode_tiled() {
+    static const EncodeTiled fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            (void)cudaGetLastError();
+            p = nullptr;
+        }
+        return (EncodeTiled)p;
+    }();
+    return fn;
+}
+
+template <int NB>
+int make_maps3(const Fwd3Args &a, int ngroups, Maps3 *maps) {
+    const EncodeTiled enc = encode_tiled();
+    if (!enc) return DD_ERR_LAUNCH;
+    for (int rows = 0; rows < 2; rows++) {
+        const cuuint64_t np = (cuuint64_t)(rows ? a.g.width : a.g.height), nl = (cuuint64_t)(rows ? a.g.height : a.g.width);
+        const cuuint64_t line_b = (cuuint64_t)pad4((int)np) * NB * sizeof(float);
+        const cuuint64_t dim[4] = {np * NB, nl, (cuuint64_t)a.g.depth, (cuuint64_t)ngroups};
+        const cuuint64_t str[3] = {line_b, line_b * nl, line_b * nl * dim[2]};
+        const cuuint32_t one[4] = {1, 1, 1, 1};
+        for (int i = 0; i < kNPitch; i++) {
+            const cuuint32_t box[4] = {(cuuint32_t)(pitch3(i) * NB), 1, kZB, 1};
+            if (enc(&maps->m[rows][i], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void *)(rows ? a.volx : a.volt), dim, str, box,
+                    one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+                return DD_ERR_LAUNCH;
+        }
+    }
+    return DD_OK;
+}
+
+template <int NB, int RR>
+int launch_fwd_rows(Fwd3Args a, int ngroups, cudaStream_t st) {
+    a.ncg = (a.g.num_col + kFC - 1) / kFC;
+    a.nrb = (a.g.num_row + RR * kCons3 - 1) / (RR * kCons3);
+    const long long nx = (long long)a.ncg * a.nrb;
+    if (nx > 0x7FFFFFFFLL) return DD_ERR_SIZE_OVERFLOW;
+    const int smem = kStage3<NB> * kTileB3<NB> + kFast * 8;   // the fast path reads up to two pixels past a row
+    if (cudaFuncSetAttribute(k_fwd3<NB, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        return DD_ERR_LAUNCH;
+    Maps3 maps;
+    const int rc = make_maps3<NB>(a, ngroups, &maps);
+    if (rc != DD_OK) return rc;
+    k_fwd3<NB, RR><<<dim3((unsigned)nx, (unsigned)a.V, (unsigned)ngroups), kFwdThreads3<NB>, smem, st>>>(a, maps);
     dd2::count_launches(1);
-    return launch_status();
+    return DD_OK;
+}
+
+// Rows per thread: 8, 4 or 2, whichever leaves least work for rows that do not
+// exist -- a step costs a thread its rows plus about 2.5 rows' worth of
+// finding the first slice and of its share of the producers.
+template <int NB>
+int launch_fwd_volumes(Fwd3Args a, int b0, int ngroups, cudaStream_t st) {
+    if (ngroups <= 0) return DD_OK;
+    a.b0 = b0;
+    a.volx += (size_t)b0 * a.g.depth * a.g.height * pad4(a.g.width);
+    a.volt += (size_t)b0 * a.g.depth * a.g.width * pad4(a.g.height);
+    const int R = a.g.num_row;
+    auto cost = [&](int rr) { return ((R + rr * kCons3 - 1) / (rr * kCons3)) * (rr + 2.5); };
+    const double c8 = cost(8), c4 = cost(4), c2 = cost(2);
+    if (c8 <= c4 && c8 <= c2) return launch_fwd_rows<NB, 8>(a, ngroups, st);
+    if (c4 <= c2) return launch_fwd_rows<NB, 4>(a, ngroups, st);
+    return launch_fwd_rows<NB, 2>(a, ngroups, st);
 }
 
 template <int GEOM, int NB, int ZS>
@@ -1005,21 +1341,22 @@ int launch_adj(const Adj3Args &a, const float *in, float *ss, cudaStream_t st) {
     return rc != DD_OK ? rc : launch_status();
 }
 
-int transpose(const dd_geom3d *g, const float *in, float *out, int B, cudaStream_t st) {
-    const int np = B * g->depth;
-    const dim3 grid((unsigned)((g->width + 31) / 32), (unsigned)((g->height + 31) / 32),
-                    (unsigned)(np < 65535 ? np : 65535));
-    dd2::ProfRec *pr = dd2::prof_begin(DD_KERNEL_TABLES, st);
-    k_transpose3<<<grid, 256, 0, st>>>(in, out, g->width, g->height, np);
-    dd2::prof_end(pr, st);
-    dd2::count_launches(1);
-    return launch_status();
-}
-
 // Forward-type operator into `out` (optionally minus `sub`).
 int forward(int scan, int op, const dd_geom3d *g, const char *planb, const float *in, float *out,
-            const float *sub, int B, int V, char *volT, int *status, cudaStream_t st) {
-    const int s1 = transpose(g, in, (float *)volT, B, st);
+            const float *sub, int B, int V, char *volx, char *volt, int *status, cudaStream_t st) {
+    const int W = g->width, H = g->height, Dp = g->depth;
+    const int pairs = B / kNB, odd = B % kNB;
+    const long long nz = (long long)Dp * (pairs > 1 ? pairs : 1);
+    const dim3 gl((unsigned)((W + 31) / 32), (unsigned)((H + 31) / 32), (unsigned)(nz < 65535 ? nz : 65535));
+    const size_t done = (size_t)pairs * kNB * Dp;   // slices of the paired volumes
+    dd2::ProfRec *pt = dd2::prof_begin(DD_KERNEL_TABLES, st);
+    if (pairs) k_lines_of3<kNB><<<gl, 256, 0, st>>>(in, (float *)volx, (float *)volt, W, H, Dp, pairs);
+    if (odd)
+        k_lines_of3<1><<<gl, 256, 0, st>>>(in + done * W * H, (float *)volx + done * H * pad4(W),
+                                           (float *)volt + done * W * pad4(H), W, H, Dp, 1);
+    dd2::prof_end(pt, st);
+    dd2::count_launches((pairs ? 1 : 0) + odd);
+    const int s1 = launch_status();
     if (s1 != DD_OK) return s1;
     if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
     Fwd3Args a;
@@ -1027,17 +1364,20 @@ int forward(int scan, int op, const dd_geom3d *g, const char *planb, const float
     a.g = *g;
     a.plan = planb;
     a.P = plan_layout(g, V);
-    a.vol = in;
-    a.volT = (const float *)volT;
+    a.volx = (const float *)volx;
+    a.volt = (const float *)volt;
     a.out = out;
     a.sub = sub;
-    a.B = B;
     a.V = V;
-    a.nrb = (g->num_row + kFR * kFwdWarps3 - 1) / (kFR * kFwdWarps3);
-    const int fam = op_family(op), geom = geom_of(scan);
-    if (geom == DD_GEOM3_CONE_FLAT) return launch_fwd<DD_GEOM3_CONE_FLAT>(fam, a, st);
-    if (geom == DD_GEOM3_CONE_ARC) return launch_fwd<DD_GEOM3_CONE_ARC>(fam, a, st);
-    return launch_fwd<DD_GEOM3_SPIRAL>(fam, a, st);
+    a.nrb = a.ncg = 0;
+    a.b0 = 0;
+    a.geom = geom_of(scan);
+    a.family = op_family(op);
+    dd2::ProfRec *pr = dd2::prof_begin(DD_KERNEL_FORWARD, st);
+    int rc = launch_fwd_volumes<kNB>(a, 0, pairs, st);
+    if (rc == DD_OK) rc = launch_fwd_volumes<1>(a, pairs * kNB, odd, st);
+    dd2::prof_end(pr, st);
+    return rc != DD_OK ? rc : launch_status();
 }
 
 // Adjoint-type operator: out = value, or out = base + scale * value.
@@ -1109,7 +1449,7 @@ extern "C" int dd3d_apply_planned(int scan, int op, const dd_geom3d *g, const vo
     char *wb = (char *)workspace;
     cudaStream_t s = (cudaStream_t)stream;
     int *status = (int *)(wb + A.status);
-    if (f) return forward(scan, op, g, (const char *)planp, in, out, nullptr, batch, num_view, wb + A.volT, status, s);
+    if (f) return forward(scan, op, g, (const char *)planp, in, out, nullptr, batch, num_view, wb + A.volx, wb + A.volt, status, s);
     return adjoint(scan, op, g, (const char *)planp, in, out, nullptr, 0.0f, batch, num_view, wb + A.ss, status, s);
 }
 
@@ -1152,7 +1492,7 @@ extern "C" int dd3d_dc_step(int scan, const dd_geom3d *g, const void *planp, flo
     cudaStream_t s = (cudaStream_t)stream;
     const char *pb = (const char *)planp;
     int *status = (int *)(wb + A.status);
-    const int s1 = forward(scan, DD_OP_PROJ, g, pb, x, resid, y, batch, num_view, wb + A.volT, status, s);
+    const int s1 = forward(scan, DD_OP_PROJ, g, pb, x, resid, y, batch, num_view, wb + A.volx, wb + A.volt, status, s);
     if (s1 != DD_OK) return s1;
     return adjoint(scan, DD_OP_PROJ_T, g, pb, resid, x, x, -eta, batch, num_view, wb + A.ss, status + 1, s);
 }

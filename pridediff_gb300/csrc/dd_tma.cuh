@@ -58,6 +58,10 @@ __device__ __forceinline__ void dd_mbar_expect_tx(uint64_t *bar, uint32_t bytes)
                  : "memory");
 }
 
+__device__ __forceinline__ void dd_mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(dd_smem_addr(bar)) : "memory");
+}
+
 // 1-D bulk copy global -> shared, completion signalled on `bar`.
 // dst, src 16-byte aligned; bytes a multiple of 16.
 __device__ __forceinline__ void dd_bulk_g2s(void *dst, const void *src, uint32_t bytes,
@@ -66,6 +70,17 @@ __device__ __forceinline__ void dd_bulk_g2s(void *dst, const void *src, uint32_t
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
             dd_smem_addr(dst)),
         "l"(src), "r"(bytes), "r"(dd_smem_addr(bar))
+        : "memory");
+}
+
+// Tiled 4-D copy global -> shared of the map's box at (c0, c1, c2, c3), zero
+// past the tensor.  dst 128-byte aligned; c0 x 4 bytes a multiple of 16.
+__device__ __forceinline__ void dd_tensor4_g2s(void *dst, const void *map, int c0, int c1, int c2, int c3,
+                                               uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+            dd_smem_addr(dst)),
+        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(dd_smem_addr(bar))
         : "memory");
 }
 
