@@ -144,8 +144,8 @@ typedef struct dd_tune2d {
     int ctas_per_sm;    /* persistent CTAs per SM (0 = as many as fit; capped at that) */
     int lpt_order;      /* items longest-first (1) or in instance order (0) */
     /* single-geometry forward (dd2d_apply_planned_tuned): */
-    int fwd_slices;     /* slices per CTA: 4 (default) or 1 */
-    int fwd_cluster;    /* CTAs sharing a view's walked lines, a cluster: 2 (default) or 1 */
+    int fwd_slices;     /* slices per CTA: 4 (default; the kernel takes up to 8, or as many as there are) or 1 */
+    int fwd_cluster;    /* CTAs sharing a view's walked lines, a cluster: 2 (default) or 1; same results */
     /* persistent forward: */
     int items_cluster;  /* CTAs sharing an item's walked lines: 1 (default) or 2 */
     int reserved[3];
@@ -157,8 +157,8 @@ int dd2d_apply_planned_tuned(int scan, int op, const dd_geom2d *g, const void *p
                              float *out, int batch, int num_view, void *workspace, size_t workspace_bytes,
                              const dd_tune2d *tune, dd_stream_t stream);
 /* The forward CTA shape a tune resolves to on this geometry (slices per CTA,
- * cluster size): 4 slices become 2 where their line tables would not fit in
- * shared memory. */
+ * cluster size): 4 slices become 1 where lines are too long for 4 (more than
+ * about 3,400 pixels). */
 int dd2d_fwd_shape(int scan, const dd_geom2d *g, const dd_tune2d *tune, int *slices, int *cluster);
 
 size_t dd2d_batch_plan_bytes(int scan, const dd_instance2d *inst, int n);

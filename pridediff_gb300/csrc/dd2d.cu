@@ -30,7 +30,7 @@
 #include <stdint.h>
 #include <string.h>
 
-#include "dd2d_kernels.cuh"
+#include "dd2d_fwd.cuh"
 #include "dd_trace.h"
 
 namespace dd2 {
@@ -73,55 +73,18 @@ __global__ void k_lines(int geom, dd_geom2d g, const float *__restrict__ angles,
 }
 
 // ---------------------------------------------------------------------------
-// Prefix tables
+// Forward: planes of rows and columns, and the single-geometry launch
 // ---------------------------------------------------------------------------
-// Row lines (x-branch): one warp per (image, row); S_j = sum_{i<j} x_i in
-// double-float arithmetic, rounded once.  Entry n = (S_n, 0).
-__global__ void k_tab_rows(const float *__restrict__ img, int B, int H, int W,
-                           float2 *__restrict__ tab) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= B * H) return;
-    const float *row = img + (size_t)warp * W;
-    warp_prefix_table(W, tab + (size_t)warp * rs_entries(W), lane, [&](int j, float *x, float *w) {
-        *x = row[j];
-        *w = 1.0f;
-    });
-}
-
-// Column lines (y-branch): line = image column, walked from the bottom row.
-// A block takes 32 columns of one image (lanes: coalesced reads along a row)
-// and splits the rows into kColChunks chunks (warps): each warp sums its
-// chunk in double-float arithmetic, the chunk totals are added in order, and
-// each warp then writes its rows' prefixes from its chunk's start -- 8 times
-// the threads of one walk per column.
-constexpr int kColChunks = 8;
-__global__ void __launch_bounds__(32 * kColChunks)
-k_tab_cols(const float *__restrict__ img, int B, int H, int W, float2 *__restrict__ tab) {
-    const int c = threadIdx.x & 31, k = threadIdx.x >> 5;
-    const int ncb = (W + 31) / 32;
-    const int b = blockIdx.x / ncb, col = (blockIdx.x - b * ncb) * 32 + c;
-    const int per = (H + kColChunks - 1) / kColChunks;
-    const int i0 = min(H, k * per), i1 = min(H, i0 + per);
-    const bool ok = b < B && col < W;
-    const float *__restrict__ im = img + (size_t)b * H * W + col;
-    __shared__ float tot_hi[kColChunks][32], tot_lo[kColChunks][32];
-    DdF run = {0.0f, 0.0f};
-    if (ok)
-        for (int i = i0; i < i1; i++) run = df_add(run, DdF{__ldg(im + (size_t)(H - 1 - i) * W), 0.0f});
-    tot_hi[k][c] = run.hi;
-    tot_lo[k][c] = run.lo;
-    __syncthreads();
-    if (!ok) return;
-    run = {0.0f, 0.0f};
-    for (int q = 0; q < k; q++) run = df_add(run, DdF{tot_hi[q][c], tot_lo[q][c]});
-    float2 *__restrict__ t = tab + ((size_t)b * W + col) * rs_entries(H);
-    for (int i = i0; i < i1; i++) {
-        const float x = __ldg(im + (size_t)(H - 1 - i) * W);
-        t[i] = make_float2(run.hi, x);
-        run = df_add(run, DdF{x, 0.0f});
-    }
-    if (i0 < H && i1 == H) t[H] = make_float2(run.hi, 0.0f);
+// Planes of P slices of a stack of B images: the rows (lines of the views
+// that walk rows) and the columns from the bottom row up (dd2d_fwd.cuh).
+template <int P>
+__global__ void __launch_bounds__(256)
+k_planes(const float *__restrict__ img, int B, int H, int W, float *__restrict__ rows, float *__restrict__ cols,
+         size_t rplane, size_t cplane) {
+    __shared__ float t[32][33 * P];
+    const int q = blockIdx.z;
+    plane_tile<P>(img + (size_t)q * P * H * W, min(P, B - q * P), W, H, blockIdx.x * 32, blockIdx.y * 32,
+                  rows + q * rplane, cols + q * cplane, t);
 }
 
 // Detector tables for the adjoint: per (image, view) G_k and g_k over the
@@ -153,33 +116,25 @@ __global__ void k_dettab(int geom, int mode, const float *__restrict__ sino, int
     });
 }
 
-// Single-geometry forward launch: grid (views, image groups).
-// Shape of the single-geometry forward CTA: kFwdWarps warps over kFwdImages
-// slices.  The per-boundary locate in a line's drift record is shared by the
-// CTA's slices while the double-buffered line tables grow with them; on the
-// 16 x 512^2, 720-view workload 8 warps x 4 slices (4.62 ms) beat 8 x 8
-// (5.39 ms), 8 x 2 (6.02 ms) and 16 x 8 (5.27 ms).
-constexpr int kFwdImages = 4;
-constexpr int kFwdWarps = 8;
-
-// blockIdx.x = view * CL + rank in the view's cluster of CL CTAs.
-template <int GEOM, int WEIGHTED, int NPASS, int NW, int BI, int CL>
-__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NW * 32, (BI == 1 && NPASS <= 4) ? 8 : 0)
-k_fwd(dd_geom2d g, int op, int B, int V, int nl, const DdView2 *__restrict__ views,
-      const float *__restrict__ dp, const float *__restrict__ bcoef,
-      const DdLine *__restrict__ lines, const DdLine *__restrict__ dlines,
-      const float2 *__restrict__ tabx, const float2 *__restrict__ taby, float *__restrict__ out,
-      const float *__restrict__ sub, int *__restrict__ status) {
+// Single-geometry forward: one item per cluster.  blockIdx.x = view * cluster
+// size + rank, blockIdx.y = group of NB slices.  3 CTAs per SM (56 registers)
+// up to 24 sums a thread.
+template <int KIND, int NPASS, int NB>
+__global__ void __launch_bounds__(fwd_threads(NB), NPASS * NB <= 24 ? 3 : 2)
+k_fwd(dd_geom2d g, int geom, int op, int B, int V, int nl, const DdView2 *__restrict__ views,
+      const float *__restrict__ dp, const float *__restrict__ bcoef, const DdLine *__restrict__ lines,
+      const DdLine *__restrict__ dlines, const float *__restrict__ rows, const float *__restrict__ cols,
+      size_t rplane, size_t cplane, float *__restrict__ out, const float *__restrict__ sub, int cl,
+      int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const int rsmax = rs_entries(g.width > g.height ? g.width : g.height);
-    const FwdSmem L = fwd_smem(GEOM, g.num_det, rsmax, BI, CL, NW);
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L.bar);
-    init_bars(bar);
-    DdPhases ph;
+    __shared__ FwdState S;
+    const FwdLay L = fwd_lay(KIND == kPara, g.num_det, max(g.width, g.height), NB, cl);
+    fwd_init<NB>(smem, L, S);
+    constexpr int planes = NB / plane_slices(NB);
     FwdItem it;
-    it.v = blockIdx.x / CL;
-    it.b0 = blockIdx.y * BI;
-    it.nb = min(BI, B - it.b0);
+    it.v = blockIdx.x / cl;
+    it.b0 = blockIdx.y * NB;
+    it.nb = min(NB, B - it.b0);
     it.V = V;
     it.nl = nl;
     it.views = views;
@@ -187,13 +142,14 @@ k_fwd(dd_geom2d g, int op, int B, int V, int nl, const DdView2 *__restrict__ vie
     it.bcoef = bcoef;
     it.lines = lines;
     it.dlines = dlines;
-    it.tabx = tabx;
-    it.taby = taby;
+    it.rows = rows + (size_t)blockIdx.y * planes * rplane;
+    it.cols = cols + (size_t)blockIdx.y * planes * cplane;
+    it.rplane = rplane;
+    it.cplane = cplane;
     it.out = out;
     it.sub = sub;
-    if (!fwd_view<GEOM, WEIGHTED, NPASS, BI, NW, CL>(g, op, it, smem, g.num_det, rsmax, ph) &&
-        threadIdx.x == 0)
-        dd_report_timeout(status);
+    uint32_t step = 0, nr = 0;
+    if (!fwd_item<KIND, NPASS, NB>(g, geom, op, it, smem, L, S, step, nr) && threadIdx.x == 0) dd_report_timeout(status);
 }
 
 // Parallel beam (plan time): the views that walk image rows and those that
@@ -580,61 +536,122 @@ int max_smem_optin() {
     return n;
 }
 
-template <int GEOM, int BI, int CL>
-static auto fwd_kernel(bool w, int D) {
-    constexpr int NW = kFwdWarps;
-    auto kern = k_fwd<GEOM, 0, 8, NW, BI, CL>;
-    switch (npass_class(D, NW)) {
-    case 1: kern = w ? k_fwd<GEOM, 1, 1, NW, BI, CL> : k_fwd<GEOM, 0, 1, NW, BI, CL>; break;
-    case 2: kern = w ? k_fwd<GEOM, 1, 2, NW, BI, CL> : k_fwd<GEOM, 0, 2, NW, BI, CL>; break;
-    case 3: kern = w ? k_fwd<GEOM, 1, 3, NW, BI, CL> : k_fwd<GEOM, 0, 3, NW, BI, CL>; break;
-    case 4: kern = w ? k_fwd<GEOM, 1, 4, NW, BI, CL> : k_fwd<GEOM, 0, 4, NW, BI, CL>; break;
-    default: kern = w ? k_fwd<GEOM, 1, 8, NW, BI, CL> : k_fwd<GEOM, 0, 8, NW, BI, CL>; break;
-    }
-    return kern;
-}
-
 // The forward CTA shape a tune asks for (slices per CTA, CTAs per view's
-// cluster), with the defaults where it asks for none, and 1 slice where the
-// line tables of 4 would not fit in shared memory (lines of more than about
-// 3,400 pixels).  One slice per CTA keeps a CTA's tables and accumulators
-// small (32 registers, 8 CTAs per SM): single-slice calls ran 5-7 % faster
-// than with 2 slices per CTA (512^2, 720 views: 0.740 vs 0.789 ms).
+// cluster), with the defaults where it asks for none, and 1 slice where lines
+// are too long for 4.
 static void fwd_shape(int geom, const dd_geom2d *g, const dd_tune2d *tune, int *bi, int *cl) {
-    const int rsmax = rs_entries(g->width > g->height ? g->width : g->height);
-    *bi = (tune && (tune->fwd_slices == 1 || tune->fwd_slices == 4)) ? tune->fwd_slices : kFwdImages;
-    *cl = (tune && (tune->fwd_cluster == 1 || tune->fwd_cluster == 2)) ? tune->fwd_cluster : kFwdCluster;
-    if (*bi == 4 && fwd_smem(geom, g->num_det, rsmax, 4, *cl, kFwdWarps).total > max_smem_optin()) *bi = 1;
+    *bi = (tune && (tune->fwd_slices == 1 || tune->fwd_slices == 4)) ? tune->fwd_slices : 4;
+    *cl = (tune && (tune->fwd_cluster == 1 || tune->fwd_cluster == 2)) ? tune->fwd_cluster : 2;
+    if (*bi == 4 && four_slice_bytes(geom == DD_GEOM_PARA, g->num_det, std::max(g->width, g->height), *cl) > max_smem_optin())
+        *bi = 1;
 }
 
-template <int GEOM>
-static int launch_fwd(int op, const dd_geom2d *g, const PlanLayout &P, const char *planb, int B,
-                      int V, const float2 *tx, const float2 *ty, float *out, const float *sub,
-                      int *status, cudaStream_t st, const dd_tune2d *tune) {
-    const int rsmax = rs_entries(g->width > g->height ? g->width : g->height);
-    const bool w = (op == DD_OP_BPROJ_TW);
-    constexpr int NW = kFwdWarps;
-    int bi, cl;
-    fwd_shape(GEOM, g, tune, &bi, &cl);
-    const FwdSmem S = fwd_smem(GEOM, g->num_det, rsmax, bi, cl, NW);
-    if (S.total > max_smem_optin()) return DD_ERR_SIZE_OVERFLOW;
-    if ((long long)V * cl > 0x7FFFFFFFLL) return DD_ERR_SIZE_OVERFLOW;
-    dim3 grid(V * cl, (B + bi - 1) / bi);
-    const DdView2 *views = (const DdView2 *)(planb + P.views);
-    const float *dp = (const float *)(planb + P.dp);
-    const float *bc = (const float *)(planb + P.bcoef);
-    const DdLine *lines = (const DdLine *)(planb + P.lines);
-    const DdLine *dlines = GEOM == DD_GEOM_PARA ? (const DdLine *)(planb + P.dlines) : nullptr;
-    auto kern = (bi == 4) ? (cl == 2 ? fwd_kernel<GEOM, 4, 2>(w, g->num_det) : fwd_kernel<GEOM, 4, 1>(w, g->num_det))
-                          : (cl == 2 ? fwd_kernel<GEOM, 1, 2>(w, g->num_det) : fwd_kernel<GEOM, 1, 1>(w, g->num_det));
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
+struct FwdCall {
+    const dd_geom2d *g;
+    int geom, op, V, nl, cl;
+    const DdView2 *views;
+    const float *dp, *bcoef;
+    const DdLine *lines, *dlines;
+    const float *sub;
+    int *status;
+    cudaStream_t st;
+};
+
+// `n` slices in groups of NB: their planes, and the groups' items.
+template <int KIND, int NPASS, int NB>
+static int launch_fwd_group(const FwdCall &c, const float *in, int n, float *rows, float *cols, float *out,
+                            const float *sub) {
+    constexpr int P = plane_slices(NB);
+    const int W = c.g->width, H = c.g->height, groups = (n + NB - 1) / NB;
+    const size_t rplane = plane_bytes(H, W, P) / sizeof(float), cplane = plane_bytes(W, H, P) / sizeof(float);
+    const int planes = groups * (NB / P);
+    if (planes > 65535) return DD_ERR_SIZE_OVERFLOW;
+    ProfRec *pt = prof_begin(DD_KERNEL_TABLES, c.st);
+    k_planes<P><<<dim3((unsigned)((W + 31) / 32), (unsigned)((H + 31) / 32), (unsigned)planes), 256, 0, c.st>>>(
+        in, n, H, W, rows, cols, rplane, cplane);
+    prof_end(pt, c.st);
+    const FwdLay L = fwd_lay(KIND == kPara, c.g->num_det, std::max(W, H), NB, c.cl);
+    auto kern = k_fwd<KIND, NPASS, NB>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total) != cudaSuccess)
         return DD_ERR_LAUNCH;
-    ProfRec *pr = prof_begin(DD_KERNEL_FORWARD, st);
-    kern<<<grid, NW * 32, S.total, st>>>(*g, op, B, V, P.nl, views, dp, bc, lines, dlines, tx, ty,
-                                         out, sub, status);
-    prof_end(pr, st);
-    g_launches++;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)c.cl;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(c.V * c.cl), (unsigned)groups);
+    cfg.blockDim = dim3(fwd_threads(NB));
+    cfg.dynamicSmemBytes = (size_t)L.total;
+    cfg.stream = c.st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    ProfRec *pr = prof_begin(DD_KERNEL_FORWARD, c.st);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, *c.g, c.geom, c.op, n, c.V, c.nl, c.views, c.dp, c.bcoef, c.lines,
+                                             c.dlines, (const float *)rows, (const float *)cols, rplane, cplane, out, sub,
+                                             c.cl, c.status);
+    prof_end(pr, c.st);
+    g_launches += 2;
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return DD_ERR_LAUNCH;
+    }
     return launch_status();
+}
+
+template <int KIND, int NB>
+static int launch_fwd_passes(const FwdCall &c, const float *in, int n, float *rows, float *cols, float *out,
+                             const float *sub) {
+    switch (pass_class(c.g->num_det)) {
+    case 1: return launch_fwd_group<KIND, 1, NB>(c, in, n, rows, cols, out, sub);
+    case 2: return launch_fwd_group<KIND, 2, NB>(c, in, n, rows, cols, out, sub);
+    case 3: return launch_fwd_group<KIND, 3, NB>(c, in, n, rows, cols, out, sub);
+    case 4: return launch_fwd_group<KIND, 4, NB>(c, in, n, rows, cols, out, sub);
+    default: return launch_fwd_group<KIND, 8, (NB > 4 ? 4 : NB)>(c, in, n, rows, cols, out, sub);   // never 8 slices
+    }
+}
+
+// Slices per CTA: 8 share a line's overlaps best; groups of 8, then 4 (of
+// which one may be empty), 2 or 1 for the rest.  5 to 7 left over take one
+// group of 8: about the time of two smaller ones.  No 8 where the stages of
+// three lines would leave room for one CTA per SM only (lines of more than
+// about 1,000 pixels) or the detector needs 8 passes (the sums' registers).
+template <int KIND>
+static int launch_fwd(const FwdCall &c, bool single, int B, const float *in, char *rows, char *cols, float *out) {
+    const int W = c.g->width, H = c.g->height, D = c.g->num_det, npix = std::max(W, H);
+    if ((long long)c.V * c.cl > 0x7FFFFFFFLL) return DD_ERR_SIZE_OVERFLOW;
+    const size_t image = (size_t)W * H, sino = (size_t)c.V * D;
+    int big = 1;
+    if (!single) {
+        const int limit = max_smem_optin();
+        big = pass_class(D) <= 4 && fwd_lay(KIND == kPara, D, npix, 8, c.cl).total <= limit / 2 ? 8
+              : fwd_lay(KIND == kPara, D, npix, 4, c.cl).total <= limit                         ? 4
+                                                                                                : 2;
+    }
+    int done = 0;
+    while (done < B) {
+        const int left = B - done;
+        int nb = big, n = left / big * big;   // whole groups of the largest kind first
+        if (n == 0) {
+            n = left;
+            nb = left > 4 ? 8 : left > 2 ? 4 : left;
+        }
+        const float *sub = c.sub ? c.sub + done * sino : nullptr;
+        float *r = (float *)rows, *k = (float *)cols, *o = out + done * sino;
+        const float *x = in + done * image;
+        int st;
+        switch (nb) {
+        case 8: st = launch_fwd_passes<KIND, 8>(c, x, n, r, k, o, sub); break;
+        case 4: st = launch_fwd_passes<KIND, 4>(c, x, n, r, k, o, sub); break;
+        case 2: st = launch_fwd_passes<KIND, 2>(c, x, n, r, k, o, sub); break;
+        default: st = launch_fwd_passes<KIND, 1>(c, x, n, r, k, o, sub); break;
+        }
+        if (st != DD_OK) return st;
+        const int p = plane_slices(nb), planes = (n + nb - 1) / nb * (nb / p);
+        rows += planes * plane_bytes(H, W, p);
+        cols += planes * plane_bytes(W, H, p);
+        done += n;
+    }
+    return DD_OK;
 }
 
 template <int GEOM>
@@ -686,18 +703,6 @@ static int launch_adj_para(int op, const dd_geom2d *g, const PlanLayout &P, cons
     return launch_status();
 }
 
-int launch_image_tables(const dd_geom2d *g, const float *in, int B, float2 *tx, float2 *ty,
-                        cudaStream_t st) {
-    const int W = g->width, H = g->height;
-    const int nw = B * H;
-    ProfRec *pr = prof_begin(DD_KERNEL_TABLES, st);
-    k_tab_rows<<<(nw * 32 + 255) / 256, 256, 0, st>>>(in, B, H, W, tx);
-    k_tab_cols<<<B * ((W + 31) / 32), 32 * kColChunks, 0, st>>>(in, B, H, W, ty);
-    prof_end(pr, st);
-    g_launches += 2;
-    return launch_status();
-}
-
 int launch_det_tables(int geom, int op, const dd_geom2d *g, const char *planb, const float *in, int B,
                       int V, float2 *dtab, cudaStream_t st) {
     const PlanLayout P = plan_layout(geom == DD_GEOM_PARA ? DD_SCAN_PARA : DD_SCAN_FLAT, g, V);
@@ -728,13 +733,26 @@ int apply_planned(int scan, int op, const dd_geom2d *g, const void *planp, const
     int *status = (int *)(wb + A.status);
     const int geom = geom_of(scan);
     if (op_is_forward(op)) {
-        float2 *tx = (float2 *)(wb + A.tabx), *ty = (float2 *)(wb + A.taby);
-        const int ts = launch_image_tables(g, in, B, tx, ty, st);
-        if (ts != DD_OK) return ts;
         if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
-        if (geom == DD_GEOM_PARA) return launch_fwd<DD_GEOM_PARA>(op, g, P, planb, B, V, tx, ty, out, sub, status, st, tune);
-        if (geom == DD_GEOM_FLAT) return launch_fwd<DD_GEOM_FLAT>(op, g, P, planb, B, V, tx, ty, out, sub, status, st, tune);
-        return launch_fwd<DD_GEOM_ARC>(op, g, P, planb, B, V, tx, ty, out, sub, status, st, tune);
+        FwdCall c;
+        c.g = g;
+        c.geom = geom;
+        c.op = op;
+        c.V = V;
+        c.nl = P.nl;
+        int bi;
+        fwd_shape(geom, g, tune, &bi, &c.cl);
+        c.views = (const DdView2 *)(planb + P.views);
+        c.dp = (const float *)(planb + P.dp);
+        c.bcoef = (const float *)(planb + P.bcoef);
+        c.lines = (const DdLine *)(planb + P.lines);
+        c.dlines = geom == DD_GEOM_PARA ? (const DdLine *)(planb + P.dlines) : nullptr;
+        c.sub = sub;
+        c.status = status;
+        c.st = st;
+        if (geom == DD_GEOM_PARA) return launch_fwd<kPara>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
+        if (op != DD_OP_PROJ) return launch_fwd<kFanScaled>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
+        return launch_fwd<kFan>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
     }
     float2 *dtab = (float2 *)(wb + A.dtab);
     const int ts = launch_det_tables(geom, op, g, planb, in, B, V, dtab, st);
@@ -927,7 +945,7 @@ extern "C" const char *dd_status_string(int status) {
     }
 }
 
-extern "C" const char *dd_version(void) { return "pridediff_dd 0.2 sm_103a"; }
+extern "C" const char *dd_version(void) { return "pridediff_dd 0.3 sm_103a"; }
 
 extern "C" unsigned long long dd_launch_count(void) { return g_launches; }
 

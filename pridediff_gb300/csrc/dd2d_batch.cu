@@ -22,17 +22,17 @@
 #include <algorithm>
 #include <vector>
 
-#include "dd2d_kernels.cuh"
+#include "dd2d_fwd.cuh"
 #include "dd_trace.h"
 
 namespace dd2 {
 
 struct BatchInst {
     dd_geom2d g;
-    int V, batch, nl, pad;
+    int V, batch, nl, ps;          // ps: slices per forward item (1, 2 or 4)
     long long plan_off;            // bytes: instance plan inside the batch plan
     long long img_off, sino_off;   // elements: packed images / sinograms
-    long long tabx_off, taby_off;  // float2: forward tables in the workspace
+    long long row_off, col_off;    // bytes: planes of rows / columns in the workspace
     long long dtab_off;            // float2: adjoint tables in the workspace
     long long views, ang, dp, bcoef, lines, dlines, amap, trange;   // PlanLayout offsets
 };
@@ -40,31 +40,34 @@ struct BatchInst {
 struct BatchLayout {
     size_t desc, fitems, aitems, plans, total;        // plan buffer
     size_t w_tabs, w_dtab, w_resid, w_counter, w_status, w_total;   // workspace
-    int nfwd, nadj, Dmax, rsmax;
-    int fi;   // slices per forward item (fwd_item_slices)
+    int nfwd, nadj, Dmax, nmax;   // items; largest detector and longest line
+    int fi;   // largest instance's slices per forward item
     std::vector<BatchInst> inst;
 };
 
-// Slices per persistent forward item: 2 where no instance has more than 2
-// slices (after instances with one geometry are merged, the usual uneven
-// batch), so that the forward kernel holds half the line tables and runs 6
-// CTAs per SM instead of 5 (24 uneven instances: 6.51 -> 6.16 ms); kBI
-// otherwise, where 4 slices share each locate.
-static int fwd_item_slices(const dd_instance2d *in, int n) {
-    int mb = 0;
-    for (int i = 0; i < n; i++) mb = std::max(mb, in[i].batch);
-    return mb <= 2 ? 2 : kBI;
+// Most slices per persistent forward item: 4, or fewer where lines of
+// thousands of pixels would not leave room for them.
+static int fwd_item_limit(int scan, const dd_instance2d *in, int n) {
+    int D = 1, npix = 1;
+    for (int i = 0; i < n; i++) {
+        D = std::max(D, in[i].geom.num_det);
+        npix = std::max(npix, std::max(in[i].geom.width, in[i].geom.height));
+    }
+    int fi = kBI;
+    while (fi > 1 && fwd_lay(scan == DD_SCAN_PARA, D, npix, fi, 1).total > max_smem_optin()) fi /= 2;
+    return fi;
 }
 
 static BatchLayout batch_layout(int scan, const dd_instance2d *in, int n, int bi) {
     BatchLayout L;
     L.inst.resize(n);
-    L.fi = fwd_item_slices(in, n);
+    const int limit = fwd_item_limit(scan, in, n);
+    L.fi = 1;
     long long img = 0, sino = 0, tabs = 0, dtab = 0;
     size_t plans = 0;
     L.nfwd = L.nadj = 0;
     L.Dmax = 1;
-    L.rsmax = 2;
+    L.nmax = 1;
     for (int i = 0; i < n; i++) {
         BatchInst &d = L.inst[i];
         memset(&d, 0, sizeof(d));
@@ -88,18 +91,20 @@ static BatchLayout batch_layout(int scan, const dd_instance2d *in, int n, int bi
         img += (long long)d.batch * H * W;
         d.sino_off = sino;
         sino += (long long)d.batch * d.V * D;
-        d.tabx_off = tabs;
-        tabs += (long long)d.batch * H * rs_entries(W);
-        d.taby_off = tabs;
-        tabs += (long long)d.batch * W * rs_entries(H);
-        tabs = (tabs + 1) & ~1LL;
+        d.ps = std::min(limit, d.batch <= 2 ? d.batch : kBI);
+        L.fi = std::max(L.fi, d.ps);
+        const long long planes = (d.batch + d.ps - 1) / d.ps;
+        d.row_off = tabs;
+        tabs += planes * (long long)plane_bytes(H, W, d.ps);
+        d.col_off = tabs;
+        tabs += planes * (long long)plane_bytes(W, H, d.ps);
         d.dtab_off = dtab;
         dtab += ((long long)d.batch * d.V * rs_entries(D) + 1) & ~1LL;
         const int groups = (d.batch + bi - 1) / bi;
-        L.nfwd += d.V * ((d.batch + L.fi - 1) / L.fi);
+        L.nfwd += d.V * ((d.batch + d.ps - 1) / d.ps);
         L.nadj += ((W + kTile - 1) / kTile) * ((H + kTile - 1) / kTile) * groups;
         L.Dmax = std::max(L.Dmax, D);
-        L.rsmax = std::max(L.rsmax, rs_entries(std::max(W, H)));
+        L.nmax = std::max(L.nmax, std::max(W, H));
     }
     size_t o = 0;
     L.desc = o; o = align_up(o + sizeof(BatchInst) * (size_t)n, 256);
@@ -108,7 +113,7 @@ static BatchLayout batch_layout(int scan, const dd_instance2d *in, int n, int bi
     L.plans = o; o = align_up(o + plans, 256);
     L.total = o;
     size_t w = 0;
-    L.w_tabs = w; w = align_up(w + sizeof(float2) * (size_t)tabs, 256);
+    L.w_tabs = w; w = align_up(w + (size_t)tabs, 256);
     L.w_dtab = w; w = align_up(w + sizeof(float2) * (size_t)dtab, 256);
     L.w_resid = w; w = align_up(w + sizeof(float) * (size_t)sino, 256);
     L.w_counter = w; w = align_up(w + 2 * sizeof(int), 256);
@@ -118,53 +123,27 @@ static BatchLayout batch_layout(int scan, const dd_instance2d *in, int n, int bi
 }
 
 // ---------------------------------------------------------------------------
-// Batched prefix tables (one launch each; blockIdx.y = instance)
+// Batched planes of rows and columns (forward) and prefix tables (adjoint);
+// one launch each, blockIdx.y = instance
 // ---------------------------------------------------------------------------
-__global__ void k_tab_rows_b(const BatchInst *__restrict__ desc, const float *__restrict__ img,
-                             float2 *__restrict__ tabs) {
-    const BatchInst &d = desc[blockIdx.y];
-    const int W = d.g.width, H = d.g.height;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= d.batch * H) return;
-    const float *row = img + d.img_off + (size_t)warp * W;
-    warp_prefix_table(W, tabs + d.tabx_off + (size_t)warp * rs_entries(W), lane, [&](int j, float *x, float *w) {
-        *x = row[j];
-        *w = 1.0f;
-    });
+template <int P>
+__device__ __forceinline__ void planes_of(const BatchInst &d, int q, int tile, const float *img, char *tabs, float *t) {
+    const int W = d.g.width, H = d.g.height, ntx = (W + 31) / 32;
+    plane_tile<P>(img + d.img_off + (size_t)q * P * H * W, min(P, d.batch - q * P), W, H, tile % ntx * 32,
+                  tile / ntx * 32, reinterpret_cast<float *>(tabs + d.row_off + q * plane_bytes(H, W, P)),
+                  reinterpret_cast<float *>(tabs + d.col_off + q * plane_bytes(W, H, P)),
+                  reinterpret_cast<float (*)[33 * P]>(t));
 }
-
-// Column tables as the single-geometry k_tab_cols builds them: a block takes
-// 32 of an instance's (image, column) lines, its 8 warps a chunk of rows each.
-__global__ void __launch_bounds__(256) k_tab_cols_b(const BatchInst *__restrict__ desc,
-                                                    const float *__restrict__ img, float2 *__restrict__ tabs) {
-    constexpr int kChunks = 8;
+__global__ void __launch_bounds__(256)
+k_planes_b(const BatchInst *__restrict__ desc, const float *__restrict__ img, char *__restrict__ tabs) {
+    __shared__ float t[32 * 33 * 4];
     const BatchInst &d = desc[blockIdx.y];
-    const int W = d.g.width, H = d.g.height;
-    const int c = threadIdx.x & 31, k = threadIdx.x >> 5;
-    const int idx = blockIdx.x * 32 + c;
-    const bool ok = idx < d.batch * W;
-    const int b = ok ? idx / W : 0, col = ok ? idx - b * W : 0;
-    const int per = (H + kChunks - 1) / kChunks;
-    const int i0 = min(H, k * per), i1 = min(H, i0 + per);
-    const float *__restrict__ im = img + d.img_off + (size_t)b * H * W + col;
-    __shared__ float tot_hi[kChunks][32], tot_lo[kChunks][32];
-    DdF run = {0.0f, 0.0f};
-    if (ok)
-        for (int i = i0; i < i1; i++) run = df_add(run, DdF{__ldg(im + (size_t)(H - 1 - i) * W), 0.0f});
-    tot_hi[k][c] = run.hi;
-    tot_lo[k][c] = run.lo;
-    __syncthreads();
-    if (!ok) return;
-    run = {0.0f, 0.0f};
-    for (int q = 0; q < k; q++) run = df_add(run, DdF{tot_hi[q][c], tot_lo[q][c]});
-    float2 *__restrict__ t = tabs + d.taby_off + (size_t)idx * rs_entries(H);
-    for (int i = i0; i < i1; i++) {
-        const float x = __ldg(im + (size_t)(H - 1 - i) * W);
-        t[i] = make_float2(run.hi, x);
-        run = df_add(run, DdF{x, 0.0f});
-    }
-    if (i0 < H && i1 == H) t[H] = make_float2(run.hi, 0.0f);
+    const int nt = ((d.g.width + 31) / 32) * ((d.g.height + 31) / 32);
+    const int q = blockIdx.x / nt, tile = blockIdx.x - q * nt;
+    if (q * d.ps >= d.batch) return;
+    if (d.ps == 1) planes_of<1>(d, q, tile, img, tabs, t);
+    else if (d.ps == 2) planes_of<2>(d, q, tile, img, tabs, t);
+    else planes_of<4>(d, q, tile, img, tabs, t);
 }
 
 __global__ void k_dettab_b(int geom, int mode, const BatchInst *__restrict__ desc,
@@ -220,49 +199,45 @@ __device__ __forceinline__ int next_item_cluster(int *counter) {
     return i;
 }
 
-// Resident CTAs per SM the persistent forward is compiled for: items of 4
-// slices, 48 registers per thread up to 4 passes (on 24 uneven one-slice
-// instances 5 CTAs per SM ran the forward in 8.13 ms, 6 in 8.20 ms); items
-// of 2 slices, 40 registers and 6 CTAs.
-__host__ __device__ constexpr int fwd_items_min_ctas(int npass, int bi) {
-    return npass <= 4 ? (bi <= 2 ? 6 : 5) : 3;
-}
-
 // CTAs per persistent-forward cluster.  Batches of many short items leave
-// little tail to split: on 24 uneven one-slice instances, clusters of 2 (an
-// item's lines shared as in the single-geometry forward) took 9.00 ms, single
-// CTAs 8.20 ms.  A single CTA sums a view's lines in one sequence, the
-// single-geometry forward's cluster as two interleaved halves, so the two
-// projections of an instance agree to FP32 rounding, not bit for bit
-// (walking the lines in the cluster's order cost 8.73 vs 8.13 ms).
-// The cluster size is a tuning choice (dd_tune2d.items_cluster): 1 unless the
-// autotuner finds 2 faster for the batch at hand.
+// little tail to split, and a cluster's start-up costs more than it saves
+// (24 uneven one-slice instances: 9.00 ms with clusters of 2, 8.20 ms without,
+// of an earlier item body).  The cluster size is a tuning choice
+// (dd_tune2d.items_cluster): 1 unless the autotuner finds 2 faster for the
+// batch at hand; the result is the same bit for bit.
 constexpr int kFwdItemsCluster = 1;
 
-template <int GEOM, int NPASS, int CL, int BI>
-__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kThreads, fwd_items_min_ctas(NPASS, BI))
-k_fwd_items(int op, const BatchInst *__restrict__ desc, const int4 *__restrict__ items, int nitems,
-            const char *__restrict__ plan, size_t plans_off, const float2 *__restrict__ tabs,
-            float *__restrict__ out, const float *__restrict__ sub, int Dmax, int rsmax,
+// An item runs with as many slices side by side as its instance has (1, 2 or
+// 4): one-slice items in a 4-slice kernel took 6.97 instead of 5.9 ms on 24
+// uneven instances of 1 to 3 slices.
+static_assert(prods(1) == prods(4) && prods(2) == prods(4), "items of 1, 2 and 4 slices share a CTA's warps");
+template <int KIND, int NPASS>
+__global__ void __launch_bounds__(fwd_threads(4), NPASS <= 4 ? 3 : 2)
+k_fwd_items(int geom, int op, const BatchInst *__restrict__ desc, const int4 *__restrict__ items, int nitems,
+            const char *__restrict__ plan, size_t plans_off, const char *__restrict__ tabs,
+            float *__restrict__ out, const float *__restrict__ sub, int Dmax, int nmax, int fi, int cl,
             int *__restrict__ counter, int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const FwdSmem L = fwd_smem(GEOM, Dmax, rsmax, BI, CL);
-    init_bars(reinterpret_cast<uint64_t *>(smem + L.bar));
+    __shared__ FwdState S;
+    const FwdLay L = fwd_lay(KIND == kPara, Dmax, nmax, fi, cl);   // of the largest items
+    fwd_init<4>(smem, L, S);
     // the item and its geometry live in shared memory: read where used, they
     // hold no registers across the line loop (the plain forward reads them
     // from kernel parameters)
     __shared__ FwdItem s_it;
     __shared__ dd_geom2d s_g;
-    DdPhases ph;
+    __shared__ int s_ps;
+    uint32_t step = 0, nr = 0;
     for (;;) {
         int i;
-        if constexpr (CL > 1) i = next_item_cluster(counter);
+        if (cl > 1) i = next_item_cluster(counter);
         else i = next_item(counter);
         if (i >= nitems) break;
         if (threadIdx.x == 0) {
             const int4 w = items[i];
             const BatchInst &d = desc[w.x];
             const char *pb = plan + plans_off + d.plan_off;
+            const int W = d.g.width, H = d.g.height, q = w.z / d.ps;
             FwdItem it;
             it.v = w.y;
             it.b0 = w.z;
@@ -274,15 +249,20 @@ k_fwd_items(int op, const BatchInst *__restrict__ desc, const int4 *__restrict__
             it.bcoef = reinterpret_cast<const float *>(pb + d.bcoef);
             it.lines = reinterpret_cast<const DdLine *>(pb + d.lines);
             it.dlines = reinterpret_cast<const DdLine *>(pb + d.dlines);
-            it.tabx = tabs + d.tabx_off;
-            it.taby = tabs + d.taby_off;
+            it.rows = reinterpret_cast<const float *>(tabs + d.row_off + q * plane_bytes(H, W, d.ps));
+            it.cols = reinterpret_cast<const float *>(tabs + d.col_off + q * plane_bytes(W, H, d.ps));
+            it.rplane = it.cplane = 0;   // one plane per item
             it.out = out + d.sino_off;
             it.sub = sub ? sub + d.sino_off : nullptr;
             s_it = it;
             s_g = d.g;
+            s_ps = d.ps;
         }
-        __syncthreads();   // every thread passed the cluster barrier above before s_it changes
-        if (!fwd_view<GEOM, 0, NPASS, BI, kWarps, CL>(s_g, op, s_it, smem, Dmax, rsmax, ph)) {
+        __syncthreads();   // every thread passed the barrier above before s_it changes
+        const bool ok = s_ps == 1   ? fwd_item<KIND, NPASS, 1>(s_g, geom, op, s_it, smem, L, S, step, nr)
+                        : s_ps == 2 ? fwd_item<KIND, NPASS, 2>(s_g, geom, op, s_it, smem, L, S, step, nr)
+                                    : fwd_item<KIND, NPASS, 4>(s_g, geom, op, s_it, smem, L, S, step, nr);
+        if (!ok) {
             if (threadIdx.x == 0) dd_report_timeout(status);
             break;
         }
@@ -364,10 +344,10 @@ static int validate_batch(int scan, int op, const dd_instance2d *inst, int n) {
         const int st = validate(scan, op, &inst[i].geom, inst[i].batch, inst[i].num_view);
         if (st != DD_OK) return st;
         if ((inst[i].geom.width + kTile - 1) / kTile > 0xFFFF) return DD_ERR_SIZE_OVERFLOW;
-        // the persistent forward stages 4 images' line tables per CTA
+        // the longest lines the persistent forward takes
         const dd_geom2d &g = inst[i].geom;
-        if (fwd_smem(geom_of(scan), g.num_det, rs_entries(std::max(g.width, g.height)), kBI,
-                     kFwdItemsCluster).total > max_smem_optin())
+        if (four_slice_bytes(scan == DD_SCAN_PARA, g.num_det, std::max(g.width, g.height), kFwdItemsCluster) >
+            max_smem_optin())
             return DD_ERR_SIZE_OVERFLOW;
     }
     return DD_OK;
@@ -383,64 +363,76 @@ static int grid_of(const dd_tune2d *t, int nitems, int fit) {
 }
 
 template <typename K>
-static int resident_ctas(K kern, int smem) {
+static int resident_ctas(K kern, int smem, int threads) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kThreads, (size_t)smem) != cudaSuccess || n < 1) n = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, (size_t)smem) != cudaSuccess || n < 1) n = 1;
     return n;
 }
 
-// Persistent grid of a clustered kernel (clusters of `cl` CTAs): grid_of's CTA
-// count rounded down to whole clusters, at most the clusters that can be
-// resident at once.
-template <typename K>
-static int cluster_grid_of(const dd_tune2d *t, int nitems, K kern, int smem, int cl) {
-    const int ctas = grid_of(t, nitems * cl, resident_ctas(kern, smem));
-    int clusters = std::max(1, std::min(nitems, ctas / cl));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(clusters * cl);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    int maxc = 0;
-    if (cudaOccupancyMaxActiveClusters(&maxc, (void *)kern, &cfg) == cudaSuccess && maxc > 0)
-        clusters = std::min(clusters, maxc);
-    else
-        (void)cudaGetLastError();
-    return clusters * cl;
-}
-
-template <int GEOM, int CL, int BI>
-static auto fwd_items_kernel(int Dmax) {
-    auto kern = k_fwd_items<GEOM, 8, CL, BI>;
-    switch (npass_class(Dmax)) {
-    case 1: kern = k_fwd_items<GEOM, 1, CL, BI>; break;
-    case 2: kern = k_fwd_items<GEOM, 2, CL, BI>; break;
-    case 3: kern = k_fwd_items<GEOM, 3, CL, BI>; break;
-    case 4: kern = k_fwd_items<GEOM, 4, CL, BI>; break;
-    default: break;
-    }
-    return kern;
-}
-
-template <int GEOM>
-static int launch_fwd_items(int op, const BatchLayout &L, const char *planb, const float2 *tabs,
-                            float *out, const float *sub, int *counter, int *status, const dd_tune2d *tune,
-                            cudaStream_t st) {
+template <int KIND, int NPASS>
+static int launch_fwd_items_as(int geom, int op, const BatchLayout &L, const char *planb, char *tabs, float *out,
+                               const float *sub, int *counter, int *status, const dd_tune2d *tune, cudaStream_t st) {
     int cl = (tune && tune->items_cluster == 2) ? 2 : kFwdItemsCluster;
-    if (cl == 2 && fwd_smem(GEOM, L.Dmax, L.rsmax, L.fi, 2).total > max_smem_optin()) cl = 1;
-    const FwdSmem S = fwd_smem(GEOM, L.Dmax, L.rsmax, L.fi, cl);
-    auto kern = (L.fi == 2)
-        ? ((cl == 2) ? fwd_items_kernel<GEOM, 2, 2>(L.Dmax) : fwd_items_kernel<GEOM, 1, 2>(L.Dmax))
-        : ((cl == 2) ? fwd_items_kernel<GEOM, 2, kBI>(L.Dmax) : fwd_items_kernel<GEOM, 1, kBI>(L.Dmax));
+    if (cl == 2 && fwd_lay(KIND == kPara, L.Dmax, L.nmax, L.fi, 2).total > max_smem_optin()) cl = 1;
+    const FwdLay S = fwd_lay(KIND == kPara, L.Dmax, L.nmax, L.fi, cl);
+    auto kern = k_fwd_items<KIND, NPASS>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
         return DD_ERR_LAUNCH;
-    const int grid = cluster_grid_of(tune, L.nfwd, kern, S.total, cl);
+    // grid_of's CTA count rounded down to whole clusters, at most the clusters
+    // that can be resident at once
+    const int ctas = grid_of(tune, L.nfwd * cl, resident_ctas(kern, S.total, fwd_threads(4)));
+    int clusters = std::max(1, std::min(L.nfwd, ctas / cl));
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)cl;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(clusters * cl));
+    cfg.blockDim = dim3(fwd_threads(4));
+    cfg.dynamicSmemBytes = (size_t)S.total;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cl > 1) {
+        int maxc = 0;
+        if (cudaOccupancyMaxActiveClusters(&maxc, (void *)kern, &cfg) == cudaSuccess && maxc > 0)
+            clusters = std::min(clusters, maxc);
+        else
+            (void)cudaGetLastError();
+        cfg.gridDim = dim3((unsigned)(clusters * cl));
+    }
     ProfRec *pr = prof_begin(DD_KERNEL_FORWARD, st);
-    kern<<<grid, kThreads, S.total, st>>>(op, (const BatchInst *)(planb + L.desc),
-                                          (const int4 *)(planb + L.fitems), L.nfwd, planb, L.plans, tabs,
-                                          out, sub, L.Dmax, L.rsmax, counter, status);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, geom, op, (const BatchInst *)(planb + L.desc),
+                                             (const int4 *)(planb + L.fitems), L.nfwd, planb, L.plans, (const char *)tabs,
+                                             out, sub, L.Dmax, L.nmax, L.fi, cl, counter, status);
     prof_end(pr, st);
     count_launches(1);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return DD_ERR_LAUNCH;
+    }
     return launch_status();
+}
+
+template <int KIND>
+static int launch_fwd_items(int geom, int op, const BatchLayout &L, const char *planb, const float *in, char *tabs,
+                            float *out, const float *sub, int *counter, int *status, const dd_tune2d *tune,
+                            cudaStream_t st) {
+    int maxt = 1;
+    for (const BatchInst &d : L.inst)
+        maxt = std::max(maxt, ((d.batch + d.ps - 1) / d.ps) * ((d.g.width + 31) / 32) * ((d.g.height + 31) / 32));
+    ProfRec *pr = prof_begin(DD_KERNEL_TABLES, st);
+    k_planes_b<<<dim3((unsigned)maxt, (unsigned)L.inst.size()), 256, 0, st>>>((const BatchInst *)(planb + L.desc), in, tabs);
+    prof_end(pr, st);
+    count_launches(1);
+    if (cudaMemsetAsync(counter, 0, 2 * sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
+    switch (pass_class(L.Dmax)) {
+    case 1: return launch_fwd_items_as<KIND, 1>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+    case 2: return launch_fwd_items_as<KIND, 2>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+    case 3: return launch_fwd_items_as<KIND, 3>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+    case 4: return launch_fwd_items_as<KIND, 4>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+    default: return launch_fwd_items_as<KIND, 8>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+    }
 }
 
 template <int GEOM>
@@ -451,7 +443,7 @@ static int launch_adj_items(int op, const BatchLayout &L, const char *planb, con
     auto kern = (op == DD_OP_PROJ_T) ? k_adj_items<GEOM, 0> : k_adj_items<GEOM, 1>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
         return DD_ERR_LAUNCH;
-    const int grid = grid_of(tune, L.nadj, resident_ctas(kern, S.total));
+    const int grid = grid_of(tune, L.nadj, resident_ctas(kern, S.total, kThreads));
     ProfRec *pr = prof_begin(DD_KERNEL_ADJOINT, st);
     kern<<<grid, kThreads, S.total, st>>>((const BatchInst *)(planb + L.desc),
                                           (const int4 *)(planb + L.aitems), L.nadj, planb, L.plans, dtabs,
@@ -465,25 +457,12 @@ static int launch_adj_items(int op, const BatchLayout &L, const char *planb, con
 static int batch_forward(int scan, int op, const BatchLayout &L, const char *planb, const float *in,
                          float *out, const float *sub, char *wb, const dd_tune2d *tune, cudaStream_t st) {
     const int geom = geom_of(scan);
-    float2 *tabs = (float2 *)(wb + L.w_tabs);
+    char *tabs = wb + L.w_tabs;
     int *counter = (int *)(wb + L.w_counter);
     int *status = (int *)(wb + L.w_status);
-    const BatchInst *desc = (const BatchInst *)(planb + L.desc);
-    int maxrows = 1, maxcols = 1;
-    for (const BatchInst &d : L.inst) {
-        maxrows = std::max(maxrows, d.batch * d.g.height);
-        maxcols = std::max(maxcols, d.batch * d.g.width);
-    }
-    const int n = (int)L.inst.size();
-    ProfRec *pr = prof_begin(DD_KERNEL_TABLES, st);
-    k_tab_rows_b<<<dim3((maxrows * 32 + 255) / 256, n), 256, 0, st>>>(desc, in, tabs);
-    k_tab_cols_b<<<dim3((maxcols + 31) / 32, n), 256, 0, st>>>(desc, in, tabs);
-    prof_end(pr, st);
-    count_launches(2);
-    if (cudaMemsetAsync(counter, 0, 2 * sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
-    if (geom == DD_GEOM_PARA) return launch_fwd_items<DD_GEOM_PARA>(op, L, planb, tabs, out, sub, counter, status, tune, st);
-    if (geom == DD_GEOM_FLAT) return launch_fwd_items<DD_GEOM_FLAT>(op, L, planb, tabs, out, sub, counter, status, tune, st);
-    return launch_fwd_items<DD_GEOM_ARC>(op, L, planb, tabs, out, sub, counter, status, tune, st);
+    if (geom == DD_GEOM_PARA) return launch_fwd_items<kPara>(geom, op, L, planb, in, tabs, out, sub, counter, status, tune, st);
+    if (op != DD_OP_PROJ) return launch_fwd_items<kFanScaled>(geom, op, L, planb, in, tabs, out, sub, counter, status, tune, st);
+    return launch_fwd_items<kFan>(geom, op, L, planb, in, tabs, out, sub, counter, status, tune, st);
 }
 
 // adjoint of all instances: out = base + scale * (A^T in)   (base may be null)
@@ -546,8 +525,8 @@ extern "C" int dd2d_batch_plan(int scan, const dd_instance2d *inst, int n, const
     for (int i = 0; i < n; i++) {
         const BatchInst &d = L.inst[i];
         const int W = d.g.width, H = d.g.height, D = d.g.num_det;
-        for (int b0 = 0; b0 < d.batch; b0 += L.fi) {
-            const int nb = std::min(L.fi, d.batch - b0);
+        for (int b0 = 0; b0 < d.batch; b0 += d.ps) {
+            const int nb = std::min(d.ps, d.batch - b0);
             for (int v = 0; v < d.V; v++)
                 fw.push_back({make_int4(i, v, b0, nb), (long long)std::max(W, H) * (D + 1) * nb});
         }

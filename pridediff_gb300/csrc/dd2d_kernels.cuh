@@ -1,11 +1,13 @@
 // Shared device code of the 2-D DD projector: layouts, the integral-form
-// evaluation and the two work-item bodies (forward = detector gathers,
-// adjoint = pixel gathers).  Included by dd2d.cu (single-geometry launches)
-// and dd2d_batch.cu (persistent launches over uneven instances).
+// evaluation and the adjoint's work-item bodies (pixel gathers; the forward's
+// is in dd2d_fwd.cuh).  Included by dd2d.cu (single-geometry launches) and
+// dd2d_batch.cu (persistent launches over uneven instances).
 #pragma once
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include <cooperative_groups.h>
 
@@ -102,6 +104,7 @@ inline ApplyLayout apply_layout(int op, const dd_geom2d *g, int B, int V) {
     size_t o = 0;
     L.tabx = L.taby = L.dtab = 0;
     if (op_is_forward(op)) {
+        // the planes of rows and columns (8 bytes a pixel hold any grouping of the slices)
         L.tabx = o; o = align_up(o + sizeof(float2) * (size_t)B * g->height * rs_entries(g->width), 256);
         L.taby = o; o = align_up(o + sizeof(float2) * (size_t)B * g->width * rs_entries(g->height), 256);
     } else {
@@ -213,321 +216,18 @@ __device__ __forceinline__ float fan_fbp_weight(float sx, float sy, float px, fl
     return t * t;
 }
 
-struct Loc {
-    int p, j;
-    float dl, r;
-};
-
-__device__ __forceinline__ Loc locate(const DdLine &L, float u) {
-    Loc l;
-    float rr;
-    dd_locate(&L, u, &l.p, &l.j, &rr);
-    l.r = rr;
-    l.dl = L.p[l.p].dl;
-    return l;
-}
-
-// ---------------------------------------------------------------------------
-// Forward-type kernel (Proj, BackProjTrans, BackProjTransWeighted): detector
-// gathers.  CTA = (view, group of kBI images); loops over the view's walked
-// lines with the line record and the kBI line tables double-buffered in
-// shared memory by TMA bulk copies.
-// ---------------------------------------------------------------------------
-// Detector passes of a 256-thread CTA (8 warps x 31 bins each) rounded up to
-// the instantiated classes; NPASS sizes the per-thread accumulators, so a
-// smaller class means fewer registers and more resident CTAs per SM.
-__host__ __device__ inline int npass_class(int D, int nw = kWarps) {
-    const int n = (D + nw * kBinsPerWarp - 1) / (nw * kBinsPerWarp);
-    return n <= 1 ? 1 : n <= 2 ? 2 : n <= 3 ? 3 : n <= 4 ? 4 : 8;
-}
-
-struct FwdSmem {
-    // dynamic layout offsets (bytes)
-    int rec, drec, tab, kt, dp, bar, total;
-};
-
-// Forward CTAs per work item: a cluster of kFwdCluster CTAs shares a view's
-// lines (rank r walks lines r, r + kFwdCluster, ...), so items are shorter and
-// the last ones leave fewer SMs idle; rank 0 adds the others' sums through
-// distributed shared memory.
-constexpr int kFwdCluster = 2;
-
-// (BackProjTransWeighted uses the same layout: its weights live in registers.)
-// cl > 1: the line tables' space also holds a CTA's sums for the combine
-// (npass_class(D) passes x bi images x 32 lanes x nw warps floats).
-__host__ __device__ inline FwdSmem fwd_smem(int geom, int D, int rsmax, int bi = kBI, int cl = 1,
-                                            int nw = kWarps) {
-    FwdSmem s;
-    int o = 0;
-    s.rec = o; o += 2 * (int)sizeof(DdLine);
-    s.drec = o; if (geom == DD_GEOM_PARA) o += 2 * (int)sizeof(DdLine);
-    s.tab = o;
-    {
-        const int tabs = 2 * bi * rsmax * (int)sizeof(float2);
-        const int red = cl > 1 ? npass_class(D, nw) * bi * nw * 32 * (int)sizeof(float) : 0;
-        o += tabs > red ? tabs : red;
-    }
-    s.kt = o; o += bi * 32 * (int)sizeof(float);   // K of the pixel pieces
-    s.dp = o; o += ((D + 1 + 3) & ~3) * (int)sizeof(float);
-    s.bar = o; o += 2 * (int)sizeof(uint64_t);
-    s.total = (o + 127) & ~127;
-    return s;
-}
-
-// One forward work item: a view of one instance and a group of <= kBI of its
-// images.  Epilogue: out = beta * acc (sub == nullptr) or beta * acc - sub
-// (data-consistency residual A x - y, written without a separate pass).
-struct FwdItem {
-    int v, b0, nb, V, nl;
-    const DdView2 *views;
-    const float *dp, *bcoef;
-    const DdLine *lines, *dlines;
-    const float2 *tabx, *taby;   // prefix tables of image 0 of the instance
-    float *out;                  // sinogram of image 0 of the instance
-    const float *sub;            // optional, same layout as out
-};
-
-// Forward (detector-gather) evaluation of one work item.  The caller has
-// initialised bar[0..1]; `ph` tracks the barriers' phases so that a
-// persistent CTA can run many items back to back.  Returns false if a
-// bounded wait timed out (copies in flight have been drained).
-// CL > 1: the CTAs of a cluster of CL run the item together, rank r walking
-// lines r, r + CL, ...; every rank returns after the combine, and all of them
-// return false if any rank timed out.
-template <int GEOM, int WEIGHTED, int NPASS, int BI = kBI, int NW = kWarps, int CL = 1>
-__device__ bool fwd_view(const dd_geom2d &g, int op, const FwdItem &it, unsigned char *smem,
-                         int Dmax, int rsmax, DdPhases &ph) {
-    const int v = it.v, b0 = it.b0, nb = it.nb;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int rank = CL > 1 ? (int)cooperative_groups::this_cluster().block_rank() : 0;
-    const int D = g.num_det;
-    const DdView2 vw = it.views[v];
-    const int xb = vw.xb;
-    const int nline = xb ? g.height : g.width;
-    const int npix = xb ? g.width : g.height;
-    const int rs = rs_entries(npix);
-    const FwdSmem L = fwd_smem(GEOM, Dmax, rsmax, BI, CL, NW);
-    DdLine *rec = reinterpret_cast<DdLine *>(smem + L.rec);
-    DdLine *drec = reinterpret_cast<DdLine *>(smem + L.drec);
-    float2 *tab = reinterpret_cast<float2 *>(smem + L.tab);
-    float *kt = reinterpret_cast<float *>(smem + L.kt);
-    float *dps = reinterpret_cast<float *>(smem + L.dp);
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L.bar);
-    __shared__ int abort_flag;
-
-    const float2 *tsrc = xb ? it.tabx : it.taby;
-    const size_t img_stride = (size_t)nline * rs;          // float2 per image
-    const uint32_t tab_bytes = (uint32_t)(rs * sizeof(float2));
-    const uint32_t rec_bytes = (uint32_t)sizeof(DdLine);
-    const uint32_t tx_bytes = nb * tab_bytes + rec_bytes + (GEOM == DD_GEOM_PARA ? rec_bytes : 0);
-
-    if (tid == 0) abort_flag = 0;
-    if (GEOM != DD_GEOM_PARA)
-        for (int k = tid; k <= D; k += (NW * 32)) dps[k] = it.dp[(size_t)v * (D + 1) + k];
-    __syncthreads();
-
-    auto issue = [&](int line, int buf) {
-        dd_mbar_expect_tx(&bar[buf], tx_bytes);
-        dd_bulk_g2s(rec + buf, it.lines + (size_t)v * it.nl + line, rec_bytes, &bar[buf]);
-        if (GEOM == DD_GEOM_PARA)
-            dd_bulk_g2s(drec + buf, it.dlines + (size_t)v * it.nl + line, rec_bytes, &bar[buf]);
-        for (int b = 0; b < nb; b++)
-            dd_bulk_g2s(tab + ((size_t)buf * BI + b) * rsmax,
-                        tsrc + (size_t)(b0 + b) * img_stride + (size_t)line * rs, tab_bytes, &bar[buf]);
-    };
-
-    const int npass = (D + NW * kBinsPerWarp - 1) / (NW * kBinsPerWarp);
-    constexpr int kMaxPass = NPASS;   // D <= NPASS * 248 detector bins
-    float acc[kMaxPass][BI];
-#pragma unroll
-    for (int m = 0; m < kMaxPass; m++)
-#pragma unroll
-        for (int b = 0; b < BI; b++) acc[m][b] = 0.0f;
-
-    const float para_beta = xb ? FDIV(g.pix_y, g.det_size) : FDIV(g.pix_x, g.det_size);
-    // fan beams: each pass's detector boundary is the same for all the lines
-    // of the view; read it once
-    float ud[kMaxPass];
-#pragma unroll
-    for (int m = 0; m < kMaxPass; m++)
-        ud[m] = (GEOM != DD_GEOM_PARA && m < npass) ? dps[min(m * (NW * kBinsPerWarp) + warp * kBinsPerWarp + lane, D)]
-                                                     : 0.0f;
-    // the last warp issues the copies: the first warps build the piece
-    // constants right after the barrier, on every line's critical path
-    const int issuer = (NW - 1) * 32;
-    if (tid == issuer && rank < nline) issue(rank, 0);
-    for (int line = rank, step = 0; line < nline; line += CL, step++) {
-        const int buf = step & 1;
-        if (!dd_mbar_wait(&bar[buf], ph.parity(buf))) abort_flag = 1;
-        ph.flip(buf);
-        // past this barrier every warp has finished line - 1, whose buffer
-        // takes the copies of line + 1
-        __syncthreads();
-        if (abort_flag) {
-            // this line's copies may still be in flight (the next line's are
-            // issued only after this wait): let them land before returning
-            if (tid == issuer) dd_mbar_drain(&bar[buf], ph.parity(buf) ^ 1u);
-            break;
-        }
-        if (tid == issuer && line + CL < nline) issue(line + CL, buf ^ 1);
-        const DdLine &R = rec[buf];
-        const int np = R.h.npiece;
-        if (WEIGHTED && np > 0) {
-            // BackProjTransWeighted: multiply every pixel by its FBP weight at
-            // this view (FanFlatDisCPU2d.cpp:693, FanArcDisCPU2d.cpp:703) and
-            // rebuild the line's prefix table in place: warp b scans image b
-            // in 128-pixel chunks (4 consecutive pixels per lane, weights in
-            // registers), then builds that image's piece constants below, so
-            // the rebuild needs no CTA barrier.
-            if (warp < nb) {
-                float2 *t = tab + ((size_t)buf * BI + warp) * rsmax;
-                const float lpos = xb
-                    ? pix_centre(0.5f * (float)g.height - (float)line - 0.5f, g.pix_y, g.pix_yshift)
-                    : pix_centre((float)line - 0.5f * (float)g.width + 0.5f, g.pix_x, g.pix_xshift);
-                const float pitch = xb ? g.pix_x : g.pix_y;
-                float carry = 0.0f;
-                // 128-pixel chunks, 4 consecutive pixels per lane (two 16-byte
-                // loads; rows are 16-byte aligned and rsmax is even)
-                for (int k0 = 0; k0 < npix; k0 += 128) {
-                    const int i0 = k0 + 4 * lane;
-                    float y[4];
-                    if (i0 + 3 < npix) {
-                        const float4 p01 = *reinterpret_cast<const float4 *>(t + i0);
-                        const float4 p23 = *reinterpret_cast<const float4 *>(t + i0 + 2);
-                        y[0] = p01.y; y[1] = p01.w; y[2] = p23.y; y[3] = p23.w;
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 4; e++) y[e] = (i0 + e < npix) ? t[i0 + e].y : 0.0f;
-                    }
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const float pc = pix_centre((float)(i0 + e) + 0.5f, pitch, vw.axis0);
-                        y[e] *= xb ? fan_fbp_weight<GEOM>(vw.srcx, vw.srcy, pc, lpos, g.iso_source)
-                                   : fan_fbp_weight<GEOM>(vw.srcx, vw.srcy, lpos, pc, g.iso_source);
-                    }
-                    const float r1 = y[0] + y[1], r2 = r1 + y[2], r3 = r2 + y[3];
-                    float inc = r3;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const float z = __shfl_up_sync(0xffffffffu, inc, o);
-                        if (lane >= o) inc += z;
-                    }
-                    float prev = __shfl_up_sync(0xffffffffu, inc, 1);
-                    if (lane == 0) prev = 0.0f;
-                    const float base = carry + prev;
-                    const float pre[4] = {base, base + y[0], base + r1, base + r2};
-                    if (i0 + 3 < npix) {
-                        *reinterpret_cast<float4 *>(t + i0) = make_float4(pre[0], y[0], pre[1], y[1]);
-                        *reinterpret_cast<float4 *>(t + i0 + 2) = make_float4(pre[2], y[2], pre[3], y[3]);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 4; e++)
-                            if (i0 + e < npix) t[i0 + e] = make_float2(pre[e], y[e]);
-                    }
-                    carry += __shfl_sync(0xffffffffu, inc, 31);
-                }
-                if (lane == 0) t[npix] = make_float2(carry, 0.0f);
-                __syncwarp();   // the piece constants read other lanes' entries
-            }
-        }
-        if (np > 0) {
-            const float2 *tb = tab + (size_t)buf * BI * rsmax;
-            // warp b: image b's piece constants (for BackProjTransWeighted the
-            // warp that rebuilt its table)
-            for (int b = warp; b < nb; b += NW) kt[b * 32 + lane] = piece_K(R, tb + (size_t)b * rsmax, lane);
-            __syncthreads();
-            const float scale = (op == DD_OP_PROJ) ? 1.0f : R.h.alpha;
-            const float bound0 = R.h.bound0, endv = R.h.endv;
-            const int idet0 = R.h.idet0;
-#pragma unroll
-            for (int m = 0; m < kMaxPass; m++) {
-                if (m >= npass) break;
-                const int kb = m * (NW * kBinsPerWarp) + warp * kBinsPerWarp + lane;
-                float u;
-                if (kb <= idet0) {
-                    u = bound0;   // lower boundary of bin idet0 is the walk start
-                } else if (GEOM == DD_GEOM_PARA) {
-                    const DdLine &Rd = drec[buf];
-                    const int idx = min(kb - 1, D - 1);
-                    const float est = Rd.p[0].Q + (float)(idx - Rd.p[0].gb) * Rd.p[0].dl;
-                    u = (Rd.h.npiece > 0) ? dd_boundary(&Rd, idx, est) : bound0;
-                } else {
-                    u = ud[m];
-                }
-                u = fminf(fmaxf(u, bound0), endv);
-                // 32 boundaries clamped to the same end of the walk give 31
-                // zero differences: the warp skips the bins this line misses
-                if (__all_sync(0xffffffffu, u == bound0) || __all_sync(0xffffffffu, u == endv)) continue;
-                const Loc lc = locate(R, u);
-#pragma unroll
-                for (int b = 0; b < BI; b++) {
-                    if (b < nb) {
-                        const float2 e = tb[(size_t)b * rsmax + lc.j];
-                        const float f = fmaf(lc.r, e.y, fmaf(lc.dl, e.x, kt[b * 32 + lc.p]));
-                        const float fn = __shfl_down_sync(0xffffffffu, f, 1);
-                        if (lane < kBinsPerWarp) acc[m][b] = fmaf(scale, fn - f, acc[m][b]);
-                    }
-                }
-            }
-        }
-    }
-    // no copy is left in flight here: the next line's copies are issued only
-    // after its predecessor's wait succeeded, and an abort drained its line's
-    __syncthreads();   // the next item's first copies reuse the buffers
-    if constexpr (CL > 1) {
-        // ranks > 0 leave their sums in the (idle) line-table space; rank 0
-        // adds them in rank order, so the result does not depend on timing
-        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-        float *red = reinterpret_cast<float *>(smem + L.tab);
-        if (rank != 0 && !abort_flag) {
-#pragma unroll
-            for (int m = 0; m < kMaxPass; m++) {
-                if (m >= npass) break;
-#pragma unroll
-                for (int b = 0; b < BI; b++) red[(m * BI + b) * (NW * 32) + tid] = acc[m][b];
-            }
-        }
-        cluster.sync();
-        int ab = 0;
-        for (int r = 0; r < CL; r++) ab |= *cluster.map_shared_rank(&abort_flag, r);
-        if (rank == 0 && !ab) {
-            for (int r = 1; r < CL; r++) {
-                const float *rr = cluster.map_shared_rank(red, r);
-#pragma unroll
-                for (int m = 0; m < kMaxPass; m++) {
-                    if (m >= npass) break;
-#pragma unroll
-                    for (int b = 0; b < BI; b++) acc[m][b] += rr[(m * BI + b) * (NW * 32) + tid];
-                }
-            }
-        }
-        cluster.sync();   // no rank leaves (or reuses its buffers) before rank 0 has read them
-        if (ab) return false;
-        if (rank != 0) return true;
-    } else {
-        if (abort_flag) return false;
-    }
-#pragma unroll
-    for (int m = 0; m < kMaxPass; m++) {
-        if (m >= npass) break;
-        const int k = m * (NW * kBinsPerWarp) + warp * kBinsPerWarp + lane;
-        if (lane < kBinsPerWarp && k < D) {
-            float beta = 1.0f;
-            if (op == DD_OP_PROJ) beta = (GEOM == DD_GEOM_PARA) ? para_beta : it.bcoef[(size_t)v * (D + 1) + k];
-            const int ko = vw.flip ? D - 1 - k : k;
-#pragma unroll
-            for (int b = 0; b < BI; b++) {   // static indices keep acc in registers
-                if (b >= nb) break;
-                const size_t o = ((size_t)(b0 + b) * it.V + v) * D + ko;
-                // rounded product, then rounded difference: bit-equal to a
-                // separate projection followed by a subtraction (no FMA)
-                float val = __fmul_rn(acc[m][b], beta);
-                if (it.sub) val = __fsub_rn(val, it.sub[o]);
-                it.out[o] = val;
-            }
-        }
-    }
-    return true;
+// The longest lines of which 4 slices run in one CTA: what a prefix-table
+// forward with two buffers takes, at 8 warps of 31 bins.  (The limit of the
+// uneven batch's instances and of dd2d_fwd_shape's 4 slices.)
+inline long long four_slice_bytes(bool para, int D, int npix, int cl) {
+    const int n = (D + kWarps * kBinsPerWarp - 1) / (kWarps * kBinsPerWarp);
+    const int npass = n <= 1 ? 1 : n <= 2 ? 2 : n <= 3 ? 3 : n <= 4 ? 4 : 8;
+    const long long tabs = 2LL * kBI * rs_entries(npix) * (long long)sizeof(float2);
+    const long long red = cl > 1 ? (long long)npass * kBI * kThreads * (long long)sizeof(float) : 0;
+    const long long o = (para ? 4LL : 2LL) * (long long)sizeof(DdLine) + std::max(tabs, red) +
+                        kBI * 32 * (long long)sizeof(float) + ((D + 1 + 3) & ~3) * (long long)sizeof(float) +
+                        2 * (long long)sizeof(uint64_t);
+    return (o + 127) / 128 * 128;
 }
 
 __device__ __forceinline__ void init_bars(uint64_t *bar, int n = 2) {
@@ -1181,8 +881,7 @@ int validate(int scan, int op, const dd_geom2d *g, int B, int V);
 int geom_of(int scan);
 int launch_status();
 int max_smem_optin();   // largest dynamic shared memory per CTA (opt-in) on this device
-// prefix tables of B images (forward) / B sinograms (adjoint) of one geometry
-int launch_image_tables(const dd_geom2d *g, const float *in, int B, float2 *tx, float2 *ty, cudaStream_t st);
+// prefix tables of B sinograms of one geometry (adjoint)
 int launch_det_tables(int geom, int op, const dd_geom2d *g, const char *planb, const float *in, int B,
                       int V, float2 *dtab, cudaStream_t st);
 
