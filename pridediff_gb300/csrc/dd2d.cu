@@ -152,8 +152,8 @@ k_fwd(dd_geom2d g, int geom, int op, int B, int V, int nl, const DdView2 *__rest
     if (!fwd_item<KIND, NPASS, NB>(g, geom, op, it, smem, L, S, step, nr) && threadIdx.x == 0) dd_report_timeout(status);
 }
 
-// Parallel beam (plan time): the views that walk image rows and those that
-// walk columns, each in view order.  One warp: ballots rank the views.
+// Plan time: the views that walk image rows and those that walk columns, each
+// in view order.  One warp: ballots rank the views.
 __global__ void __launch_bounds__(32)
 k_axis_views(int V, const DdView2 *__restrict__ views, int *__restrict__ axisv) {
     const int lane = threadIdx.x;
@@ -377,46 +377,36 @@ k_trange(dd_geom2d g, int V, const DdView2 *__restrict__ views, const float *__r
     trange[i] = make_int2(kb, kn | (views[v].xb ? 1 << 16 : 0));   // the view's axis in bit 16
 }
 
-// Single-geometry adjoint launch: grid (tiles x * image groups, tiles y).
-// Fan beams: 4 CTAs per SM (64 registers), as the persistent adjoint.
-template <int GEOM, int OPK>
-__global__ void __launch_bounds__(kThreads, GEOM == DD_GEOM_PARA ? 1 : 4)
-k_adj(dd_geom2d g, int B, int V, int nl, const float *__restrict__ angles,
-      const DdView2 *__restrict__ views, const float *__restrict__ dp,
-      const DdLine *__restrict__ lines, const DdLine *__restrict__ dlines, const unsigned char *__restrict__ amap,
-      const int2 *__restrict__ trange, const float2 *__restrict__ dtab,
-      float *__restrict__ out,
-      const float *__restrict__ base, float scale, int *__restrict__ status) {
+// Single-geometry fan-beam adjoint launch: grid (tiles x * image groups *
+// cluster, tiles y); 4 CTAs per SM (64 registers), as the persistent adjoint.
+template <int GEOM, int OPK, int NB>
+__global__ void __cluster_dims__(kAdjCluster, 1, 1) __launch_bounds__(kThreads, 4)
+k_adj(dd_geom2d g, int B, int V, const DdView2 *__restrict__ views, const unsigned char *__restrict__ amap,
+      const int2 *__restrict__ trange, const int *__restrict__ axisv, const float2 *__restrict__ dtab,
+      float *__restrict__ out, const float *__restrict__ base, float scale, int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
     const AdjSmem SL = adj_smem(GEOM);
-    init_bars(reinterpret_cast<uint64_t *>(smem + SL.bar), GEOM == DD_GEOM_PARA ? 2 : kAdjBufs);
+    init_bars(reinterpret_cast<uint64_t *>(smem + SL.bar), kAdjBufs);
     DdPhases ph;
-    AdjItem it;
+    AdjItem it = {};
     // the image groups of a tile are adjacent in launch order: they run at the
     // same time, walk the views in step and read each view's map block of the
     // tile once from DRAM between them (the others hit L2)
-    const int ngroups = (B + kBI - 1) / kBI;
-    it.c0 = (blockIdx.x / ngroups) * kTile;
+    const int ngroups = (B + NB - 1) / NB, at = blockIdx.x / kAdjCluster;
+    it.c0 = (at / ngroups) * kTile;
     it.r0 = blockIdx.y * kTile;
-    it.b0 = (blockIdx.x % ngroups) * kBI;
-    it.nb = min(kBI, B - it.b0);
+    it.b0 = (at % ngroups) * NB;
+    it.nb = min(NB, B - it.b0);
     it.V = V;
-    it.nl = nl;
-    it.angles = angles;
     it.views = views;
-    it.dp = dp;
-    it.lines = lines;
-    it.dlines = dlines;
     it.amap = amap;
     it.trange = trange;
+    it.axisv = axisv;
     it.dtab = dtab;
     it.out = out;
     it.base = base;
     it.scale = scale;
-    bool ok;
-    if constexpr (GEOM == DD_GEOM_PARA) ok = adj_tile<GEOM, OPK>(g, it, smem, ph);
-    else ok = adj_tile_map<GEOM, OPK>(g, it, smem, ph);
-    if (!ok && threadIdx.x == 0) dd_report_timeout(status);
+    if (!adj_tile_map<GEOM, OPK, NB>(g, it, smem, ph) && threadIdx.x == 0) dd_report_timeout(status);
 }
 
 // ---------------------------------------------------------------------------
@@ -497,7 +487,7 @@ int plan(int scan, const dd_geom2d *g, const float *angles, int V, void *planp, 
     DdLine *dlines = scan == DD_SCAN_PARA ? (DdLine *)(base + P.dlines) : nullptr;
     ProfRec *pr = prof_begin(DD_KERNEL_PLAN, st);
     k_views<<<V, 256, 0, st>>>(geom, *g, angles, V, views, (float *)(base + P.ang), dp, bc);
-    if (geom == DD_GEOM_PARA) {
+    if (geom == DD_GEOM_PARA || with_map) {
         k_axis_views<<<1, 32, 0, st>>>(V, views, (int *)(base + P.axisv));
         g_launches++;
     }
@@ -654,28 +644,37 @@ static int launch_fwd(const FwdCall &c, bool single, int B, const float *in, cha
     return DD_OK;
 }
 
-template <int GEOM>
-static int launch_adj(int op, const dd_geom2d *g, const PlanLayout &P, const char *planb,
-                      const float *angles, int B, int V, const float2 *dtab, float *out,
-                      const float *base, float scale, int *status, cudaStream_t st) {
-    const unsigned ngroups = (unsigned)((B + kBI - 1) / kBI);
-    dim3 grid((unsigned)((g->width + kTile - 1) / kTile) * ngroups, (g->height + kTile - 1) / kTile);
-    const DdView2 *views = (const DdView2 *)(planb + P.views);
-    const float *dp = (const float *)(planb + P.dp);
-    const DdLine *lines = (const DdLine *)(planb + P.lines);
-    const DdLine *dlines = GEOM == DD_GEOM_PARA ? (const DdLine *)(planb + P.dlines) : nullptr;
-    const unsigned char *amap = GEOM == DD_GEOM_PARA ? nullptr : (const unsigned char *)(planb + P.amap);
-    const int2 *trange = GEOM == DD_GEOM_PARA ? nullptr : (const int2 *)(planb + P.trange);
+template <int GEOM, int OPK, int NB>
+static int launch_adj_as(const dd_geom2d *g, const PlanLayout &P, const char *planb, int B, int V, const float2 *dtab,
+                         float *out, const float *base, float scale, int *status, cudaStream_t st) {
+    const unsigned ngroups = (unsigned)((B + NB - 1) / NB);
+    const dim3 grid((unsigned)((g->width + kTile - 1) / kTile) * ngroups * kAdjCluster, (g->height + kTile - 1) / kTile);
     const AdjSmem S = adj_smem(GEOM);
-    auto kern = (op == DD_OP_PROJ_T) ? k_adj<GEOM, 0> : (op == DD_OP_BPROJ) ? k_adj<GEOM, 1> : k_adj<GEOM, 2>;
+    auto kern = k_adj<GEOM, OPK, NB>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
         return DD_ERR_LAUNCH;
     ProfRec *pr = prof_begin(DD_KERNEL_ADJOINT, st);
-    kern<<<grid, kThreads, S.total, st>>>(*g, B, V, P.nl, angles, views, dp, lines, dlines, amap, trange,
-                                          dtab, out, base, scale, status);
+    kern<<<grid, kThreads, S.total, st>>>(*g, B, V, (const DdView2 *)(planb + P.views),
+                                          (const unsigned char *)(planb + P.amap), (const int2 *)(planb + P.trange),
+                                          (const int *)(planb + P.axisv), dtab, out, base, scale, status);
     prof_end(pr, st);
     g_launches++;
     return launch_status();
+}
+
+template <int GEOM, int OPK>
+static int launch_adj_op(const dd_geom2d *g, const PlanLayout &P, const char *planb, int B, int V, const float2 *dtab,
+                         float *out, const float *base, float scale, int *status, cudaStream_t st) {
+    if (B == 1) return launch_adj_as<GEOM, OPK, 1>(g, P, planb, B, V, dtab, out, base, scale, status, st);
+    return launch_adj_as<GEOM, OPK, kBI>(g, P, planb, B, V, dtab, out, base, scale, status, st);
+}
+
+template <int GEOM>
+static int launch_adj(int op, const dd_geom2d *g, const PlanLayout &P, const char *planb, int B, int V,
+                      const float2 *dtab, float *out, const float *base, float scale, int *status, cudaStream_t st) {
+    if (op == DD_OP_PROJ_T) return launch_adj_op<GEOM, 0>(g, P, planb, B, V, dtab, out, base, scale, status, st);
+    if (op == DD_OP_BPROJ) return launch_adj_op<GEOM, 1>(g, P, planb, B, V, dtab, out, base, scale, status, st);
+    return launch_adj_op<GEOM, 2>(g, P, planb, B, V, dtab, out, base, scale, status, st);
 }
 
 // Parallel-beam adjoint: the rows' launch writes, the columns' launch adds.
@@ -724,7 +723,6 @@ int apply_planned(int scan, int op, const dd_geom2d *g, const void *planp, const
                   const float *sub = nullptr, const float *base = nullptr, float scale = 1.0f,
                   const dd_tune2d *tune = nullptr) {
     const PlanLayout P = plan_layout(scan, g, V);
-    const float *angles = (const float *)((const char *)planp + P.ang);
     const ApplyLayout A = apply_layout(op, g, B, V);
     if (!ws || wsb < A.total) return DD_ERR_WORKSPACE;
     if (!in || !out || !planp) return DD_ERR_INVALID_ARG;
@@ -759,8 +757,8 @@ int apply_planned(int scan, int op, const dd_geom2d *g, const void *planp, const
     if (ts != DD_OK) return ts;
     if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
     if (geom == DD_GEOM_PARA) return launch_adj_para(op, g, P, planb, B, V, dtab, out, base, scale, status, st);
-    if (geom == DD_GEOM_FLAT) return launch_adj<DD_GEOM_FLAT>(op, g, P, planb, angles, B, V, dtab, out, base, scale, status, st);
-    return launch_adj<DD_GEOM_ARC>(op, g, P, planb, angles, B, V, dtab, out, base, scale, status, st);
+    if (geom == DD_GEOM_FLAT) return launch_adj<DD_GEOM_FLAT>(op, g, P, planb, B, V, dtab, out, base, scale, status, st);
+    return launch_adj<DD_GEOM_ARC>(op, g, P, planb, B, V, dtab, out, base, scale, status, st);
 }
 
 }  // namespace dd2

@@ -34,7 +34,7 @@ struct BatchInst {
     long long img_off, sino_off;   // elements: packed images / sinograms
     long long row_off, col_off;    // bytes: planes of rows / columns in the workspace
     long long dtab_off;            // float2: adjoint tables in the workspace
-    long long views, ang, dp, bcoef, lines, dlines, amap, trange;   // PlanLayout offsets
+    long long views, ang, dp, bcoef, lines, dlines, amap, trange, axisv;   // PlanLayout offsets
 };
 
 struct BatchLayout {
@@ -86,6 +86,7 @@ static BatchLayout batch_layout(int scan, const dd_instance2d *in, int n, int bi
         d.dlines = (long long)P.dlines;
         d.amap = (long long)P.amap;
         d.trange = (long long)P.trange;
+        d.axisv = (long long)P.axisv;
         const int W = d.g.width, H = d.g.height, D = d.g.num_det;
         d.img_off = img;
         img += (long long)d.batch * H * W;
@@ -269,18 +270,42 @@ k_fwd_items(int geom, int op, const BatchInst *__restrict__ desc, const int4 *__
     }
 }
 
-// Fan beams: held to the plain adjoint's 4 CTAs per SM (64 registers per
-// thread); parallel beams (two sets of accumulators): 3.  The item and its
-// geometry live in shared memory, as in the forward.
-template <int GEOM, int OPK>
-__global__ void __launch_bounds__(kThreads, GEOM == DD_GEOM_PARA ? 3 : 4)
-k_adj_items(const BatchInst *__restrict__ desc, const int4 *__restrict__ items, int nitems,
-            const char *__restrict__ plan, size_t plans_off, const float2 *__restrict__ dtabs,
-            float *__restrict__ out, const float *__restrict__ base, float scale,
-            int *__restrict__ counter, int *__restrict__ status) {
+// Adjoint items of parallel beams: persistent, 3 CTAs per SM (two sets of
+// accumulators).  The item and its geometry live in shared memory, as in the
+// forward.
+__device__ __forceinline__ AdjItem adj_item(const BatchInst &d, const int4 w, const char *pb, const float2 *dtabs,
+                                            float *out, const float *base, float scale) {
+    AdjItem it;
+    it.c0 = (w.y & 0xFFFF) * kTile;
+    it.r0 = (w.y >> 16) * kTile;
+    it.b0 = w.z;
+    it.nb = w.w;
+    it.V = d.V;
+    it.nl = d.nl;
+    it.angles = reinterpret_cast<const float *>(pb + d.ang);
+    it.views = reinterpret_cast<const DdView2 *>(pb + d.views);
+    it.dp = reinterpret_cast<const float *>(pb + d.dp);
+    it.lines = reinterpret_cast<const DdLine *>(pb + d.lines);
+    it.dlines = reinterpret_cast<const DdLine *>(pb + d.dlines);
+    it.amap = reinterpret_cast<const unsigned char *>(pb + d.amap);
+    it.trange = reinterpret_cast<const int2 *>(pb + d.trange);
+    it.axisv = reinterpret_cast<const int *>(pb + d.axisv);
+    it.dtab = dtabs + d.dtab_off;
+    it.out = out + d.img_off;
+    it.base = base ? base + d.img_off : nullptr;
+    it.scale = scale;
+    return it;
+}
+
+template <int OPK>
+__global__ void __launch_bounds__(kThreads, 3)
+k_adj_items_para(const BatchInst *__restrict__ desc, const int4 *__restrict__ items, int nitems,
+                 const char *__restrict__ plan, size_t plans_off, const float2 *__restrict__ dtabs,
+                 float *__restrict__ out, const float *__restrict__ base, float scale,
+                 int *__restrict__ counter, int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const AdjSmem SL = adj_smem(GEOM);
-    init_bars(reinterpret_cast<uint64_t *>(smem + SL.bar), GEOM == DD_GEOM_PARA ? 2 : kAdjBufs);
+    const AdjSmem SL = adj_smem(DD_GEOM_PARA);
+    init_bars(reinterpret_cast<uint64_t *>(smem + SL.bar), 2);
     __shared__ AdjItem s_it;
     __shared__ dd_geom2d s_g;
     DdPhases ph;
@@ -290,37 +315,44 @@ k_adj_items(const BatchInst *__restrict__ desc, const int4 *__restrict__ items, 
         if (threadIdx.x == 0) {
             const int4 w = items[i];
             const BatchInst &d = desc[w.x];
-            const char *pb = plan + plans_off + d.plan_off;
-            AdjItem it;
-            it.c0 = (w.y & 0xFFFF) * kTile;
-            it.r0 = (w.y >> 16) * kTile;
-            it.b0 = w.z;
-            it.nb = w.w;
-            it.V = d.V;
-            it.nl = d.nl;
-            it.angles = reinterpret_cast<const float *>(pb + d.ang);
-            it.views = reinterpret_cast<const DdView2 *>(pb + d.views);
-            it.dp = reinterpret_cast<const float *>(pb + d.dp);
-            it.lines = reinterpret_cast<const DdLine *>(pb + d.lines);
-            it.dlines = reinterpret_cast<const DdLine *>(pb + d.dlines);
-            it.amap = reinterpret_cast<const unsigned char *>(pb + d.amap);
-            it.trange = reinterpret_cast<const int2 *>(pb + d.trange);
-            it.dtab = dtabs + d.dtab_off;
-            it.out = out + d.img_off;
-            it.base = base ? base + d.img_off : nullptr;
-            it.scale = scale;
-            s_it = it;
+            s_it = adj_item(d, w, plan + plans_off + d.plan_off, dtabs, out, base, scale);
             s_g = d.g;
         }
         __syncthreads();
-        bool ok;
-        if constexpr (GEOM == DD_GEOM_PARA) ok = adj_tile<GEOM, OPK>(s_g, s_it, smem, ph);
-        else ok = adj_tile_map<GEOM, OPK>(s_g, s_it, smem, ph);
-        if (!ok) {
+        if (!adj_tile<DD_GEOM_PARA, OPK>(s_g, s_it, smem, ph)) {
             if (threadIdx.x == 0) dd_report_timeout(status);
             break;
         }
     }
+}
+
+// Adjoint items of fan beams: a cluster per item, in the list's order; 4 CTAs
+// per SM (64 registers), as the single-geometry adjoint.  Not persistent: the
+// clusters behind the resident ones start as these finish, and an item's
+// start (its view list, its first copies) then hides behind the SM's other
+// CTAs, where a persistent cluster goes through it between two cluster
+// barriers (24 uneven instances: 2.60 ms persistent, 2.41 ms so; the map's 14
+// GB take 2.06 ms at the copy rate).
+template <int GEOM, int OPK>
+__global__ void __cluster_dims__(kAdjCluster, 1, 1) __launch_bounds__(kThreads, 4)
+k_adj_items(const BatchInst *__restrict__ desc, const int4 *__restrict__ items, const char *__restrict__ plan,
+            size_t plans_off, const float2 *__restrict__ dtabs, float *__restrict__ out,
+            const float *__restrict__ base, float scale, int *__restrict__ status) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const AdjSmem SL = adj_smem(GEOM);
+    __shared__ AdjItem s_it;
+    __shared__ dd_geom2d s_g;
+    if (threadIdx.x == 0) {
+        const int4 w = items[blockIdx.x / kAdjCluster];
+        const BatchInst &d = desc[w.x];
+        s_it = adj_item(d, w, plan + plans_off + d.plan_off, dtabs, out, base, scale);
+        s_g = d.g;
+    }
+    init_bars(reinterpret_cast<uint64_t *>(smem + SL.bar), kAdjBufs);   // ends with a CTA barrier
+    DdPhases ph;
+    const bool ok = s_it.nb == 1 ? adj_tile_map<GEOM, OPK, 1>(s_g, s_it, smem, ph)
+                                 : adj_tile_map<GEOM, OPK, kBI>(s_g, s_it, smem, ph);
+    if (!ok && threadIdx.x == 0) dd_report_timeout(status);
 }
 
 // ---------------------------------------------------------------------------
@@ -440,14 +472,23 @@ static int launch_adj_items(int op, const BatchLayout &L, const char *planb, con
                             float *out, const float *base, float scale, int *counter, int *status,
                             const dd_tune2d *tune, cudaStream_t st) {
     const AdjSmem S = adj_smem(GEOM);
-    auto kern = (op == DD_OP_PROJ_T) ? k_adj_items<GEOM, 0> : k_adj_items<GEOM, 1>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
-        return DD_ERR_LAUNCH;
-    const int grid = grid_of(tune, L.nadj, resident_ctas(kern, S.total, kThreads));
+    const BatchInst *desc = (const BatchInst *)(planb + L.desc);
+    const int4 *items = (const int4 *)(planb + L.aitems);
     ProfRec *pr = prof_begin(DD_KERNEL_ADJOINT, st);
-    kern<<<grid, kThreads, S.total, st>>>((const BatchInst *)(planb + L.desc),
-                                          (const int4 *)(planb + L.aitems), L.nadj, planb, L.plans, dtabs,
-                                          out, base, scale, counter, status);
+    if constexpr (GEOM == DD_GEOM_PARA) {
+        auto kern = (op == DD_OP_PROJ_T) ? k_adj_items_para<0> : k_adj_items_para<1>;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
+            return DD_ERR_LAUNCH;
+        const int grid = grid_of(tune, L.nadj, resident_ctas(kern, S.total, kThreads));
+        kern<<<grid, kThreads, S.total, st>>>(desc, items, L.nadj, planb, L.plans, dtabs, out, base, scale, counter,
+                                              status);
+    } else {
+        auto kern = (op == DD_OP_PROJ_T) ? k_adj_items<GEOM, 0> : k_adj_items<GEOM, 1>;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
+            return DD_ERR_LAUNCH;
+        kern<<<(unsigned)L.nadj * kAdjCluster, kThreads, S.total, st>>>(desc, items, planb, L.plans, dtabs, out, base,
+                                                                       scale, status);
+    }
     prof_end(pr, st);
     count_launches(1);
     return launch_status();

@@ -78,14 +78,15 @@ inline PlanLayout plan_layout(int scan, const dd_geom2d *g, int V, bool with_map
     L.lines = o; o = align_up(o + sizeof(DdLine) * (size_t)V * L.nl, 256);
     L.dlines = o;
     if (scan == DD_SCAN_PARA) o = align_up(o + sizeof(DdLine) * (size_t)V * L.nl, 256);
-    // parallel beam: the views that walk rows and those that walk columns
-    // ({count rows, count columns, rows' views[V], columns' views[V]})
+    // the adjoint's view lists: those that walk rows and those that walk
+    // columns ({count rows, count columns, rows' views[V], columns' views[V]})
     L.axisv = o;
     if (scan == DD_SCAN_PARA) o = align_up(o + sizeof(int) * (2 * (size_t)V + 2), 256);
     L.amap = L.trange = o;
     if (scan != DD_SCAN_PARA && with_map) {
         L.amap = o; o = align_up(o + (size_t)kMapBlkBytes * V * tiles_n(g), 256);
         L.trange = o; o = align_up(o + sizeof(int2) * (size_t)V * tiles_n(g), 256);
+        L.axisv = o; o = align_up(o + sizeof(int) * (2 * (size_t)V + 2), 256);
     }
     L.total = o;
     return L;
@@ -377,6 +378,7 @@ struct AdjItem {
     const DdLine *lines, *dlines;
     const unsigned char *amap;   // fan beams: adjoint-map blocks (plan)
     const int2 *trange;          // fan beams, per (view, tile): {first staged bin, bins | xb << 16} (plan)
+    const int *axisv;            // view lists (plan)
     const float2 *dtab;          // detector tables of image 0 of the instance
     float *out;                  // image 0 of the instance
     const float *base;
@@ -627,25 +629,47 @@ __device__ bool adj_tile(const dd_geom2d &g, const AdjItem &it, unsigned char *s
 
 
 // ---------------------------------------------------------------------------
-// Fan-beam adjoint through the adjoint map.  For every view the CTA copies by
-// TMA, for its 32 walked lines, the map entries {bin, offset} of the tile's
-// pixel boundaries, the per-line scales and the slice of every image's
-// detector prefix table the tile can reach.  A thread owns fixed pixels (4
-// consecutive rows of one column: warp = row group, lane = column) for every
-// view, so one set of accumulators serves both projection axes: pixel value
-// += w (H(upper) - H(lower)), with H(u) = G_k + (u - d_k) g_k read at the two
-// staged boundary entries (for views that walk columns the 4 pixels share
-// boundaries: 5 values of H serve them).
+// Fan-beam adjoint through the adjoint map, one 32 x 32 tile by a cluster of
+// kAdjCluster CTAs.  Each CTA takes a part of the views that walk one axis and
+// sums them on its own; the ranks' sums meet in shared memory at the end and
+// are added in rank order, each rank writing a quarter of the tile.  So a
+// tile's views are not one serial chain of copies, waits and barriers, and
+// every view is walked along its own axis: a thread owns 4 consecutive pixels
+// of one line (lane = line, warp = group of 4), whose 5 boundaries serve the
+// 4 pixels.
+//
+// For every view the CTA copies by TMA the tile's map block -- the entries
+// {bin, offset} of its lines' pixel boundaries and the lines' scales -- and
+// the slice of every image's detector prefix table the tile can reach: pixel
+// value += w (H(upper) - H(lower)), H(u) = G_k + (u - d_k) g_k.
+//
+// Bound by the map's stream from HBM for one slice (1.78 GB at 5.8 TB/s, 86 %
+// of the copy rate) and by instruction issue (73 %) from 4 on.  512^2, 720
+// views, 736 bins, 1 / 2 / 4 / 16 slices, by one CTA per tile with the pixels
+// of views that walk rows on 4 lines a thread: 0.64 / 0.80 / 1.05 / 2.23 ms;
+// here 0.35 / 0.41 / 0.53 / 1.87 ms (tables included).
 // ---------------------------------------------------------------------------
-template <int GEOM, int OPK>   // OPK: 0 ProjTrans, 1 BackProj, 2 BackProjWeighted
+constexpr int kAdjCluster = 4;
+static_assert(kTile % kAdjCluster == 0 && kTile / kAdjCluster == kWarps, "a rank writes one row per warp");
+
+// Ranks that take the views walking rows (the others: columns), by their shares.
+__device__ __forceinline__ int row_ranks(int nr, int nc) {
+    if (nc == 0) return kAdjCluster;
+    if (nr == 0) return 0;
+    return min(max((int)((2ll * kAdjCluster * nr + nr + nc) / (2ll * (nr + nc))), 1), kAdjCluster - 1);
+}
+
+template <int GEOM, int OPK, int NB>   // OPK: 0 ProjTrans, 1 BackProj, 2 BackProjWeighted; NB: most images
 __device__ bool adj_tile_map(const dd_geom2d &g, const AdjItem &it, unsigned char *smem, DdPhases &ph) {
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int rank = (int)cluster.block_rank();
     const AdjSmem SL = adj_smem(GEOM);
     const int V = it.V;
     const int W = g.width, H = g.height, D = g.num_det;
     const int rsd = rs_entries(D);
     unsigned char *mapb = smem + SL.map;                           // [kAdjBufs] map blocks
     float2 *stage = reinterpret_cast<float2 *>(smem + SL.stage);   // [kAdjBufs][kBI][kStage]
-    int *krange = reinterpret_cast<int *>(smem + SL.krange);       // per buffer: first bin, bins, first entry
+    int *krange = reinterpret_cast<int *>(smem + SL.krange);       // per buffer: first bin, bins, first entry, view
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + SL.bar);
     __shared__ int abort_flag;
     const int c0 = it.c0, r0 = it.r0, b0 = it.b0, nb = it.nb;
@@ -654,219 +678,193 @@ __device__ bool adj_tile_map(const dd_geom2d &g, const AdjItem &it, unsigned cha
     if (tid == 0) abort_flag = 0;
     __syncthreads();
 
-    // What view v's copies move, from its staged range {first bin, bins | xb << 16}.
-    struct Cp {
-        int xb, elo, kb, kn;
-    };
+    // this rank's views: a part of one axis's list
+    const int nr = it.axisv[0], nc = it.axisv[1], rk = row_ranks(nr, nc);
+    const int xb = rank < rk;
+    const int part = xb ? rank : rank - rk, parts = xb ? rk : kAdjCluster - rk, na = xb ? nr : nc;
+    const int i0 = (int)((long long)na * part / parts), NV = (int)((long long)na * (part + 1) / parts) - i0;
+    const int *__restrict__ vlist = it.axisv + 2 + (xb ? 0 : V) + i0;
     const int tile = (r0 / kTile) * tiles_x(&g) + c0 / kTile, ntiles = tiles_n(&g);
-    auto desc = [&](int2 tr) {
-        Cp d;
-        d.xb = tr.y >> 16;
-        d.elo = map_first(&g, d.xb, c0, r0);
-        d.kb = tr.x;
-        d.kn = tr.y & 0xFFFF;
-        return d;
-    };
-    // thread 0 arms a buffer's barrier with the byte count of its next view,
-    // before any warp issues a copy into it
-    auto arm = [&](int buf, const Cp &d) {
-        dd_mbar_expect_tx(&bar[buf], (uint32_t)(kMapBlkBytes + nb * d.kn * (int)sizeof(float2)));
+    const int elo = map_first(&g, xb, c0, r0);
+
+    // thread 0 arms a buffer's barrier with the byte count of its next view
+    // ({first staged bin, bins | xb << 16}), before any warp issues a copy into it
+    auto arm = [&](int buf, int2 tr) {
+        dd_mbar_expect_tx(&bar[buf], (uint32_t)(kMapBlkBytes + nb * (tr.y & 0xFFFF) * (int)sizeof(float2)));
     };
     // View v's copies, one per warp: warp 0 moves the tile's map block, warp
     // b + 1 (b < nb) the detector-table slice of image b.
-    auto issue = [&](int v, int buf, const Cp &d) {
-        if (tid == 0) {
-            krange[4 * buf] = d.kb;
-            krange[4 * buf + 1] = d.kn;
-            krange[4 * buf + 2] = d.elo;
-            krange[4 * buf + 3] = d.xb;
-        }
+    auto issue = [&](int v, int buf, int2 tr) {
+        const int kn = tr.y & 0xFFFF;
+        if (tid == 0) reinterpret_cast<int4 *>(krange)[buf] = make_int4(tr.x, kn, v, 0);
         if (lane == 0) {
             if (warp == 0)
                 dd_bulk_g2s(mapb + (size_t)buf * kMapBlkBytes, it.amap + ((size_t)v * ntiles + tile) * kMapBlkBytes,
                             (uint32_t)kMapBlkBytes, &bar[buf]);
-            else if (warp <= nb && d.kn > 0)
+            else if (warp <= nb && kn > 0)
                 dd_bulk_g2s(stage + ((size_t)buf * kBI + warp - 1) * kStage,
-                            dtab + ((size_t)(b0 + warp - 1) * V + v) * rsd + d.kb, (uint32_t)(d.kn * sizeof(float2)),
+                            dtab + ((size_t)(b0 + warp - 1) * V + v) * rsd + tr.x, (uint32_t)(kn * sizeof(float2)),
                             &bar[buf]);
         }
     };
 
-    float acc[kLinesPerWarp][kBI];
+    float acc[kLinesPerWarp][NB];
 #pragma unroll
     for (int q = 0; q < kLinesPerWarp; q++)
 #pragma unroll
-        for (int b = 0; b < kBI; b++) acc[q][b] = 0.0f;
+        for (int b = 0; b < NB; b++) acc[q][b] = 0.0f;
 
+    // only the warps that issue a view's copies (warp 0: the map block, warps
+    // 1 .. nb: the detector slices) follow the list ahead
+    const bool issuing = warp <= nb;
+    int vn = 0;                        // view i + 2 of the list, its range, and view i + 3
+    int2 trn = make_int2(0, 0);
+    int vnn = 0;
     {
-        const Cp d0 = desc(it.trange[tile]);
-        const Cp d1 = desc(V > 1 ? it.trange[(size_t)ntiles + tile] : make_int2(0, 0));
+        const int va = NV > 0 ? vlist[0] : 0, vb = NV > 1 ? vlist[1] : 0;
+        const int2 ta = NV > 0 ? it.trange[(size_t)va * ntiles + tile] : make_int2(0, 0);
+        const int2 tb = NV > 1 ? it.trange[(size_t)vb * ntiles + tile] : make_int2(0, 0);
         if (tid == 0) {
-            arm(0, d0);
-            if (V > 1) arm(1, d1);
+            if (NV > 0) arm(0, ta);
+            if (NV > 1) arm(1, tb);
         }
         __syncthreads();
-        issue(0, 0, d0);
-        if (V > 1) issue(1, 1, d1);
-    }
-    // only the warps that issue a view's copies (warp 0: the map block, warps
-    // 1 .. nb: the detector slices) need its descriptor
-    const bool issuing = warp <= nb;
-    int2 tr_next = (V > 2 && issuing) ? it.trange[(size_t)2 * ntiles + tile] : make_int2(0, 0);   // view v + 2
-    int vstop = V;   // first view not waited for (the copies of vstop may be in flight)
-    int buf = 0, buf2 = 2 % kAdjBufs;   // buffers of views v and v + 2
-    for (int v = 0; v < V; v++, buf = (buf + 1 == kAdjBufs) ? 0 : buf + 1,
-                                buf2 = (buf2 + 1 == kAdjBufs) ? 0 : buf2 + 1) {
-        const bool more = v + 2 < V;
-        Cp dn;
-        if (more && issuing) {
-            dn = desc(tr_next);
-            // the phase of view v - 1 on this barrier was waited for before the
-            // previous barrier, so it can be armed for view v + 2 now
-            if (tid == 0) arm(buf2, dn);
+        if (NV > 0) issue(va, 0, ta);
+        if (NV > 1) issue(vb, 1, tb);
+        if (issuing) {
+            if (NV > 2) {
+                vn = vlist[2];
+                trn = it.trange[(size_t)vn * ntiles + tile];
+            }
+            if (NV > 3) vnn = vlist[3];
         }
+    }
+    // this thread's 4 pixels: pixel q lies between entries E - q - 1 and E - q of its line
+    const int rq0 = r0 + kLinesPerWarp * warp;
+    const int E = xb ? kLinesPerWarp * (warp + 1) : H - rq0 - elo;
+    const int nv = xb ? kLinesPerWarp : min(kLinesPerWarp, H - rq0);   // rows: absent pixels have no entries
+    int vstop = NV;   // first view of the list not waited for (its copies may be in flight)
+    int buf = 0, buf2 = 2 % kAdjBufs;   // buffers of views i and i + 2
+    for (int i = 0; i < NV; i++, buf = (buf + 1 == kAdjBufs) ? 0 : buf + 1,
+                                buf2 = (buf2 + 1 == kAdjBufs) ? 0 : buf2 + 1) {
+        // the phase of view i - 1 on this barrier was waited for before the
+        // previous barrier, so it can be armed for view i + 2 now
+        if (tid == 0 && i + 2 < NV) arm(buf2, trn);
         if (!dd_mbar_wait(&bar[buf], ph.parity(buf))) abort_flag = 1;
         ph.flip(buf);
-        // one barrier per view: past it every warp has finished view v - 1
+        // one barrier per view: past it every warp has finished view i - 1
         __syncthreads();
         if (abort_flag) {
-            // view v's copies (not waited for) may still be in flight
+            // view i's copies (not waited for) may still be in flight
             if (tid == 0) dd_mbar_drain(&bar[buf], ph.parity(buf) ^ 1u);
-            vstop = v + 1;
+            vstop = i + 1;
             break;
         }
-        // so the copies of view v + 2 go into the buffer of view v - 1
-        if (more && issuing) {
-            issue(v + 2, buf2, dn);
-            if (v + 3 < V) tr_next = it.trange[(size_t)(v + 3) * ntiles + tile];
+        // so the copies of view i + 2 go into the buffer of view i - 1
+        if (issuing && i + 2 < NV) {
+            issue(vn, buf2, trn);
+            if (i + 3 < NV) {
+                vn = vnn;
+                trn = it.trange[(size_t)vn * ntiles + tile];
+                if (i + 4 < NV) vnn = vlist[i + 4];
+            }
         }
         const int4 kr = reinterpret_cast<const int4 *>(krange)[buf];   // one 16-byte load
-        const int kb = kr.x, kn = kr.y, elo = kr.z, xb = kr.w;
+        const int kb = kr.x, kn = kr.y, v = kr.z;
         const int2 *mp = reinterpret_cast<const int2 *>(mapb + (size_t)buf * kMapBlkBytes);
         const float *alb = reinterpret_cast<const float *>(mp + kTile * kMapE);   // line scales
         const float2 *sb = stage + (size_t)buf * kBI * kStage;
-        DdView2 vw;   // BackProjWeighted: the view's source and first pixel edge
-        if (OPK == 2) vw = it.views[v];
-        // this thread's pixels: rows rq0 .. rq0 + 3 of column c
-        const int rq0 = r0 + kLinesPerWarp * warp, c = c0 + lane;
-        if (!xb) {
-            // views that walk columns: the thread's 4 pixels are consecutive
-            // on its line and pixel q's lower boundary is pixel q + 1's upper
-            // one, so 5 boundary values serve the 4 pixels (the same values:
-            // results are unchanged)
-            const int nv = (c < W) ? min(kLinesPerWarp, H - rq0) : 0;
-            if (nv > 0) {
-                const int lr = c - c0, E = H - rq0 - elo;   // pixel q: upper entry E - q, lower E - q - 1
-                int2 m[kLinesPerWarp + 1];
-                bool all_in = true;   // every used entry in the staged slice (the usual case)
+        if (nv > 0) {
+            int2 m[kLinesPerWarp + 1];
+            bool all_in = true;   // every used entry in the staged slice (the usual case)
 #pragma unroll
-                for (int i = 0; i <= kLinesPerWarp; i++) {
-                    m[i] = (i <= nv) ? mp[lr * kMapE + E - i] : make_int2(-1, 0);
-                    if (m[i].x >= 0 && (unsigned)(m[i].x - kb) >= (unsigned)kn) all_in = false;
-                }
-                float wq[kLinesPerWarp];
+            for (int e = 0; e <= kLinesPerWarp; e++) {
+                m[e] = (e <= nv) ? mp[lane * kMapE + E - e] : make_int2(-1, 0);
+                if (m[e].x >= 0 && (unsigned)(m[e].x - kb) >= (unsigned)kn) all_in = false;
+            }
+            float wq[kLinesPerWarp];
+            if (OPK == 2) {
+                const DdView2 *vw = it.views + v;   // the view's source and first pixel edge
+                const float sx = vw->srcx, sy = vw->srcy, ax = vw->axis0;
 #pragma unroll
                 for (int q = 0; q < kLinesPerWarp; q++) {
-                    float wgt = (OPK == 0) ? 1.0f : alb[lr];
-                    if (OPK == 2) {
-                        const float pcx = pix_centre((float)c - 0.5f * (float)W + 0.5f, g.pix_x, g.pix_xshift);
-                        const float pcy = pix_centre((float)(H - 1 - (rq0 + q)) + 0.5f, g.pix_y, vw.axis0);
-                        wgt = wgt * fan_fbp_weight<GEOM>(vw.srcx, vw.srcy, pcx, pcy, g.iso_source);
-                    }
-                    wq[q] = wgt;
+                    const float pi = (float)(xb ? c0 + kLinesPerWarp * warp + 3 - q : H - 1 - (rq0 + q)) + 0.5f;
+                    const float along = pix_centre(pi, xb ? g.pix_x : g.pix_y, ax);
+                    const float across = xb ? pix_centre(0.5f * (float)H - (float)(r0 + lane) - 0.5f, g.pix_y, g.pix_yshift)
+                                            : pix_centre((float)(c0 + lane) - 0.5f * (float)W + 0.5f, g.pix_x, g.pix_xshift);
+                    wq[q] = alb[lane] * fan_fbp_weight<GEOM>(sx, sy, xb ? along : across, xb ? across : along, g.iso_source);
                 }
+            } else {
 #pragma unroll
-                for (int b = 0; b < kBI; b++) {
-                    if (b >= nb) break;
-                    const float2 *t = dtab + ((size_t)(b0 + b) * V + v) * rsd;   // per image
-                    float h[kLinesPerWarp + 1];
-                    if (all_in) {
-#pragma unroll
-                        for (int i = 0; i <= kLinesPerWarp; i++) {
-                            const float2 e = sb[b * kStage + max(m[i].x - kb, 0)];
-                            h[i] = fmaf(__int_as_float(m[i].y), e.y, e.x);   // unused where m[i].x < 0
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i <= kLinesPerWarp; i++) {
-                            h[i] = 0.0f;
-                            if (m[i].x >= 0) {
-                                const bool in = (unsigned)(m[i].x - kb) < (unsigned)kn;
-                                const float2 e = in ? sb[b * kStage + (m[i].x - kb)] : __ldg(t + m[i].x);
-                                h[i] = fmaf(__int_as_float(m[i].y), e.y, e.x);
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int q = 0; q < kLinesPerWarp; q++)
-                        if (q < nv && m[q].x >= 0 && m[q + 1].x >= 0) acc[q][b] += wq[q] * (h[q] - h[q + 1]);
-                }
+                for (int q = 0; q < kLinesPerWarp; q++) wq[q] = (OPK == 0) ? 1.0f : alb[lane];
             }
-        } else {
 #pragma unroll
-            for (int q = 0; q < kLinesPerWarp; q++) {
-                const int r = rq0 + q;
-                if (r >= H || c >= W) continue;
-                const int lr = r - r0, eu = c + 1 - elo;   // line r, pixel c
-                const int2 up = mp[lr * kMapE + eu], low = mp[lr * kMapE + eu - 1];
-                if (up.x < 0 || low.x < 0) continue;
-                float wgt = (OPK == 0) ? 1.0f : alb[lr];
-                if (OPK == 2) {
-                    const float pcx = pix_centre((float)c + 0.5f, g.pix_x, vw.axis0);
-                    const float pcy = pix_centre(0.5f * (float)H - (float)r - 0.5f, g.pix_y, g.pix_yshift);
-                    wgt = wgt * fan_fbp_weight<GEOM>(vw.srcx, vw.srcy, pcx, pcy, g.iso_source);
-                }
-                const float offU = __int_as_float(up.y), offL = __int_as_float(low.y);
-                const bool inU = (unsigned)(up.x - kb) < (unsigned)kn;
-                const bool inL = (unsigned)(low.x - kb) < (unsigned)kn;
-                if (inU && inL) {   // both entries in the staged slice (the usual case)
-                    const float2 *su = sb + (up.x - kb), *sl = sb + (low.x - kb);
+            for (int b = 0; b < NB; b++) {
+                if (b >= nb) break;
+                float h[kLinesPerWarp + 1];
+                if (all_in) {
 #pragma unroll
-                    for (int b = 0; b < kBI; b++) {
-                        if (b >= nb) break;
-                        const float2 e = su[b * kStage], e2 = sl[b * kStage];
-                        const float hu = fmaf(offU, e.y, e.x);
-                        const float hl = fmaf(offL, e2.y, e2.x);
-                        acc[q][b] += wgt * (hu - hl);
+                    for (int e = 0; e <= kLinesPerWarp; e++) {
+                        const float2 t = sb[b * kStage + max(m[e].x - kb, 0)];
+                        h[e] = fmaf(__int_as_float(m[e].y), t.y, t.x);   // unused where m[e].x < 0
                     }
                 } else {
+                    const float2 *t = dtab + ((size_t)(b0 + b) * V + v) * rsd;   // per image
 #pragma unroll
-                    for (int b = 0; b < kBI; b++) {
-                        if (b >= nb) break;
-                        const float2 *t = dtab + ((size_t)(b0 + b) * V + v) * rsd;   // per image
-                        const float2 e = inU ? sb[b * kStage + (up.x - kb)] : __ldg(t + up.x);
-                        const float2 e2 = inL ? sb[b * kStage + (low.x - kb)] : __ldg(t + low.x);
-                        const float hu = fmaf(offU, e.y, e.x);
-                        const float hl = fmaf(offL, e2.y, e2.x);
-                        acc[q][b] += wgt * (hu - hl);
+                    for (int e = 0; e <= kLinesPerWarp; e++) {
+                        h[e] = 0.0f;
+                        if (m[e].x >= 0) {
+                            const bool in = (unsigned)(m[e].x - kb) < (unsigned)kn;
+                            const float2 x = in ? sb[b * kStage + (m[e].x - kb)] : __ldg(t + m[e].x);
+                            h[e] = fmaf(__int_as_float(m[e].y), x.y, x.x);
+                        }
                     }
                 }
+#pragma unroll
+                for (int q = 0; q < kLinesPerWarp; q++)
+                    if (q < nv && m[q].x >= 0 && m[q + 1].x >= 0) acc[q][b] += wq[q] * (h[q] - h[q + 1]);
             }
         }
     }
-    __syncthreads();   // the next item's first copies reuse the buffers
+    __syncthreads();   // the buffers are free: the last copies have been waited for ...
     if (abort_flag) {
-        // let the copies of view vstop (issued, not waited for) land
-        for (int u = vstop; u < V && u < vstop + 1; u++) {
-            const int b = u % kAdjBufs;
+        // ... or, after a timeout, are let land (those of view vstop, issued and not waited for)
+        if (vstop < NV) {
+            const int b = vstop % kAdjBufs;
             if (tid == 0) dd_mbar_drain(&bar[b], ph.parity(b));
             ph.flip(b);
         }
         __syncthreads();
-        return false;
     }
+    // the ranks' sums, added in rank order
+    float *sums = reinterpret_cast<float *>(mapb);   // [NB][kTile][kTile + 1]
 #pragma unroll
-    for (int q = 0; q < kLinesPerWarp; q++) {
-        const int r = r0 + kLinesPerWarp * warp + q, c = c0 + lane;
-        if (r >= H || c >= W) continue;
+    for (int b = 0; b < NB; b++)
 #pragma unroll
-        for (int b = 0; b < kBI; b++) {   // static indices keep acc in registers
-            if (b >= nb) break;
-            const size_t o = ((size_t)(b0 + b) * H + r) * W + c;
-            it.out[o] = it.base ? fmaf(it.scale, acc[q][b], it.base[o]) : acc[q][b];
+        for (int q = 0; q < kLinesPerWarp; q++) {
+            const int row = xb ? lane : kLinesPerWarp * warp + q, col = xb ? kLinesPerWarp * warp + 3 - q : lane;
+            sums[(b * kTile + row) * (kTile + 1) + col] = acc[q][b];
+        }
+    cluster.sync();
+    int ab = 0;
+    for (int k = 0; k < kAdjCluster; k++) ab |= *cluster.map_shared_rank(&abort_flag, k);
+    if (!ab) {
+        const int row = rank * kWarps + warp, r = r0 + row, c = c0 + lane;
+        if (r < H && c < W) {
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                if (b >= nb) break;
+                const int at = (b * kTile + row) * (kTile + 1) + lane;
+                float val = cluster.map_shared_rank(sums, 0)[at];
+#pragma unroll
+                for (int k = 1; k < kAdjCluster; k++) val += cluster.map_shared_rank(sums, k)[at];
+                const size_t o = ((size_t)(b0 + b) * H + r) * W + c;
+                it.out[o] = it.base ? fmaf(it.scale, val, it.base[o]) : val;
+            }
         }
     }
-    return true;
+    cluster.sync();   // no rank leaves (or reuses its buffers) before the others have read its sums
+    return !ab;
 }
 
 
