@@ -161,9 +161,18 @@ _forward_choice: Dict[str, dict] = {}   # in-process copy of the cache's choices
 _forward_about: Dict[str, dict] = {}    # what each key is
 
 
+_forward_keys: Dict[tuple, str] = {}    # keys by the values they are made of
+
+
 def forward2d_key(scan: int, geom_fields: tuple, batch: int, views: int, device) -> str:
-    return make_key(kind="forward2d", scan=scan, geom=list(geom_fields), batch=batch, views=views,
-                    **gpu_signature(device))
+    parts = (scan, geom_fields, batch, views, str(device))
+    key = _forward_keys.get(parts)
+    if key is None:
+        if len(_forward_keys) >= 1024:
+            _forward_keys.clear()
+        key = _forward_keys[parts] = make_key(kind="forward2d", scan=scan, geom=list(geom_fields), batch=batch,
+                                              views=views, **gpu_signature(device))
+    return key
 
 
 def tune_forward2d(key: str, run, reps: int = 3, path=None, about: Optional[dict] = None) -> dict:

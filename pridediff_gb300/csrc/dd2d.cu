@@ -80,8 +80,9 @@ __global__ void k_lines(int geom, dd_geom2d g, const float *__restrict__ angles,
 template <int P>
 __global__ void __launch_bounds__(256)
 k_planes(const float *__restrict__ img, int B, int H, int W, float *__restrict__ rows, float *__restrict__ cols,
-         size_t rplane, size_t cplane) {
+         size_t rplane, size_t cplane, int *__restrict__ clear) {
     __shared__ float t[32][33 * P];
+    if (clear && threadIdx.x == 0 && blockIdx.x + blockIdx.y + blockIdx.z == 0) *clear = 0;   // the call's status word
     const int q = blockIdx.z;
     plane_tile<P>(img + (size_t)q * P * H * W, min(P, B - q * P), W, H, blockIdx.x * 32, blockIdx.y * 32,
                   rows + q * rplane, cols + q * cplane, t);
@@ -94,9 +95,10 @@ k_planes(const float *__restrict__ img, int B, int H, int W, float *__restrict__
 __global__ void k_dettab(int geom, int mode, const float *__restrict__ sino, int B, int V, int D,
                          const DdView2 *__restrict__ views, const float *__restrict__ dp,
                          const float *__restrict__ bcoef, float para_coef_x, float para_coef_y,
-                         float2 *__restrict__ tab) {
+                         float2 *__restrict__ tab, int *__restrict__ clear) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
+    if (blockIdx.x + threadIdx.x == 0) *clear = 0;   // the call's status word
     if (warp >= B * V) return;
     const int b = warp / V, v = warp - b * V;
     const DdView2 vw = views[v];
@@ -544,6 +546,7 @@ struct FwdCall {
     const DdLine *lines, *dlines;
     const float *sub;
     int *status;
+    bool first;   // the call's first launch, which clears its status word
     cudaStream_t st;
 };
 
@@ -558,7 +561,7 @@ static int launch_fwd_group(const FwdCall &c, const float *in, int n, float *row
     if (planes > 65535) return DD_ERR_SIZE_OVERFLOW;
     ProfRec *pt = prof_begin(DD_KERNEL_TABLES, c.st);
     k_planes<P><<<dim3((unsigned)((W + 31) / 32), (unsigned)((H + 31) / 32), (unsigned)planes), 256, 0, c.st>>>(
-        in, n, H, W, rows, cols, rplane, cplane);
+        in, n, H, W, rows, cols, rplane, cplane, c.first ? c.status : nullptr);
     prof_end(pt, c.st);
     const FwdLay L = fwd_lay(KIND == kPara, c.g->num_det, std::max(W, H), NB, c.cl);
     auto kern = k_fwd<KIND, NPASS, NB>;
@@ -606,7 +609,7 @@ static int launch_fwd_passes(const FwdCall &c, const float *in, int n, float *ro
 // three lines would leave room for one CTA per SM only (lines of more than
 // about 1,000 pixels) or the detector needs 8 passes (the sums' registers).
 template <int KIND>
-static int launch_fwd(const FwdCall &c, bool single, int B, const float *in, char *rows, char *cols, float *out) {
+static int launch_fwd(FwdCall c, bool single, int B, const float *in, char *rows, char *cols, float *out) {
     const int W = c.g->width, H = c.g->height, D = c.g->num_det, npix = std::max(W, H);
     if ((long long)c.V * c.cl > 0x7FFFFFFFLL) return DD_ERR_SIZE_OVERFLOW;
     const size_t image = (size_t)W * H, sino = (size_t)c.V * D;
@@ -636,6 +639,7 @@ static int launch_fwd(const FwdCall &c, bool single, int B, const float *in, cha
         default: st = launch_fwd_passes<KIND, 1>(c, x, n, r, k, o, sub); break;
         }
         if (st != DD_OK) return st;
+        c.first = false;
         const int p = plane_slices(nb), planes = (n + nb - 1) / nb * (nb / p);
         rows += planes * plane_bytes(H, W, p);
         cols += planes * plane_bytes(W, H, p);
@@ -703,7 +707,7 @@ static int launch_adj_para(int op, const dd_geom2d *g, const PlanLayout &P, cons
 }
 
 int launch_det_tables(int geom, int op, const dd_geom2d *g, const char *planb, const float *in, int B,
-                      int V, float2 *dtab, cudaStream_t st) {
+                      int V, float2 *dtab, int *status, cudaStream_t st) {
     const PlanLayout P = plan_layout(geom == DD_GEOM_PARA ? DD_SCAN_PARA : DD_SCAN_FLAT, g, V);
     const int mode = (op == DD_OP_PROJ_T) ? 0 : 1;
     const float pcx = g->pix_y / g->det_size, pcy = g->pix_x / g->det_size;
@@ -712,7 +716,7 @@ int launch_det_tables(int geom, int op, const dd_geom2d *g, const char *planb, c
     k_dettab<<<(nw * 32 + 255) / 256, 256, 0, st>>>(geom, mode, in, B, V, g->num_det,
                                                      (const DdView2 *)(planb + P.views),
                                                      (const float *)(planb + P.dp),
-                                                     (const float *)(planb + P.bcoef), pcx, pcy, dtab);
+                                                     (const float *)(planb + P.bcoef), pcx, pcy, dtab, status);
     prof_end(pr, st);
     g_launches++;
     return launch_status();
@@ -731,8 +735,8 @@ int apply_planned(int scan, int op, const dd_geom2d *g, const void *planp, const
     int *status = (int *)(wb + A.status);
     const int geom = geom_of(scan);
     if (op_is_forward(op)) {
-        if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
         FwdCall c;
+        c.first = true;
         c.g = g;
         c.geom = geom;
         c.op = op;
@@ -753,9 +757,8 @@ int apply_planned(int scan, int op, const dd_geom2d *g, const void *planp, const
         return launch_fwd<kFan>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
     }
     float2 *dtab = (float2 *)(wb + A.dtab);
-    const int ts = launch_det_tables(geom, op, g, planb, in, B, V, dtab, st);
+    const int ts = launch_det_tables(geom, op, g, planb, in, B, V, dtab, status, st);
     if (ts != DD_OK) return ts;
-    if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
     if (geom == DD_GEOM_PARA) return launch_adj_para(op, g, P, planb, B, V, dtab, out, base, scale, status, st);
     if (geom == DD_GEOM_FLAT) return launch_adj<DD_GEOM_FLAT>(op, g, P, planb, B, V, dtab, out, base, scale, status, st);
     return launch_adj<DD_GEOM_ARC>(op, g, P, planb, B, V, dtab, out, base, scale, status, st);

@@ -881,6 +881,6 @@ int launch_status();
 int max_smem_optin();   // largest dynamic shared memory per CTA (opt-in) on this device
 // prefix tables of B sinograms of one geometry (adjoint)
 int launch_det_tables(int geom, int op, const dd_geom2d *g, const char *planb, const float *in, int B,
-                      int V, float2 *dtab, cudaStream_t st);
+                      int V, float2 *dtab, int *status, cudaStream_t st);   // clears *status
 
 }  // namespace dd2

@@ -228,7 +228,9 @@ template <> struct Vox<2> {
 //   vx[s][y][x][b] = vol[b][s][y][x],  vt[s][x][H-1-y][b] = vol[b][s][y][x].
 template <int NB>
 __global__ void __launch_bounds__(256) k_lines_of3(const float *__restrict__ in, float *__restrict__ vx,
-                                                   float *__restrict__ vt, int W, int H, int Dp, int ngroups) {
+                                                   float *__restrict__ vt, int W, int H, int Dp, int ngroups,
+                                                   int *__restrict__ clear) {
+    if (clear && threadIdx.x == 0 && blockIdx.x + blockIdx.y + blockIdx.z == 0) *clear = 0;   // the call's status word
     using T = typename Vox<NB>::T;
     __shared__ T t[32][33];
     const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
@@ -268,7 +270,9 @@ __global__ void __launch_bounds__(256) k_lines_of3(const float *__restrict__ in,
 // group of its own).
 template <int GEOM, int FAMILY>
 __global__ void __launch_bounds__(128) k_sino3(dd_geom3d g, const char *__restrict__ plan, PlanLayout P,
-                                               const float *__restrict__ in, float *__restrict__ ss, int B, int V) {
+                                               const float *__restrict__ in, float *__restrict__ ss, int B, int V,
+                                               int *__restrict__ clear) {
+    if (threadIdx.x + blockIdx.x + blockIdx.y + blockIdx.z == 0) *clear = 0;   // the call's status word
     const int C = g.num_col, R = g.num_row;
     const int k = blockIdx.x * 128 + threadIdx.x, r = blockIdx.y, v = blockIdx.z;
     if (k >= C) return;
@@ -1330,8 +1334,8 @@ int launch_adj(const Adj3Args &a, const float *in, float *ss, cudaStream_t st) {
     const dd_geom3d &g = a.g;
     const dim3 gs((unsigned)((g.num_col + 127) / 128), (unsigned)g.num_row, (unsigned)a.V);
     dd2::ProfRec *pt = dd2::prof_begin(DD_KERNEL_TABLES, st);
-    if (a.family == 0) k_sino3<GEOM, 0><<<gs, 128, 0, st>>>(g, a.plan, a.P, in, ss, a.B, a.V);
-    else k_sino3<GEOM, 1><<<gs, 128, 0, st>>>(g, a.plan, a.P, in, ss, a.B, a.V);
+    if (a.family == 0) k_sino3<GEOM, 0><<<gs, 128, 0, st>>>(g, a.plan, a.P, in, ss, a.B, a.V, a.status);
+    else k_sino3<GEOM, 1><<<gs, 128, 0, st>>>(g, a.plan, a.P, in, ss, a.B, a.V, a.status);
     dd2::prof_end(pt, st);
     dd2::count_launches(1);
     dd2::ProfRec *pr = dd2::prof_begin(DD_KERNEL_ADJOINT, st);
@@ -1350,15 +1354,14 @@ int forward(int scan, int op, const dd_geom3d *g, const char *planb, const float
     const dim3 gl((unsigned)((W + 31) / 32), (unsigned)((H + 31) / 32), (unsigned)(nz < 65535 ? nz : 65535));
     const size_t done = (size_t)pairs * kNB * Dp;   // slices of the paired volumes
     dd2::ProfRec *pt = dd2::prof_begin(DD_KERNEL_TABLES, st);
-    if (pairs) k_lines_of3<kNB><<<gl, 256, 0, st>>>(in, (float *)volx, (float *)volt, W, H, Dp, pairs);
+    if (pairs) k_lines_of3<kNB><<<gl, 256, 0, st>>>(in, (float *)volx, (float *)volt, W, H, Dp, pairs, status);
     if (odd)
         k_lines_of3<1><<<gl, 256, 0, st>>>(in + done * W * H, (float *)volx + done * H * pad4(W),
-                                           (float *)volt + done * W * pad4(H), W, H, Dp, 1);
+                                           (float *)volt + done * W * pad4(H), W, H, Dp, 1, pairs ? nullptr : status);
     dd2::prof_end(pt, st);
     dd2::count_launches((pairs ? 1 : 0) + odd);
     const int s1 = launch_status();
     if (s1 != DD_OK) return s1;
-    if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
     Fwd3Args a;
     a.status = status;
     a.g = *g;
@@ -1383,7 +1386,6 @@ int forward(int scan, int op, const dd_geom3d *g, const char *planb, const float
 // Adjoint-type operator: out = value, or out = base + scale * value.
 int adjoint(int scan, int op, const dd_geom3d *g, const char *planb, const float *in, float *out,
             const float *basep, float scale, int B, int V, char *ss, int *status, cudaStream_t st) {
-    if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
     Adj3Args a;
     a.status = status;
     a.g = *g;

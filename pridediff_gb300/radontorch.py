@@ -22,6 +22,8 @@ Deliberate differences (all in the caller's favour):
 """
 from __future__ import annotations
 
+import contextlib
+
 import torch
 
 from . import _native as N
@@ -56,13 +58,55 @@ def host_options(options):
     return vals
 
 
+# What a call derives from plain values alone, kept by those values: geometry
+# records by the options' numbers, workspace sizes of validated calls.
+_geoms: dict = {}
+_sizes: dict = {}
+
+
+def _remember(table: dict, key, value):
+    if len(table) >= 1024:
+        table.clear()
+    table[key] = value
+    return value
+
+
+def _geometry(options, kind: str):
+    """(record, fields) of an options vector: kind "2d", "3d" or "spiral"."""
+    key = (kind, *host_options(options))
+    hit = _geoms.get(key)
+    if hit is None:
+        g = N.geom2d(key[1:]) if kind == "2d" else N.geom3d(key[1:], spiral=(kind == "spiral"))
+        hit = _remember(_geoms, key, (g, tuple(getattr(g, f) for f, _ in g._fields_)))
+    return hit
+
+
+def _workspace(dim: int, sc: int, opc: int, g, fields, batch: int, views: int, what: str) -> int:
+    """Workspace bytes of a call, once the library has accepted its geometry."""
+    key = (dim, sc, opc, fields, batch, views)
+    n = _sizes.get(key)
+    if n is None:
+        lib = N.load()
+        validate, size = ((lib.dd2d_validate, lib.dd2d_apply_workspace_bytes) if dim == 2 else
+                          (lib.dd3d_validate, lib.dd3d_apply_workspace_bytes))
+        N.check(validate(sc, opc, g, batch, views), what)
+        n = _remember(_sizes, key, int(size(sc, opc, g, batch, views)))
+    return n
+
+
+def _on(dev):
+    """The device as the current one (no context switch where it already is)."""
+    if torch.cuda.current_device() == dev.index:
+        return contextlib.nullcontext()
+    return torch.cuda.device(dev)
+
+
 def _check_inputs(x: torch.Tensor, angles: torch.Tensor, extra=None):
     # CHECK_DEVICE / CHECK_CONTIGUOUS (RadonTorch.cpp:12-14)
-    tensors = [x, angles] + ([extra] if extra is not None else [])
     dev = x.device
-    if any(t.device != dev for t in tensors):
+    if angles.device != dev or (extra is not None and extra.device != dev):
         raise RuntimeError("Expected all tensors to be on the same device")
-    if any(not t.is_contiguous() for t in tensors):
+    if not (x.is_contiguous() and angles.is_contiguous() and (extra is None or extra.is_contiguous())):
         raise RuntimeError("Expected all tensors to be contiguous")
     if dev.type != "cuda":
         raise RuntimeError("pridediff_gb300 runs on CUDA devices only; got a tensor on " + str(dev))
@@ -132,12 +176,14 @@ class _PlanCache:
 plans = _PlanCache()
 
 
-def plan2d(scan: str, g, angles: torch.Tensor):
-    """Device plan of a 2-D geometry (cached)."""
+def plan2d(scan: str, g, angles: torch.Tensor, fields: tuple = None):
+    """Device plan of a 2-D geometry (cached); fields: the record's values, if at hand."""
     lib = N.load()
     sc = N.SCAN2D[scan]
     V = int(angles.shape[0])
-    key = ("2d", sc, tuple(getattr(g, f) for f, _ in g._fields_), V, angles.device.index)
+    if fields is None:
+        fields = tuple(getattr(g, f) for f, _ in g._fields_)
+    key = ("2d", sc, fields, V, angles.device.index)
 
     def build():
         nbytes = int(lib.dd2d_plan_bytes(sc, g, V))
@@ -152,8 +198,7 @@ def plan2d(scan: str, g, angles: torch.Tensor):
 def _apply2d(scan: str, op: str, x: torch.Tensor, options, angles: torch.Tensor) -> torch.Tensor:
     _check_inputs(x, angles)
     lib = N.load()
-    o = host_options(options)
-    g = N.geom2d(o)
+    g, fields = _geometry(options, "2d")
     if x.dim() != 4:
         raise RuntimeError("expected a 4-D (B, C, ., .) tensor")
     B, C = x.shape[0], x.shape[1]
@@ -171,18 +216,17 @@ def _apply2d(scan: str, op: str, x: torch.Tensor, options, angles: torch.Tensor)
         return out.zero_()
     sc, opc = N.SCAN2D[scan], N.OPS[op]
     _status.check(x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         # the library validates the geometry before anything is enqueued
-        N.check(lib.dd2d_validate(sc, opc, g, B * C, V), f"{scan} {op}")
-        plan = plan2d(scan, g, angles)
-        nbytes = int(lib.dd2d_apply_workspace_bytes(sc, opc, g, B * C, V))
+        nbytes = _workspace(2, sc, opc, g, fields, B * C, V, f"{scan} {op}")
+        plan = plan2d(scan, g, angles, fields)
         ws = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=x.device)
 
         def run(cfg):
             return lib.dd2d_apply_planned_tuned(sc, opc, g, plan.data_ptr(), x.data_ptr(), out.data_ptr(), B * C,
                                                 V, ws.data_ptr(), nbytes, forward_tune(cfg),
                                                 _stream_ptr(x.device))
-        cfg = forward_shape(sc, g, B * C, V, x.device, run) if image_in else None
+        cfg = forward_shape(sc, g, B * C, V, x.device, run, fields) if image_in else None
         st = run(cfg)
     N.check(st, f"{scan} {op}")
     return out
@@ -197,7 +241,7 @@ def forward_tune(cfg):
     return t
 
 
-def forward_shape(sc: int, g, batch: int, views: int, device, run):
+def forward_shape(sc: int, g, batch: int, views: int, device, run, fields: tuple = None):
     """The single-geometry forward's CTA shape for this geometry and batch,
     chosen by the autotuner on first use (timing every candidate on the
     call's own buffers, which the chosen shape then overwrites) and kept for
@@ -206,7 +250,9 @@ def forward_shape(sc: int, g, batch: int, views: int, device, run):
     from . import autotune
     if not autotune.enabled():
         return None
-    key = autotune.forward2d_key(sc, tuple(getattr(g, f) for f, _ in g._fields_), batch, views, device)
+    if fields is None:
+        fields = tuple(getattr(g, f) for f, _ in g._fields_)
+    key = autotune.forward2d_key(sc, fields, batch, views, device)
     if key in autotune._forward_choice:
         return autotune._forward_choice[key]
     if torch.cuda.is_current_stream_capturing():
@@ -219,14 +265,16 @@ def forward_shape(sc: int, g, batch: int, views: int, device, run):
     return autotune.tune_forward2d(key, launch, about=about)
 
 
-def plan3d(scan: str, g, angles: torch.Tensor, source_pos=None):
+def plan3d(scan: str, g, angles: torch.Tensor, source_pos=None, fields: tuple = None):
     """Device plan of a 3-D geometry (cached; spiral plans also key on the
     source table's identity and version)."""
     lib = N.load()
     sc = N.SCAN3D[scan]
     V = int(angles.shape[0])
     sp_key = None if source_pos is None else (id(source_pos), source_pos._version)
-    key = ("3d", sc, tuple(getattr(g, f) for f, _ in g._fields_), V, angles.device.index, sp_key)
+    if fields is None:
+        fields = tuple(getattr(g, f) for f, _ in g._fields_)
+    key = ("3d", sc, fields, V, angles.device.index, sp_key)
 
     def build():
         nbytes = int(lib.dd3d_plan_bytes(sc, g, V))
@@ -245,8 +293,7 @@ def _apply3d(scan: str, op: str, x: torch.Tensor, options, angles: torch.Tensor,
     if source_pos is not None and source_pos.dtype != torch.float32:
         raise RuntimeError("Expected float32 tensors")
     lib = N.load()
-    o = host_options(options)
-    g = N.geom3d(o, spiral=(scan == "spiral"))
+    g, fields = _geometry(options, "spiral" if scan == "spiral" else "3d")
     if x.dim() != 5:
         raise RuntimeError("expected a 5-D (B, C, ., ., .) tensor")
     B, Ch = x.shape[0], x.shape[1]
@@ -266,10 +313,9 @@ def _apply3d(scan: str, op: str, x: torch.Tensor, options, angles: torch.Tensor,
         return out.zero_()
     sc, opc = N.SCAN3D[scan], N.OPS[op]
     _status.check(x.device)
-    with torch.cuda.device(x.device):
-        N.check(lib.dd3d_validate(sc, opc, g, B * Ch, V), f"{scan} {op}")
-        plan = plan3d(scan, g, angles, source_pos)
-        nbytes = int(lib.dd3d_apply_workspace_bytes(sc, opc, g, B * Ch, V))
+    with _on(x.device):
+        nbytes = _workspace(3, sc, opc, g, fields, B * Ch, V, f"{scan} {op}")
+        plan = plan3d(scan, g, angles, source_pos, fields)
         ws = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=x.device)
         st = lib.dd3d_apply_planned(sc, opc, g, plan.data_ptr(), x.data_ptr(), out.data_ptr(), B * Ch, V,
                                     ws.data_ptr(), nbytes, _stream_ptr(x.device))

@@ -28,19 +28,21 @@ from . import _native as N
 
 _lock = threading.Lock()
 _word = None          # pinned int32 host tensor, shared by every device
+_view = None          # the same memory as a numpy array: read on every call
 _registered = set()   # device indices whose kernels write _word
 
 
 def _sink():
-    global _word
+    global _word, _view
     if _word is None:
         _word = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        _view = _word.numpy()
     return _word
 
 
 def register(device) -> None:
     """Make the kernels on `device` write timeouts into the host word."""
-    idx = torch.device(device).index
+    idx = device.index if isinstance(device, torch.device) else torch.device(device).index
     if idx is None:
         idx = torch.cuda.current_device()
     if idx in _registered:
@@ -61,7 +63,7 @@ def check(device) -> None:
     registration copies to device memory, which a capture does not allow)."""
     if not torch.cuda.is_current_stream_capturing():
         register(device)
-    w = _word
+    w = _view
     if w is None:
         return
     code = int(w[0])
