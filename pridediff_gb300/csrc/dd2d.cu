@@ -177,139 +177,30 @@ k_axis_views(int V, const DdView2 *__restrict__ views, int *__restrict__ axisv) 
     }
 }
 
-// ---------------------------------------------------------------------------
-// Parallel-beam adjoint, line-major.  The parallel beam's detector boundaries
-// drift per walked line (ParaDisCPU2d.cpp:76, :100: the recurrence restarts
-// at each line's first bin), so every (view, line, image) needs its own piece
-// constants of the detector table.  One CTA takes one walked line and a group
-// of kBI images over all the views that walk its axis, builds the line's
-// piece constants once per view and serves all the line's pixels from them
-// (a 32 x 32 tile rebuilds them for each tile the line crosses).  A thread
-// owns fixed pixels of the line; their sums stay in shared memory.  The rows
-// (x-branch views) are written by one launch and the columns added by a
-// second, the same order as the tiled kernel's merge of its two ownerships,
-// with the same per-pixel arithmetic.
-// ---------------------------------------------------------------------------
-struct ParaSmem {
-    int rec, drec, tab, kt, acc, bar, total;
-};
-__host__ __device__ inline ParaSmem para_smem(int D, int npix) {
-    ParaSmem s;
-    int o = 0;
-    s.rec = o; o += 2 * (int)sizeof(DdLine);
-    s.drec = o; o += 2 * (int)sizeof(DdLine);
-    s.tab = o; o += 2 * kBI * rs_entries(D) * (int)sizeof(float2);
-    s.kt = o; o += kBI * 32 * (int)sizeof(float);
-    s.acc = o; o += ((kBI * npix + 3) & ~3) * (int)sizeof(float);
-    s.bar = o; o += 2 * (int)sizeof(uint64_t);
-    s.total = (o + 127) & ~127;
-    return s;
-}
-
+// Single-geometry parallel-beam adjoint launch: grid (lines * cluster, image groups).
 template <int OPK>   // 0 ProjTrans, 1 BackProj
-__global__ void __launch_bounds__(kThreads)
+__global__ void __cluster_dims__(kAdjCluster, 1, 1) __launch_bounds__(kThreads)
 k_adj_para(dd_geom2d g, int B, int V, int nl, int axis, const int *__restrict__ axisv,
            const DdLine *__restrict__ lines, const DdLine *__restrict__ dlines,
            const float2 *__restrict__ dtab, float *__restrict__ out, const float *__restrict__ base,
-           float scale, int add, int *__restrict__ status) {
+           float scale, int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const int W = g.width, H = g.height, D = g.num_det;
-    const int npix = axis ? W : H;
-    const int line = blockIdx.x, b0 = blockIdx.y * kBI, nb = min(kBI, B - b0);
-    const int nv = axisv[axis ? 0 : 1];
-    const int *vlist = axisv + 2 + (axis ? 0 : V);
-    const int rsd = rs_entries(D);
-    const ParaSmem S = para_smem(D, npix);
-    DdLine *rec = reinterpret_cast<DdLine *>(smem + S.rec);
-    DdLine *drec = reinterpret_cast<DdLine *>(smem + S.drec);
-    float2 *tabs = reinterpret_cast<float2 *>(smem + S.tab);   // [2][kBI][rsd]
-    float *kt = reinterpret_cast<float *>(smem + S.kt);        // [kBI][32]
-    float *accs = reinterpret_cast<float *>(smem + S.acc);     // [kBI][npix]
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + S.bar);
-    __shared__ int abort_flag;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < kBI * npix; i += kThreads) accs[i] = 0.0f;
-    if (tid == 0) abort_flag = 0;
-    init_bars(bar);   // synchronises the CTA
-    DdPhases ph;
-
-    const uint32_t rec_bytes = (uint32_t)sizeof(DdLine);
-    const uint32_t tab_bytes = (uint32_t)(rsd * sizeof(float2));
-    auto issue = [&](int idx, int buf) {
-        const int v = vlist[idx];
-        dd_mbar_expect_tx(&bar[buf], 2 * rec_bytes + nb * tab_bytes);
-        dd_bulk_g2s(rec + buf, lines + (size_t)v * nl + line, rec_bytes, &bar[buf]);
-        dd_bulk_g2s(drec + buf, dlines + (size_t)v * nl + line, rec_bytes, &bar[buf]);
-        for (int b = 0; b < nb; b++)
-            dd_bulk_g2s(tabs + ((size_t)buf * kBI + b) * rsd, dtab + ((size_t)(b0 + b) * V + v) * rsd, tab_bytes,
-                        &bar[buf]);
-    };
-    const int issuer = (kWarps - 1) * 32;
-    if (tid == issuer && nv > 0) issue(0, 0);
-    for (int idx = 0; idx < nv; idx++) {
-        const int buf = idx & 1;
-        if (!dd_mbar_wait(&bar[buf], ph.parity(buf))) abort_flag = 1;
-        ph.flip(buf);
-        // past this barrier every warp has finished view idx - 1, whose
-        // buffer takes the copies of view idx + 1
-        __syncthreads();
-        if (abort_flag) {
-            // view idx's copies (the wait gave up on them) may be in flight
-            if (tid == issuer) dd_mbar_drain(&bar[buf], ph.parity(buf) ^ 1u);
-            break;
-        }
-        if (tid == issuer && idx + 1 < nv) issue(idx + 1, buf ^ 1);
-        const DdLine &L = rec[buf], &Ld = drec[buf];
-        if (L.h.npiece == 0) continue;   // the same for the whole CTA
-        const int npd = Ld.h.npiece;
-        const float2 *tb = tabs + (size_t)buf * kBI * rsd;
-        for (int b = warp; b < nb; b += kWarps) kt[b * 32 + lane] = npd > 0 ? piece_K(Ld, tb + (size_t)b * rsd, lane) : 0.0f;
-        __syncthreads();
-        const int i0 = L.h.i0, nend = L.h.nend;
-        const float bound0 = L.h.bound0;
-        const float alpha = (OPK == 0) ? 1.0f : L.h.alpha;
-        // a warp takes 32 consecutive pixel boundaries (lane l: the upper
-        // boundary of pixel q0 + l - 1) and 31 pixels: each boundary is
-        // located once and neighbours difference by one shuffle
-        for (int q0 = warp * kBinsPerWarp; q0 < npix; q0 += kWarps * kBinsPerWarp) {   // warp-uniform
-            const int bi = q0 + lane - 1;   // boundary index (upper boundary of pixel bi)
-            float u = bound0;               // boundary i0 - 1 is the walk start; below it H is constant
-            if (bi >= i0 && bi < nend) u = dd_boundary(&L, bi, L.p[0].Q + (float)(bi - L.p[0].gb) * L.p[0].dl);
-            int pU = 0, jU = 0;
-            float rU = 0.0f, dlU = 0.0f;
-            if (npd > 0) {
-                dd_locate(&Ld, fminf(fmaxf(u, bound0), Ld.h.endv), &pU, &jU, &rU);
-                dlU = Ld.p[pU].dl;
-            }
-            const int pi = bi;   // the pixel this lane closes (lanes 1..31)
-            const bool valid = lane > 0 && pi < npix && pi >= i0 && pi < nend;
-#pragma unroll
-            for (int b = 0; b < kBI; b++) {
-                if (b >= nb) break;
-                float hu = 0.0f;
-                if (npd > 0) {
-                    const float2 e = tb[(size_t)b * rsd + jU];
-                    hu = fmaf(rU, e.y, fmaf(dlU, e.x, kt[b * 32 + pU]));
-                }
-                const float hl = __shfl_up_sync(0xffffffffu, hu, 1);
-                if (valid) accs[b * npix + pi] += alpha * (hu - hl);
-            }
-        }
-    }
-    __syncthreads();
-    if (abort_flag) {
-        if (tid == 0) dd_report_timeout(status);
-        return;
-    }
-    for (int b = 0; b < nb; b++) {
-        for (int pi = tid; pi < npix; pi += kThreads) {
-            const int r = axis ? line : H - 1 - pi, c = axis ? pi : line;
-            const size_t o = ((size_t)(b0 + b) * H + r) * W + c;
-            const float val = accs[b * npix + pi];
-            if (!add) out[o] = base ? fmaf(scale, val, base[o]) : val;
-            else out[o] = base ? fmaf(scale, val, out[o]) : out[o] + val;
-        }
-    }
+    AdjItem it = {};
+    it.c0 = blockIdx.x / kAdjCluster;
+    it.r0 = axis;
+    it.b0 = blockIdx.y * kBI;
+    it.nb = min(kBI, B - it.b0);
+    it.V = V;
+    it.nl = nl;
+    it.lines = lines;
+    it.dlines = dlines;
+    it.axisv = axisv;
+    it.dtab = dtab;
+    it.out = out;
+    it.base = base;
+    it.scale = scale;
+    const ParaSmem S = para_smem(g.num_det, axis ? g.width : g.height, min(kBI, B));
+    if (!adj_para_line<OPK>(g, it, smem, S) && threadIdx.x == 0) dd_report_timeout(status);
 }
 
 // Adjoint map of fan beams (plan time): one CTA per (tile, view) fills the
@@ -387,7 +278,7 @@ k_adj(dd_geom2d g, int B, int V, const DdView2 *__restrict__ views, const unsign
       const int2 *__restrict__ trange, const int *__restrict__ axisv, const float2 *__restrict__ dtab,
       float *__restrict__ out, const float *__restrict__ base, float scale, int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const AdjSmem SL = adj_smem(GEOM);
+    const AdjSmem SL = adj_smem();
     init_bars(reinterpret_cast<uint64_t *>(smem + SL.bar), kAdjBufs);
     DdPhases ph;
     AdjItem it = {};
@@ -653,7 +544,7 @@ static int launch_adj_as(const dd_geom2d *g, const PlanLayout &P, const char *pl
                          float *out, const float *base, float scale, int *status, cudaStream_t st) {
     const unsigned ngroups = (unsigned)((B + NB - 1) / NB);
     const dim3 grid((unsigned)((g->width + kTile - 1) / kTile) * ngroups * kAdjCluster, (g->height + kTile - 1) / kTile);
-    const AdjSmem S = adj_smem(GEOM);
+    const AdjSmem S = adj_smem();
     auto kern = k_adj<GEOM, OPK, NB>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
         return DD_ERR_LAUNCH;
@@ -689,7 +580,8 @@ static int launch_adj_para(int op, const dd_geom2d *g, const PlanLayout &P, cons
     const DdLine *dlines = (const DdLine *)(planb + P.dlines);
     const int *axisv = (const int *)(planb + P.axisv);
     const int W = g->width, H = g->height, D = g->num_det;
-    const int smax = std::max(para_smem(D, W).total, para_smem(D, H).total);
+    const int nbm = std::min(kBI, B);
+    const int smax = std::max(para_smem(D, W, nbm).total, para_smem(D, H, nbm).total);
     if (smax > max_smem_optin()) return DD_ERR_SIZE_OVERFLOW;
     auto kern = (op == DD_OP_PROJ_T) ? k_adj_para<0> : k_adj_para<1>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) != cudaSuccess)
@@ -697,9 +589,9 @@ static int launch_adj_para(int op, const dd_geom2d *g, const PlanLayout &P, cons
     ProfRec *pr = prof_begin(DD_KERNEL_ADJOINT, st);
     for (int axis = 1; axis >= 0; axis--) {
         const int npix = axis ? W : H, nline = axis ? H : W;
-        const dim3 grid((unsigned)nline, (unsigned)((B + kBI - 1) / kBI));
-        kern<<<grid, kThreads, para_smem(D, npix).total, st>>>(*g, B, V, P.nl, axis, axisv, lines, dlines, dtab,
-                                                                out, base, scale, axis == 0, status);
+        const dim3 grid((unsigned)nline * kAdjCluster, (unsigned)((B + kBI - 1) / kBI));
+        kern<<<grid, kThreads, para_smem(D, npix, nbm).total, st>>>(*g, B, V, P.nl, axis, axisv, lines, dlines, dtab,
+                                                                     out, base, scale, status);
     }
     prof_end(pr, st);
     g_launches += 2;

@@ -40,7 +40,7 @@ struct BatchInst {
 struct BatchLayout {
     size_t desc, fitems, aitems, plans, total;        // plan buffer
     size_t w_tabs, w_dtab, w_resid, w_counter, w_status, w_total;   // workspace
-    int nfwd, nadj, Dmax, nmax;   // items; largest detector and longest line
+    int nfwd, nadj, nrow, Dmax, nmax;   // items (nrow of the parallel beam's are rows); largest detector and line
     int fi;   // largest instance's slices per forward item
     std::vector<BatchInst> inst;
 };
@@ -65,7 +65,7 @@ static BatchLayout batch_layout(int scan, const dd_instance2d *in, int n, int bi
     L.fi = 1;
     long long img = 0, sino = 0, tabs = 0, dtab = 0;
     size_t plans = 0;
-    L.nfwd = L.nadj = 0;
+    L.nfwd = L.nadj = L.nrow = 0;
     L.Dmax = 1;
     L.nmax = 1;
     for (int i = 0; i < n; i++) {
@@ -103,7 +103,12 @@ static BatchLayout batch_layout(int scan, const dd_instance2d *in, int n, int bi
         dtab += ((long long)d.batch * d.V * rs_entries(D) + 1) & ~1LL;
         const int groups = (d.batch + bi - 1) / bi;
         L.nfwd += d.V * ((d.batch + d.ps - 1) / d.ps);
-        L.nadj += ((W + kTile - 1) / kTile) * ((H + kTile - 1) / kTile) * groups;
+        if (scan == DD_SCAN_PARA) {
+            L.nrow += H * groups;
+            L.nadj += (H + W) * groups;
+        } else {
+            L.nadj += ((W + kTile - 1) / kTile) * ((H + kTile - 1) / kTile) * groups;
+        }
         L.Dmax = std::max(L.Dmax, D);
         L.nmax = std::max(L.nmax, std::max(W, H));
     }
@@ -270,9 +275,6 @@ k_fwd_items(int geom, int op, const BatchInst *__restrict__ desc, const int4 *__
     }
 }
 
-// Adjoint items of parallel beams: persistent, 3 CTAs per SM (two sets of
-// accumulators).  The item and its geometry live in shared memory, as in the
-// forward.
 __device__ __forceinline__ AdjItem adj_item(const BatchInst &d, const int4 w, const char *pb, const float2 *dtabs,
                                             float *out, const float *base, float scale) {
     AdjItem it;
@@ -282,9 +284,7 @@ __device__ __forceinline__ AdjItem adj_item(const BatchInst &d, const int4 w, co
     it.nb = w.w;
     it.V = d.V;
     it.nl = d.nl;
-    it.angles = reinterpret_cast<const float *>(pb + d.ang);
     it.views = reinterpret_cast<const DdView2 *>(pb + d.views);
-    it.dp = reinterpret_cast<const float *>(pb + d.dp);
     it.lines = reinterpret_cast<const DdLine *>(pb + d.lines);
     it.dlines = reinterpret_cast<const DdLine *>(pb + d.dlines);
     it.amap = reinterpret_cast<const unsigned char *>(pb + d.amap);
@@ -297,33 +297,27 @@ __device__ __forceinline__ AdjItem adj_item(const BatchInst &d, const int4 w, co
     return it;
 }
 
+// Adjoint items of parallel beams: a cluster per line, the rows by one launch,
+// then the columns.
 template <int OPK>
-__global__ void __launch_bounds__(kThreads, 3)
-k_adj_items_para(const BatchInst *__restrict__ desc, const int4 *__restrict__ items, int nitems,
+__global__ void __cluster_dims__(kAdjCluster, 1, 1) __launch_bounds__(kThreads)
+k_adj_items_para(const BatchInst *__restrict__ desc, const int4 *__restrict__ items, int axis,
                  const char *__restrict__ plan, size_t plans_off, const float2 *__restrict__ dtabs,
-                 float *__restrict__ out, const float *__restrict__ base, float scale,
-                 int *__restrict__ counter, int *__restrict__ status) {
+                 float *__restrict__ out, const float *__restrict__ base, float scale, int Dmax, int nmax,
+                 int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const AdjSmem SL = adj_smem(DD_GEOM_PARA);
-    init_bars(reinterpret_cast<uint64_t *>(smem + SL.bar), 2);
     __shared__ AdjItem s_it;
     __shared__ dd_geom2d s_g;
-    DdPhases ph;
-    for (;;) {
-        const int i = next_item(counter + 1);   // its barriers also order s_it's reuse
-        if (i >= nitems) break;
-        if (threadIdx.x == 0) {
-            const int4 w = items[i];
-            const BatchInst &d = desc[w.x];
-            s_it = adj_item(d, w, plan + plans_off + d.plan_off, dtabs, out, base, scale);
-            s_g = d.g;
-        }
-        __syncthreads();
-        if (!adj_tile<DD_GEOM_PARA, OPK>(s_g, s_it, smem, ph)) {
-            if (threadIdx.x == 0) dd_report_timeout(status);
-            break;
-        }
+    if (threadIdx.x == 0) {
+        const int4 w = items[blockIdx.x / kAdjCluster];
+        const BatchInst &d = desc[w.x];
+        s_it = adj_item(d, w, plan + plans_off + d.plan_off, dtabs, out, base, scale);
+        s_it.c0 = w.y;
+        s_it.r0 = axis;
+        s_g = d.g;
     }
+    __syncthreads();
+    if (!adj_para_line<OPK>(s_g, s_it, smem, para_smem(Dmax, nmax, kBI)) && threadIdx.x == 0) dd_report_timeout(status);
 }
 
 // Adjoint items of fan beams: a cluster per item, in the list's order; 4 CTAs
@@ -339,7 +333,7 @@ k_adj_items(const BatchInst *__restrict__ desc, const int4 *__restrict__ items, 
             size_t plans_off, const float2 *__restrict__ dtabs, float *__restrict__ out,
             const float *__restrict__ base, float scale, int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
-    const AdjSmem SL = adj_smem(GEOM);
+    const AdjSmem SL = adj_smem();
     __shared__ AdjItem s_it;
     __shared__ dd_geom2d s_g;
     if (threadIdx.x == 0) {
@@ -469,20 +463,24 @@ static int launch_fwd_items(int geom, int op, const BatchLayout &L, const char *
 
 template <int GEOM>
 static int launch_adj_items(int op, const BatchLayout &L, const char *planb, const float2 *dtabs,
-                            float *out, const float *base, float scale, int *counter, int *status,
-                            const dd_tune2d *tune, cudaStream_t st) {
-    const AdjSmem S = adj_smem(GEOM);
+                            float *out, const float *base, float scale, int *status, cudaStream_t st) {
     const BatchInst *desc = (const BatchInst *)(planb + L.desc);
     const int4 *items = (const int4 *)(planb + L.aitems);
     ProfRec *pr = prof_begin(DD_KERNEL_ADJOINT, st);
     if constexpr (GEOM == DD_GEOM_PARA) {
         auto kern = (op == DD_OP_PROJ_T) ? k_adj_items_para<0> : k_adj_items_para<1>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
+        const int smem = para_smem(L.Dmax, L.nmax, kBI).total;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return DD_ERR_LAUNCH;
-        const int grid = grid_of(tune, L.nadj, resident_ctas(kern, S.total, kThreads));
-        kern<<<grid, kThreads, S.total, st>>>(desc, items, L.nadj, planb, L.plans, dtabs, out, base, scale, counter,
-                                              status);
+        for (int axis = 1; axis >= 0; axis--) {
+            const int4 *from = axis ? items : items + L.nrow;
+            const int n = axis ? L.nrow : L.nadj - L.nrow;
+            kern<<<(unsigned)n * kAdjCluster, kThreads, smem, st>>>(desc, from, axis, planb, L.plans, dtabs, out, base, scale,
+                                                                   L.Dmax, L.nmax, status);
+        }
+        count_launches(1);
     } else {
+        const AdjSmem S = adj_smem();
         auto kern = (op == DD_OP_PROJ_T) ? k_adj_items<GEOM, 0> : k_adj_items<GEOM, 1>;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
             return DD_ERR_LAUNCH;
@@ -508,11 +506,9 @@ static int batch_forward(int scan, int op, const BatchLayout &L, const char *pla
 
 // adjoint of all instances: out = base + scale * (A^T in)   (base may be null)
 static int batch_adjoint(int scan, int op, const BatchLayout &L, const char *planb, const float *in,
-                         float *out, const float *base, float scale, char *wb, const dd_tune2d *tune,
-                         cudaStream_t st) {
+                         float *out, const float *base, float scale, char *wb, cudaStream_t st) {
     const int geom = geom_of(scan);
     float2 *dtabs = (float2 *)(wb + L.w_dtab);
-    int *counter = (int *)(wb + L.w_counter);
     int *status = (int *)(wb + L.w_status);
     const BatchInst *desc = (const BatchInst *)(planb + L.desc);
     int maxw = 1;
@@ -523,10 +519,9 @@ static int batch_adjoint(int scan, int op, const BatchLayout &L, const char *pla
                                                                   planb, L.plans, in, dtabs);
     prof_end(pr, st);
     count_launches(1);
-    if (cudaMemsetAsync(counter, 0, 2 * sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
-    if (geom == DD_GEOM_PARA) return launch_adj_items<DD_GEOM_PARA>(op, L, planb, dtabs, out, base, scale, counter, status, tune, st);
-    if (geom == DD_GEOM_FLAT) return launch_adj_items<DD_GEOM_FLAT>(op, L, planb, dtabs, out, base, scale, counter, status, tune, st);
-    return launch_adj_items<DD_GEOM_ARC>(op, L, planb, dtabs, out, base, scale, counter, status, tune, st);
+    if (geom == DD_GEOM_PARA) return launch_adj_items<DD_GEOM_PARA>(op, L, planb, dtabs, out, base, scale, status, st);
+    if (geom == DD_GEOM_FLAT) return launch_adj_items<DD_GEOM_FLAT>(op, L, planb, dtabs, out, base, scale, status, st);
+    return launch_adj_items<DD_GEOM_ARC>(op, L, planb, dtabs, out, base, scale, status, st);
 }
 
 }  // namespace dd2
@@ -560,7 +555,7 @@ extern "C" int dd2d_batch_plan(int scan, const dd_instance2d *inst, int n, const
         int4 w;
         long long cost;
     };
-    std::vector<Item> fw, aw;
+    std::vector<Item> fw, aw, ac;   // ac: the parallel beam's columns
     fw.reserve(L.nfwd);
     aw.reserve(L.nadj);
     for (int i = 0; i < n; i++) {
@@ -573,6 +568,11 @@ extern "C" int dd2d_batch_plan(int scan, const dd_instance2d *inst, int n, const
         }
         for (int b0 = 0; b0 < d.batch; b0 += kBI) {
             const int nb = std::min(kBI, d.batch - b0);
+            if (scan == DD_SCAN_PARA) {
+                for (int y = 0; y < H; y++) aw.push_back({make_int4(i, y, b0, nb), (long long)d.V * W * nb});
+                for (int x = 0; x < W; x++) ac.push_back({make_int4(i, x, b0, nb), (long long)d.V * H * nb});
+                continue;
+            }
             for (int ty = 0; ty < (H + kTile - 1) / kTile; ty++)
                 for (int tx = 0; tx < (W + kTile - 1) / kTile; tx++)
                     aw.push_back({make_int4(i, tx | (ty << 16), b0, nb), (long long)d.V * nb});
@@ -582,7 +582,9 @@ extern "C" int dd2d_batch_plan(int scan, const dd_instance2d *inst, int n, const
     if (lpt) {
         std::stable_sort(fw.begin(), fw.end(), [](const Item &a, const Item &b) { return a.cost > b.cost; });
         std::stable_sort(aw.begin(), aw.end(), [](const Item &a, const Item &b) { return a.cost > b.cost; });
+        std::stable_sort(ac.begin(), ac.end(), [](const Item &a, const Item &b) { return a.cost > b.cost; });
     }
+    aw.insert(aw.end(), ac.begin(), ac.end());
     std::vector<int4> fi(fw.size()), ai(aw.size());
     for (size_t k = 0; k < fw.size(); k++) fi[k] = fw[k].w;
     for (size_t k = 0; k < aw.size(); k++) ai[k] = aw[k].w;
@@ -615,7 +617,7 @@ extern "C" int dd2d_batch_apply(int scan, int op, const dd_instance2d *inst, int
     if (cudaMemsetAsync(wb + L.w_status, 0, sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
     if (op_is_forward(op))
         return batch_forward(scan, op, L, (const char *)planp, in, out, nullptr, wb, tune, st);
-    return batch_adjoint(scan, op, L, (const char *)planp, in, out, nullptr, 1.0f, wb, tune, st);
+    return batch_adjoint(scan, op, L, (const char *)planp, in, out, nullptr, 1.0f, wb, st);
 }
 
 extern "C" int dd2d_batch_dc_step(int scan, const dd_instance2d *inst, int n, const void *planp, float *x,
@@ -634,7 +636,7 @@ extern "C" int dd2d_batch_dc_step(int scan, const dd_instance2d *inst, int n, co
     if (cudaMemsetAsync(wb + L.w_status, 0, sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
     int s1 = batch_forward(scan, DD_OP_PROJ, L, pb, x, resid, y, wb, tune, st);
     if (s1 != DD_OK) return s1;
-    return batch_adjoint(scan, DD_OP_PROJ_T, L, pb, resid, x, x, -eta, wb, tune, st);
+    return batch_adjoint(scan, DD_OP_PROJ_T, L, pb, resid, x, x, -eta, wb, st);
 }
 
 int dd2b_set_sink(int *sink) { return dd_set_status_sink_tu(sink); }

@@ -284,36 +284,19 @@ constexpr int kAdjBufs = 3;
 static_assert((kAdjBufs * kMapBlkBytes + kAdjBufs * kBI * kStage * 8) % 16 == 0,
               "the fan adjoint's per-buffer copy descriptors must be 16-byte aligned");
 
-// Shared-memory layout of the adjoint kernel (bytes).  Parallel beam: line
-// records (and detector-side records); fan beams: adjoint-map rows, detector
-// table slices and per-line scales.
+// Shared-memory layout of the fan-beam adjoint (bytes): adjoint-map rows,
+// detector table slices and per-line scales.
 struct AdjSmem {
-    int rec, drec, kd, stage, krange, bar, total;
-    int map;
+    int map, stage, krange, bar, total;
 };
 
-__host__ __device__ inline AdjSmem adj_smem(int geom) {
+__host__ __device__ inline AdjSmem adj_smem() {
     AdjSmem s;
     int o = 0;
-    s.map = 0;
-    if (geom != DD_GEOM_PARA) {
-        s.rec = s.drec = s.kd = 0;
-        s.map = o; o += kAdjBufs * kMapBlkBytes;
-        s.stage = o; o += kAdjBufs * kBI * kStage * (int)sizeof(float2);
-        s.krange = o; o += 4 * kAdjBufs * (int)sizeof(int);   // 16-byte aligned: read as int4
-        s.bar = o; o += kAdjBufs * (int)sizeof(uint64_t);
-        s.total = (o + 127) & ~127;
-        return s;
-    }
-    s.rec = o; o += 2 * kTile * (int)sizeof(DdLine);
-    s.drec = o; if (geom == DD_GEOM_PARA) o += 2 * kTile * (int)sizeof(DdLine);
-    s.kd = o; if (geom == DD_GEOM_PARA) o += kWarps * kBI * 32 * (int)sizeof(float);
-    s.stage = o; if (geom != DD_GEOM_PARA) o += 2 * kBI * kStage * (int)sizeof(float2);
-    s.krange = o; o += 4 * (int)sizeof(int);
-    s.bar = o; o += 2 * (int)sizeof(uint64_t);
-    // the final merge of the two pixel ownerships reuses the record buffers
-    const int merge = kBI * kTile * (kTile + 1) * (int)sizeof(float);
-    if (o < merge + 16) o = merge + 16;
+    s.map = o; o += kAdjBufs * kMapBlkBytes;
+    s.stage = o; o += kAdjBufs * kBI * kStage * (int)sizeof(float2);
+    s.krange = o; o += 4 * kAdjBufs * (int)sizeof(int);   // 16-byte aligned: read as int4
+    s.bar = o; o += kAdjBufs * (int)sizeof(uint64_t);
     s.total = (o + 127) & ~127;
     return s;
 }
@@ -367,15 +350,14 @@ __device__ __forceinline__ int fan_bin(int geom, const dd_geom2d &g, const DdVie
     return k;
 }
 
-// One adjoint work item: a 32x32 tile of one instance and a group of <= kBI
-// of its images, accumulated over all views.  Epilogue: out = value, or
-// out = base + scale * value (base may alias out: in-place update).
+// One adjoint work item of one instance and a group of <= kBI of its images:
+// fan beams, a 32x32 tile over all views; parallel beam, a walked line over
+// the views that walk its axis.  Epilogue: out = value, or out = base + scale
+// * value (base may alias out: in-place update).
 struct AdjItem {
-    int c0, r0, b0, nb, V, nl;
-    const float *angles;
+    int c0, r0, b0, nb, V, nl;   // parallel beam: c0 = line, r0 = 1 for rows, 0 for columns
     const DdView2 *views;
-    const float *dp;
-    const DdLine *lines, *dlines;
+    const DdLine *lines, *dlines;   // parallel beam
     const unsigned char *amap;   // fan beams: adjoint-map blocks (plan)
     const int2 *trange;          // fan beams, per (view, tile): {first staged bin, bins | xb << 16} (plan)
     const int *axisv;            // view lists (plan)
@@ -385,248 +367,9 @@ struct AdjItem {
     float scale;
 };
 
-template <int GEOM, int OPK>   // OPK: 0 ProjTrans, 1 BackProj, 2 BackProjWeighted
-__device__ bool adj_tile(const dd_geom2d &g, const AdjItem &it, unsigned char *smem, DdPhases &ph) {
-    const AdjSmem SL = adj_smem(GEOM);
-    const int V = it.V, nl = it.nl;
-    const float *__restrict__ angles = it.angles;
-    const DdView2 *__restrict__ views = it.views;
-    const float *__restrict__ dp = it.dp;
-    const DdLine *__restrict__ lines = it.lines;
-    const DdLine *__restrict__ dlines = it.dlines;
-    const float2 *__restrict__ dtab = it.dtab;
-    DdLine *recs = reinterpret_cast<DdLine *>(smem + SL.rec);
-    DdLine *drecs = reinterpret_cast<DdLine *>(smem + SL.drec);
-    float *kdp = reinterpret_cast<float *>(smem + SL.kd);
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + SL.bar);
-    float2 *stage = reinterpret_cast<float2 *>(smem + SL.stage);
-    int *krange = reinterpret_cast<int *>(smem + SL.krange);   // per buffer: first staged bin, count
-    __shared__ int abort_flag;
-
-    const int c0 = it.c0, r0 = it.r0;
-    const int b0 = it.b0;
-    const int nb = it.nb;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int W = g.width, H = g.height, D = g.num_det;
-    const int rsd = rs_entries(D);
-
-    if (tid == 0) abort_flag = 0;
-    __syncthreads();
-
-    // records of the tile's lines of view v: rows r0.. (x-branch) or columns c0..
-    // plus, for fan beams, the slice of every image's detector table that the
-    // tile can reach (16-byte aligned: even first bin, even count)
-    auto issue = [&](int v, int buf) {
-        const DdView2 vwv = views[v];
-        const int xbv = vwv.xb;
-        const int line0 = xbv ? r0 : c0;
-        const int nline = xbv ? H : W;
-        const int n = min(kTile, nline - line0);
-        const uint32_t bytes = (uint32_t)(n * sizeof(DdLine));
-        uint32_t tx = bytes * (GEOM == DD_GEOM_PARA ? 2u : 1u);
-        int kb = 0, kn = 0;
-        if (GEOM != DD_GEOM_PARA) {
-            int kmin, kmax;
-            tile_bin_range(GEOM, g, vwv, angles[v], c0, r0, &kmin, &kmax);
-            kb = kmin & ~1;
-            kn = (kmax - kb + 2) & ~1;
-            if (kb + kn > rsd) kn = rsd - kb;
-            if (kn > kStage || kn <= 0) kn = 0;
-            tx += (uint32_t)(nb * kn * (int)sizeof(float2));
-        }
-        krange[2 * buf] = kb;
-        krange[2 * buf + 1] = kn;
-        dd_mbar_expect_tx(&bar[buf], tx);
-        dd_bulk_g2s(recs + buf * kTile, lines + (size_t)v * nl + line0, bytes, &bar[buf]);
-        if (GEOM == DD_GEOM_PARA)
-            dd_bulk_g2s(drecs + buf * kTile, dlines + (size_t)v * nl + line0, bytes, &bar[buf]);
-        if (kn > 0)
-            for (int b = 0; b < nb; b++)
-                dd_bulk_g2s(stage + ((size_t)buf * kBI + b) * kStage, dtab + ((size_t)(b0 + b) * V + v) * rsd + kb,
-                            (uint32_t)(kn * sizeof(float2)), &bar[buf]);
-    };
-
-    float ax[kLinesPerWarp][kBI], ay[kLinesPerWarp][kBI];
-#pragma unroll
-    for (int q = 0; q < kLinesPerWarp; q++)
-#pragma unroll
-        for (int b = 0; b < kBI; b++) ax[q][b] = ay[q][b] = 0.0f;
-
-    if (tid == 0) issue(0, 0);
-    int inflight = -1;
-    for (int v = 0; v < V; v++) {
-        const int buf = v & 1;
-        if (tid == 0 && v + 1 < V) issue(v + 1, buf ^ 1);
-        if (!dd_mbar_wait(&bar[buf], ph.parity(buf))) abort_flag = 1;
-        ph.flip(buf);
-        __syncthreads();
-        if (abort_flag) {
-            // view v's copies (not waited for) and view v + 1's may be in flight
-            if (tid == 0) dd_mbar_drain(&bar[buf], ph.parity(buf) ^ 1u);
-            inflight = (v + 1 < V) ? (buf ^ 1) : -1;
-            break;
-        }
-        const DdView2 vw = views[v];
-        const float view = angles[v];
-        const float *dpv = dp + (size_t)v * (D + 1);
-        const float dend = (GEOM == DD_GEOM_PARA) ? 0.0f : __ldg(dpv + D);
-#pragma unroll
-        for (int q = 0; q < kLinesPerWarp; q++) {
-            const int rel = warp + kWarps * q;
-            int line, pi;
-            if (vw.xb) {
-                line = r0 + rel;
-                pi = c0 + lane;
-                if (line >= H) continue;
-            } else {
-                line = c0 + rel;
-                pi = H - r0 - kTile + lane;
-                if (line >= W) continue;
-            }
-            const DdLine &L = recs[buf * kTile + rel];
-            const int np = L.h.npiece;
-            if (np == 0) continue;   // warp-uniform
-            const int i0 = L.h.i0, nend = L.h.nend;
-            const float bound0 = L.h.bound0;
-            const int idet0 = L.h.idet0;
-            const bool valid = (pi >= i0) && (pi < nend) && (pi >= 0);
-            const bool need_low = valid && (lane == 0 || pi == i0);
-            // image-independent geometry: boundary values and their detector positions
-            float up = bound0, low = bound0;
-            if (valid) up = dd_boundary(&L, pi, L.p[0].Q + (float)(pi - L.p[0].gb) * L.p[0].dl);
-            if (need_low && pi > i0) low = dd_boundary(&L, pi - 1, L.p[0].Q + (float)(pi - 1 - L.p[0].gb) * L.p[0].dl);
-            const float alpha = (OPK == 0) ? 1.0f : L.h.alpha;
-            float wgt = alpha;
-            if (OPK == 2 && valid) {
-                float pcx, pcy;
-                if (vw.xb) {
-                    pcx = pix_centre((float)pi + 0.5f, g.pix_x, vw.axis0);
-                    pcy = pix_centre(0.5f * (float)H - (float)line - 0.5f, g.pix_y, g.pix_yshift);
-                } else {
-                    pcx = pix_centre((float)line - 0.5f * (float)W + 0.5f, g.pix_x, g.pix_xshift);
-                    pcy = pix_centre((float)pi + 0.5f, g.pix_y, vw.axis0);
-                }
-                wgt = alpha * fan_fbp_weight<GEOM>(vw.srcx, vw.srcy, pcx, pcy, g.iso_source);
-            }
-            if (GEOM == DD_GEOM_PARA) {
-                const DdLine &Ld = drecs[buf * kTile + rel];
-                const int npd = Ld.h.npiece;
-                float *kd = kdp + warp * kBI * 32;
-                for (int b = 0; b < nb; b++) {
-                    const float Kb = npd > 0 ? piece_K(Ld, dtab + ((size_t)(b0 + b) * V + v) * rsd, lane) : 0.0f;
-                    kd[b * 32 + lane] = Kb;
-                }
-                __syncwarp();
-                int pU = 0, jU = 0, pL = 0, jL = 0;
-                float rU = 0.0f, rL = 0.0f, dlU = 0.0f, dlL = 0.0f;
-                if (npd > 0) {
-                    const float uu = fminf(fmaxf(up, bound0), Ld.h.endv);
-                    dd_locate(&Ld, uu, &pU, &jU, &rU);
-                    dlU = Ld.p[pU].dl;
-                    const float ul = fminf(fmaxf(low, bound0), Ld.h.endv);
-                    dd_locate(&Ld, ul, &pL, &jL, &rL);
-                    dlL = Ld.p[pL].dl;
-                }
-#pragma unroll
-                for (int b = 0; b < kBI; b++) {
-                    if (b >= nb) break;
-                    const float2 *t = dtab + ((size_t)(b0 + b) * V + v) * rsd;   // per image
-                    float hu = 0.0f, hl2 = 0.0f;
-                    if (npd > 0) {
-                        const float2 e = __ldg(t + jU);
-                        hu = fmaf(rU, e.y, fmaf(dlU, e.x, kd[b * 32 + pU]));
-                        if (need_low) {
-                            const float2 e2 = __ldg(t + jL);
-                            hl2 = fmaf(rL, e2.y, fmaf(dlL, e2.x, kd[b * 32 + pL]));
-                        }
-                    }
-                    float hl = __shfl_up_sync(0xffffffffu, hu, 1);
-                    if (need_low) hl = hl2;
-                    if (valid) {
-                        const float val = wgt * (hu - hl);
-                        if (vw.xb) ax[q][b] += val;
-                        else ay[q][b] += val;
-                    }
-                }
-                __syncwarp();
-            } else {
-                const float uu = fminf(fmaxf(up, bound0), dend);
-                float dkU;
-                const int kU = fan_bin(GEOM, g, vw, view, dpv, uu, idet0, &dkU);
-                const float offU = uu - dkU;
-                int kL = kU;
-                float offL = 0.0f;
-                if (need_low) {
-                    const float ul = fminf(fmaxf(low, bound0), dend);
-                    float dkL;
-                    kL = fan_bin(GEOM, g, vw, view, dpv, ul, idet0, &dkL);
-                    offL = ul - dkL;
-                }
-                const int kb = krange[2 * buf], kn = krange[2 * buf + 1];
-                const bool inU = (unsigned)(kU - kb) < (unsigned)kn;
-                const bool inL = (unsigned)(kL - kb) < (unsigned)kn;
-                const float2 *sb = stage + (size_t)buf * kBI * kStage;
-#pragma unroll
-                for (int b = 0; b < kBI; b++) {
-                    if (b >= nb) break;
-                    const float2 *t = dtab + ((size_t)(b0 + b) * V + v) * rsd;   // per image
-                    const float2 e = inU ? sb[b * kStage + (kU - kb)] : __ldg(t + kU);
-                    const float hu = fmaf(offU, e.y, e.x);
-                    float hl = __shfl_up_sync(0xffffffffu, hu, 1);
-                    if (need_low) {
-                        const float2 e2 = inL ? sb[b * kStage + (kL - kb)] : __ldg(t + kL);
-                        hl = fmaf(offL, e2.y, e2.x);
-                    }
-                    if (valid) {
-                        const float val = wgt * (hu - hl);
-                        if (vw.xb) ax[q][b] += val;
-                        else ay[q][b] += val;
-                    }
-                }
-            }
-        }
-        __syncthreads();   // buffer `buf` is refilled by the next iteration's issue
-    }
-    if (abort_flag) {
-        if (tid == 0 && inflight >= 0) dd_mbar_drain(&bar[inflight], ph.parity(inflight));
-        if (inflight >= 0) ph.flip(inflight);
-        __syncthreads();
-        return false;
-    }
-    // merge the two ownerships through shared memory (reusing the record buffers)
-    float (*tile)[kTile][kTile + 1] = reinterpret_cast<float (*)[kTile][kTile + 1]>(smem + SL.rec);
-    // (b loops unrolled over kBI: static indices keep ax / ay in registers)
-#pragma unroll
-    for (int b = 0; b < kBI; b++) {
-        if (b >= nb) break;
-#pragma unroll
-        for (int q = 0; q < kLinesPerWarp; q++) tile[b][warp + kWarps * q][lane] = ax[q][b];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < kBI; b++) {
-        if (b >= nb) break;
-#pragma unroll
-        for (int q = 0; q < kLinesPerWarp; q++) tile[b][kTile - 1 - lane][warp + kWarps * q] += ay[q][b];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < kBI; b++) {
-        if (b >= nb) break;
-#pragma unroll
-        for (int q = 0; q < kLinesPerWarp; q++) {
-            const int r = r0 + warp + kWarps * q, c = c0 + lane;
-            if (r < H && c < W) {
-                const size_t o = ((size_t)(b0 + b) * H + r) * W + c;
-                const float val = tile[b][warp + kWarps * q][lane];
-                it.out[o] = it.base ? fmaf(it.scale, val, it.base[o]) : val;
-            }
-        }
-    }
-    __syncthreads();   // the tile buffer aliases the record buffers of the next item
-    return true;
-}
-
+// An adjoint tile or line is shared by a cluster of kAdjCluster CTAs, each
+// taking a part of its views; the ranks' sums are added in rank order.
+constexpr int kAdjCluster = 4;
 
 // ---------------------------------------------------------------------------
 // Fan-beam adjoint through the adjoint map, one 32 x 32 tile by a cluster of
@@ -649,7 +392,6 @@ __device__ bool adj_tile(const dd_geom2d &g, const AdjItem &it, unsigned char *s
 // of views that walk rows on 4 lines a thread: 0.64 / 0.80 / 1.05 / 2.23 ms;
 // here 0.35 / 0.41 / 0.53 / 1.87 ms (tables included).
 // ---------------------------------------------------------------------------
-constexpr int kAdjCluster = 4;
 static_assert(kTile % kAdjCluster == 0 && kTile / kAdjCluster == kWarps, "a rank writes one row per warp");
 
 // Ranks that take the views walking rows (the others: columns), by their shares.
@@ -663,7 +405,7 @@ template <int GEOM, int OPK, int NB>   // OPK: 0 ProjTrans, 1 BackProj, 2 BackPr
 __device__ bool adj_tile_map(const dd_geom2d &g, const AdjItem &it, unsigned char *smem, DdPhases &ph) {
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const int rank = (int)cluster.block_rank();
-    const AdjSmem SL = adj_smem(GEOM);
+    const AdjSmem SL = adj_smem();
     const int V = it.V;
     const int W = g.width, H = g.height, D = g.num_det;
     const int rsd = rs_entries(D);
@@ -867,6 +609,146 @@ __device__ bool adj_tile_map(const dd_geom2d &g, const AdjItem &it, unsigned cha
     return !ab;
 }
 
+
+// ---------------------------------------------------------------------------
+// Parallel-beam adjoint, line-major.  The parallel beam's detector boundaries
+// drift per walked line (ParaDisCPU2d.cpp:76, :100: the recurrence restarts
+// at each line's first bin), so every (view, line, image) needs its own piece
+// constants of the detector table.  A cluster takes one walked line and a
+// group of images over all the views that walk its axis, each CTA a part of
+// them: it builds the line's piece constants once per view and serves all the
+// line's pixels from them, whose sums stay in shared memory.  The rows
+// (x-branch views) are written by one launch and the columns added by a
+// second.
+//
+// Bound by the chain of a view's steps (copy, piece constants, barrier, the
+// locates) for a few slices: 256^2, 180 views, both launches, 1 / 4 slices 0.26 /
+// 0.37 ms by one CTA a line, 0.17 / 0.23 ms here; by the locates where the
+// lines fill the chip by themselves: 16 slices of 512^2, 720 views, 9.3 -> 9.0.
+// ---------------------------------------------------------------------------
+struct ParaSmem {
+    int rec, drec, tab, kt, acc, bar, total;
+};
+__host__ __device__ inline ParaSmem para_smem(int D, int npix, int nb) {
+    ParaSmem s;
+    int o = 0;
+    s.rec = o; o += 2 * (int)sizeof(DdLine);
+    s.drec = o; o += 2 * (int)sizeof(DdLine);
+    s.tab = o; o += 2 * nb * rs_entries(D) * (int)sizeof(float2);
+    s.kt = o; o += nb * 32 * (int)sizeof(float);
+    s.acc = o; o += ((nb * npix + 3) & ~3) * (int)sizeof(float);
+    s.bar = o; o += 2 * (int)sizeof(uint64_t);
+    s.total = (o + 127) & ~127;
+    return s;
+}
+
+// S: laid out for at least the item's detector, line and images.
+template <int OPK>   // 0 ProjTrans, 1 BackProj
+__device__ bool adj_para_line(const dd_geom2d &g, const AdjItem &it, unsigned char *smem, const ParaSmem &S) {
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int rank = (int)cluster.block_rank();
+    const int W = g.width, H = g.height, D = g.num_det, V = it.V;
+    const int axis = it.r0, line = it.c0, b0 = it.b0, nb = it.nb;
+    const int npix = axis ? W : H;
+    const int na = it.axisv[axis ? 0 : 1];
+    const int v0 = (int)((long long)na * rank / kAdjCluster), nv = (int)((long long)na * (rank + 1) / kAdjCluster) - v0;
+    const int *vlist = it.axisv + 2 + (axis ? 0 : V) + v0;
+    const int rsd = rs_entries(D);
+    DdLine *rec = reinterpret_cast<DdLine *>(smem + S.rec);
+    DdLine *drec = reinterpret_cast<DdLine *>(smem + S.drec);
+    float2 *tabs = reinterpret_cast<float2 *>(smem + S.tab);   // [2][nb][rsd]
+    float *kt = reinterpret_cast<float *>(smem + S.kt);        // [nb][32]
+    float *accs = reinterpret_cast<float *>(smem + S.acc);     // [nb][npix]
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + S.bar);
+    __shared__ int abort_flag;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < nb * npix; i += kThreads) accs[i] = 0.0f;
+    if (tid == 0) abort_flag = 0;
+    init_bars(bar);   // synchronises the CTA
+    DdPhases ph;
+
+    const uint32_t rec_bytes = (uint32_t)sizeof(DdLine);
+    const uint32_t tab_bytes = (uint32_t)(rsd * sizeof(float2));
+    auto issue = [&](int idx, int buf) {
+        const int v = vlist[idx];
+        dd_mbar_expect_tx(&bar[buf], 2 * rec_bytes + nb * tab_bytes);
+        dd_bulk_g2s(rec + buf, it.lines + (size_t)v * it.nl + line, rec_bytes, &bar[buf]);
+        dd_bulk_g2s(drec + buf, it.dlines + (size_t)v * it.nl + line, rec_bytes, &bar[buf]);
+        for (int b = 0; b < nb; b++)
+            dd_bulk_g2s(tabs + ((size_t)buf * nb + b) * rsd, it.dtab + ((size_t)(b0 + b) * V + v) * rsd, tab_bytes,
+                        &bar[buf]);
+    };
+    const int issuer = (kWarps - 1) * 32;
+    if (tid == issuer && nv > 0) issue(0, 0);
+    for (int idx = 0; idx < nv; idx++) {
+        const int buf = idx & 1;
+        if (!dd_mbar_wait(&bar[buf], ph.parity(buf))) abort_flag = 1;
+        ph.flip(buf);
+        // past this barrier every warp has finished view idx - 1, whose
+        // buffer takes the copies of view idx + 1
+        __syncthreads();
+        if (abort_flag) {
+            // view idx's copies (the wait gave up on them) may be in flight
+            if (tid == issuer) dd_mbar_drain(&bar[buf], ph.parity(buf) ^ 1u);
+            break;
+        }
+        if (tid == issuer && idx + 1 < nv) issue(idx + 1, buf ^ 1);
+        const DdLine &L = rec[buf], &Ld = drec[buf];
+        if (L.h.npiece == 0) continue;   // the same for the whole CTA
+        const int npd = Ld.h.npiece;
+        const float2 *tb = tabs + (size_t)buf * nb * rsd;
+        for (int b = warp; b < nb; b += kWarps) kt[b * 32 + lane] = npd > 0 ? piece_K(Ld, tb + (size_t)b * rsd, lane) : 0.0f;
+        __syncthreads();
+        const int i0 = L.h.i0, nend = L.h.nend;
+        const float bound0 = L.h.bound0;
+        const float alpha = (OPK == 0) ? 1.0f : L.h.alpha;
+        // a warp takes 32 consecutive pixel boundaries (lane l: the upper
+        // boundary of pixel q0 + l - 1) and 31 pixels: each boundary is
+        // located once and neighbours difference by one shuffle
+        for (int q0 = warp * kBinsPerWarp; q0 < npix; q0 += kWarps * kBinsPerWarp) {   // warp-uniform
+            const int bi = q0 + lane - 1;   // boundary index (upper boundary of pixel bi)
+            float u = bound0;               // boundary i0 - 1 is the walk start; below it H is constant
+            if (bi >= i0 && bi < nend) u = dd_boundary(&L, bi, L.p[0].Q + (float)(bi - L.p[0].gb) * L.p[0].dl);
+            int pU = 0, jU = 0;
+            float rU = 0.0f, dlU = 0.0f;
+            if (npd > 0) {
+                dd_locate(&Ld, fminf(fmaxf(u, bound0), Ld.h.endv), &pU, &jU, &rU);
+                dlU = Ld.p[pU].dl;
+            }
+            const int pi = bi;   // the pixel this lane closes (lanes 1..31)
+            const bool valid = lane > 0 && pi < npix && pi >= i0 && pi < nend;
+#pragma unroll
+            for (int b = 0; b < kBI; b++) {
+                if (b >= nb) break;
+                float hu = 0.0f;
+                if (npd > 0) {
+                    const float2 e = tb[(size_t)b * rsd + jU];
+                    hu = fmaf(rU, e.y, fmaf(dlU, e.x, kt[b * 32 + pU]));
+                }
+                const float hl = __shfl_up_sync(0xffffffffu, hu, 1);
+                if (valid) accs[b * npix + pi] += alpha * (hu - hl);
+            }
+        }
+    }
+    cluster.sync();
+    int ab = 0;
+    for (int k = 0; k < kAdjCluster; k++) ab |= *cluster.map_shared_rank(&abort_flag, k);
+    if (!ab) {
+        const int n = nb * npix;
+        for (int i = rank * kThreads + tid; i < n; i += kAdjCluster * kThreads) {
+            const int b = i / npix, pi = i - b * npix;
+            const int r = axis ? line : H - 1 - pi, c = axis ? pi : line;
+            const size_t o = ((size_t)(b0 + b) * H + r) * W + c;
+            float val = cluster.map_shared_rank(accs, 0)[i];
+#pragma unroll
+            for (int k = 1; k < kAdjCluster; k++) val += cluster.map_shared_rank(accs, k)[i];
+            if (axis) it.out[o] = it.base ? fmaf(it.scale, val, it.base[o]) : val;
+            else it.out[o] = it.base ? fmaf(it.scale, val, it.out[o]) : it.out[o] + val;
+        }
+    }
+    cluster.sync();   // no rank leaves before the others have read its sums
+    return !ab;
+}
 
 // ---- host launchers shared by both translation units (dd2d.cu) -----------
 struct ProfRec;
