@@ -13,16 +13,20 @@
 //                                F(u) = integral of the pixel function to u;
 //   adjoint (pixel gathers):     pix_i  += H(b_i) - H(b_{i-1}),
 //                                H(u) = integral of the detector function.
-// F is evaluated from a per-line prefix table (S_j, x_j) staged in shared
-// memory by TMA bulk copies; H from a per-view prefix table of the detector
-// row.  Both are branch-free interpolations, so a warp processes 32 adjacent
-// boundaries in lock step and neighbouring lanes exchange values with one
-// shuffle.  The adjoint is a gather: no atomics, deterministic.
+// H is evaluated from a per-view prefix table of the detector row, staged in
+// shared memory by TMA bulk copies: branch-free interpolations, so a warp
+// processes 32 adjacent boundaries in lock step and neighbouring lanes
+// exchange values with one shuffle.  The adjoint is a gather: no atomics,
+// deterministic.  The forward's difference of integrals is the sum of a
+// bin's overlaps with the line's pixels, at most a few: they are taken from a
+// table of the line's boundaries, once for all the slices of a group
+// (dd2d_fwd.cuh).  One or two slices of an arc fan take F from a per-line
+// prefix table as well (dd2d_prefix.cuh).
 //
 // The pixel boundaries are deeprecon's drifted FP32 sequence
 // (`Point1Proj += PixInterval`), represented exactly by per-line binade
-// pieces (dd_geom.cuh); the integral over a drifted pixel is then
-//   F(u) = K_p + dl_p * S_j + r * x_j
+// pieces (dd_geom.cuh); an integral over drifted pixels is then
+//   K_p + dl_p * S_j + r * x_j
 // with a per-piece constant K_p computed once per line by a warp scan.
 #include <cuda_runtime.h>
 
@@ -31,6 +35,7 @@
 #include <string.h>
 
 #include "dd2d_fwd.cuh"
+#include "dd2d_prefix.cuh"
 #include "dd_trace.h"
 
 namespace dd2 {
@@ -494,6 +499,36 @@ static int launch_fwd_passes(const FwdCall &c, const float *in, int n, float *ro
     }
 }
 
+// One or two slices of an arc fan (dd2d_prefix.cuh).
+template <int NPASS, int BI>
+static int launch_prefix_as(const FwdCall &c, int B, const float *in, float2 *tx, float2 *ty, float *out) {
+    const int W = c.g->width, H = c.g->height;
+    ProfRec *pt = prof_begin(DD_KERNEL_TABLES, c.st);
+    k_tab_rows<<<(unsigned)(((size_t)B * H * 32 + 255) / 256), 256, 0, c.st>>>(in, B, H, W, tx, c.status);
+    k_tab_cols<<<B * ((W + 31) / 32), 32 * kColChunks, 0, c.st>>>(in, B, H, W, ty);
+    prof_end(pt, c.st);
+    const PrefixSmem S = prefix_smem(c.g->num_det, rs_entries(std::max(W, H)), BI);
+    auto kern = k_fwd_prefix<NPASS, BI>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
+        return DD_ERR_LAUNCH;
+    ProfRec *pr = prof_begin(DD_KERNEL_FORWARD, c.st);
+    kern<<<(unsigned)c.V * 2, kThreads, S.total, c.st>>>(*c.g, B, c.V, c.nl, c.views, c.dp, c.bcoef, c.lines, tx, ty,
+                                                         out, c.sub, c.status);
+    prof_end(pr, c.st);
+    g_launches += 3;
+    return launch_status();
+}
+template <int BI>
+static int launch_prefix(const FwdCall &c, int B, const float *in, float2 *tx, float2 *ty, float *out) {
+    switch (prefix_passes(c.g->num_det)) {
+    case 1: return launch_prefix_as<1, BI>(c, B, in, tx, ty, out);
+    case 2: return launch_prefix_as<2, BI>(c, B, in, tx, ty, out);
+    case 3: return launch_prefix_as<3, BI>(c, B, in, tx, ty, out);
+    case 4: return launch_prefix_as<4, BI>(c, B, in, tx, ty, out);
+    default: return launch_prefix_as<8, BI>(c, B, in, tx, ty, out);
+    }
+}
+
 // Slices per CTA: 8 share a line's overlaps best; groups of 8, then 4 (of
 // which one may be empty), 2 or 1 for the rest.  5 to 7 left over take one
 // group of 8: about the time of two smaller ones.  No 8 where the stages of
@@ -645,6 +680,14 @@ int apply_planned(int scan, int op, const dd_geom2d *g, const void *planp, const
         c.status = status;
         c.st = st;
         if (geom == DD_GEOM_PARA) return launch_fwd<kPara>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
+        if (op == DD_OP_BPROJ_TW) return launch_fwd<kFanScaled>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
+        // (the reason stands at dd2d_prefix.cuh's head; not where the lines'
+        // tables are too long for shared memory)
+        if (geom == DD_GEOM_ARC && op == DD_OP_PROJ && B <= 2 &&
+            prefix_smem(g->num_det, rs_entries(std::max(g->width, g->height)), B).total <= max_smem_optin()) {
+            float2 *tx = (float2 *)(wb + A.tabx), *ty = (float2 *)(wb + A.taby);
+            return B == 1 ? launch_prefix<1>(c, B, in, tx, ty, out) : launch_prefix<2>(c, B, in, tx, ty, out);
+        }
         if (op != DD_OP_PROJ) return launch_fwd<kFanScaled>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
         return launch_fwd<kFan>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
     }

@@ -5,11 +5,12 @@
 // The reference has no batching beyond folding the batch into gridDim.x with
 // one uniform geometry per call (ParaDisCUDA2d.cu:334-337); here every
 // instance's geometry plan lives in one plan buffer, the work of all
-// instances is cut into items (forward: one view x a group of slices;
-// adjoint: one 32x32 tile x a group of slices), and a persistent grid of
-// `ctas_per_sm` CTAs per SM pulls items from a device counter in
-// longest-first order.  The item bodies are the single-geometry ones
-// (dd2d_kernels.cuh), so results are identical to per-instance calls.
+// instances is cut into items, longest first: forward, one view x a group of
+// slices, pulled from a device counter by a persistent grid; adjoint, one
+// 32x32 tile (parallel beam: one image line) x a group of slices, a cluster
+// each.  The adjoint's item bodies are the single-geometry ones
+// (dd2d_kernels.cuh), so its results are identical to per-instance calls; the
+// forward's sum the same overlaps (dd2d_fwd.cuh).
 //
 // The data-consistency step x <- x - eta * A^T (A x - y) is four launches:
 // image tables, forward items writing the residual A x - y directly, detector

@@ -26,7 +26,7 @@
 // buffer: two calls whose work overlaps on the GPU (different streams, or
 // different host threads, without ordering between them) race on it and
 // produce garbage.  Each call rewrites everything it reads from the buffer
-// (geometry plan, prefix tables, and a zeroed status word), so nothing left
+// (geometry plan, image or detector tables, and a zeroed status word), so nothing left
 // by the previous call leaks into the next.
 #include <cuda_runtime.h>
 
