@@ -88,9 +88,9 @@ def test_uneven_batch_of_many_slices(scan):
         assert torch.equal(b, p.projection_t(r, a))
 
 
-def _check3d(oracle_mod, geom, op, W, H, dep, cols, rows, V, B, cell=1.5, pz=1.0, row=1.5):
-    col = cell * 2 * (1.0 if geom == "cone_flat" else 1.0 / 600)
-    opt = [W, H, dep, cols, rows, 1.0, 1.1, pz, col, row, 300.0, 600.0, 0.3, -0.2]
+def _check3d(oracle_mod, geom, op, W, H, dep, cols, rows, V, B, cell=1.5, pz=1.0, row=1.5, sid=300.0):
+    col = cell * 2 * (1.0 if geom == "cone_flat" else 0.5 / sid)
+    opt = [W, H, dep, cols, rows, 1.0, 1.1, pz, col, row, sid, 2 * sid, 0.3, -0.2]
     opt += [0.1 * col, 0.3] if geom == "spiral" else [0.4, 0.1 * col, 0.3]
     opt = np.array(opt, np.float32)
     ang = _turn(V).astype(np.float32)
@@ -123,5 +123,19 @@ def test_forward3d_columns_and_windows(oracle_mod, geom, op, B, W, H, dep, cols,
 @pytest.mark.parametrize("geom,op", [("cone_arc", "proj_t"), ("spiral", "bproj_w")])
 def test_adjoint3d_slabs(oracle_mod, geom, op, W, H, dep, B):
     big = W > 100
-    # the large ones with a far source's scaling of the volume, few views
-    _check3d(oracle_mod, geom, op, W, H, dep, 300 if big else 80, 24, 2 if big else 7, B, cell=0.8 if big else 1.5)
+    # the source outside the volume; few views of the large ones
+    _check3d(oracle_mod, geom, op, W, H, dep, 300 if big else 80, 24, 2 if big else 7, B, sid=600.0 if big else 300.0)
+
+
+# steps of 4 bins and 4 outputs and their remainders, groups of 4 rows, more
+# outputs than a CTA's threads take at a time.  A sum of D terms in sequence
+# rounds D partial sums that grow like a random walk: 2^-24 sqrt(D / 2) of it.
+@pytest.mark.parametrize("D", [1, 2, 3, 4, 5, 7, 127, 128, 1023, 1025, 4098])
+@pytest.mark.parametrize("rows", [1, 3, 4, 5])
+def test_filter_steps(D, rows):
+    from pridediff_gb300 import fbp
+    rng = np.random.default_rng(D + rows)
+    x, w, taps = (rng.standard_normal(s).astype(np.float32) for s in ((rows, D), (1, D), 2 * D - 1))
+    out = fbp.FbpFilter.apply(*(torch.from_numpy(a).cuda() for a in (x, w, taps)))
+    ref = np.stack([np.convolve(r, taps[::-1].astype(np.float64))[D - 1:2 * D - 1] for r in (x * w).astype(np.float64)])
+    assert rel_l2(out.cpu().numpy(), ref) <= max(5e-7, 6e-8 * (D / 2) ** 0.5)
