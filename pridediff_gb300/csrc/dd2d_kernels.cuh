@@ -105,7 +105,8 @@ inline ApplyLayout apply_layout(int op, const dd_geom2d *g, int B, int V) {
     size_t o = 0;
     L.tabx = L.taby = L.dtab = 0;
     if (op_is_forward(op)) {
-        // the planes of rows and columns (8 bytes a pixel hold any grouping of the slices)
+        // the planes of rows and columns (8 bytes a pixel hold any grouping of
+        // the slices), or their prefix tables
         L.tabx = o; o = align_up(o + sizeof(float2) * (size_t)B * g->height * rs_entries(g->width), 256);
         L.taby = o; o = align_up(o + sizeof(float2) * (size_t)B * g->width * rs_entries(g->height), 256);
     } else {

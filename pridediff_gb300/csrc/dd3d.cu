@@ -387,7 +387,7 @@ __device__ __noinline__ typename Vox<NB>::T column_sum3(const Fwd3Args &a, const
 // kStage3 stages; full / empty mbarriers order them and the consumer warps,
 // which run apart by up to a stage (no CTA barrier in the loop).
 //
-// Bound by instruction issue, about 3,400 per line and CTA (63 % of the issue
+// Bound by instruction issue, about 3,400 per line and CTA (58 % of the issue
 // slots; a third of them the producers').  With every row's slices walked and
 // each of its segments' voxels gathered from global memory it was about four
 // times that.  2 x 256^3 cone beam, 36 views: 12.9 -> 4.1 ms; one 512 x 512 x
