@@ -226,7 +226,10 @@ def _apply2d(scan: str, op: str, x: torch.Tensor, options, angles: torch.Tensor)
             return lib.dd2d_apply_planned_tuned(sc, opc, g, plan.data_ptr(), x.data_ptr(), out.data_ptr(), B * C,
                                                 V, ws.data_ptr(), nbytes, forward_tune(cfg),
                                                 _stream_ptr(x.device))
-        cfg = forward_shape(sc, g, B * C, V, x.device, run, fields) if image_in else None
+        # one or two arc slices are projected in one shape: nothing to choose
+        # (and no choice to leave to the geometry's other operators)
+        one_shape = scan == "arc" and op == "proj" and B * C <= 2
+        cfg = forward_shape(sc, g, B * C, V, x.device, run, fields) if image_in and not one_shape else None
         st = run(cfg)
     N.check(st, f"{scan} {op}")
     return out
