@@ -680,7 +680,7 @@ int apply_planned(int scan, int op, const dd_geom2d *g, const void *planp, const
         c.status = status;
         c.st = st;
         if (geom == DD_GEOM_PARA) return launch_fwd<kPara>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
-        if (op == DD_OP_BPROJ_TW) return launch_fwd<kFanScaled>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
+        if (op == DD_OP_BPROJ_TW) return launch_fwd<kFanWeighted>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
         // (the reason stands at dd2d_prefix.cuh's head; not where the lines'
         // tables are too long for shared memory)
         if (geom == DD_GEOM_ARC && op == DD_OP_PROJ && B <= 2 &&

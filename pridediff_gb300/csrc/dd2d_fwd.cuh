@@ -49,9 +49,10 @@ __host__ __device__ constexpr int fwd_threads(int nb) { return (kCons + prods(nb
 static_assert(prods(1) <= stages(1) && prods(2) <= stages(2) && prods(4) <= stages(4) && prods(8) <= stages(8),
               "a producer must not wait for a stage two uses ahead of the consumers");
 
-// Proj of a fan beam; the DD back-projector's transposes of a fan beam (parts
-// scaled per line, and per pixel where weighted); the parallel beam.
-enum { kFan = 0, kFanScaled = 1, kPara = 2 };
+// Proj of a fan beam; the weighted DD back-projector's transpose of a fan beam
+// (parts scaled per line and pixel); the parallel beam; the unweighted
+// transpose of a fan beam (parts scaled per line).
+enum { kFan = 0, kFanWeighted = 1, kPara = 2, kFanScaled = 3 };
 
 // Passes over the detector, rounded up to the instantiated classes (the
 // accumulators of a thread are NPASS x NB).
@@ -247,7 +248,6 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
     auto line_of = [&](int i) { return CL > 1 ? 2 * i + rank : i < half ? 2 * i : 2 * (i - half) + 1; };
     float *red = reinterpret_cast<float *>(smem + L.red);
     const int npass = (D + kBins - 1) / kBins;
-    const bool weighted = op == DD_OP_BPROJ_TW;
     Slices<NB> acc[NPASS];
 #pragma unroll
     for (int m = 0; m < NPASS; m++) acc[m].clear();
@@ -352,7 +352,7 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
                 const float *dt = reinterpret_cast<const float *>(smem + L.det + st * L.det_b) + kB0;
                 const float *pix = reinterpret_cast<const float *>(smem + L.pix + st * L.pix_b);
                 float lpos = 0.0f;
-                if (KIND == kFanScaled && weighted) {
+                if (KIND == kFanWeighted) {
                     const int line = line_of(i);
                     lpos = xb ? pix_centre(0.5f * (float)g.height - (float)line - 0.5f, g.pix_y, g.pix_yshift)
                               : pix_centre((float)line - 0.5f * (float)g.width + 0.5f, g.pix_x, g.pix_xshift);
@@ -380,7 +380,7 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
                     auto add = [&](float w, int i) {   // a part of pixel j + i
                         if (!(w > 0.0f)) return;
                         if (KIND != kFan) w *= h1.w;
-                        if (KIND == kFanScaled && weighted) {
+                        if (KIND == kFanWeighted) {
                             const float pc = pix_centre((float)(j + i) + 0.5f, xb ? g.pix_x : g.pix_y, vwp->axis0);
                             const float cx = xb ? pc : lpos, cy = xb ? lpos : pc;
                             w *= geom == DD_GEOM_ARC
