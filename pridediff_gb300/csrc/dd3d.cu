@@ -1291,7 +1291,10 @@ int launch_fwd_rows(Fwd3Args a, int ngroups, cudaStream_t st) {
 
 // Rows per thread: 8, 4 or 2, whichever leaves least work for rows that do not
 // exist -- a step costs a thread its rows plus about 2.5 rows' worth of
-// finding the first slice and of its share of the producers.
+// finding the first slice and of its share of the producers -- or for SMs that
+// get no CTA: where CTAs do not fill the chip (3 per SM with one volume, 2 with
+// two) fewer rows are more CTAs.  128 x 128 x 64, 24 views, 200 x 64 cells, 1 /
+// 2 / 3 volumes: 0.60 / 0.54 / 1.15 ms with 8 rows, 0.18 / 0.26 / 0.44 with 4.
 template <int NB>
 int launch_fwd_volumes(Fwd3Args a, int b0, int ngroups, cudaStream_t st) {
     if (ngroups <= 0) return DD_OK;
@@ -1299,7 +1302,8 @@ int launch_fwd_volumes(Fwd3Args a, int b0, int ngroups, cudaStream_t st) {
     a.volx += (size_t)b0 * a.g.depth * a.g.height * pad4(a.g.width);
     a.volt += (size_t)b0 * a.g.depth * a.g.width * pad4(a.g.height);
     const int R = a.g.num_row;
-    auto cost = [&](int rr) { return ((R + rr * kCons3 - 1) / (rr * kCons3)) * (rr + 2.5); };
+    const double full = 152.0 * kFwdMin3<NB>, per_block = (double)((a.g.num_col + kFC - 1) / kFC) * a.V * ngroups;
+    auto cost = [&](int rr) { return std::max(((R + rr * kCons3 - 1) / (rr * kCons3)) * per_block, full) * (rr + 2.5); };
     const double c8 = cost(8), c4 = cost(4), c2 = cost(2);
     if (c8 <= c4 && c8 <= c2) return launch_fwd_rows<NB, 8>(a, ngroups, st);
     if (c4 <= c2) return launch_fwd_rows<NB, 4>(a, ngroups, st);
