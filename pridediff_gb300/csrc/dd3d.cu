@@ -1295,6 +1295,10 @@ int launch_fwd_rows(Fwd3Args a, int ngroups, cudaStream_t st) {
 // get no CTA: where CTAs do not fill the chip (3 per SM with one volume, 2 with
 // two) fewer rows are more CTAs.  128 x 128 x 64, 24 views, 200 x 64 cells, 1 /
 // 2 / 3 volumes: 0.60 / 0.54 / 1.15 ms with 8 rows, 0.18 / 0.26 / 0.44 with 4.
+// Rows that meet more slices than a step holds take each line in parts, without
+// the usual path's registers: at least twice the time.  224 x 224 x 200, 60
+// views, 300 x 180 cells, 1 / 2 volumes: 6.7 / 7.2 ms with 8 rows, 2.1 / 2.8
+// with 4.
 template <int NB>
 int launch_fwd_volumes(Fwd3Args a, int b0, int ngroups, cudaStream_t st) {
     if (ngroups <= 0) return DD_OK;
@@ -1303,7 +1307,14 @@ int launch_fwd_volumes(Fwd3Args a, int b0, int ngroups, cudaStream_t st) {
     a.volt += (size_t)b0 * a.g.depth * a.g.width * pad4(a.g.height);
     const int R = a.g.num_row;
     const double full = 152.0 * kFwdMin3<NB>, per_block = (double)((a.g.num_col + kFC - 1) / kFC) * a.V * ngroups;
-    auto cost = [&](int rr) { return std::max(((R + rr * kCons3 - 1) / (rr * kCons3)) * per_block, full) * (rr + 2.5); };
+    // slices the rows of a CTA meet on the farthest line
+    const double row_slices = a.g.row_size * (a.g.iso_source + 0.6 * std::max(a.g.width * a.g.pix_x, a.g.height * a.g.pix_y)) /
+                              (a.g.source_detector * a.g.pix_z);
+    auto cost = [&](int rr) {
+        const double blocks = std::max(((R + rr * kCons3 - 1) / (rr * kCons3)) * per_block, full);
+        const bool parts = a.g.depth > kZW && std::min(R, rr * kCons3) * row_slices + 4 > kZW;
+        return blocks * (rr + 2.5) * (parts ? 2 : 1);
+    };
     const double c8 = cost(8), c4 = cost(4), c2 = cost(2);
     if (c8 <= c4 && c8 <= c2) return launch_fwd_rows<NB, 8>(a, ngroups, st);
     if (c4 <= c2) return launch_fwd_rows<NB, 4>(a, ngroups, st);

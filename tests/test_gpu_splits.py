@@ -118,6 +118,13 @@ def test_forward3d_columns_and_windows(oracle_mod, geom, op, B, W, H, dep, cols,
     _check3d(oracle_mod, geom, op, W, H, dep, cols, 20, 4, B, cell, pz)
 
 
+# 64 rows that meet more slices than a step holds, 32 that do not
+@pytest.mark.parametrize("rows", [33, 64, 65])
+@pytest.mark.parametrize("geom,op,B", [("cone_flat", "proj", 1), ("cone_arc", "bproj_tw", 2), ("spiral", "proj", 2)])
+def test_forward3d_rows_of_many_slices(oracle_mod, geom, op, B, rows):
+    _check3d(oracle_mod, geom, op, 37, 44, 90, 45, rows, 5, B, pz=0.5, row=1.5)
+
+
 # 16 slices a thread from 912 (tile, slab) CTAs on: 512 x 512 x 50 is past it
 @pytest.mark.parametrize("W,H,dep,B", [(33, 40, 7, 3), (65, 31, 17, 1), (512, 512, 50, 1), (512, 512, 49, 3)])
 @pytest.mark.parametrize("geom,op", [("cone_arc", "proj_t"), ("spiral", "bproj_w")])
