@@ -157,6 +157,7 @@ DD_HD float dd_from_mant(int m, int e) {
 // ---------------------------------------------------------------------------
 // Piece builder: the drifted sequence b_{i+1} = fl(b_i + pint) for
 // i = i0 .. nend-1, starting from b_{i0} = v0.  Returns the number of pieces.
+// For pint > 0 their last boundaries gb ascend within [i0, nend - 1].
 // ---------------------------------------------------------------------------
 DD_HD int dd_build_pieces(float v0, float pint, int i0, int nend, DdPiece *P, int *flags) {
     int np = 0;
@@ -201,9 +202,10 @@ DD_HD int dd_build_pieces(float v0, float pint, int i0, int nend, DdPiece *P, in
         // constant increment from x1 on (round-to-even ties settle after one step)
         const int e = dd_fexp(x1);
         const int M1 = dd_mant(x1);
-        const int Dm = dd_mant(x2) - M1;          // increment in ulps (> 0)
+        const int Dm = dd_mant(x2) - M1;          // increment in ulps (>= 0)
         long long k;
-        if (M1 > 0) k = ((long long)(1 << 24) - 1 - M1) / Dm;   // stay below 2^(e+1)
+        if (Dm <= 0) k = last - (i + 1);          // below half an ulp: the walk stands still here
+        else if (M1 > 0) k = ((long long)(1 << 24) - 1 - M1) / Dm;   // stay below 2^(e+1)
         else k = ((long long)(-(1 << 23)) - M1) / Dm;            // stay at or below -2^e
         if (k > (long long)(last - (i + 1))) k = last - (i + 1);
         const int MQ = M1 + (int)k * Dm;

@@ -203,12 +203,16 @@ DD_HD void dd_line2_setup(int geom, const dd_geom2d *g, float view, const DdView
     if (geom == DD_GEOM_PARA) h.alpha = FDIV(g->det_size, pint);
     else if (geom == DD_GEOM_FLAT) h.alpha = FDIV(FMUL(FDIV(g->iso_source, g->source_detector), g->det_size), pint);
     else h.alpha = FDIV(FMUL(g->iso_source, g->det_size), pint);
-    if (i0 >= npix || idet0 >= D) {
+    // first upper boundary: (idxcol + 1) * PixInterval + Point0Proj
+    const float b0 = i0 < npix ? FADD(FMUL((float)(i0 + 1), pint), p0) : 0.0f;
+    // A fan-beam line level with the source or behind it (the source inside
+    // the image's rectangle) has no ascending boundaries: it meets nothing.
+    // Its record must not keep runs whose indices lie outside the line.
+    const bool ahead = pint > 0.0f && FSUB(pint, pint) == 0.0f && FSUB(b0, b0) == 0.0f;
+    if (i0 >= npix || idet0 >= D || !ahead) {
         h.npiece = 0;
         h.endv = bound0;
     } else {
-        // first upper boundary: (idxcol + 1) * PixInterval + Point0Proj
-        const float b0 = FADD(FMUL((float)(i0 + 1), pint), p0);
         int fl = 0;
         h.npiece = dd_build_pieces(b0, pint, i0, npix, L->p, &fl);
         h.flags = fl;
