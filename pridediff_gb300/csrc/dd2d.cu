@@ -534,6 +534,7 @@ static int launch_prefix(const FwdCall &c, int B, const float *in, float2 *tx, f
 // group of 8: about the time of two smaller ones.  No 8 where the stages of
 // three lines would leave room for one CTA per SM only (lines of more than
 // about 1,000 pixels) or the detector needs 8 passes (the sums' registers).
+// 4 or 2 where they fit; one slice always does (4,096 pixels, 1,984 cells).
 template <int KIND>
 static int launch_fwd(FwdCall c, bool single, int B, const float *in, char *rows, char *cols, float *out) {
     const int W = c.g->width, H = c.g->height, D = c.g->num_det, npix = std::max(W, H);
@@ -543,8 +544,9 @@ static int launch_fwd(FwdCall c, bool single, int B, const float *in, char *rows
     if (!single) {
         const int limit = max_smem_optin();
         big = pass_class(D) <= 4 && fwd_lay(KIND == kPara, D, npix, 8, c.cl).total <= limit / 2 ? 8
-              : fwd_lay(KIND == kPara, D, npix, 4, c.cl).total <= limit                         ? 4
-                                                                                                : 2;
+              : fwd_fits(KIND == kPara, D, npix, 4, c.cl, limit)                                ? 4
+              : fwd_fits(KIND == kPara, D, npix, 2, c.cl, limit)                                ? 2
+                                                                                                : 1;
     }
     int done = 0;
     while (done < B) {

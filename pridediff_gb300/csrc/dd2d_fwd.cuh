@@ -80,6 +80,7 @@ struct FwdLay {
     int ks;                    // stages: stages(nb), or as many as fit
 };
 constexpr int kSmemMax = 227 * 1024;
+constexpr int kFwdStatic = 512;   // of which the kernels' static arrays take no more than this
 // boundary e of a line sits at entry e + kB0 of its table
 constexpr int kB0 = 4;
 __host__ __device__ inline FwdLay fwd_lay(bool para, int D, int npix, int nb, int cl) {
@@ -90,7 +91,7 @@ __host__ __device__ inline FwdLay fwd_lay(bool para, int D, int npix, int nb, in
     s.pix_b = nb / p * plane_pitch(npix, p) * p * (int)sizeof(float);
     int o = 0;
     const int kP = prods(nb), red = pass_class(D) * nb * kCons * 32 * (int)sizeof(float);
-    const int fixed = (para ? 2 : 1) * kP * kRecs * (int)sizeof(DdLine) + (2 * stages(nb) + kRecs * kP) * 8 + 512;
+    const int fixed = (para ? 2 : 1) * kP * kRecs * (int)sizeof(DdLine) + (2 * stages(nb) + kRecs * kP) * 8 + kFwdStatic;
     int kS = stages(nb);
     while (kS > kP && fixed + kS * (s.bnd_b + s.det_b + s.pix_b + 32) + (cl == 1 ? red : 0) > kSmemMax) kS--;
     s.ks = kS;
@@ -108,6 +109,11 @@ __host__ __device__ inline FwdLay fwd_lay(bool para, int D, int npix, int nb, in
     if (cl == 1) o += red;
     s.total = (o + 127) & ~127;
     return s;
+}
+
+// Do NB slices side by side fit a CTA?
+inline bool fwd_fits(bool para, int D, int npix, int nb, int cl, int limit) {
+    return fwd_lay(para, D, npix, nb, cl).total + kFwdStatic <= limit;
 }
 
 struct FwdItem {

@@ -44,3 +44,40 @@ def test_source_inside_the_image(oracle_mod, geom, op, B, view):
     lhs, rhs = float((out.astype(np.float64) * y).sum()), float((x * b.astype(np.float64)).sum())
     # each side's FP32 sums: some 30 roundings of 2^-24 of the magnitudes, on either
     assert abs(lhs - rhs) <= 5e-6 * float(np.abs(out.astype(np.float64) * y).sum())
+
+
+def _apply(scan, op, opt, ang, x, slices, cluster):
+    """One call through the C ABI with a forward shape asked for."""
+    import ctypes
+    from pridediff_gb300 import _native as N
+    from pridediff_gb300 import radontorch as R
+    lib, g = N.load(), N.geom2d(opt)
+    a = torch.from_numpy(np.asarray(ang, np.float32)).cuda()
+    xt = torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    B, V, sc, opc = x.shape[0], len(ang), N.SCAN2D[scan], N.OPS[op]
+    out = torch.full((B, V, g.num_det), np.nan, device="cuda")
+    plan = R.plan2d(scan, g, a)
+    n = lib.dd2d_apply_workspace_bytes(sc, opc, g, B, V)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    t = R.forward_tune(dict(fwd_slices=slices, fwd_cluster=cluster))
+    N.check(lib.dd2d_apply_planned_tuned(sc, opc, g, plan.data_ptr(), xt.data_ptr(), out.data_ptr(), B, V, ws.data_ptr(),
+                                         n, ctypes.byref(t), R._stream_ptr(a.device)), f"{scan} {op}")
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+# Lines of which 8, 4, 2 or 1 slices fit a CTA: about 1,000, 2,750 (2,490 of
+# the parallel beam with a full detector) and 3,430 pixels, the last only with
+# the sums of a single CTA.
+@pytest.mark.parametrize("W,D", [(1080, 700), (2480, 1984), (2790, 300), (3450, 1984), (3465, 1900), (4096, 1984)])
+@pytest.mark.parametrize("scan,B", [("para", 1), ("para", 2), ("para", 3), ("flat", 9)])
+def test_long_lines_in_every_shape(oracle_mod, scan, B, W, D):
+    pix = 0.7 * 1080 / W
+    opt = [W, 3, D, pix, pix, {"para": 1.0, "flat": 1085.6 / 595.0}[scan] * 1.1 * W * pix / D, 595.0, 1085.6, 0.1, -0.2, 0.1]
+    ang = np.array([0.2, 1.4, 3.3], np.float32)
+    x = np.random.default_rng(W + B).random((B, 3, W), dtype=np.float32)
+    ref = oracle_mod.run2d(scan, "proj", x, ang, opt, nthreads=8)
+    out = [_apply(scan, "proj", opt, ang, x, s, c) for s in (4, 1) for c in (2, 1)] + [run2d(scan, "proj", x, ang, opt)]
+    assert rel_l2(out[0], ref) <= 1e-5
+    for o in out[1:]:
+        assert np.array_equal(o, out[0])
