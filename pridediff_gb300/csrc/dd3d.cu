@@ -781,20 +781,21 @@ struct Adj3Args {
     int *status;
     int B, V, ntx;
     int b0, family;      // first volume of the launch; operator family (dd3_coef)
+    int bufs;            // buffers of staged units: 3, or 2 (adj3_smem)
 };
 
-// Shared memory of the adjoint kernel: kAdj3Bufs buffers of one (view, walk
-// block)'s data (the records of the tile's 16 lines, the block's column
-// boundary and magnification tables, the row table, the lines' z quantities
-// and the view record), each moved by bulk copies; all sizes are multiples of
-// 16 bytes.
+// Shared memory of the adjoint kernel: buffers of one (view, walk block)'s data
+// (the records of the tile's 16 lines, the block's column boundary and
+// magnification tables, the row table, the lines' z quantities and the view
+// record), each moved by bulk copies; all sizes are multiples of 16 bytes.
+// kAdj3Bufs of them, or 2 where 3 row tables (8 bytes a row) do not fit.
 constexpr int kAdj3Bufs = 3;
 struct Adj3Smem {
     int rec, dp, mag, rz, lz, vw, bar, total;
     uint32_t rec_b, dp_b, mag_b, rz_b, lz_b;
 };
 
-__host__ __device__ inline Adj3Smem adj3_smem(const PlanLayout &P) {
+__host__ __device__ inline Adj3Smem adj3_smem(const PlanLayout &P, int bufs) {
     Adj3Smem s;
     s.rec_b = (uint32_t)(kTile * sizeof(DdLine));
     s.dp_b = (uint32_t)((DD3_CHUNK + 4) * sizeof(float));
@@ -802,19 +803,20 @@ __host__ __device__ inline Adj3Smem adj3_smem(const PlanLayout &P) {
     s.rz_b = (uint32_t)(P.srz * sizeof(float));
     s.lz_b = (uint32_t)(kTile * sizeof(float4));
     int o = 0;
-    s.rec = o; o += kAdj3Bufs * (int)s.rec_b;
-    s.dp = o; o += kAdj3Bufs * (int)s.dp_b;
-    s.mag = o; o += kAdj3Bufs * (int)s.mag_b;
-    s.rz = o; o += kAdj3Bufs * (int)s.rz_b;
-    s.lz = o; o += kAdj3Bufs * (int)s.lz_b;
-    s.vw = o; o += kAdj3Bufs * (int)sizeof(DdView3);
-    s.bar = o; o += kAdj3Bufs * (int)sizeof(uint64_t);
+    s.rec = o; o += bufs * (int)s.rec_b;
+    s.dp = o; o += bufs * (int)s.dp_b;
+    s.mag = o; o += bufs * (int)s.mag_b;
+    s.rz = o; o += bufs * (int)s.rz_b;
+    s.lz = o; o += bufs * (int)s.lz_b;
+    s.vw = o; o += bufs * (int)sizeof(DdView3);
+    s.bar = o; o += bufs * (int)sizeof(uint64_t);
     s.total = (o + 127) & ~127;
     return s;
 }
 
-// The size limit of a view's tables: what two buffers of a whole view (all
-// its walk blocks) take beside 200 KB.
+// The size limit of a view's tables: what two buffers of a whole view (all its
+// walk blocks) take beside 200 KB.  Two of the adjoint's buffers, which hold one
+// block each, fit whatever passes it.
 inline bool view_too_wide(const PlanLayout &P, int R) {
     const size_t one = (size_t)kTile * P.nch * sizeof(DdLine) + sizeof(float) * ((size_t)P.sdp + P.smag + pad4(2 * R)) +
                        kTile * sizeof(float4) + sizeof(DdView3) + sizeof(uint64_t);
@@ -894,7 +896,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_adj3(const Adj3Args a) {
     const dd_geom3d &g = a.g;
     const int W = g.width, H = g.height, Dp = g.depth, C = g.num_col, R = g.num_row;
     const PlanLayout &P = a.P;
-    const Adj3Smem S = adj3_smem(P);
+    const int bufs = a.bufs;
+    const Adj3Smem S = adj3_smem(P, bufs);
     const int tid = threadIdx.x, lane = tid & 31;
     const int tX = blockIdx.x % a.ntx, tY = blockIdx.x / a.ntx;
     const int xlo = tX * kTile, ylo = tY * kTile;
@@ -915,7 +918,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_adj3(const Adj3Args a) {
 
     if (tid == 0) {
         abort_flag = 0;
-        for (int i = 0; i < kAdj3Bufs; i++) dd_mbar_init(&bar[i], 1);
+        for (int i = 0; i < bufs; i++) dd_mbar_init(&bar[i], 1);
         dd_fence_mbar_init();
     }
     __syncthreads();
@@ -1043,35 +1046,36 @@ __global__ void __launch_bounds__(kThreads, 3) k_adj3(const Adj3Args a) {
     for (int q = 0; q < ZS; q++) acc[q] = VT::zero();
 
     DdPhases ph;
-    // unit i uses buffer i % 3; units i + 1 and i + 2 are in flight behind it
+    // unit i uses buffer i % bufs; the bufs - 1 units behind it are in flight
+    const int ahead = bufs - 1;
     if (tid < 32) {
         next(&units[0]);
-        next(&units[1]);
+        if (ahead > 1) next(&units[1]);
         if (tid == 0) {
             if (units[0].v >= 0) issue(units[0].v, units[0].cc, 0);
-            if (units[1].v >= 0) issue(units[1].v, units[1].cc, 1);
+            if (ahead > 1 && units[1].v >= 0) issue(units[1].v, units[1].cc, 1);
         }
     }
     __syncthreads();
     int buf = 0;
-    for (int i = 0; units[i & 3].v >= 0; i++, buf = buf == 2 ? 0 : buf + 1) {
-        const int buf2 = buf == 0 ? 2 : buf - 1;   // buffer of unit i + 2 (and of unit i - 1)
-        // slot i + 2 was last read before the barrier of unit i - 1
-        if (tid < 32) next(&units[(i + 2) & 3]);
+    for (int i = 0; units[i & 3].v >= 0; i++, buf = buf == ahead ? 0 : buf + 1) {
+        const int buf2 = buf == 0 ? ahead : buf - 1;   // buffer of unit i + ahead (and of unit i - 1)
+        // slot i + ahead was last read before the barrier of unit i - 1
+        if (tid < 32) next(&units[(i + ahead) & 3]);
         if (!dd_mbar_wait(&bar[buf], ph.parity(buf))) abort_flag = 1;
         ph.flip(buf);
         // past this barrier every warp has finished unit i - 1
         __syncthreads();
         if (abort_flag) {
-            // this unit's copies (the wait gave up on them) and the next one's may be in flight
+            // this unit's copies (the wait gave up on them) and, of three buffers, the next one's may be in flight
             if (tid == 0) {
-                const int b1 = buf == 2 ? 0 : buf + 1;
+                const int b1 = buf == ahead ? 0 : buf + 1;
                 dd_mbar_drain(&bar[buf], ph.parity(buf) ^ 1u);
-                if (units[(i + 1) & 3].v >= 0) dd_mbar_drain(&bar[b1], ph.parity(b1));
+                if (ahead > 1 && units[(i + 1) & 3].v >= 0) dd_mbar_drain(&bar[b1], ph.parity(b1));
             }
             break;
         }
-        if (tid == 0 && units[(i + 2) & 3].v >= 0) issue(units[(i + 2) & 3].v, units[(i + 2) & 3].cc, buf2);
+        if (tid == 0 && units[(i + ahead) & 3].v >= 0) issue(units[(i + ahead) & 3].v, units[(i + ahead) & 3].cc, buf2);
         const DdView3 &w = *reinterpret_cast<const DdView3 *>(sm + S.vw + buf * (int)sizeof(DdView3));
         const int xb = w.xb;
         const int rl = xb ? (y - ylo) : (x - xlo);
@@ -1323,7 +1327,7 @@ int launch_fwd_volumes(Fwd3Args a, int b0, int ngroups, cudaStream_t st) {
 
 template <int GEOM, int NB, int ZS>
 int launch_adj_slabs(const Adj3Args &a, int ngroups, cudaStream_t st) {
-    const int smem = adj3_smem(a.P).total;
+    const int smem = adj3_smem(a.P, a.bufs).total;
     if (cudaFuncSetAttribute(k_adj3<GEOM, NB, ZS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
         return DD_ERR_LAUNCH;
     const int nty = (a.g.height + kTile - 1) / kTile;
@@ -1415,6 +1419,8 @@ int adjoint(int scan, int op, const dd_geom3d *g, const char *planb, const float
     a.ntx = (g->width + kTile - 1) / kTile;
     a.b0 = 0;
     a.family = op_family(op);
+    // (1 KB: the kernel's static arrays, which come out of the same 227 KB)
+    a.bufs = adj3_smem(a.P, kAdj3Bufs).total + 1024 <= 227 * 1024 ? kAdj3Bufs : 2;
     const int geom = geom_of(scan);
     if (geom == DD_GEOM3_CONE_FLAT) return launch_adj<DD_GEOM3_CONE_FLAT>(a, in, (float *)ss, st);
     if (geom == DD_GEOM3_CONE_ARC) return launch_adj<DD_GEOM3_CONE_ARC>(a, in, (float *)ss, st);

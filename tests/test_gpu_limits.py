@@ -7,8 +7,10 @@ import numpy as np
 import pytest
 import torch
 
+from cases3d import spiral_source
 from conftest import rel_l2
 from test_gpu_2d import run as run2d
+from test_gpu_3d import run as run3d
 
 pytestmark = pytest.mark.gpu
 
@@ -81,3 +83,22 @@ def test_long_lines_in_every_shape(oracle_mod, scan, B, W, D):
     assert rel_l2(out[0], ref) <= 1e-5
     for o in out[1:]:
         assert np.array_equal(o, out[0])
+
+
+# A row table of 8,190 to 11,300 rows: three of them do not fit the adjoint's
+# shared memory, two do.
+@pytest.mark.parametrize("rows", [8100, 8191, 9000, 11300])
+@pytest.mark.parametrize("geom,fwd,adj", [("cone_flat", "proj", "proj_t"), ("spiral", "bproj_tw", "bproj_w")])
+def test_tall_detector(oracle_mod, geom, fwd, adj, rows):
+    W, H, dep, cols, V, sid = 20, 24, 18, 12, 4, 300.0
+    col, row = 5.0 * (1.0 if geom == "cone_flat" else 0.5 / sid), 60.0 / rows
+    opt = [W, H, dep, cols, rows, 1.0, 1.1, 1.0, col, row, sid, 2 * sid, 0.3, -0.2]
+    opt = np.array(opt + ([0.1 * col, 0.3] if geom == "spiral" else [0.4, 0.1 * col, 0.3]), np.float32)
+    ang = (np.arange(V) * 2 * np.pi / V + 0.1).astype(np.float32)
+    sp = spiral_source(V, 0.5, -0.25 * V) if geom == "spiral" else None
+    rng = np.random.default_rng(rows)
+    for op, shape in ((fwd, (1, dep, H, W)), (adj, (1, V, rows, cols))):
+        x = rng.random(shape).astype(np.float32)
+        ref = oracle_mod.run3d(geom, op, x, ang, opt, source_pos=sp, nthreads=8)
+        assert np.any(ref)
+        assert rel_l2(run3d(geom, op, x, ang, opt, sp), ref) <= 5e-5
