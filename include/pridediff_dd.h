@@ -27,6 +27,10 @@
  *   rows [axial position, radius shift, angle shift, axial shift]
  *   (RadonTorch.cpp:1040-1043).
  * B is the product of the reference's batch and channel sizes.
+ *
+ * Alignment: inputs and outputs 4 bytes (a float); plans and 2-D workspaces 16
+ * bytes (bulk copies read them); 3-D workspaces any (the calls use them from
+ * their first 16-byte boundary on, within the size that the query gives).
  */
 #ifndef PRIDEDIFF_DD_H
 #define PRIDEDIFF_DD_H

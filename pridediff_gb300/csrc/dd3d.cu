@@ -104,6 +104,11 @@ inline ApplyLayout apply_layout(bool fwd, bool adj, const dd_geom3d *g, int B, i
     return L;
 }
 
+// A caller's workspace from its first 16-byte boundary on (tensor maps and the
+// paired volumes' 8-byte loads need it).  The 256 bytes of the status words,
+// which close every layout, leave room for the shift.
+inline char *ws_base(const void *ws) { return (char *)(((uintptr_t)ws + 15) & ~(uintptr_t)15); }
+
 // ---------------------------------------------------------------------------
 // Plan kernels
 // ---------------------------------------------------------------------------
@@ -1469,7 +1474,7 @@ extern "C" int dd3d_apply_planned(int scan, int op, const dd_geom3d *g, const vo
     const bool f = op_is_forward(op);
     const ApplyLayout A = apply_layout(f, !f, g, batch, num_view);
     if (!workspace || workspace_bytes < A.total) return DD_ERR_WORKSPACE;
-    char *wb = (char *)workspace;
+    char *wb = ws_base(workspace);
     cudaStream_t s = (cudaStream_t)stream;
     int *status = (int *)(wb + A.status);
     if (f) return forward(scan, op, g, (const char *)planp, in, out, nullptr, batch, num_view, wb + A.volx, wb + A.volt, status, s);
@@ -1490,10 +1495,10 @@ extern "C" int dd3d_apply(int scan, int op, const dd_geom3d *g, const float *in,
     if (!in || !out || !angles || (scan == DD_SCAN_SPIRAL && !source_pos)) return DD_ERR_INVALID_ARG;
     const size_t pb = dd3d_plan_bytes(scan, g, num_view);
     if (!workspace || workspace_bytes < dd3d_workspace_bytes(scan, op, g, batch, num_view)) return DD_ERR_WORKSPACE;
-    const int s1 = plan(scan, g, angles, source_pos, num_view, workspace, pb, (cudaStream_t)stream);
+    char *wb = ws_base(workspace);
+    const int s1 = plan(scan, g, angles, source_pos, num_view, wb, pb, (cudaStream_t)stream);
     if (s1 != DD_OK) return s1;
-    return dd3d_apply_planned(scan, op, g, workspace, in, out, batch, num_view, (char *)workspace + pb,
-                              workspace_bytes - pb, stream);
+    return dd3d_apply_planned(scan, op, g, wb, in, out, batch, num_view, wb + pb, workspace_bytes - pb, stream);
 }
 
 extern "C" size_t dd3d_dc_workspace_bytes(int scan, const dd_geom3d *g, int batch, int num_view) {
@@ -1511,7 +1516,7 @@ extern "C" int dd3d_dc_step(int scan, const dd_geom3d *g, const void *planp, flo
     if (!planp || !x || !y || !resid) return DD_ERR_INVALID_ARG;
     const ApplyLayout A = apply_layout(true, true, g, batch, num_view);
     if (!workspace || workspace_bytes < A.total) return DD_ERR_WORKSPACE;
-    char *wb = (char *)workspace;
+    char *wb = ws_base(workspace);
     cudaStream_t s = (cudaStream_t)stream;
     const char *pb = (const char *)planp;
     int *status = (int *)(wb + A.status);
@@ -1525,7 +1530,7 @@ extern "C" int dd3d_status(int scan, int op, const dd_geom3d *g, int batch, int 
     if (validate(scan, op, g, batch, num_view) != DD_OK || !workspace || !status) return DD_ERR_INVALID_ARG;
     const bool f = op_is_forward(op);
     const size_t off = dd3d_plan_bytes(scan, g, num_view) + apply_layout(f, !f, g, batch, num_view).status;
-    if (cudaMemcpy(status, (const char *)workspace + off, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+    if (cudaMemcpy(status, ws_base(workspace) + off, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
         return DD_ERR_LAUNCH;
     return DD_OK;
 }
@@ -1535,7 +1540,7 @@ extern "C" int dd3d_planned_status(int op, const dd_geom3d *g, int batch, int nu
     if (!g || batch <= 0 || num_view <= 0 || !workspace || !status) return DD_ERR_INVALID_ARG;
     const bool f = op_is_forward(op);
     const size_t off = apply_layout(f, !f, g, batch, num_view).status;
-    if (cudaMemcpy(status, (const char *)workspace + off, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+    if (cudaMemcpy(status, ws_base(workspace) + off, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
         return DD_ERR_LAUNCH;
     return DD_OK;
 }

@@ -102,3 +102,42 @@ def test_tall_detector(oracle_mod, geom, fwd, adj, rows):
         ref = oracle_mod.run3d(geom, op, x, ang, opt, source_pos=sp, nthreads=8)
         assert np.any(ref)
         assert rel_l2(run3d(geom, op, x, ang, opt, sp), ref) <= 5e-5
+
+
+# A 3-D workspace that starts on any address: every call works from its first
+# 16-byte boundary on and stays inside the bytes it asked for.
+@pytest.mark.parametrize("shift", [0, 1, 4, 8, 15])
+@pytest.mark.parametrize("op,B", [("proj", 1), ("proj", 3), ("proj_t", 1), ("proj_t", 2), ("dc", 2)])
+def test_workspace_at_any_address(op, B, shift):
+    import ctypes
+    from pridediff_gb300 import _native as N
+    from pridediff_gb300 import radontorch as R
+    lib, sc = N.load(), N.SCAN3D["cone_flat"]
+    g = N.geom3d([30, 26, 21, 40, 18, 1.0, 1.0, 1.0, 1.6, 1.6, 300.0, 600.0, 0.0, 0.0, 0.0, 0.0, 0.0])
+    V = 5
+    a = torch.arange(V, dtype=torch.float32, device="cuda") * (2 * np.pi / V)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    vol, sino = torch.rand((B, 21, 26, 30), device="cuda", generator=gen), torch.rand((B, V, 18, 40), device="cuda", generator=gen)
+    plan = R.plan3d("cone_flat", g, a)
+    n = int(lib.dd3d_dc_workspace_bytes(sc, g, B, V) if op == "dc" else
+            lib.dd3d_apply_workspace_bytes(sc, N.OPS[op], g, B, V))
+
+    def call(at):
+        buf = torch.full((n + 32,), 0xA5, dtype=torch.uint8, device="cuda")
+        st = R._stream_ptr(a.device)
+        if op == "dc":
+            x, resid = vol.clone(), torch.empty_like(sino)
+            N.check(lib.dd3d_dc_step(sc, g, plan.data_ptr(), x.data_ptr(), sino.data_ptr(), resid.data_ptr(),
+                                     ctypes.c_float(1e-4), B, V, buf.data_ptr() + at, n, st), op)
+            res = x
+        else:
+            src, res = (vol, torch.empty_like(sino)) if op == "proj" else (sino, torch.empty_like(vol))
+            N.check(lib.dd3d_apply_planned(sc, N.OPS[op], g, plan.data_ptr(), src.data_ptr(), res.data_ptr(), B, V,
+                                           buf.data_ptr() + at, n, st), op)
+            word = ctypes.c_int(-1)
+            assert lib.dd3d_planned_status(N.OPS[op], g, B, V, buf.data_ptr() + at, ctypes.byref(word)) == N.DD_OK
+            assert word.value == N.DD_OK
+        torch.cuda.synchronize()
+        assert bool((buf[:at] == 0xA5).all()) and bool((buf[at + n:] == 0xA5).all())
+        return res
+    assert torch.equal(call(shift), call(0))
