@@ -317,16 +317,18 @@ template <int NB> constexpr int kStage3 = 3;
 template <int NB> constexpr int kFwdMin3 = NB == 1 ? 3 : 2;
 // (a producer must not wait for a stage two uses ahead of the consumers)
 static_assert(kProd3<1> <= kStage3<1> && kProd3<2> <= kStage3<2>, "at least a stage per producer");
-constexpr int kSeg = 8;      // column segments of one line held in shared memory
+constexpr int kSeg = 16;     // column segments of one line held in shared memory
 constexpr int kFast = 3;     // ... and held in registers by the usual path
 constexpr int kZB = 16;      // slices of one copy
-constexpr int kZW = 62;      // most slices of a line in one step
 // pixels per slice of a tile: a CTA takes the narrowest that holds what its
-// columns meet on any line (one tensor map each)
-constexpr int kNPitch = 5;
-__host__ __device__ constexpr int pitch3(int i) { return i == 0 ? 16 : i == 1 ? 24 : i == 2 ? 32 : i == 3 ? 48 : 64; }
-// bytes of a step's voxel tile: 62 slices of 64 pixels and a neighbour at either end
-template <int NB> constexpr int kTileB3 = (kZW + 2) * 64 * 4 * NB;
+// columns meet on any line (one tensor map each); most slices of a line in one
+// step: the tile holds them and a neighbour at either end
+constexpr int kNPitch = 7, kNarrow3 = 5;
+__host__ __device__ constexpr int pitch3(int i) { return i < 3 ? 16 + 8 * i : i < 5 ? 16 * i : 32 * i - 64; }
+__host__ __device__ constexpr int zwindow3(int pitch) { return pitch <= 64 ? 62 : 30; }
+// bytes of a step's voxel tile: 64 slices of 64 pixels, 32 of 128
+constexpr int kTileSlices3 = 64;
+template <int NB> constexpr int kTileB3 = kTileSlices3 * 64 * 4 * NB;
 
 // Tensor maps of the volumes' rows and columns (k_lines_of3): {pixel x
 // volumes, line, slice, group}, boxes of one line, pitch3(i) pixels and kZB slices.
@@ -350,30 +352,12 @@ struct Fwd3Args {
 template <int NB>
 struct Step3 {
     float4 h;                   // p0z, 1 / pintz, first slice, slices (0: nothing to do)
-    int pitch, line;            // pixels per slice of the tile (0: no tile, read global memory)
+    int pitch, line;            // pixels per slice of the tile (0: no tile, the pixels are read from global memory)
     int fast, pad;              // tile present, no column with more than kFast segments, and the line in one step
-    int nseg[kFC], j0[kFC];     // per column: segments, first pixel in the tile
+    int nseg[kFC], j0[kFC];     // per column: segments (kSeg + 1: more), first pixel in the tile (on the line without one)
     float c[kSeg][kFC];         // coefficients
-    float top[kZW + 2];         // entry i: top of slice first + i - 1; +inf behind the last
+    float top[kTileSlices3];    // entry i: top of slice first + i - 1; +inf behind the last
 };
-
-// One column's sum over the pixels of a line at slice s, from global memory:
-// where a column meets more than kSeg pixels, or the 32 columns more pixels
-// than a tile holds.
-template <int NB>
-__device__ __noinline__ typename Vox<NB>::T column_sum3(const Fwd3Args &a, const DdView3 &w, const DdLine *Lg,
-                                                        const float *sdp, int lane, int kk, float lpos, float parea,
-                                                        const typename Vox<NB>::T *row) {
-    typename Vox<NB>::T x = Vox<NB>::zero();
-    DdColWalk cw;
-    if (dd3_colwalk_init(Lg, sdp, lane, kk, &cw)) {
-        int j;
-        float wd;
-        while (dd3_colwalk_next(Lg, &cw, &j, &wd))
-            x = Vox<NB>::fma(dd3_coef(a.geom, a.family, &a.g, &w, lpos, j, wd, parea), __ldg(row + j), x);
-    }
-    return x;
-}
 
 // grid: (row block x group of 32 columns inside one walk block, view, volume
 // group).  Lane = column, consumer warp w = rows r0 + RR w .. r0 + RR (w + 1) - 1.
@@ -392,14 +376,25 @@ __device__ __noinline__ typename Vox<NB>::T column_sum3(const Fwd3Args &a, const
 // kStage3 stages; full / empty mbarriers order them and the consumer warps,
 // which run apart by up to a stage (no CTA barrier in the loop).
 //
-// Bound by instruction issue, about 3,400 per line and CTA (58 % of the issue
-// slots; a third of them the producers').  With every row's slices walked and
+// Where the CTA's columns meet more pixels than its tile holds, the pixels are
+// read from global memory by the step's segments; where a column meets more
+// than kSeg, the consumers walk its record pixel by pixel.
+//
+// Bound by instruction issue (58 % of the slots, about 3,400 per line and CTA, a
+// third of them the producers') and the latency of a merge's dependent steps
+// at 30 warps an SM or fewer.  With every row's slices walked and
 // each of its segments' voxels gathered from global memory it was about four
 // times that.  2 x 256^3 cone beam, 36 views: 12.9 -> 4.1 ms; one 512 x 512 x
 // 128 volume, 96 spiral views: 12.6 -> 3.5 ms.  On the way: the sums of all
 // (column, slice) pairs formed first, lanes along z from global memory, 8.5 /
 // 10.1 ms (7,100 instructions); per-slice bulk copies instead of boxes and the
 // segments by the record walk, 5.0 / 7.2 ms.
+// Columns of several pixels, ms by gathers per row and slice / by the record
+// once per slice wherever the tile or 8 segments did not do / now: spiral,
+// 512 x 512 x 128, 64 rows, 512 columns and 180 views 18.3 / 28.0 / 7.7, 256
+// columns and 90 views 6.9 / 28.7 / 3.7; cone, 2 x 256^2 x 128, 128 rows, 60
+// views, 128 columns 4.6 / 16.3 / 2.7; one 256^2 x 64, 64 rows, 60 views, 32
+// columns 17.7 / 18.2 / 1.9, 16 columns 29.8 / 27.6 / 13.5.
 template <int NB, int RR>
 __global__ void __launch_bounds__(kFwdThreads3<NB>, kFwdMin3<NB>) k_fwd3(const __grid_constant__ Fwd3Args a, const __grid_constant__ Maps3 maps) {
     constexpr int kP = kProd3<NB>, kS = kStage3<NB>;
@@ -506,8 +501,10 @@ __global__ void __launch_bounds__(kFwdThreads3<NB>, kFwdMin3<NB>) k_fwd3(const _
         const float pm = fminf(la.z, lb.z), px = fminf(la.w / la.z, lb.w / lb.z), span = sdp[kFC] - sdp[0];
         const float widest = (pm > 0.0f && zmin < zmax) ? fminf((zmax - zmin) / pm + 4.0f, (float)Dp) : (float)Dp;
         const float npx = (pm > 0.0f && px > 0.0f && span >= 0.0f) ? span / px + (float)(2 + kAl) : 1.0e6f;
-        for (pi = 0; pi < kNPitch - 1 && npx > (float)pitch3(pi); pi++) {}
-        zstep = kZW;
+        // (tiles of more than 64 pixels only where they hold a line's slices at once)
+        const int np = widest <= (float)zwindow3(pitch3(kNPitch - 1)) ? kNPitch : kNarrow3;
+        for (pi = 0; pi < np - 1 && npx > (float)pitch3(pi); pi++) {}
+        zstep = zwindow3(pitch3(pi));
         nchunk = max(1, ((int)widest + zstep - 1) / zstep);
         nstep = nline * nchunk;
     }
@@ -613,7 +610,8 @@ __global__ void __launch_bounds__(kFwdThreads3<NB>, kFwdMin3<NB>) k_fwd3(const _
                     ns = 0;   // no column meets the line
                 } else {
                     jb = lo / kAl * kAl;
-                    pitch = (wide || hi - jb > tpitch) ? 0 : tpitch;
+                    pitch = tpitch;
+                    if (wide || hi - jb > tpitch) jb = pitch = 0;
                 }
                 fast = __all_sync(0xffffffffu, nseg <= kFast) && pitch > 0 && nchunk == 1;
                 S.nseg[lane] = nseg;
@@ -698,32 +696,60 @@ __global__ void __launch_bounds__(kFwdThreads3<NB>, kFwdMin3<NB>) k_fwd3(const _
                         }
                     }
                 } else {
-                    auto column = [&](int e) -> T {
-                        T x = VT::zero();
-                        if ((unsigned)(e - 1) < (unsigned)n) {
-                            if (pitch > 0) {
-                                for (int t = 0; t < nseg; t++) x = VT::fma(S.c[t][lane], tile[e * pitch + t], x);
-                            } else {
-                                const int line = S.line;
-                                x = column_sum3<NB>(a, w, lines + line, sdp, lane, kk,
-                                                    a.family == 2 ? dd3_line_pos_f(&g, &w, line) : 0.0f, linez[line].w,
-                                                    src + ((size_t)(first + e - 1) * nline + line) * np4);
+                    // rows and slices as above; column(e): the column's sum over entry e's pixels
+                    auto merge = [&](auto column) {
+                        int e = i;
+                        T x = column(e);
+                        float zhi = S.top[e];
+#pragma unroll
+                        for (int q = 0; q < RR; q++) {
+                            const float w0 = FSUB(fminf(rp1[q], zhi), rp0[q]);
+                            if (w0 > 0.0f) acc[q] = VT::fma(w0, x, acc[q]);
+                            while (zhi < rp1[q]) {
+                                const float lo = fmaxf(zhi, rp0[q]);
+                                x = column(++e);
+                                zhi = S.top[e];
+                                const float w1 = FSUB(fminf(rp1[q], zhi), lo);
+                                if (w1 > 0.0f) acc[q] = VT::fma(w1, x, acc[q]);
                             }
                         }
-                        return x;
                     };
-                    T x = column(i);
-                    float zhi = *zp;
+                    const int line = S.line;
+                    const T *__restrict__ rows = src + ((size_t)(first - 1) * nline + line) * np4;   // entry 0's row
+                    const size_t slice = (size_t)nline * np4;
+                    if (nseg <= kSeg) {
+                        const float *cs = &S.c[0][lane];
+                        merge([&](int e) -> T {
+                            T x = VT::zero();
+                            if ((unsigned)(e - 1) >= (unsigned)n) return x;
+                            if (pitch > 0) {
+                                for (int t = 0; t < nseg; t++) x = VT::fma(cs[t * kFC], tile[e * pitch + t], x);
+                                return x;
+                            }
+                            const T *__restrict__ r = rows + e * slice + S.j0[lane];
+                            for (int t = 0; t < nseg; t += 4) {   // four loads in flight
+                                T v[4];
 #pragma unroll
-                    for (int q = 0; q < RR; q++) {
-                        const float w0 = FSUB(fminf(rp1[q], zhi), rp0[q]);
-                        if (w0 > 0.0f) acc[q] = VT::fma(w0, x, acc[q]);
-                        while (zhi < rp1[q]) {
-                            const float lo = fmaxf(zhi, rp0[q]);
-                            x = column(++i);
-                            zhi = S.top[i];
-                            const float w1 = FSUB(fminf(rp1[q], zhi), lo);
-                            if (w1 > 0.0f) acc[q] = VT::fma(w1, x, acc[q]);
+                                for (int q = 0; q < 4; q++) v[q] = t + q < nseg ? __ldg(r + t + q) : VT::zero();
+#pragma unroll
+                                for (int q = 0; q < 4; q++)
+                                    if (t + q < nseg) x = VT::fma(cs[(t + q) * kFC], v[q], x);
+                            }
+                            return x;
+                        });
+                    } else {   // more pixels than that: by the record, pixel by pixel
+                        const DdLine *Lg = lines + line;
+                        const float lpos = a.family == 2 ? dd3_line_pos_f(&g, &w, line) : 0.0f, parea = linez[line].w;
+                        DdColWalk cw;
+                        if (dd3_colwalk_init(Lg, sdp, lane, kk, &cw)) {
+                            int j;
+                            float wd;
+                            while (dd3_colwalk_next(Lg, &cw, &j, &wd)) {
+                                const float cf = dd3_coef(a.geom, a.family, &g, &w, lpos, j, wd, parea);
+                                merge([&](int e) -> T {
+                                    return (unsigned)(e - 1) < (unsigned)n ? VT::fma(cf, __ldg(rows + e * slice + j), VT::zero()) : VT::zero();
+                                });
+                            }
                         }
                     }
                 }
@@ -1307,7 +1333,10 @@ int launch_fwd_rows(Fwd3Args a, int ngroups, cudaStream_t st) {
 // Rows that meet more slices than a step holds take each line in parts, without
 // the usual path's registers: at least twice the time.  224 x 224 x 200, 60
 // views, 300 x 180 cells, 1 / 2 volumes: 6.7 / 7.2 ms with 8 rows, 2.1 / 2.8
-// with 4.
+// with 4.  Where 32 columns meet more than 64 pixels on some views, rows that
+// meet more slices than a tile of 128 pixels holds gather from global memory
+// there: 1.3 times (spiral, 512 x 512 x 128, 64 rows, 512 columns and 180 views /
+// 256 columns and 90 views: 11.5 / 9.7 ms with 8 rows, 7.7 / 3.7 with 4).
 template <int NB>
 int launch_fwd_volumes(Fwd3Args a, int b0, int ngroups, cudaStream_t st) {
     if (ngroups <= 0) return DD_OK;
@@ -1319,10 +1348,16 @@ int launch_fwd_volumes(Fwd3Args a, int b0, int ngroups, cudaStream_t st) {
     // slices the rows of a CTA meet on the farthest line
     const double row_slices = a.g.row_size * (a.g.iso_source + 0.6 * std::max(a.g.width * a.g.pix_x, a.g.height * a.g.pix_y)) /
                               (a.g.source_detector * a.g.pix_z);
+    // pixels its columns meet there, on views halfway to 45 degrees
+    const double cell = a.geom == DD_GEOM3_CONE_FLAT ? a.g.col_size * a.g.iso_source / a.g.source_detector : a.g.col_size * a.g.iso_source;
+    const double far = 1.0 + 0.6 * std::max(a.g.width * a.g.pix_x, a.g.height * a.g.pix_y) / a.g.iso_source;
+    const bool wide = 1.15 * kFC * cell * far / std::min(a.g.pix_x, a.g.pix_y) + 3 > pitch3(kNarrow3 - 1);
+    const int most = zwindow3(pitch3(kNarrow3 - 1)), few = zwindow3(pitch3(kNPitch - 1));
     auto cost = [&](int rr) {
         const double blocks = std::max(((R + rr * kCons3 - 1) / (rr * kCons3)) * per_block, full);
-        const bool parts = a.g.depth > kZW && std::min(R, rr * kCons3) * row_slices + 4 > kZW;
-        return blocks * (rr + 2.5) * (parts ? 2 : 1);
+        const double meet = std::min(R, rr * kCons3) * row_slices + 4;
+        const bool parts = a.g.depth > most && meet > most, gather = wide && a.g.depth > few && meet > few;
+        return blocks * (rr + 2.5) * (parts ? 2 : 1) * (gather ? 1.3 : 1);
     };
     const double c8 = cost(8), c4 = cost(4), c2 = cost(2);
     if (c8 <= c4 && c8 <= c2) return launch_fwd_rows<NB, 8>(a, ngroups, st);

@@ -11,6 +11,7 @@ from cases3d import spiral_source
 from conftest import rel_l2
 from test_gpu_2d import run as run2d
 from test_gpu_3d import run as run3d
+from test_gpu_splits import _check3d
 
 pytestmark = pytest.mark.gpu
 
@@ -141,3 +142,13 @@ def test_workspace_at_any_address(op, B, shift):
         assert bool((buf[:at] == 0xA5).all()) and bool((buf[at + n:] == 0xA5).all())
         return res
     assert torch.equal(call(shift), call(0))
+
+
+# 3-D forward, 32 columns that meet more than 64 pixels: a tile of 96 or 128
+# where it holds a line's slices (20 rows), else the step's segments with
+# pixels from global memory (thin slices); columns of 9 to 16 pixels, and more.
+@pytest.mark.parametrize("rows,pz", [(20, 1.0), (65, 0.3)])
+@pytest.mark.parametrize("cell,cols", [(2.0, 70), (2.6, 45), (3.6, 40), (7.0, 33), (11.0, 14), (14.5, 10), (25.0, 6)])
+@pytest.mark.parametrize("geom,op,B", [("cone_flat", "proj", 2), ("cone_arc", "bproj_t", 1), ("spiral", "bproj_tw", 3)])
+def test_forward3d_columns_of_several_pixels(oracle_mod, geom, op, B, cell, cols, rows, pz):
+    _check3d(oracle_mod, geom, op, 150, 117, 40, cols, rows, 4, B, cell, pz)
