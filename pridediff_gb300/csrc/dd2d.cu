@@ -135,7 +135,7 @@ k_fwd(dd_geom2d g, int geom, int op, int B, int V, int nl, const DdView2 *__rest
       int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ FwdState S;
-    const FwdLay L = fwd_lay(KIND == kPara, g.num_det, max(g.width, g.height), NB, cl);
+    const FwdLay L = fwd_lay(KIND, g.num_det, max(g.width, g.height), NB, cl);
     fwd_init<NB>(smem, L, S);
     constexpr int planes = NB / plane_slices(NB);
     FwdItem it;
@@ -459,7 +459,7 @@ static int launch_fwd_group(const FwdCall &c, const float *in, int n, float *row
     k_planes<P><<<dim3((unsigned)((W + 31) / 32), (unsigned)((H + 31) / 32), (unsigned)planes), 256, 0, c.st>>>(
         in, n, H, W, rows, cols, rplane, cplane, c.first ? c.status : nullptr);
     prof_end(pt, c.st);
-    const FwdLay L = fwd_lay(KIND == kPara, c.g->num_det, std::max(W, H), NB, c.cl);
+    const FwdLay L = fwd_lay(KIND, c.g->num_det, std::max(W, H), NB, c.cl);
     auto kern = k_fwd<KIND, NPASS, NB>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total) != cudaSuccess)
         return DD_ERR_LAUNCH;
@@ -543,9 +543,9 @@ static int launch_fwd(FwdCall c, bool single, int B, const float *in, char *rows
     int big = 1;
     if (!single) {
         const int limit = max_smem_optin();
-        big = pass_class(D) <= 4 && fwd_lay(KIND == kPara, D, npix, 8, c.cl).total <= limit / 2 ? 8
-              : fwd_fits(KIND == kPara, D, npix, 4, c.cl, limit)                                ? 4
-              : fwd_fits(KIND == kPara, D, npix, 2, c.cl, limit)                                ? 2
+        big = pass_class(D) <= 4 && fwd_lay(KIND, D, npix, 8, c.cl).total <= limit / 2 ? 8
+              : fwd_fits(KIND, D, npix, 4, c.cl, limit)                                ? 4
+              : fwd_fits(KIND, D, npix, 2, c.cl, limit)                                ? 2
                                                                                                 : 1;
     }
     int done = 0;

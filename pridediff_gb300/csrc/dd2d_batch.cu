@@ -55,7 +55,7 @@ static int fwd_item_limit(int scan, const dd_instance2d *in, int n) {
         npix = std::max(npix, std::max(in[i].geom.width, in[i].geom.height));
     }
     int fi = kBI;
-    while (fi > 1 && !fwd_fits(scan == DD_SCAN_PARA, D, npix, fi, 1, max_smem_optin())) fi /= 2;
+    while (fi > 1 && !fwd_fits(scan == DD_SCAN_PARA ? kPara : kFan, D, npix, fi, 1, max_smem_optin())) fi /= 2;
     return fi;
 }
 
@@ -226,7 +226,7 @@ k_fwd_items(int geom, int op, const BatchInst *__restrict__ desc, const int4 *__
             int *__restrict__ counter, int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ FwdState S;
-    const FwdLay L = fwd_lay(KIND == kPara, Dmax, nmax, fi, cl);   // of the largest items
+    const FwdLay L = fwd_lay(KIND, Dmax, nmax, fi, cl);   // of the largest items
     fwd_init<4>(smem, L, S);
     // the item and its geometry live in shared memory: read where used, they
     // hold no registers across the line loop (the plain forward reads them
@@ -400,8 +400,8 @@ template <int KIND, int NPASS>
 static int launch_fwd_items_as(int geom, int op, const BatchLayout &L, const char *planb, char *tabs, float *out,
                                const float *sub, int *counter, int *status, const dd_tune2d *tune, cudaStream_t st) {
     int cl = (tune && tune->items_cluster == 2) ? 2 : kFwdItemsCluster;
-    if (cl == 2 && !fwd_fits(KIND == kPara, L.Dmax, L.nmax, L.fi, 2, max_smem_optin())) cl = 1;
-    const FwdLay S = fwd_lay(KIND == kPara, L.Dmax, L.nmax, L.fi, cl);
+    if (cl == 2 && !fwd_fits(KIND, L.Dmax, L.nmax, L.fi, 2, max_smem_optin())) cl = 1;
+    const FwdLay S = fwd_lay(KIND, L.Dmax, L.nmax, L.fi, cl);
     auto kern = k_fwd_items<KIND, NPASS>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
         return DD_ERR_LAUNCH;

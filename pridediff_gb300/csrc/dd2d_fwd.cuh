@@ -73,7 +73,7 @@ __host__ __device__ inline size_t plane_bytes(int lines, int n, int p) {
 }
 
 // Shared memory: a stage per line in flight {header, pixel boundaries, detector boundaries
-// (parallel beam), pixels}, line records, barriers.
+// (parallel beam) or pixel weights (kFanWeighted), pixels}, line records, barriers.
 struct FwdLay {
     int hdr, bnd, det, pix, red, rec, drec, bar, total;
     int bnd_b, det_b, pix_b;   // bytes of one stage
@@ -83,11 +83,14 @@ constexpr int kSmemMax = 227 * 1024;
 constexpr int kFwdStatic = 512;   // of which the kernels' static arrays take no more than this
 // boundary e of a line sits at entry e + kB0 of its table
 constexpr int kB0 = 4;
-__host__ __device__ inline FwdLay fwd_lay(bool para, int D, int npix, int nb, int cl) {
+__host__ __device__ inline FwdLay fwd_lay(int kind, int D, int npix, int nb, int cl) {
     FwdLay s;
     const int p = plane_slices(nb);
     s.bnd_b = ((npix + kB0 + 8 + 3) & ~3) * (int)sizeof(float);
-    s.det_b = para ? ((D + kB0 + 8 + 3) & ~3) * (int)sizeof(float) : 0;
+    const bool para = kind == kPara;
+    s.det_b = para                   ? ((D + kB0 + 8 + 3) & ~3) * (int)sizeof(float)
+              : kind == kFanWeighted ? ((npix + 3) & ~3) * (int)sizeof(float)
+                                     : 0;
     s.pix_b = nb / p * plane_pitch(npix, p) * p * (int)sizeof(float);
     int o = 0;
     const int kP = prods(nb), red = pass_class(D) * nb * kCons * 32 * (int)sizeof(float);
@@ -112,8 +115,8 @@ __host__ __device__ inline FwdLay fwd_lay(bool para, int D, int npix, int nb, in
 }
 
 // Do NB slices side by side fit a CTA?
-inline bool fwd_fits(bool para, int D, int npix, int nb, int cl, int limit) {
-    return fwd_lay(para, D, npix, nb, cl).total + kFwdStatic <= limit;
+inline bool fwd_fits(int kind, int D, int npix, int nb, int cl, int limit) {
+    return fwd_lay(kind, D, npix, nb, cl).total + kFwdStatic <= limit;
 }
 
 struct FwdItem {
@@ -204,6 +207,28 @@ __device__ __forceinline__ void fill_boundaries(const DdLine &L, float *t, int l
     __syncwarp();
     // the walk's start takes the place of the boundary below its first pixel
     if (lane == 0) t[i0 - 1 + kB0] = L.h.bound0;
+}
+
+// FBP weights of a line's pixels i0 .. nend - 1, one warp: once a pixel, where a
+// weight per overlap is one per cell and pixel that meet.  Weighted transpose, 1
+// / 4 / 8 / 16 slices, ms with the pixels weighed ahead of prefix tables / a
+// weight per overlap / here: 512^2, 360 views, 736 bins 0.83, 1.29, 2.50, 4.69
+// / 0.76, 0.88, 1.25, 2.26 / 0.45, 0.59, 0.80, 1.53; 300^2, 200 views, 1,200
+// bins 0.44, 0.59, 1.12, 2.11 / 0.51, 0.75, 1.18, 2.24 / 0.27, 0.43, 0.69, 1.29.
+// (The table takes lines of 900 to 1,000 pixels from 8 slices to 4: 1000^2, 60
+// views, 900 bins, 16 slices 5.1 / 1.27 / 1.61; 8 slices 2.6 / 1.05 / 0.84.)
+template <int GEOM>
+__device__ __forceinline__ void fill_weights(const dd_geom2d &g, const DdView2 &vw, int line, int i0, int nend, float *wt,
+                                             int lane) {
+    const int xb = vw.xb;
+    const float sx = vw.srcx, sy = vw.srcy, axis0 = vw.axis0, pitch = xb ? g.pix_x : g.pix_y;
+    const float lpos = xb ? pix_centre(0.5f * (float)g.height - (float)line - 0.5f, g.pix_y, g.pix_yshift)
+                          : pix_centre((float)line - 0.5f * (float)g.width + 0.5f, g.pix_x, g.pix_xshift);
+#pragma unroll 4
+    for (int e = i0 + lane; e < nend; e += 32) {
+        const float pc = pix_centre((float)e + 0.5f, pitch, axis0);
+        wt[e] = fan_fbp_weight<GEOM>(sx, sy, xb ? pc : lpos, xb ? lpos : pc, g.iso_source);
+    }
 }
 
 // Sets up a CTA's barriers and state (all threads; ends with a CTA barrier).
@@ -300,6 +325,11 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
                                 src + (size_t)lane * plane + (size_t)line_of(i) * pitch * P, row_b, &full[st]);
                 fill_boundaries(R, reinterpret_cast<float *>(smem + L.bnd + st * L.bnd_b), lane);
                 if (KIND == kPara) fill_boundaries(drec[buf], reinterpret_cast<float *>(smem + L.det + st * L.det_b), lane);
+                if (KIND == kFanWeighted) {
+                    float *wt = reinterpret_cast<float *>(smem + L.det + st * L.det_b);
+                    if (geom == DD_GEOM_ARC) fill_weights<DD_GEOM_ARC>(g, *vwp, line_of(i), i0, nend, wt, lane);
+                    else fill_weights<DD_GEOM_FLAT>(g, *vwp, line_of(i), i0, nend, wt, lane);
+                }
             }
             if (lane == 0) {
                 // pixel of axis position u: inv u + off, the chord of the
@@ -355,14 +385,9 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
                 const int idet0 = __float_as_int(h1.z);
                 const int i0 = __float_as_int(h1.x), last = i0 + n - 1;
                 const float *bt = reinterpret_cast<const float *>(smem + L.bnd + st * L.bnd_b) + kB0;
-                const float *dt = reinterpret_cast<const float *>(smem + L.det + st * L.det_b) + kB0;
+                // the detector's boundaries, or the pixels' weights
+                const float *dt = reinterpret_cast<const float *>(smem + L.det + st * L.det_b) + (KIND == kPara ? kB0 : 0);
                 const float *pix = reinterpret_cast<const float *>(smem + L.pix + st * L.pix_b);
-                float lpos = 0.0f;
-                if (KIND == kFanWeighted) {
-                    const int line = line_of(i);
-                    lpos = xb ? pix_centre(0.5f * (float)g.height - (float)line - 0.5f, g.pix_y, g.pix_yshift)
-                              : pix_centre((float)line - 0.5f * (float)g.width + 0.5f, g.pix_x, g.pix_xshift);
-                }
 #pragma unroll
                 for (int m = 0; m < NPASS; m++) {
                     if (m >= npass) break;
@@ -386,13 +411,7 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
                     auto add = [&](float w, int i) {   // a part of pixel j + i
                         if (!(w > 0.0f)) return;
                         if (KIND != kFan) w *= h1.w;
-                        if (KIND == kFanWeighted) {
-                            const float pc = pix_centre((float)(j + i) + 0.5f, xb ? g.pix_x : g.pix_y, vwp->axis0);
-                            const float cx = xb ? pc : lpos, cy = xb ? lpos : pc;
-                            w *= geom == DD_GEOM_ARC
-                                     ? fan_fbp_weight<DD_GEOM_ARC>(vwp->srcx, vwp->srcy, cx, cy, g.iso_source)
-                                     : fan_fbp_weight<DD_GEOM_FLAT>(vwp->srcx, vwp->srcy, cx, cy, g.iso_source);
-                        }
+                        if (KIND == kFanWeighted) w *= dt[j + i];
                         acc[m].add(w, pix + (j + i) * P, pitch * P);
                     };
                     // (past the last boundary, which bounds hi, the table may

@@ -152,3 +152,19 @@ def test_workspace_at_any_address(op, B, shift):
 @pytest.mark.parametrize("geom,op,B", [("cone_flat", "proj", 2), ("cone_arc", "bproj_t", 1), ("spiral", "bproj_tw", 3)])
 def test_forward3d_columns_of_several_pixels(oracle_mod, geom, op, B, cell, cols, rows, pz):
     _check3d(oracle_mod, geom, op, 150, 117, 40, cols, rows, 4, B, cell, pz)
+
+
+# The weighted transpose's table of a line's weights: many cells a pixel, cells
+# of many pixels, lines of which 8, 4, 2 and 1 slices fit beside it.
+@pytest.mark.parametrize("W,H,D,cell,B", [(60, 45, 300, 0.25, 1), (45, 60, 1984, 0.04, 8), (60, 45, 9, 12.0, 4), (1, 50, 40, 1.0, 2),
+                                          (890, 4, 300, 3.2, 9), (1000, 4, 300, 3.6, 9), (2500, 3, 700, 3.9, 5), (3450, 3, 1984, 1.8, 2),
+                                          (4096, 3, 1984, 2.2, 2)])
+@pytest.mark.parametrize("geom", ["flat", "arc"])
+def test_weighted_transpose(oracle_mod, geom, W, H, D, cell, B):
+    pix = 0.7 * min(1.0, 1000.0 / W)
+    det = cell * pix * {"flat": 1085.6 / 595.0, "arc": 1.0 / 595.0}[geom]
+    opt = [W, H, D, pix, 0.9 * pix, det, 595.0, 1085.6, 0.1, -0.2, 0.1 * det]
+    ang = (np.arange(5) * 2 * np.pi / 5 + 0.1).astype(np.float32)
+    x = np.random.default_rng(D).random((B, H, W), dtype=np.float32)
+    ref = oracle_mod.run2d(geom, "bproj_tw", x, ang, opt, nthreads=8)
+    assert np.any(ref) and rel_l2(run2d(geom, "bproj_tw", x, ang, opt), ref) <= 1e-5
