@@ -126,16 +126,16 @@ __global__ void k_dettab(int geom, int mode, const float *__restrict__ sino, int
 // Single-geometry forward: one item per cluster.  blockIdx.x = view * cluster
 // size + rank, blockIdx.y = group of NB slices.  3 CTAs per SM (56 registers)
 // up to 24 sums a thread.
-template <int KIND, int NPASS, int NB>
+template <int KIND, int NPASS, int NB, bool WIDE>
 __global__ void __launch_bounds__(fwd_threads(NB), NPASS * NB <= 24 ? 3 : 2)
 k_fwd(dd_geom2d g, int geom, int op, int B, int V, int nl, const DdView2 *__restrict__ views,
       const float *__restrict__ dp, const float *__restrict__ bcoef, const DdLine *__restrict__ lines,
       const DdLine *__restrict__ dlines, const float *__restrict__ rows, const float *__restrict__ cols,
-      size_t rplane, size_t cplane, float *__restrict__ out, const float *__restrict__ sub, int cl,
+      size_t rplane, size_t cplane, float *__restrict__ out, const float *__restrict__ sub, int cl, int sh,
       int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ FwdState S;
-    const FwdLay L = fwd_lay(KIND, g.num_det, max(g.width, g.height), NB, cl);
+    const FwdLay L = fwd_lay(KIND, g.num_det, g.num_det << sh, max(g.width, g.height), NB, cl);
     fwd_init<NB>(smem, L, S);
     constexpr int planes = NB / plane_slices(NB);
     FwdItem it;
@@ -144,6 +144,7 @@ k_fwd(dd_geom2d g, int geom, int op, int B, int V, int nl, const DdView2 *__rest
     it.nb = min(NB, B - it.b0);
     it.V = V;
     it.nl = nl;
+    it.sh = sh;
     it.views = views;
     it.dp = dp;
     it.bcoef = bcoef;
@@ -156,7 +157,7 @@ k_fwd(dd_geom2d g, int geom, int op, int B, int V, int nl, const DdView2 *__rest
     it.out = out;
     it.sub = sub;
     uint32_t step = 0, nr = 0;
-    if (!fwd_item<KIND, NPASS, NB>(g, geom, op, it, smem, L, S, step, nr) && threadIdx.x == 0) dd_report_timeout(status);
+    if (!fwd_item<KIND, NPASS, NB, WIDE>(g, geom, op, it, smem, L, S, step, nr) && threadIdx.x == 0) dd_report_timeout(status);
 }
 
 // Plan time: the views that walk image rows and those that walk columns, each
@@ -436,7 +437,7 @@ static void fwd_shape(int geom, const dd_geom2d *g, const dd_tune2d *tune, int *
 
 struct FwdCall {
     const dd_geom2d *g;
-    int geom, op, V, nl, cl;
+    int geom, op, V, nl, cl, sh;
     const DdView2 *views;
     const float *dp, *bcoef;
     const DdLine *lines, *dlines;
@@ -447,7 +448,7 @@ struct FwdCall {
 };
 
 // `n` slices in groups of NB: their planes, and the groups' items.
-template <int KIND, int NPASS, int NB>
+template <int KIND, int NPASS, int NB, bool WIDE>
 static int launch_fwd_group(const FwdCall &c, const float *in, int n, float *rows, float *cols, float *out,
                             const float *sub) {
     constexpr int P = plane_slices(NB);
@@ -459,8 +460,8 @@ static int launch_fwd_group(const FwdCall &c, const float *in, int n, float *row
     k_planes<P><<<dim3((unsigned)((W + 31) / 32), (unsigned)((H + 31) / 32), (unsigned)planes), 256, 0, c.st>>>(
         in, n, H, W, rows, cols, rplane, cplane, c.first ? c.status : nullptr);
     prof_end(pt, c.st);
-    const FwdLay L = fwd_lay(KIND, c.g->num_det, std::max(W, H), NB, c.cl);
-    auto kern = k_fwd<KIND, NPASS, NB>;
+    const FwdLay L = fwd_lay(KIND, c.g->num_det, c.g->num_det << c.sh, std::max(W, H), NB, c.cl);
+    auto kern = k_fwd<KIND, NPASS, NB, WIDE>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total) != cudaSuccess)
         return DD_ERR_LAUNCH;
     cudaLaunchAttribute at;
@@ -477,7 +478,7 @@ static int launch_fwd_group(const FwdCall &c, const float *in, int n, float *row
     ProfRec *pr = prof_begin(DD_KERNEL_FORWARD, c.st);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, *c.g, c.geom, c.op, n, c.V, c.nl, c.views, c.dp, c.bcoef, c.lines,
                                              c.dlines, (const float *)rows, (const float *)cols, rplane, cplane, out, sub,
-                                             c.cl, c.status);
+                                             c.cl, c.sh, c.status);
     prof_end(pr, c.st);
     g_launches += 2;
     if (e != cudaSuccess) {
@@ -490,12 +491,15 @@ static int launch_fwd_group(const FwdCall &c, const float *in, int n, float *row
 template <int KIND, int NB>
 static int launch_fwd_passes(const FwdCall &c, const float *in, int n, float *rows, float *cols, float *out,
                              const float *sub) {
+    if (c.sh > 0)   // wide bins: at most two passes
+        return c.g->num_det << c.sh <= kBins ? launch_fwd_group<KIND, 1, NB, true>(c, in, n, rows, cols, out, sub)
+                                             : launch_fwd_group<KIND, 2, NB, true>(c, in, n, rows, cols, out, sub);
     switch (pass_class(c.g->num_det)) {
-    case 1: return launch_fwd_group<KIND, 1, NB>(c, in, n, rows, cols, out, sub);
-    case 2: return launch_fwd_group<KIND, 2, NB>(c, in, n, rows, cols, out, sub);
-    case 3: return launch_fwd_group<KIND, 3, NB>(c, in, n, rows, cols, out, sub);
-    case 4: return launch_fwd_group<KIND, 4, NB>(c, in, n, rows, cols, out, sub);
-    default: return launch_fwd_group<KIND, 8, (NB > 4 ? 4 : NB)>(c, in, n, rows, cols, out, sub);   // never 8 slices
+    case 1: return launch_fwd_group<KIND, 1, NB, false>(c, in, n, rows, cols, out, sub);
+    case 2: return launch_fwd_group<KIND, 2, NB, false>(c, in, n, rows, cols, out, sub);
+    case 3: return launch_fwd_group<KIND, 3, NB, false>(c, in, n, rows, cols, out, sub);
+    case 4: return launch_fwd_group<KIND, 4, NB, false>(c, in, n, rows, cols, out, sub);
+    default: return launch_fwd_group<KIND, 8, (NB > 4 ? 4 : NB), false>(c, in, n, rows, cols, out, sub);   // never 8 slices
     }
 }
 
@@ -537,15 +541,15 @@ static int launch_prefix(const FwdCall &c, int B, const float *in, float2 *tx, f
 // 4 or 2 where they fit; one slice always does (4,096 pixels, 1,984 cells).
 template <int KIND>
 static int launch_fwd(FwdCall c, bool single, int B, const float *in, char *rows, char *cols, float *out) {
-    const int W = c.g->width, H = c.g->height, D = c.g->num_det, npix = std::max(W, H);
+    const int W = c.g->width, H = c.g->height, D = c.g->num_det, npix = std::max(W, H), lanes = D << c.sh;
     if ((long long)c.V * c.cl > 0x7FFFFFFFLL) return DD_ERR_SIZE_OVERFLOW;
     const size_t image = (size_t)W * H, sino = (size_t)c.V * D;
     int big = 1;
     if (!single) {
         const int limit = max_smem_optin();
-        big = pass_class(D) <= 4 && fwd_lay(KIND, D, npix, 8, c.cl).total <= limit / 2 ? 8
-              : fwd_fits(KIND, D, npix, 4, c.cl, limit)                                ? 4
-              : fwd_fits(KIND, D, npix, 2, c.cl, limit)                                ? 2
+        big = pass_class(lanes) <= 4 && fwd_lay(KIND, D, lanes, npix, 8, c.cl).total <= limit / 2 ? 8
+              : fwd_fits(KIND, D, lanes, npix, 4, c.cl, limit)                                ? 4
+              : fwd_fits(KIND, D, lanes, npix, 2, c.cl, limit)                                ? 2
                                                                                                 : 1;
     }
     int done = 0;
@@ -673,6 +677,7 @@ int apply_planned(int scan, int op, const dd_geom2d *g, const void *planp, const
         c.nl = P.nl;
         int bi;
         fwd_shape(geom, g, tune, &bi, &c.cl);
+        c.sh = fwd_lanes(geom, *g);
         c.views = (const DdView2 *)(planb + P.views);
         c.dp = (const float *)(planb + P.dp);
         c.bcoef = (const float *)(planb + P.bcoef);

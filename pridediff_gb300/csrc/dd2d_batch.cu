@@ -30,7 +30,7 @@ namespace dd2 {
 
 struct BatchInst {
     dd_geom2d g;
-    int V, batch, nl, ps;          // ps: slices per forward item (1, 2 or 4)
+    int V, batch, nl, ps, sh;      // forward items: ps slices (1, 2 or 4), 2^sh lanes a bin
     long long plan_off;            // bytes: instance plan inside the batch plan
     long long img_off, sino_off;   // elements: packed images / sinograms
     long long row_off, col_off;    // bytes: planes of rows / columns in the workspace
@@ -42,6 +42,7 @@ struct BatchLayout {
     size_t desc, fitems, aitems, plans, total;        // plan buffer
     size_t w_tabs, w_dtab, w_resid, w_counter, w_status, w_total;   // workspace
     int nfwd, nadj, nrow, Dmax, nmax;   // items (nrow of the parallel beam's are rows); largest detector and line
+    int lanes;   // most lanes that an instance's bins take
     int fi;   // largest instance's slices per forward item
     std::vector<BatchInst> inst;
 };
@@ -49,13 +50,14 @@ struct BatchLayout {
 // Most slices per persistent forward item: 4, or fewer where lines of
 // thousands of pixels would not leave room for them.
 static int fwd_item_limit(int scan, const dd_instance2d *in, int n) {
-    int D = 1, npix = 1;
+    int D = 1, npix = 1, lanes = 1;
     for (int i = 0; i < n; i++) {
         D = std::max(D, in[i].geom.num_det);
+        lanes = std::max(lanes, in[i].geom.num_det << fwd_lanes(geom_of(scan), in[i].geom));
         npix = std::max(npix, std::max(in[i].geom.width, in[i].geom.height));
     }
     int fi = kBI;
-    while (fi > 1 && !fwd_fits(scan == DD_SCAN_PARA ? kPara : kFan, D, npix, fi, 1, max_smem_optin())) fi /= 2;
+    while (fi > 1 && !fwd_fits(scan == DD_SCAN_PARA ? kPara : kFan, D, lanes, npix, fi, 1, max_smem_optin())) fi /= 2;
     return fi;
 }
 
@@ -67,7 +69,7 @@ static BatchLayout batch_layout(int scan, const dd_instance2d *in, int n, int bi
     long long img = 0, sino = 0, tabs = 0, dtab = 0;
     size_t plans = 0;
     L.nfwd = L.nadj = L.nrow = 0;
-    L.Dmax = 1;
+    L.Dmax = L.lanes = 1;
     L.nmax = 1;
     for (int i = 0; i < n; i++) {
         BatchInst &d = L.inst[i];
@@ -111,6 +113,8 @@ static BatchLayout batch_layout(int scan, const dd_instance2d *in, int n, int bi
             L.nadj += ((W + kTile - 1) / kTile) * ((H + kTile - 1) / kTile) * groups;
         }
         L.Dmax = std::max(L.Dmax, D);
+        d.sh = fwd_lanes(geom_of(scan), d.g);
+        L.lanes = std::max(L.lanes, D << d.sh);
         L.nmax = std::max(L.nmax, std::max(W, H));
     }
     size_t o = 0;
@@ -218,15 +222,16 @@ constexpr int kFwdItemsCluster = 1;
 // 4): one-slice items in a 4-slice kernel took 6.97 instead of 5.9 ms on 24
 // uneven instances of 1 to 3 slices.
 static_assert(prods(1) == prods(4) && prods(2) == prods(4), "items of 1, 2 and 4 slices share a CTA's warps");
-template <int KIND, int NPASS>
+// WIDE: some instance's bins take more than one lane.
+template <int KIND, int NPASS, bool WIDE>
 __global__ void __launch_bounds__(fwd_threads(4), NPASS <= 4 ? 3 : 2)
 k_fwd_items(int geom, int op, const BatchInst *__restrict__ desc, const int4 *__restrict__ items, int nitems,
             const char *__restrict__ plan, size_t plans_off, const char *__restrict__ tabs,
-            float *__restrict__ out, const float *__restrict__ sub, int Dmax, int nmax, int fi, int cl,
+            float *__restrict__ out, const float *__restrict__ sub, int Dmax, int lanes, int nmax, int fi, int cl,
             int *__restrict__ counter, int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ FwdState S;
-    const FwdLay L = fwd_lay(KIND, Dmax, nmax, fi, cl);   // of the largest items
+    const FwdLay L = fwd_lay(KIND, Dmax, lanes, nmax, fi, cl);   // of the largest items
     fwd_init<4>(smem, L, S);
     // the item and its geometry live in shared memory: read where used, they
     // hold no registers across the line loop (the plain forward reads them
@@ -251,6 +256,7 @@ k_fwd_items(int geom, int op, const BatchInst *__restrict__ desc, const int4 *__
             it.nb = w.w;
             it.V = d.V;
             it.nl = d.nl;
+            it.sh = d.sh;
             it.views = reinterpret_cast<const DdView2 *>(pb + d.views);
             it.dp = reinterpret_cast<const float *>(pb + d.dp);
             it.bcoef = reinterpret_cast<const float *>(pb + d.bcoef);
@@ -266,9 +272,9 @@ k_fwd_items(int geom, int op, const BatchInst *__restrict__ desc, const int4 *__
             s_ps = d.ps;
         }
         __syncthreads();   // every thread passed the barrier above before s_it changes
-        const bool ok = s_ps == 1   ? fwd_item<KIND, NPASS, 1>(s_g, geom, op, s_it, smem, L, S, step, nr)
-                        : s_ps == 2 ? fwd_item<KIND, NPASS, 2>(s_g, geom, op, s_it, smem, L, S, step, nr)
-                                    : fwd_item<KIND, NPASS, 4>(s_g, geom, op, s_it, smem, L, S, step, nr);
+        const bool ok = s_ps == 1   ? fwd_item<KIND, NPASS, 1, WIDE>(s_g, geom, op, s_it, smem, L, S, step, nr)
+                        : s_ps == 2 ? fwd_item<KIND, NPASS, 2, WIDE>(s_g, geom, op, s_it, smem, L, S, step, nr)
+                                    : fwd_item<KIND, NPASS, 4, WIDE>(s_g, geom, op, s_it, smem, L, S, step, nr);
         if (!ok) {
             if (threadIdx.x == 0) dd_report_timeout(status);
             break;
@@ -396,13 +402,13 @@ static int resident_ctas(K kern, int smem, int threads) {
     return n;
 }
 
-template <int KIND, int NPASS>
+template <int KIND, int NPASS, bool WIDE>
 static int launch_fwd_items_as(int geom, int op, const BatchLayout &L, const char *planb, char *tabs, float *out,
                                const float *sub, int *counter, int *status, const dd_tune2d *tune, cudaStream_t st) {
     int cl = (tune && tune->items_cluster == 2) ? 2 : kFwdItemsCluster;
-    if (cl == 2 && !fwd_fits(KIND, L.Dmax, L.nmax, L.fi, 2, max_smem_optin())) cl = 1;
-    const FwdLay S = fwd_lay(KIND, L.Dmax, L.nmax, L.fi, cl);
-    auto kern = k_fwd_items<KIND, NPASS>;
+    if (cl == 2 && !fwd_fits(KIND, L.Dmax, L.lanes, L.nmax, L.fi, 2, max_smem_optin())) cl = 1;
+    const FwdLay S = fwd_lay(KIND, L.Dmax, L.lanes, L.nmax, L.fi, cl);
+    auto kern = k_fwd_items<KIND, NPASS, WIDE>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total) != cudaSuccess)
         return DD_ERR_LAUNCH;
     // grid_of's CTA count rounded down to whole clusters, at most the clusters
@@ -431,7 +437,7 @@ static int launch_fwd_items_as(int geom, int op, const BatchLayout &L, const cha
     ProfRec *pr = prof_begin(DD_KERNEL_FORWARD, st);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, geom, op, (const BatchInst *)(planb + L.desc),
                                              (const int4 *)(planb + L.fitems), L.nfwd, planb, L.plans, (const char *)tabs,
-                                             out, sub, L.Dmax, L.nmax, L.fi, cl, counter, status);
+                                             out, sub, L.Dmax, L.lanes, L.nmax, L.fi, cl, counter, status);
     prof_end(pr, st);
     count_launches(1);
     if (e != cudaSuccess) {
@@ -453,12 +459,20 @@ static int launch_fwd_items(int geom, int op, const BatchLayout &L, const char *
     prof_end(pr, st);
     count_launches(1);
     if (cudaMemsetAsync(counter, 0, 2 * sizeof(int), st) != cudaSuccess) return DD_ERR_LAUNCH;
-    switch (pass_class(L.Dmax)) {
-    case 1: return launch_fwd_items_as<KIND, 1>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
-    case 2: return launch_fwd_items_as<KIND, 2>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
-    case 3: return launch_fwd_items_as<KIND, 3>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
-    case 4: return launch_fwd_items_as<KIND, 4>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
-    default: return launch_fwd_items_as<KIND, 8>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+    bool wide = false;
+    for (const BatchInst &d : L.inst) wide = wide || d.sh > 0;
+    const int passes = pass_class(L.lanes);
+    if (wide) {   // (few classes: batches with coarse detectors)
+        if (passes <= 2) return launch_fwd_items_as<KIND, 2, true>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+        if (passes <= 4) return launch_fwd_items_as<KIND, 4, true>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+        return launch_fwd_items_as<KIND, 8, true>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+    }
+    switch (passes) {
+    case 1: return launch_fwd_items_as<KIND, 1, false>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+    case 2: return launch_fwd_items_as<KIND, 2, false>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+    case 3: return launch_fwd_items_as<KIND, 3, false>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+    case 4: return launch_fwd_items_as<KIND, 4, false>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
+    default: return launch_fwd_items_as<KIND, 8, false>(geom, op, L, planb, tabs, out, sub, counter, status, tune, st);
     }
 }
 

@@ -26,6 +26,8 @@
 // 0.79 / 2.18 ms.
 #pragma once
 
+#include <cmath>
+
 #include "dd2d_kernels.cuh"
 
 namespace dd2 {
@@ -67,6 +69,41 @@ __host__ __device__ inline int pass_class(int D) {
 __host__ __device__ constexpr int plane_slices(int nb) { return nb < 4 ? nb : 4; }
 // Pixels a line of a plane takes (a multiple of 16 bytes).
 __host__ __device__ inline int plane_pitch(int n, int p) { return p == 1 ? (n + 3) & ~3 : p == 2 ? (n + 1) & ~1 : n; }
+// Lanes a bin takes, as a power of two.  Bins of up to 4 pixels (parallel beam,
+// whose passes cost more: 6) are one lane's; of wider ones a lane takes every
+// 2nd, 4th ... 32nd pixel, three at a time: as many lanes as make passes x steps
+// of three pixels fewest, within one pass, or two from 8 pixels on (fan beams).
+// By the geometry alone: a slice's sums do not depend on how many are in the call.
+//
+// Flat fan, 1 / 8 slices, ms by prefix sums, a lane a bin, so.  512^2, 180 views:
+// 16 cells 0.22, 0.34; 1.02, 1.52; 0.18, 0.27.  64 cells 0.22, 0.35; 0.36, 0.54;
+// 0.19, 0.30.  128 cells 0.22, 0.36; 0.24, 0.37; 0.19, 0.32.  180 cells (3.4 pixels)
+// 0.22, 0.37; 0.21, 0.33; two lanes 0.21, 0.37.  1000^2, 90 views: 16 cells 0.39,
+// 0.61; 3.67, 5.56; 0.34, 0.61.  64 cells 0.40, 0.63; 1.14, 1.78; 0.37, 0.75.  180
+// cells (6.7 pixels) 0.39, 0.64; 0.52, 0.88; two lanes 0.43, 0.93: on lines of that
+// length 5 and more slices of wide cells stay 0.6 to 0.95 times as fast as they
+// were by prefix sums.
+inline int fwd_lanes(int geom, const dd_geom2d &g) {
+    const bool para = geom == DD_GEOM_PARA;
+    const double cell = para                   ? (double)g.det_size
+                        : geom == DD_GEOM_FLAT ? (double)g.det_size * g.iso_source / g.source_detector
+                                               : (double)g.det_size * g.iso_source;
+    const double c = std::min(cell / std::min(g.pix_x, g.pix_y), 4096.0);   // pixels a bin, at the isocentre
+    if (!(c > (para ? 6.0 : 4.0)) || g.num_det > kBins) return 0;
+    double best = 1.0 + 0.7 * (c - 2.0);   // one lane: three pixels at once, the others in turn
+    int sh = 0;
+    for (int s = 1; s <= 5 && g.num_det << s <= 2 * kBins; s++) {
+        const bool two = g.num_det << s > kBins;
+        if (two && (para || !(c > 8.0))) break;
+        const double cost = (two ? 2.0 : 1.0) * std::ceil((c + 1.0) / (3 << s));
+        if (cost < best || (cost == best && two && g.num_det >= 64)) {   // (even: as measured)
+            best = cost;
+            sh = s;
+        }
+    }
+    return sh;
+}
+
 // Bytes of a plane of P slices: its rows (h lines of w pixels) or columns.
 __host__ __device__ inline size_t plane_bytes(int lines, int n, int p) {
     return sizeof(float) * (size_t)lines * plane_pitch(n, p) * p;
@@ -83,7 +120,8 @@ constexpr int kSmemMax = 227 * 1024;
 constexpr int kFwdStatic = 512;   // of which the kernels' static arrays take no more than this
 // boundary e of a line sits at entry e + kB0 of its table
 constexpr int kB0 = 4;
-__host__ __device__ inline FwdLay fwd_lay(int kind, int D, int npix, int nb, int cl) {
+// lanes: the lanes that all bins take (D << fwd_lanes).
+__host__ __device__ inline FwdLay fwd_lay(int kind, int D, int lanes, int npix, int nb, int cl) {
     FwdLay s;
     const int p = plane_slices(nb);
     s.bnd_b = ((npix + kB0 + 8 + 3) & ~3) * (int)sizeof(float);
@@ -93,7 +131,7 @@ __host__ __device__ inline FwdLay fwd_lay(int kind, int D, int npix, int nb, int
                                      : 0;
     s.pix_b = nb / p * plane_pitch(npix, p) * p * (int)sizeof(float);
     int o = 0;
-    const int kP = prods(nb), red = pass_class(D) * nb * kCons * 32 * (int)sizeof(float);
+    const int kP = prods(nb), red = pass_class(lanes) * nb * kCons * 32 * (int)sizeof(float);
     const int fixed = (para ? 2 : 1) * kP * kRecs * (int)sizeof(DdLine) + (2 * stages(nb) + kRecs * kP) * 8 + kFwdStatic;
     int kS = stages(nb);
     while (kS > kP && fixed + kS * (s.bnd_b + s.det_b + s.pix_b + 32) + (cl == 1 ? red : 0) > kSmemMax) kS--;
@@ -115,12 +153,12 @@ __host__ __device__ inline FwdLay fwd_lay(int kind, int D, int npix, int nb, int
 }
 
 // Do NB slices side by side fit a CTA?
-inline bool fwd_fits(int kind, int D, int npix, int nb, int cl, int limit) {
-    return fwd_lay(kind, D, npix, nb, cl).total + kFwdStatic <= limit;
+inline bool fwd_fits(int kind, int D, int lanes, int npix, int nb, int cl, int limit) {
+    return fwd_lay(kind, D, lanes, npix, nb, cl).total + kFwdStatic <= limit;
 }
 
 struct FwdItem {
-    int v, b0, nb, V, nl;
+    int v, b0, nb, V, nl, sh;   // sh: log2 of the lanes a bin takes
     const DdView2 *views;
     const float *dp, *bcoef;
     const DdLine *lines, *dlines;
@@ -259,7 +297,8 @@ __device__ __forceinline__ void fwd_init(unsigned char *smem, const FwdLay &L, F
 // the odd lines are summed apart and then added: by a cluster of two CTAs
 // side by side (rank 0 adds rank 1's sums through distributed shared memory),
 // by a single CTA one after the other, with the same result bit for bit.
-template <int KIND, int NPASS, int NB>
+// WIDE: a bin may take more than one lane.
+template <int KIND, int NPASS, int NB, bool WIDE>
 __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it, unsigned char *smem,
                          const FwdLay &L, FwdState &S, uint32_t &step, uint32_t &nr) {
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
@@ -278,7 +317,8 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
     const int nstep = CL == 1 ? nline : rank == 0 ? half : nline - half;
     auto line_of = [&](int i) { return CL > 1 ? 2 * i + rank : i < half ? 2 * i : 2 * (i - half) + 1; };
     float *red = reinterpret_cast<float *>(smem + L.red);
-    const int npass = (D + kBins - 1) / kBins;
+    const int sh = WIDE ? it.sh : 0, lanes = 1 << sh, sub = lane & (lanes - 1);
+    const int npass = ((D << sh) + kBins - 1) / kBins;
     Slices<NB> acc[NPASS];
 #pragma unroll
     for (int m = 0; m < NPASS; m++) acc[m].clear();
@@ -362,7 +402,7 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
         float u0[NPASS], u1[NPASS];
 #pragma unroll
         for (int m = 0; m < NPASS; m++) {
-            const int k = m * kBins + warp * 32 + lane;
+            const int k = (m * kBins + warp * 32 + lane) >> sh;
             u0[m] = 0.0f;
             u1[m] = -3.0e38f;   // past the detector: an empty interval
             if (KIND != kPara && k < D) {
@@ -391,7 +431,7 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
 #pragma unroll
                 for (int m = 0; m < NPASS; m++) {
                     if (m >= npass) break;
-                    const int k = m * kBins + warp * 32 + lane;
+                    const int k = (m * kBins + warp * 32 + lane) >> sh;
                     // the bin's interval, clamped to the walk
                     float lo, hi;
                     if (KIND == kPara) {
@@ -414,20 +454,32 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
                         if (KIND == kFanWeighted) w *= dt[j + i];
                         acc[m].add(w, pix + (j + i) * P, pitch * P);
                     };
-                    // (past the last boundary, which bounds hi, the table may
-                    // hold anything: what starts there is empty)
-                    const float f0 = b[0], f1 = b[1], f2 = b[2];
-                    const float g1 = fmaxf(f0, lo), g2 = fmaxf(f1, g1);
-                    add(FSUB(fminf(f0, hi), lo), 0);
-                    add(FSUB(fminf(f1, hi), g1), 1);
-                    add(FSUB(fminf(f2, hi), g2), 2);
-                    float from = fmaxf(f2, g2);
-                    if (__any_sync(0xffffffffu, from < hi)) {   // wide bins
-                        for (int i = 3; from < hi && j + i <= last; i++) {
-                            const float f = b[i];
-                            add(FSUB(fminf(f, hi), from), i);
-                            from = fmaxf(f, from);
+                    if constexpr (!WIDE) {
+                        // (past the last boundary, which bounds hi, the table may
+                        // hold anything: what starts there is empty)
+                        const float f0 = b[0], f1 = b[1], f2 = b[2];
+                        const float g1 = fmaxf(f0, lo), g2 = fmaxf(f1, g1);
+                        add(FSUB(fminf(f0, hi), lo), 0);
+                        add(FSUB(fminf(f1, hi), g1), 1);
+                        add(FSUB(fminf(f2, hi), g2), 2);
+                        float from = fmaxf(f2, g2);
+                        if (__any_sync(0xffffffffu, from < hi)) {   // bins of a few pixels more
+                            for (int i = 3; from < hi && j + i <= last; i++) {
+                                const float f = b[i];
+                                add(FSUB(fminf(f, hi), from), i);
+                                from = fmaxf(f, from);
+                            }
                         }
+                    } else {   // wide bins: a lane takes every lanes-th pixel, three at a time
+                        int e = j + sub;
+                        do {
+#pragma unroll
+                            for (int q = 0; q < 3; q++) {   // (entry last + 1, as above: empty)
+                                const int i = min(e + q * lanes, last + 1);
+                                add(FSUB(fminf(bt[i], hi), fmaxf(bt[i - 1], lo)), i - j);
+                            }
+                            e += 3 * lanes;
+                        } while (e <= last && bt[e - 1] < hi);
                     }
                 }
             }
@@ -485,12 +537,24 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
     }
     if (ab) return false;
     if (rank != 0 || warp >= kCons) return true;
+    if constexpr (WIDE) {   // a bin's lanes, each other's sums by halves: the same order for any group of slices
+#pragma unroll
+        for (int m = 0; m < NPASS; m++) {
+            if (m >= npass) break;
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                float x = acc[m].get(b);
+                for (int o = 1; o < lanes; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+                acc[m].set(b, x);
+            }
+        }
+    }
     const float para_beta = xb ? FDIV(g.pix_y, g.det_size) : FDIV(g.pix_x, g.det_size);
 #pragma unroll
     for (int m = 0; m < NPASS; m++) {
         if (m >= npass) break;
-        const int k = m * kBins + warp * 32 + lane;
-        if (k >= D) continue;
+        const int k = (m * kBins + warp * 32 + lane) >> sh;
+        if (k >= D || sub != 0) continue;
         float beta = 1.0f;
         if (op == DD_OP_PROJ) beta = (KIND == kPara) ? para_beta : it.bcoef[(size_t)v * (D + 1) + k];
         const int ko = vwp->flip ? D - 1 - k : k;
