@@ -184,15 +184,15 @@ k_axis_views(int V, const DdView2 *__restrict__ views, int *__restrict__ axisv) 
 }
 
 // Single-geometry parallel-beam adjoint launch: grid (lines * cluster, image groups).
-template <int OPK>   // 0 ProjTrans, 1 BackProj
-__global__ void __cluster_dims__(kAdjCluster, 1, 1) __launch_bounds__(kThreads)
+template <int OPK, int NQ>   // OPK: 0 ProjTrans, 1 BackProj; NQ: pixels a thread without clusters (0: clusters)
+__global__ void __launch_bounds__(kThreads)
 k_adj_para(dd_geom2d g, int B, int V, int nl, int axis, const int *__restrict__ axisv,
            const DdLine *__restrict__ lines, const DdLine *__restrict__ dlines,
            const float2 *__restrict__ dtab, float *__restrict__ out, const float *__restrict__ base,
            float scale, int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
     AdjItem it = {};
-    it.c0 = blockIdx.x / kAdjCluster;
+    it.c0 = blockIdx.x / (NQ > 0 ? 1 : kAdjCluster);
     it.r0 = axis;
     it.b0 = blockIdx.y * kBI;
     it.nb = min(kBI, B - it.b0);
@@ -206,7 +206,7 @@ k_adj_para(dd_geom2d g, int B, int V, int nl, int axis, const int *__restrict__ 
     it.base = base;
     it.scale = scale;
     const ParaSmem S = para_smem(g.num_det, axis ? g.width : g.height, min(kBI, B));
-    if (!adj_para_line<OPK>(g, it, smem, S) && threadIdx.x == 0) dd_report_timeout(status);
+    if (!adj_para_line<OPK, NQ>(g, it, smem, S) && threadIdx.x == 0) dd_report_timeout(status);
 }
 
 // Adjoint map of fan beams (plan time): one CTA per (tile, view) fills the
@@ -425,6 +425,17 @@ int max_smem_optin() {
     return n;
 }
 
+int sm_count() {
+    static int n = 0;
+    if (n == 0) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+            n = 1;
+    }
+    return n;
+}
+
 // The forward CTA shape a tune asks for (slices per CTA, CTAs per view's
 // cluster), with the defaults where it asks for none, and 1 slice where lines
 // are too long for 4.
@@ -613,26 +624,56 @@ static int launch_adj(int op, const dd_geom2d *g, const PlanLayout &P, const cha
     return launch_adj_op<GEOM, 2>(g, P, planb, B, V, dtab, out, base, scale, status, st);
 }
 
+// Does one CTA take a line of the parallel beam's adjoint, instead of a cluster
+// of kAdjCluster?  It does where the detector tables leave room for no more than
+// two CTAs on an SM (the starts of three more are then not hidden by others) and
+// the lines fill the chip's waves of them to 0.85.  ms by four / by one, 4 / 8 /
+// 12 slices: 300^2, 200 views, 1,200 cells 0.54, 0.95, 1.35 / 0.45, 0.86, 1.26;
+// 400^2, 100 views, 1,600 cells 0.41, 0.73, 1.07 / (66 % full) 0.70, 0.72, 0.97.
+// With three CTAs and more by one: 256^2, 180 views, 1,024 cells, 12 slices
+// 0.75 / 1.18; 512^2, 360 views, 736 cells, 3 slices 0.83 / 1.11.
+static bool para_alone(int smem, int npix, long long lines) {
+    const int resident = 228 * 1024 / (smem + 1024 + 128);   // of 228 KB an SM, 1 KB goes to each CTA beside its own
+    if (resident > 2 || para_pixels(npix) > 4) return false;
+    const long long slots = (long long)sm_count() * resident;
+    return (double)lines >= 0.85 * (double)((lines + slots - 1) / slots * slots);
+}
+
 // Parallel-beam adjoint: the rows' launch writes, the columns' launch adds.
-static int launch_adj_para(int op, const dd_geom2d *g, const PlanLayout &P, const char *planb, int B, int V,
-                           const float2 *dtab, float *out, const float *base, float scale, int *status,
-                           cudaStream_t st) {
+template <int OPK>
+static int launch_adj_para(const dd_geom2d *g, const PlanLayout &P, const char *planb, int B, int V, const float2 *dtab,
+                           float *out, const float *base, float scale, int *status, cudaStream_t st) {
     const DdLine *lines = (const DdLine *)(planb + P.lines);
     const DdLine *dlines = (const DdLine *)(planb + P.dlines);
     const int *axisv = (const int *)(planb + P.axisv);
     const int W = g->width, H = g->height, D = g->num_det;
-    const int nbm = std::min(kBI, B);
-    const int smax = std::max(para_smem(D, W, nbm).total, para_smem(D, H, nbm).total);
-    if (smax > max_smem_optin()) return DD_ERR_SIZE_OVERFLOW;
-    auto kern = (op == DD_OP_PROJ_T) ? k_adj_para<0> : k_adj_para<1>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) != cudaSuccess)
-        return DD_ERR_LAUNCH;
+    const int nbm = std::min(kBI, B), groups = (B + kBI - 1) / kBI;
     ProfRec *pr = prof_begin(DD_KERNEL_ADJOINT, st);
     for (int axis = 1; axis >= 0; axis--) {
         const int npix = axis ? W : H, nline = axis ? H : W;
-        const dim3 grid((unsigned)nline * kAdjCluster, (unsigned)((B + kBI - 1) / kBI));
-        kern<<<grid, kThreads, para_smem(D, npix, nbm).total, st>>>(*g, B, V, P.nl, axis, axisv, lines, dlines, dtab,
-                                                                     out, base, scale, status);
+        const int smem = para_smem(D, npix, nbm).total;
+        if (smem > max_smem_optin()) return DD_ERR_SIZE_OVERFLOW;
+        const bool alone = para_alone(smem, npix, (long long)nline * groups);
+        const int cl = alone ? 1 : kAdjCluster;
+        auto kern = !alone ? k_adj_para<OPK, 0> : para_pixels(npix) <= 2 ? k_adj_para<OPK, 2> : k_adj_para<OPK, 4>;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+            return DD_ERR_LAUNCH;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)cl;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(nline * cl), (unsigned)groups);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = (size_t)smem;
+        cfg.stream = st;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        if (cudaLaunchKernelEx(&cfg, kern, *g, B, V, P.nl, axis, axisv, lines, dlines, dtab, out, base, scale, status) !=
+            cudaSuccess) {
+            (void)cudaGetLastError();
+            return DD_ERR_LAUNCH;
+        }
     }
     prof_end(pr, st);
     g_launches += 2;
@@ -701,7 +742,9 @@ int apply_planned(int scan, int op, const dd_geom2d *g, const void *planp, const
     float2 *dtab = (float2 *)(wb + A.dtab);
     const int ts = launch_det_tables(geom, op, g, planb, in, B, V, dtab, status, st);
     if (ts != DD_OK) return ts;
-    if (geom == DD_GEOM_PARA) return launch_adj_para(op, g, P, planb, B, V, dtab, out, base, scale, status, st);
+    if (geom == DD_GEOM_PARA)
+        return op == DD_OP_PROJ_T ? launch_adj_para<0>(g, P, planb, B, V, dtab, out, base, scale, status, st)
+                                  : launch_adj_para<1>(g, P, planb, B, V, dtab, out, base, scale, status, st);
     if (geom == DD_GEOM_FLAT) return launch_adj<DD_GEOM_FLAT>(op, g, P, planb, B, V, dtab, out, base, scale, status, st);
     return launch_adj<DD_GEOM_ARC>(op, g, P, planb, B, V, dtab, out, base, scale, status, st);
 }

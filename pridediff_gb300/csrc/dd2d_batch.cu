@@ -324,7 +324,7 @@ k_adj_items_para(const BatchInst *__restrict__ desc, const int4 *__restrict__ it
         s_g = d.g;
     }
     __syncthreads();
-    if (!adj_para_line<OPK>(s_g, s_it, smem, para_smem(Dmax, nmax, kBI)) && threadIdx.x == 0) dd_report_timeout(status);
+    if (!adj_para_line<OPK, 0>(s_g, s_it, smem, para_smem(Dmax, nmax, kBI)) && threadIdx.x == 0) dd_report_timeout(status);
 }
 
 // Adjoint items of fan beams: a cluster per item, in the list's order; 4 CTAs
@@ -359,17 +359,6 @@ k_adj_items(const BatchInst *__restrict__ desc, const int4 *__restrict__ items, 
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
-static int sm_count() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-            n = 1;
-    }
-    return n;
-}
-
 static int validate_batch(int scan, int op, const dd_instance2d *inst, int n) {
     if (!inst || n <= 0 || n > 65535) return DD_ERR_INVALID_ARG;
     if (op == DD_OP_BPROJ_W || op == DD_OP_BPROJ_TW) return DD_ERR_UNSUPPORTED;

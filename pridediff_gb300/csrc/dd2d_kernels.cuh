@@ -622,9 +622,13 @@ __device__ bool adj_tile_map(const dd_geom2d &g, const AdjItem &it, unsigned cha
 // (x-branch views) are written by one launch and the columns added by a
 // second.
 //
+// Where the lines fill the chip by themselves, one CTA takes a line: the same
+// parts of its views in turn, added in the same order, so with equal bits, and
+// without three more starts and a cluster's barriers.
+//
 // Bound by the chain of a view's steps (copy, piece constants, barrier, the
 // locates) for a few slices: 256^2, 180 views, both launches, 1 / 4 slices 0.26 /
-// 0.37 ms by one CTA a line, 0.17 / 0.23 ms here; by the locates where the
+// 0.37 ms by one CTA a line, 0.17 / 0.23 ms by four; by the locates where the
 // lines fill the chip by themselves: 16 slices of 512^2, 720 views, 9.3 -> 9.0.
 // ---------------------------------------------------------------------------
 struct ParaSmem {
@@ -642,17 +646,23 @@ __host__ __device__ inline ParaSmem para_smem(int D, int npix, int nb) {
     s.total = (o + 127) & ~127;
     return s;
 }
+// Pixels of a line that a thread adds to (its warp takes 31 of every 248).
+__host__ __device__ inline int para_pixels(int npix) { return (npix + kWarps * kBinsPerWarp - 1) / (kWarps * kBinsPerWarp); }
 
 // S: laid out for at least the item's detector, line and images.
-template <int OPK>   // 0 ProjTrans, 1 BackProj
+// NQ > 0: one CTA, not a cluster, for lines of at most NQ pixels a thread.
+template <int OPK, int NQ>   // OPK: 0 ProjTrans, 1 BackProj
 __device__ bool adj_para_line(const dd_geom2d &g, const AdjItem &it, unsigned char *smem, const ParaSmem &S) {
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    constexpr bool ALONE = NQ > 0;
     const int rank = (int)cluster.block_rank();
     const int W = g.width, H = g.height, D = g.num_det, V = it.V;
     const int axis = it.r0, line = it.c0, b0 = it.b0, nb = it.nb;
     const int npix = axis ? W : H;
     const int na = it.axisv[axis ? 0 : 1];
-    const int v0 = (int)((long long)na * rank / kAdjCluster), nv = (int)((long long)na * (rank + 1) / kAdjCluster) - v0;
+    // part p of the axis's views ends before index part_end(p); a rank takes its own part, a single CTA all of them
+    auto part_end = [&](int p) { return (int)((long long)na * (p + 1) / kAdjCluster); };
+    const int v0 = ALONE ? 0 : part_end(rank - 1), nv = (ALONE ? na : part_end(rank)) - v0;
     const int *vlist = it.axisv + 2 + (axis ? 0 : V) + v0;
     const int rsd = rs_entries(D);
     DdLine *rec = reinterpret_cast<DdLine *>(smem + S.rec);
@@ -664,6 +674,24 @@ __device__ bool adj_para_line(const dd_geom2d &g, const AdjItem &it, unsigned ch
     __shared__ int abort_flag;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i < nb * npix; i += kThreads) accs[i] = 0.0f;
+    // a single CTA: the sums of the parts so far of the pixels that the thread adds to
+    int part = 0;
+    float sum[ALONE ? NQ : 1][kBI];
+    auto close_part = [&]() {
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            const int pi = (q * kWarps + warp) * kBinsPerWarp + lane - 1;
+            const bool mine = lane > 0 && pi < npix;
+#pragma unroll
+            for (int b = 0; b < kBI; b++) {
+                if (b >= nb || !mine) continue;
+                float *x = accs + b * npix + pi;
+                sum[q][b] = part == 0 ? *x : sum[q][b] + *x;
+                *x = 0.0f;
+            }
+        }
+        part++;
+    };
     if (tid == 0) abort_flag = 0;
     init_bars(bar);   // synchronises the CTA
     DdPhases ph;
@@ -694,6 +722,8 @@ __device__ bool adj_para_line(const dd_geom2d &g, const AdjItem &it, unsigned ch
             break;
         }
         if (tid == issuer && idx + 1 < nv) issue(idx + 1, buf ^ 1);
+        if constexpr (ALONE)
+            while (idx >= part_end(part)) close_part();
         const DdLine &L = rec[buf], &Ld = drec[buf];
         if (L.h.npiece == 0) continue;   // the same for the whole CTA
         const int npd = Ld.h.npiece;
@@ -731,6 +761,26 @@ __device__ bool adj_para_line(const dd_geom2d &g, const AdjItem &it, unsigned ch
             }
         }
     }
+    auto put = [&](int b, int pi, float val) {
+        const int r = axis ? line : H - 1 - pi, c = axis ? pi : line;
+        const size_t o = ((size_t)(b0 + b) * H + r) * W + c;
+        if (axis) it.out[o] = it.base ? fmaf(it.scale, val, it.base[o]) : val;
+        else it.out[o] = it.base ? fmaf(it.scale, val, it.out[o]) : it.out[o] + val;
+    };
+    if constexpr (ALONE) {
+        __syncthreads();
+        if (abort_flag) return false;
+        while (part < kAdjCluster) close_part();
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            const int pi = (q * kWarps + warp) * kBinsPerWarp + lane - 1;
+            if (lane == 0 || pi >= npix) continue;
+#pragma unroll
+            for (int b = 0; b < kBI; b++)
+                if (b < nb) put(b, pi, sum[q][b]);
+        }
+        return true;
+    }
     cluster.sync();
     int ab = 0;
     for (int k = 0; k < kAdjCluster; k++) ab |= *cluster.map_shared_rank(&abort_flag, k);
@@ -738,13 +788,10 @@ __device__ bool adj_para_line(const dd_geom2d &g, const AdjItem &it, unsigned ch
         const int n = nb * npix;
         for (int i = rank * kThreads + tid; i < n; i += kAdjCluster * kThreads) {
             const int b = i / npix, pi = i - b * npix;
-            const int r = axis ? line : H - 1 - pi, c = axis ? pi : line;
-            const size_t o = ((size_t)(b0 + b) * H + r) * W + c;
             float val = cluster.map_shared_rank(accs, 0)[i];
 #pragma unroll
             for (int k = 1; k < kAdjCluster; k++) val += cluster.map_shared_rank(accs, k)[i];
-            if (axis) it.out[o] = it.base ? fmaf(it.scale, val, it.base[o]) : val;
-            else it.out[o] = it.base ? fmaf(it.scale, val, it.out[o]) : it.out[o] + val;
+            put(b, pi, val);
         }
     }
     cluster.sync();   // no rank leaves before the others have read its sums
@@ -762,6 +809,7 @@ int validate(int scan, int op, const dd_geom2d *g, int B, int V);
 int geom_of(int scan);
 int launch_status();
 int max_smem_optin();   // largest dynamic shared memory per CTA (opt-in) on this device
+int sm_count();
 // prefix tables of B sinograms of one geometry (adjoint)
 int launch_det_tables(int geom, int op, const dd_geom2d *g, const char *planb, const float *in, int B,
                       int V, float2 *dtab, int *status, cudaStream_t st);   // clears *status

@@ -202,3 +202,22 @@ def test_uneven_batch_of_wide_and_narrow_bins(scan):
     for p, a, x, y in zip(projs, angs, xs, ub.unpack_sinos(ub.forward(ub.pack(xs)))):
         # the two forwards' roundings, each within 1e-5 of exact arithmetic
         assert rel_l2(y.cpu().numpy(), p.projection(x, a).cpu().numpy()) <= 2e-5
+
+
+# Parallel adjoint: a line by one CTA (the lines fill the chip and the tables
+# leave room for two CTAs an SM) or by a cluster of four, with the same bits --
+# the uneven batch always takes the cluster.  1 to 4 pixels a thread, fewer
+# views than parts.
+@pytest.mark.parametrize("W,H,D,V,B", [(300, 270, 1200, 6, 4), (300, 270, 1200, 1, 4), (270, 560, 1300, 9, 5), (249, 300, 1800, 3, 9),
+                                       (900, 300, 1250, 4, 8), (300, 40, 1200, 5, 4)])
+def test_parallel_adjoint_by_one_and_four(oracle_mod, W, H, D, V, B):
+    import pridediff_gb300 as P
+    from pridediff_gb300.batch import UnevenBatch2d
+    proj = P.projector2d((W, H), D, 0.7, 0.7 * 1.3 * W / D, 595.0, 1085.6, scan_type="para").cuda()
+    ang = torch.arange(V, dtype=torch.float32, device="cuda") * (np.pi / V) + 0.3
+    y = torch.randn((B, 1, V, D), device="cuda", generator=torch.Generator(device="cuda").manual_seed(W))
+    out = proj.projection_t(y, ang)
+    ub = UnevenBatch2d([proj], [ang], [B])
+    assert torch.equal(ub.adjoint(y.reshape(-1)).reshape(out.shape), out)
+    ref = oracle_mod.run2d("para", "proj_t", y[:, 0].cpu().numpy(), ang.cpu().numpy(), proj.options.cpu().numpy(), nthreads=8)
+    assert rel_l2(out[:, 0].cpu().numpy(), ref) <= 1e-5
