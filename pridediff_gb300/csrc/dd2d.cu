@@ -136,7 +136,7 @@ k_fwd(dd_geom2d g, int geom, int op, int B, int V, int nl, const DdView2 *__rest
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ FwdState S;
     const FwdLay L = fwd_lay(KIND, g.num_det, g.num_det << sh, max(g.width, g.height), NB, cl);
-    fwd_init<NB>(smem, L, S);
+    fwd_init<KIND, NB>(smem, L, S);
     constexpr int planes = NB / plane_slices(NB);
     FwdItem it;
     it.v = blockIdx.x / cl;

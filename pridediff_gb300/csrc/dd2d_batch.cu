@@ -225,14 +225,13 @@ static_assert(prods(1) == prods(4) && prods(2) == prods(4), "items of 1, 2 and 4
 // WIDE: some instance's bins take more than one lane.
 template <int KIND, int NPASS, bool WIDE>
 __global__ void __launch_bounds__(fwd_threads(4), NPASS <= 4 ? 3 : 2)
-k_fwd_items(int geom, int op, const BatchInst *__restrict__ desc, const int4 *__restrict__ items, int nitems,
-            const char *__restrict__ plan, size_t plans_off, const char *__restrict__ tabs,
-            float *__restrict__ out, const float *__restrict__ sub, int Dmax, int lanes, int nmax, int fi, int cl,
+k_fwd_items(const __grid_constant__ FwdLay L, int geom, int op, const BatchInst *__restrict__ desc,
+            const int4 *__restrict__ items, int nitems, const char *__restrict__ plan, size_t plans_off,
+            const char *__restrict__ tabs, float *__restrict__ out, const float *__restrict__ sub, int cl,
             int *__restrict__ counter, int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ FwdState S;
-    const FwdLay L = fwd_lay(KIND, Dmax, lanes, nmax, fi, cl);   // of the largest items
-    fwd_init<4>(smem, L, S);
+    fwd_init<KIND, 4>(smem, L, S);
     // the item and its geometry live in shared memory: read where used, they
     // hold no registers across the line loop (the plain forward reads them
     // from kernel parameters)
@@ -424,9 +423,9 @@ static int launch_fwd_items_as(int geom, int op, const BatchLayout &L, const cha
         cfg.gridDim = dim3((unsigned)(clusters * cl));
     }
     ProfRec *pr = prof_begin(DD_KERNEL_FORWARD, st);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, geom, op, (const BatchInst *)(planb + L.desc),
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, S, geom, op, (const BatchInst *)(planb + L.desc),
                                              (const int4 *)(planb + L.fitems), L.nfwd, planb, L.plans, (const char *)tabs,
-                                             out, sub, L.Dmax, L.lanes, L.nmax, L.fi, cl, counter, status);
+                                             out, sub, cl, counter, status);
     prof_end(pr, st);
     count_launches(1);
     if (e != cudaSuccess) {

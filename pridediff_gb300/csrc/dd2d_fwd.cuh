@@ -44,7 +44,7 @@ __host__ __device__ constexpr int pick4(int nb, int a, int b, int c, int d) { re
 __host__ __device__ constexpr int prods(int nb) { return pick4(nb, 4, 4, 4, 3); }
 __host__ __device__ constexpr int stages(int nb) { return pick4(nb, 8, 6, 4, 3); }
 constexpr int kCons = 8;
-constexpr int kRecs = 4;   // line records in flight per producer
+constexpr int kMaxRecs = 4;
 constexpr int kMaxProd = 4, kMaxStages = 8;
 constexpr int kBins = kCons * 32;   // bins of one pass of the consumers
 __host__ __device__ constexpr int fwd_threads(int nb) { return (kCons + prods(nb)) * 32; }
@@ -55,6 +55,8 @@ static_assert(prods(1) <= stages(1) && prods(2) <= stages(2) && prods(4) <= stag
 // (parts scaled per line and pixel); the parallel beam; the unweighted
 // transpose of a fan beam (parts scaled per line).
 enum { kFan = 0, kFanWeighted = 1, kPara = 2, kFanScaled = 3 };
+// Line records in flight per producer (the parallel beam's are twice as large).
+__host__ __device__ constexpr int recs(int kind) { return kind == kPara ? 2 : kMaxRecs; }
 
 // Passes over the detector, rounded up to the instantiated classes (the
 // accumulators of a thread are NPASS x NB).
@@ -117,7 +119,9 @@ struct FwdLay {
     int ks;                    // stages: stages(nb), or as many as fit
 };
 constexpr int kSmemMax = 227 * 1024;
-constexpr int kFwdStatic = 512;   // of which the kernels' static arrays take no more than this
+// ... and to each of three CTAs on an SM, whose 228 KB also hold 1 KB per CTA
+constexpr int kSmemThird = 228 * 1024 / 3 - 1024;
+constexpr int kFwdStatic = 256;   // of either the kernels' static arrays take no more than this
 // boundary e of a line sits at entry e + kB0 of its table
 constexpr int kB0 = 4;
 // lanes: the lanes that all bins take (D << fwd_lanes).
@@ -130,25 +134,36 @@ __host__ __device__ inline FwdLay fwd_lay(int kind, int D, int lanes, int npix, 
               : kind == kFanWeighted ? ((npix + 3) & ~3) * (int)sizeof(float)
                                      : 0;
     s.pix_b = nb / p * plane_pitch(npix, p) * p * (int)sizeof(float);
-    int o = 0;
     const int kP = prods(nb), red = pass_class(lanes) * nb * kCons * 32 * (int)sizeof(float);
-    const int fixed = (para ? 2 : 1) * kP * kRecs * (int)sizeof(DdLine) + (2 * stages(nb) + kRecs * kP) * 8 + kFwdStatic;
+    const int kRecs = recs(kind);
+    auto lay = [&](int kS) {
+        int o = 0;
+        s.ks = kS;
+        s.hdr = o; o += kS * 2 * (int)sizeof(float4);
+        s.rec = o; o += kP * kRecs * (int)sizeof(DdLine);
+        s.drec = o; o += para ? kP * kRecs * (int)sizeof(DdLine) : 0;
+        s.bar = o; o += (2 * kS + kRecs * kP) * (int)sizeof(uint64_t);
+        o = (o + 15) & ~15;
+        s.bnd = o; o += kS * s.bnd_b;
+        s.det = o; o += kS * s.det_b;
+        // the sums of the even lines (cl = 1) or of the other CTA (cl = 2, after
+        // the last line: in the pixels' space)
+        s.pix = o; o += cl > 1 && red > kS * s.pix_b ? red : kS * s.pix_b;
+        s.red = cl > 1 ? s.pix : o;
+        if (cl == 1) o += red;
+        s.total = (o + 127) & ~127;
+        return s.total + kFwdStatic;
+    };
     int kS = stages(nb);
-    while (kS > kP && fixed + kS * (s.bnd_b + s.det_b + s.pix_b + 32) + (cl == 1 ? red : 0) > kSmemMax) kS--;
-    s.ks = kS;
-    s.hdr = o; o += kS * 2 * (int)sizeof(float4);
-    s.rec = o; o += kP * kRecs * (int)sizeof(DdLine);
-    s.drec = o; o += para ? kP * kRecs * (int)sizeof(DdLine) : 0;
-    s.bar = o; o += (2 * kS + kRecs * kP) * (int)sizeof(uint64_t);
-    o = (o + 15) & ~15;
-    s.bnd = o; o += kS * s.bnd_b;
-    s.det = o; o += kS * s.det_b;
-    // the sums of the even lines (cl = 1) or of the other CTA (cl = 2, after
-    // the last line: in the pixels' space)
-    s.pix = o; o += cl > 1 && red > kS * s.pix_b ? red : kS * s.pix_b;
-    s.red = cl > 1 ? s.pix : o;
-    if (cl == 1) o += red;
-    s.total = (o + 127) & ~127;
+    while (lay(kS) > kSmemMax && kS > kP) kS--;
+    // a third CTA on an SM before the last stages, where the sums leave it
+    // registers (24 uneven parallel-beam instances of 1 to 3 slices: 10.3 ms with
+    // two CTAs, of 4 records a producer and all stages; 7.9 ms with three)
+    if (pass_class(lanes) * nb <= 24) {
+        int k = kS;
+        while (lay(k) > kSmemThird && k > kP) k--;
+        if (k == kP) lay(kS);
+    }
     return s;
 }
 
@@ -172,7 +187,7 @@ struct FwdItem {
 struct FwdState {
     int abort;
     int armed[kMaxStages];       // uses of each stage so far
-    int nrec[kMaxProd][kRecs];   // copies into each record buffer so far
+    int nrec[kMaxProd][kMaxRecs];   // copies into each record buffer so far
 };
 
 // NB slices' values of one pixel, and sums of them.
@@ -270,9 +285,9 @@ __device__ __forceinline__ void fill_weights(const dd_geom2d &g, const DdView2 &
 }
 
 // Sets up a CTA's barriers and state (all threads; ends with a CTA barrier).
-template <int NB>
+template <int KIND, int NB>
 __device__ __forceinline__ void fwd_init(unsigned char *smem, const FwdLay &L, FwdState &S) {
-    constexpr int kP = prods(NB);
+    constexpr int kP = prods(NB), kRecs = recs(KIND);
     const int kS = L.ks;
     if (threadIdx.x == 0) {
         uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L.bar);
@@ -303,7 +318,7 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
                          const FwdLay &L, FwdState &S, uint32_t &step, uint32_t &nr) {
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const int CL = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-    constexpr int P = plane_slices(NB), NPL = NB / P, kP = prods(NB);
+    constexpr int P = plane_slices(NB), NPL = NB / P, kP = prods(NB), kRecs = recs(KIND);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int D = g.num_det, v = it.v;
     const int kS = L.ks;

@@ -221,3 +221,19 @@ def test_parallel_adjoint_by_one_and_four(oracle_mod, W, H, D, V, B):
     assert torch.equal(ub.adjoint(y.reshape(-1)).reshape(out.shape), out)
     ref = oracle_mod.run2d("para", "proj_t", y[:, 0].cpu().numpy(), ang.cpu().numpy(), proj.options.cpu().numpy(), nthreads=8)
     assert rel_l2(out[:, 0].cpu().numpy(), ref) <= 1e-5
+
+
+# Stages given up for a third CTA on an SM (parallel beam, 2 records a
+# producer): 8, 7, 6 and 5 stages of one and two slices, both cluster sizes.
+@pytest.mark.parametrize("W,D", [(512, 736), (600, 800), (700, 900), (900, 1000)])
+@pytest.mark.parametrize("scan,B", [("para", 1), ("para", 2), ("flat", 1)])
+def test_forward_stages(oracle_mod, scan, B, W, D):
+    pix = 0.5
+    opt = [W, 24, D, pix, pix, {"para": 1.0, "flat": 1085.6 / 595.0}[scan] * 1.1 * W * pix / D, 595.0, 1085.6, 0.1, -0.2, 0.1]
+    ang = (np.arange(5) * 2 * np.pi / 5 + 0.1).astype(np.float32)
+    x = np.random.default_rng(W + B).random((B, 24, W), dtype=np.float32)
+    ref = oracle_mod.run2d(scan, "proj", x, ang, opt, nthreads=8)
+    out = [_apply(scan, "proj", opt, ang, x, s, c) for s in (4, 1) for c in (2, 1)]
+    assert rel_l2(out[0], ref) <= 1e-5
+    for o in out[1:]:
+        assert np.array_equal(o, out[0])
