@@ -542,6 +542,7 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
 #pragma unroll
                 for (int b = 0; b < NB; b++) red[(m * NB + b) * (kCons * 32) + tid] = acc[m].get(b);
             }
+            dd_fence_async();   // the next item's copies land where these sums lie
         }
         cluster.sync();
         for (int r = 0; r < CL; r++) ab = ab || *cluster.map_shared_rank(&S.abort, r) != 0;

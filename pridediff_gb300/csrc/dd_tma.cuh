@@ -84,6 +84,12 @@ __device__ __forceinline__ void dd_tensor4_g2s(void *dst, const void *map, int c
         : "memory");
 }
 
+// Orders this thread's plain stores to shared memory before later bulk copies
+// into the same bytes (issued by any thread past the next barrier).
+__device__ __forceinline__ void dd_fence_async() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 __device__ __forceinline__ bool dd_mbar_try_wait(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
