@@ -731,7 +731,7 @@ int apply_planned(int scan, int op, const dd_geom2d *g, const void *planp, const
         if (op == DD_OP_BPROJ_TW) return launch_fwd<kFanWeighted>(c, bi == 1, B, in, wb + A.tabx, wb + A.taby, out);
         // (the reason stands at dd2d_prefix.cuh's head; not where the lines'
         // tables are too long for shared memory)
-        if (geom == DD_GEOM_ARC && op == DD_OP_PROJ && B <= 2 &&
+        if (geom == DD_GEOM_ARC && op == DD_OP_PROJ && B <= 2 && prefix_near(*g) &&
             prefix_smem(g->num_det, rs_entries(std::max(g->width, g->height)), B).total <= max_smem_optin()) {
             float2 *tx = (float2 *)(wb + A.tabx), *ty = (float2 *)(wb + A.taby);
             return B == 1 ? launch_prefix<1>(c, B, in, tx, ty, out) : launch_prefix<2>(c, B, in, tx, ty, out);

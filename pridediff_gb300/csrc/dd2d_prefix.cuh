@@ -4,18 +4,27 @@
 //     F(u) = K_p + dl_p S_j + r x_j
 // from the line's prefix table (S_j, x_j) and per-run constants.
 //
-// Why it stays beside the overlap forward (dd2d_fwd.cuh): an arc fan's A x is
-// what a data-consistency block feeds to the ramp filter, which amplifies a
-// different rounding of A x from 6.6e-7 to 5.7e-6 (relative, 2 x 512^2, 720
-// views, 768 cells); the gradient of the block's learned weight, a sum over
-// the image that cancels, then moved by up to 2.4e-5.  For one or two slices
-// the overlaps gain too little for that (512^2, 720 views, 736 bins: 0.64 /
-// 0.72 ms against 0.69 / 0.80 ms here); from three on they serve up to 8
-// slices at once (3 / 16 slices: 0.77 / 2.2 ms against 0.94 / 3.6 ms).
+// Why it stays beside the overlap forward (dd2d_fwd.cuh): for the values of the
+// arc fan's A x that one or two slices have had, not for their accuracy.  A data-
+// consistency block feeds A x to the ramp filter, and the gradient of its learned
+// weight is a sum over the image that cancels: with overlaps it moved by up to
+// 4.5e-4 (2 slices 3.1e-5; 2 x 512^2, 720 views, 768 cells, 10 inputs).  Against 64-bit sums over
+// the same boundaries the overlaps are the nearer ones: A x 1.8e-7 against
+// 6.7e-7 here, its filtered back-projection 1.5e-6 against 6.2e-6.  From three
+// slices on they serve up to 8 at once (3 / 16 slices: 0.77 / 2.2 ms against
+// 0.94 / 3.6 ms; 1 / 2 slices 0.64 / 0.72 against 0.69 / 0.80).
+//
+// A difference of two prefix sums rounds as the line's whole integral does: of
+// N pixels, at c pixels a cell, over L lines, 2^-25 (N / c) sqrt(2 / L) of a bin's
+// sum.  prefix_near keeps it below 1.4e-6; where cells are a small part of a pixel
+// or lines few and long (1090 x 5 pixels, 1,984 cells: 1.4e-5 off the
+// reference), overlaps serve one and two slices too.
 //
 // Bound by the shared-memory gathers and the search of the drift record per
 // boundary, which one or two slices hardly share.
 #pragma once
+
+#include <cmath>
 
 #include "dd2d_kernels.cuh"
 
@@ -33,6 +42,11 @@ __device__ __forceinline__ Loc locate(const DdLine &L, float u) {
     l.r = rr;
     l.dl = L.p[l.p].dl;
     return l;
+}
+
+inline bool prefix_near(const dd_geom2d &g) {
+    const double c = (double)g.det_size * g.iso_source / std::max(g.pix_x, g.pix_y), w = g.width, h = g.height;
+    return std::max(w / std::sqrt(h), h / std::sqrt(w)) <= 32.0 * c;
 }
 
 // Detector passes of 8 warps x 31 bins, rounded up to the instantiated classes.
