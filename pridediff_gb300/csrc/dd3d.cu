@@ -812,7 +812,6 @@ struct Adj3Args {
     int *status;
     int B, V, ntx;
     int b0, family;      // first volume of the launch; operator family (dd3_coef)
-    int bufs;            // buffers of staged units: 3, or 2 (adj3_smem)
 };
 
 // Shared memory of the adjoint kernel: buffers of one (view, walk block)'s data
@@ -919,7 +918,7 @@ __global__ void __launch_bounds__(256) k_slab_views3(dd_geom3d g, char *plan, Pl
 // view staged and searched, and 8 slices a thread; 192 ms with the carried
 // row walk alone; 108 ms with the unit list, the linear column estimate and
 // 16 slices.  2 x 256^3 cone beam, 360 views: 145, 63, 49 ms.
-template <int GEOM, int NB, int ZS>
+template <int GEOM, int NB, int ZS, int BUFS>
 __global__ void __launch_bounds__(kThreads, 3) k_adj3(const Adj3Args a) {
     using VT = Vox<NB>;
     using T = typename VT::T;
@@ -927,8 +926,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_adj3(const Adj3Args a) {
     const dd_geom3d &g = a.g;
     const int W = g.width, H = g.height, Dp = g.depth, C = g.num_col, R = g.num_row;
     const PlanLayout &P = a.P;
-    const int bufs = a.bufs;
-    const Adj3Smem S = adj3_smem(P, bufs);
+    const Adj3Smem S = adj3_smem(P, BUFS);
     const int tid = threadIdx.x, lane = tid & 31;
     const int tX = blockIdx.x % a.ntx, tY = blockIdx.x / a.ntx;
     const int xlo = tX * kTile, ylo = tY * kTile;
@@ -949,7 +947,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_adj3(const Adj3Args a) {
 
     if (tid == 0) {
         abort_flag = 0;
-        for (int i = 0; i < bufs; i++) dd_mbar_init(&bar[i], 1);
+        for (int i = 0; i < BUFS; i++) dd_mbar_init(&bar[i], 1);
         dd_fence_mbar_init();
     }
     __syncthreads();
@@ -1077,8 +1075,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_adj3(const Adj3Args a) {
     for (int q = 0; q < ZS; q++) acc[q] = VT::zero();
 
     DdPhases ph;
-    // unit i uses buffer i % bufs; the bufs - 1 units behind it are in flight
-    const int ahead = bufs - 1;
+    // unit i uses buffer i % BUFS; the BUFS - 1 units behind it are in flight
+    constexpr int ahead = BUFS - 1;
     if (tid < 32) {
         next(&units[0]);
         if (ahead > 1) next(&units[1]);
@@ -1365,27 +1363,31 @@ int launch_fwd_volumes(Fwd3Args a, int b0, int ngroups, cudaStream_t st) {
     return launch_fwd_rows<NB, 2>(a, ngroups, st);
 }
 
-template <int GEOM, int NB, int ZS>
+template <int GEOM, int NB, int ZS, int BUFS>
 int launch_adj_slabs(const Adj3Args &a, int ngroups, cudaStream_t st) {
-    const int smem = adj3_smem(a.P, a.bufs).total;
-    if (cudaFuncSetAttribute(k_adj3<GEOM, NB, ZS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return DD_ERR_LAUNCH;
+    const int smem = adj3_smem(a.P, BUFS).total;
+    auto kern = k_adj3<GEOM, NB, ZS, BUFS>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return DD_ERR_LAUNCH;
     const int nty = (a.g.height + kTile - 1) / kTile;
     const dim3 grid((unsigned)(a.ntx * nty), (unsigned)((a.g.depth + ZS - 1) / ZS), (unsigned)ngroups);
-    k_adj3<GEOM, NB, ZS><<<grid, kThreads, smem, st>>>(a);
+    kern<<<grid, kThreads, smem, st>>>(a);
     dd2::count_launches(1);
     return DD_OK;
 }
 
 // 16 slices per thread share a pixel's columns and boundaries; 8 where 16
 // would leave the chip's 456 resident CTAs (3 per SM) less than twice full.
+// Detectors whose row tables leave no room for three buffers (1 KB is for the
+// kernel's static arrays) take two, 8 slices a thread.
 template <int GEOM, int NB>
 int launch_adj_kernel(Adj3Args a, int b0, int ngroups, cudaStream_t st) {
     if (ngroups <= 0) return DD_OK;
     a.b0 = b0;
+    if (adj3_smem(a.P, kAdj3Bufs).total + 1024 > 227 * 1024) return launch_adj_slabs<GEOM, NB, kZS, 2>(a, ngroups, st);
     const long long tiles = (long long)a.ntx * ((a.g.height + kTile - 1) / kTile) * ngroups;
-    if (tiles * ((a.g.depth + 2 * kZS - 1) / (2 * kZS)) >= 2 * 456) return launch_adj_slabs<GEOM, NB, 2 * kZS>(a, ngroups, st);
-    return launch_adj_slabs<GEOM, NB, kZS>(a, ngroups, st);
+    if (tiles * ((a.g.depth + 2 * kZS - 1) / (2 * kZS)) >= 2 * 456)
+        return launch_adj_slabs<GEOM, NB, 2 * kZS, kAdj3Bufs>(a, ngroups, st);
+    return launch_adj_slabs<GEOM, NB, kZS, kAdj3Bufs>(a, ngroups, st);
 }
 
 template <int GEOM>
@@ -1459,8 +1461,6 @@ int adjoint(int scan, int op, const dd_geom3d *g, const char *planb, const float
     a.ntx = (g->width + kTile - 1) / kTile;
     a.b0 = 0;
     a.family = op_family(op);
-    // (1 KB: the kernel's static arrays, which come out of the same 227 KB)
-    a.bufs = adj3_smem(a.P, kAdj3Bufs).total + 1024 <= 227 * 1024 ? kAdj3Bufs : 2;
     const int geom = geom_of(scan);
     if (geom == DD_GEOM3_CONE_FLAT) return launch_adj<DD_GEOM3_CONE_FLAT>(a, in, (float *)ss, st);
     if (geom == DD_GEOM3_CONE_ARC) return launch_adj<DD_GEOM3_CONE_ARC>(a, in, (float *)ss, st);
