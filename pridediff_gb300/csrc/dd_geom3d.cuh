@@ -452,6 +452,8 @@ DD_HD int dd3_pixel_of(const DdLine *L, float u, int *p) {
 // ---------------------------------------------------------------------------
 DD_HD float dd3_zb(float p0z, float pintz, int s) { return dd3_mul_add((float)s, pintz, p0z); }
 
+// The width of one (row, slice) cell, and the first slice of a row's own walk:
+// the host model's; the kernels carry both through one merge of rows and slices.
 DD_HD float dd3_cell(float bz0, float bz1, float zlo, float zhi) {
     const float lo = bz0 > zlo ? bz0 : zlo;
     const float hi = bz1 < zhi ? bz1 : zhi;
@@ -573,7 +575,8 @@ DD_HD bool dd3_colwalk_next(const DdLine *L, DdColWalk *cw, int *j, float *w) {
 }
 
 // ---------------------------------------------------------------------------
-// Segments of one pixel in one walk block (adjoint-type kernels)
+// Segments of one pixel in one walk block (the host model's walk; k_adj3 takes
+// dd3_pix_bounds and settles a linear estimate of the first column)
 // ---------------------------------------------------------------------------
 struct DdPixWalk {
     int k, klo, khi;
@@ -639,7 +642,8 @@ DD_HD float dd3_coef(int geom, int family, const dd_geom3d *g, const DdView3 *w,
 }
 
 // ---------------------------------------------------------------------------
-// Rows of one column that may meet a slice (adjoint-type kernels)
+// Rows of one column that may meet a slice (the host model of the per-slice
+// walk; k_adj3 carries the row from slice to slice)
 // ---------------------------------------------------------------------------
 // rowz: the view's row table {row0z, row1z} x R.  Returns the first row
 // whose upper boundary on the line plane may exceed zlo - margin; callers
