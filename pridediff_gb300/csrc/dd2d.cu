@@ -131,11 +131,13 @@ __global__ void __launch_bounds__(fwd_threads(NB), NPASS * NB <= 24 ? 3 : 2)
 k_fwd(dd_geom2d g, int geom, int op, int B, int V, int nl, const DdView2 *__restrict__ views,
       const float *__restrict__ dp, const float *__restrict__ bcoef, const DdLine *__restrict__ lines,
       const DdLine *__restrict__ dlines, const float *__restrict__ rows, const float *__restrict__ cols,
-      size_t rplane, size_t cplane, float *__restrict__ out, const float *__restrict__ sub, int cl, int sh,
+      size_t rplane, size_t cplane, float *__restrict__ out, const float *__restrict__ sub, int cl, int sh, int ks,
       int *__restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ FwdState S;
-    const FwdLay L = fwd_lay(KIND, g.num_det, g.num_det << sh, max(g.width, g.height), NB, cl);
+    // (a constant where there is no choice: the stages' indices are then cheaper)
+    const FwdLay L = fwd_lay(KIND, g.num_det, g.num_det << sh, max(g.width, g.height), NB, cl,
+                             stages(NB) > prods(NB) ? ks : stages(NB));
     fwd_init<KIND, NB>(smem, L, S);
     constexpr int planes = NB / plane_slices(NB);
     FwdItem it;
@@ -489,7 +491,7 @@ static int launch_fwd_group(const FwdCall &c, const float *in, int n, float *row
     ProfRec *pr = prof_begin(DD_KERNEL_FORWARD, c.st);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, *c.g, c.geom, c.op, n, c.V, c.nl, c.views, c.dp, c.bcoef, c.lines,
                                              c.dlines, (const float *)rows, (const float *)cols, rplane, cplane, out, sub,
-                                             c.cl, c.sh, c.status);
+                                             c.cl, c.sh, L.ks, c.status);
     prof_end(pr, c.st);
     g_launches += 2;
     if (e != cudaSuccess) {
@@ -931,7 +933,7 @@ extern "C" const char *dd_status_string(int status) {
     }
 }
 
-extern "C" const char *dd_version(void) { return "pridediff_dd 0.3 sm_103a"; }
+extern "C" const char *dd_version(void) { return "pridediff_dd 0.4 sm_103a"; }
 
 extern "C" unsigned long long dd_launch_count(void) { return g_launches; }
 

@@ -124,8 +124,8 @@ constexpr int kSmemThird = 228 * 1024 / 3 - 1024;
 constexpr int kFwdStatic = 256;   // of either the kernels' static arrays take no more than this
 // boundary e of a line sits at entry e + kB0 of its table
 constexpr int kB0 = 4;
-// lanes: the lanes that all bins take (D << fwd_lanes).
-__host__ __device__ inline FwdLay fwd_lay(int kind, int D, int lanes, int npix, int nb, int cl) {
+// lanes: the lanes that all bins take (D << fwd_lanes); ks: the stages.
+__host__ __device__ inline FwdLay fwd_lay(int kind, int D, int lanes, int npix, int nb, int cl, int ks) {
     FwdLay s;
     const int p = plane_slices(nb);
     s.bnd_b = ((npix + kB0 + 8 + 3) & ~3) * (int)sizeof(float);
@@ -135,36 +135,36 @@ __host__ __device__ inline FwdLay fwd_lay(int kind, int D, int lanes, int npix, 
                                      : 0;
     s.pix_b = nb / p * plane_pitch(npix, p) * p * (int)sizeof(float);
     const int kP = prods(nb), red = pass_class(lanes) * nb * kCons * 32 * (int)sizeof(float);
-    const int kRecs = recs(kind);
-    auto lay = [&](int kS) {
-        int o = 0;
-        s.ks = kS;
-        s.hdr = o; o += kS * 2 * (int)sizeof(float4);
-        s.rec = o; o += kP * kRecs * (int)sizeof(DdLine);
-        s.drec = o; o += para ? kP * kRecs * (int)sizeof(DdLine) : 0;
-        s.bar = o; o += (2 * kS + kRecs * kP) * (int)sizeof(uint64_t);
-        o = (o + 15) & ~15;
-        s.bnd = o; o += kS * s.bnd_b;
-        s.det = o; o += kS * s.det_b;
-        // the sums of the even lines (cl = 1) or of the other CTA (cl = 2, after
-        // the last line: in the pixels' space)
-        s.pix = o; o += cl > 1 && red > kS * s.pix_b ? red : kS * s.pix_b;
-        s.red = cl > 1 ? s.pix : o;
-        if (cl == 1) o += red;
-        s.total = (o + 127) & ~127;
-        return s.total + kFwdStatic;
-    };
-    int kS = stages(nb);
-    while (lay(kS) > kSmemMax && kS > kP) kS--;
-    // a third CTA on an SM before the last stages, where the sums leave it
-    // registers (24 uneven parallel-beam instances of 1 to 3 slices: 10.3 ms with
-    // two CTAs, of 4 records a producer and all stages; 7.9 ms with three)
-    if (pass_class(lanes) * nb <= 24) {
-        int k = kS;
-        while (lay(k) > kSmemThird && k > kP) k--;
-        if (k == kP) lay(kS);
-    }
+    int o = 0;
+    s.ks = ks;
+    s.hdr = o; o += ks * 2 * (int)sizeof(float4);
+    s.rec = o; o += kP * recs(kind) * (int)sizeof(DdLine);
+    s.drec = o; o += para ? kP * recs(kind) * (int)sizeof(DdLine) : 0;
+    s.bar = o; o += (2 * ks + recs(kind) * kP) * (int)sizeof(uint64_t);
+    o = (o + 15) & ~15;
+    s.bnd = o; o += ks * s.bnd_b;
+    s.det = o; o += ks * s.det_b;
+    // the sums of the even lines (cl = 1) or of the other CTA (cl = 2, after
+    // the last line: in the pixels' space)
+    s.pix = o; o += cl > 1 && red > ks * s.pix_b ? red : ks * s.pix_b;
+    s.red = cl > 1 ? s.pix : o;
+    if (cl == 1) o += red;
+    s.total = (o + 127) & ~127;
     return s;
+}
+// With stages(nb) of them, or as many as fit; fewer for a third CTA on an SM,
+// where the sums leave it registers and there is more than one a producer (24
+// uneven parallel-beam instances of 1 to 3 slices: 10.3 ms with two CTAs, of 4
+// records a producer and all stages; 7.9 ms with three).
+inline FwdLay fwd_lay(int kind, int D, int lanes, int npix, int nb, int cl) {
+    const int kP = prods(nb);
+    auto of = [&](int ks) { return fwd_lay(kind, D, lanes, npix, nb, cl, ks); };
+    int ks = stages(nb);
+    while (ks > kP && of(ks).total + kFwdStatic > kSmemMax) ks--;
+    if (pass_class(lanes) * nb <= 24)
+        for (int k = ks; k > kP; k--)
+            if (of(k).total + kFwdStatic <= kSmemThird) return of(k);
+    return of(ks);
 }
 
 // Do NB slices side by side fit a CTA?
