@@ -21,8 +21,8 @@ arc (the 512^2 fan geometry above; --size, --dets change it), para (1 mm
 pixels and cells, views over 180 deg), --op fbp for filtered_backprojection, cone_flat or cone_arc (256^3, 512 x 384
 detector, SID 500 / SDD 1000, --views of 360 angles over 360 deg), spiral
 (512 x 512 x 128, 64 x 736 arc detector, the first --views views of the
-comparator's middle turn) or uneven (the 24-instance uneven batch, one persistent launch
-per call; --op proj or proj_t).  With --impl reference it times deeprecon's
+comparator's middle turn) or uneven (the 24-instance uneven batch, all instances in one
+launch; --op proj or proj_t).  With --impl reference it times deeprecon's
 own CUDA kernel for the same operator (built from the reference sources into
 oracle/_ref/cuda where they exist).
 
@@ -396,8 +396,8 @@ def run_extras(dev, flush, peak, step2d, x0, y, B):
         ms_eager = _timed(lambda: ub.dc_step(xe, yb, 1e-3), 3, flush, ev)
         out["batched_dc_24_uneven"] = {
             "what": "24 uneven fan-flat instances (image {256,384,512}^2, views {360,576,720}, dets "
-                    "{368,512,736}), x <- x - 1e-3 A^T(Ax - y), 50 steps in one CUDA graph, one persistent "
-                    "launch per operator, launch shape autotuned",
+                    "{368,512,736}), x <- x - 1e-3 A^T(Ax - y), 50 steps in one CUDA graph, one launch "
+                    "per operator, launch shape autotuned",
             "tune": tune, "ms_per_step": ms / steps, "ms_per_step_eager_no_graph": ms_eager,
             "value": 24 * steps / (ms / 1e3), "unit": UNIT, **frac(nbytes, ms / steps),
             "bytes_model": "view-swept 4*V*(H*W + D) per instance and operator, FP + BP per step"}

@@ -126,7 +126,7 @@ int dd2d_dc_step(int scan, const dd_geom2d *g, const void *plan, float *x, const
                  float eta, int batch, int num_view, void *workspace, size_t workspace_bytes,
                  dd_stream_t stream);
 
-/* ---- 2-D: uneven batches in one persistent launch --------------------------
+/* ---- 2-D: uneven batches, all instances in one launch -----------------------
  * No counterpart in the reference, which runs one uniform geometry per call
  * (batch folded into gridDim.x, ParaDisCUDA2d.cu:334-337).  An uneven batch
  * is n instances of one scan type, each with its own geometry, view count and
@@ -162,7 +162,8 @@ int dd2d_apply_planned_tuned(int scan, int op, const dd_geom2d *g, const void *p
                              const dd_tune2d *tune, dd_stream_t stream);
 /* The forward CTA shape a tune resolves to on this geometry (slices per CTA,
  * cluster size): 4 slices become 1 where lines are too long for 4 (more than
- * about 3,400 pixels). */
+ * about 3,400 pixels).  "4" is groups of up to 8, of 4 or of 2, by what fits the
+ * lines. */
 int dd2d_fwd_shape(int scan, const dd_geom2d *g, const dd_tune2d *tune, int *slices, int *cluster);
 
 size_t dd2d_batch_plan_bytes(int scan, const dd_instance2d *inst, int n);

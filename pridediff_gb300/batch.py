@@ -1,12 +1,13 @@
-"""Uneven batches of 2-D projections in one persistent launch, and the
+"""Uneven batches of 2-D projections, one launch for all instances, and the
 graph-captured data-consistency (DC) loop.
 
 ``UnevenBatch2d`` takes a list of ``projector2d`` modules of one scan type
 (each with its own image size, detector count and angles) and runs the
 forward projection, the exact adjoint, or the DC step
-``x <- x - eta * A^T (A x - y)`` of all of them together: one persistent
-kernel launch per operator, work items pulled longest-first from a device
-counter (``libpridediff_dd.so``: dd2d_batch_*).
+``x <- x - eta * A^T (A x - y)`` of all of them together: one launch per
+operator beside its tables' (two for the adjoint of a parallel beam), work
+items longest first, the forward's pulled from a device counter by a persistent
+grid (``libpridediff_dd.so``: dd2d_batch_*).
 
 Tensors are packed into flat float32 tensors; ``pack`` and ``unpack_*``
 convert from/to lists of (batch_i, 1, H_i, W_i) images or (batch_i, 1, V_i,

@@ -1,4 +1,5 @@
-// Batched 2-D DD projection over uneven instances in one persistent launch.
+// Batched 2-D DD projection over uneven instances, one launch an operator (two
+// for the adjoint of a parallel beam) beside the tables'.
 //
 // An uneven batch is a list of instances, each with its own image size,
 // view count, detector count and number of slices (one scan type per batch).
@@ -10,7 +11,9 @@
 // 32x32 tile (parallel beam: one image line) x a group of slices, a cluster
 // each.  The adjoint's item bodies are the single-geometry ones
 // (dd2d_kernels.cuh), so its results are identical to per-instance calls; the
-// forward's sum the same overlaps (dd2d_fwd.cuh).
+// forward's sum the same overlaps (dd2d_fwd.cuh) in another order.  (One or two
+// slices of an arc fan are projected by prefix sums in a call of their own,
+// dd2d_prefix.cuh: there the two differ by those sums' rounding, 7e-7.)
 //
 // The data-consistency step x <- x - eta * A^T (A x - y) is four launches:
 // image tables, forward items writing the residual A x - y directly, detector

@@ -218,9 +218,10 @@ __device__ __forceinline__ float fan_fbp_weight(float sx, float sy, float px, fl
     return t * t;
 }
 
-// The longest lines of which 4 slices run in one CTA: what a prefix-table
-// forward with two buffers takes, at 8 warps of 31 bins.  (The limit of the
-// uneven batch's instances and of dd2d_fwd_shape's 4 slices.)
+// The longest lines for which dd2d_fwd_shape says 4 slices and the uneven batch
+// takes an instance: those of which 4 slices' prefix tables fit one CTA twice, at
+// 8 warps of 31 bins.  (A limit of the interface; how many slices a CTA then
+// takes is a matter of dd2d_fwd.cuh's fwd_fits.)
 inline long long four_slice_bytes(bool para, int D, int npix, int cl) {
     const int n = (D + kWarps * kBinsPerWarp - 1) / (kWarps * kBinsPerWarp);
     const int npass = n <= 1 ? 1 : n <= 2 ? 2 : n <= 3 ? 3 : n <= 4 ? 4 : 8;
@@ -241,14 +242,12 @@ __device__ __forceinline__ void init_bars(uint64_t *bar, int n = 2) {
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint-type kernel (ProjTrans, BackProj, BackProjWeighted): pixel gathers.
-// CTA = 32x32 image tile x kBI images; loops over all views, accumulating in
-// registers (row-major ownership for x-branch views, column-major for
-// y-branch views, merged through shared memory at the end).
+// Adjoint-type kernels (ProjTrans, BackProj, BackProjWeighted): pixel gathers.
 // ---------------------------------------------------------------------------
-constexpr int kLinesPerWarp = kTile / kWarps;   // 4
+constexpr int kLinesPerWarp = kTile / kWarps;   // fan beams: a thread's pixels
 
-// Fan: integral of the detector function up to u (clamped) for image b.
+// Fan: the detector bin of axis position u, by the inverse of the fan's map
+// (within one bin; fan_bin settles it on the exact boundaries).
 __device__ __forceinline__ void det_index_fan(int geom, const dd_geom2d &g, const DdView2 &vw,
                                               float view, float u, int *kk) {
     const int D = g.num_det;

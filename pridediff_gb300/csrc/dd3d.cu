@@ -380,9 +380,9 @@ struct Step3 {
 // read from global memory by the step's segments; where a column meets more
 // than kSeg, the consumers walk its record pixel by pixel.
 //
-// Bound by instruction issue (58 % of the slots, about 3,400 per line and CTA, a
-// third of them the producers') and the latency of a merge's dependent steps
-// at 30 warps an SM or fewer.  With every row's slices walked and
+// Bound by the latency of a merge's dependent steps at 20 to 33 warps an SM and by
+// instruction issue (53 to 56 % of the slots, about 3,300 per line and CTA, a
+// third of them the producers').  With every row's slices walked and
 // each of its segments' voxels gathered from global memory it was about four
 // times that.  2 x 256^3 cone beam, 36 views: 12.9 -> 4.1 ms; one 512 x 512 x
 // 128 volume, 96 spiral views: 12.6 -> 3.5 ms.  On the way: the sums of all
@@ -912,7 +912,8 @@ __global__ void __launch_bounds__(256) k_slab_views3(dd_geom3d g, char *plan, Pl
 // loaded once per segment, and a step is an overlap of the two intervals and
 // one multiply-add per volume.
 //
-// Bound by instruction issue on that walk and on finding each pixel's columns
+// Bound by the loads of the sinogram inside that walk (long scoreboard is the first
+// stall; 54 to 60 % of the issue slots are used) and by finding each pixel's columns
 // and boundaries, which ZS slices share.  One 512 x 512 x 128 volume, 1140
 // spiral views: 317 ms with a row search per slice, every walk block of every
 // view staged and searched, and 8 slices a thread; 192 ms with the carried
