@@ -516,6 +516,16 @@ static int launch_fwd_passes(const FwdCall &c, const float *in, int n, float *ro
     }
 }
 
+// Groups of 8 slices of the weighted transpose without its table.
+static int launch_fwd_each(const FwdCall &c, const float *in, int n, float *rows, float *cols, float *out, const float *sub) {
+    switch (pass_class(c.g->num_det)) {
+    case 1: return launch_fwd_group<kFanWeightedEach, 1, 8, false>(c, in, n, rows, cols, out, sub);
+    case 2: return launch_fwd_group<kFanWeightedEach, 2, 8, false>(c, in, n, rows, cols, out, sub);
+    case 3: return launch_fwd_group<kFanWeightedEach, 3, 8, false>(c, in, n, rows, cols, out, sub);
+    default: return launch_fwd_group<kFanWeightedEach, 4, 8, false>(c, in, n, rows, cols, out, sub);
+    }
+}
+
 // One or two slices of an arc fan (dd2d_prefix.cuh).
 template <int NPASS, int BI>
 static int launch_prefix_as(const FwdCall &c, int B, const float *in, float2 *tx, float2 *ty, float *out) {
@@ -565,11 +575,17 @@ static int launch_fwd(FwdCall c, bool single, int B, const float *in, char *rows
               : fwd_fits(KIND, D, lanes, npix, 2, c.cl, limit)                                ? 2
                                                                                                 : 1;
     }
+    // 8 slices fit, but not beside the weights of the line's pixels
+    const bool each = KIND == kFanWeighted && !single && big < 8 && c.sh == 0 && pass_class(D) <= 4 &&
+                      fwd_lay(kFanWeightedEach, D, lanes, npix, 8, c.cl).total <= max_smem_optin() / 2;
     int done = 0;
     while (done < B) {
         const int left = B - done;
         int nb = big, n = left / big * big;   // whole groups of the largest kind first
-        if (n == 0) {
+        if (each && left >= 8) {
+            nb = 8;
+            n = left / 8 * 8;
+        } else if (n == 0) {
             n = left;
             nb = left > 4 ? 8 : left > 2 ? 4 : left;
         }
@@ -578,7 +594,9 @@ static int launch_fwd(FwdCall c, bool single, int B, const float *in, char *rows
         const float *x = in + done * image;
         int st;
         switch (nb) {
-        case 8: st = launch_fwd_passes<KIND, 8>(c, x, n, r, k, o, sub); break;
+        case 8:
+            st = each ? launch_fwd_each(c, x, n, r, k, o, sub) : launch_fwd_passes<KIND, 8>(c, x, n, r, k, o, sub);
+            break;
         case 4: st = launch_fwd_passes<KIND, 4>(c, x, n, r, k, o, sub); break;
         case 2: st = launch_fwd_passes<KIND, 2>(c, x, n, r, k, o, sub); break;
         default: st = launch_fwd_passes<KIND, 1>(c, x, n, r, k, o, sub); break;

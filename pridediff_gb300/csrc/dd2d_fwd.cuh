@@ -53,8 +53,9 @@ static_assert(prods(1) <= stages(1) && prods(2) <= stages(2) && prods(4) <= stag
 
 // Proj of a fan beam; the weighted DD back-projector's transpose of a fan beam
 // (parts scaled per line and pixel); the parallel beam; the unweighted
-// transpose of a fan beam (parts scaled per line).
-enum { kFan = 0, kFanWeighted = 1, kPara = 2, kFanScaled = 3 };
+// transpose of a fan beam (parts scaled per line); the weighted one without its
+// table of weights.
+enum { kFan = 0, kFanWeighted = 1, kPara = 2, kFanScaled = 3, kFanWeightedEach = 4 };
 // Line records in flight per producer (the parallel beam's are twice as large).
 __host__ __device__ constexpr int recs(int kind) { return kind == kPara ? 2 : kMaxRecs; }
 
@@ -80,11 +81,11 @@ __host__ __device__ inline int plane_pitch(int n, int p) { return p == 1 ? (n + 
 // Flat fan, 1 / 8 slices, ms by prefix sums, a lane a bin, so.  512^2, 180 views:
 // 16 cells 0.22, 0.34; 1.02, 1.52; 0.18, 0.27.  64 cells 0.22, 0.35; 0.36, 0.54;
 // 0.19, 0.30.  128 cells 0.22, 0.36; 0.24, 0.37; 0.19, 0.32.  180 cells (3.4 pixels)
-// 0.22, 0.37; 0.21, 0.33; two lanes 0.21, 0.37.  1000^2, 90 views: 16 cells 0.39,
-// 0.61; 3.67, 5.56; 0.34, 0.61.  64 cells 0.40, 0.63; 1.14, 1.78; 0.37, 0.75.  180
-// cells (6.7 pixels) 0.39, 0.64; 0.52, 0.88; two lanes 0.43, 0.93: on lines of that
-// length 5 and more slices of wide cells stay 0.6 to 0.95 times as fast as they
-// were by prefix sums.
+// 0.22, 0.37; 0.21, 0.33; two lanes 0.21, 0.37.  1000^2, 360 views: 16 cells 0.49,
+// 1.98; 6.3, 12.5; 0.72, 1.50.  100 cells 0.49, 2.00; 1.41, 2.86; 0.96, 2.00.
+// (Prefix sums ask for nothing per pixel but the tables' build: where views fill
+// the chip they stay ahead for 1 to 4 slices of cells wider than 3 pixels -- 512^2,
+// 720 views, 64 cells, 1 / 4 / 8 slices 0.45, 0.59, 1.07; so 0.55, 0.70, 0.90.)
 inline int fwd_lanes(int geom, const dd_geom2d &g) {
     const bool para = geom == DD_GEOM_PARA;
     const double cell = para                   ? (double)g.det_size
@@ -268,8 +269,9 @@ __device__ __forceinline__ void fill_boundaries(const DdLine &L, float *t, int l
 // weight per overlap / here: 512^2, 360 views, 736 bins 0.83, 1.29, 2.50, 4.69
 // / 0.76, 0.88, 1.25, 2.26 / 0.45, 0.59, 0.80, 1.53; 300^2, 200 views, 1,200
 // bins 0.44, 0.59, 1.12, 2.11 / 0.51, 0.75, 1.18, 2.24 / 0.27, 0.43, 0.69, 1.29.
-// (The table takes lines of 900 to 1,000 pixels from 8 slices to 4: 1000^2, 60
-// views, 900 bins, 16 slices 5.1 / 1.27 / 1.61; 8 slices 2.6 / 1.05 / 0.84.)
+// Lines of 900 to 1,000 pixels leave no room for 8 slices beside it: whole groups
+// of 8 weigh each overlap there (kFanWeightedEach; 1000^2, 360 views, 900 bins, 8 /
+// 16 slices 10.6, 18.5 / 3.3, 5.9, by groups of 4 with the table 3.9, 7.4).
 template <int GEOM>
 __device__ __forceinline__ void fill_weights(const dd_geom2d &g, const DdView2 &vw, int line, int i0, int nend, float *wt,
                                              int lane) {
@@ -440,6 +442,12 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
                 const int idet0 = __float_as_int(h1.z);
                 const int i0 = __float_as_int(h1.x), last = i0 + n - 1;
                 const float *bt = reinterpret_cast<const float *>(smem + L.bnd + st * L.bnd_b) + kB0;
+                float lpos = 0.0f;
+                if (KIND == kFanWeightedEach) {
+                    const int line = line_of(i);
+                    lpos = xb ? pix_centre(0.5f * (float)g.height - (float)line - 0.5f, g.pix_y, g.pix_yshift)
+                              : pix_centre((float)line - 0.5f * (float)g.width + 0.5f, g.pix_x, g.pix_xshift);
+                }
                 // the detector's boundaries, or the pixels' weights
                 const float *dt = reinterpret_cast<const float *>(smem + L.det + st * L.det_b) + (KIND == kPara ? kB0 : 0);
                 const float *pix = reinterpret_cast<const float *>(smem + L.pix + st * L.pix_b);
@@ -467,6 +475,13 @@ __device__ bool fwd_item(const dd_geom2d &g, int geom, int op, const FwdItem &it
                         if (!(w > 0.0f)) return;
                         if (KIND != kFan) w *= h1.w;
                         if (KIND == kFanWeighted) w *= dt[j + i];
+                        if (KIND == kFanWeightedEach) {
+                            const float pc = pix_centre((float)(j + i) + 0.5f, xb ? g.pix_x : g.pix_y, vwp->axis0);
+                            const float cx = xb ? pc : lpos, cy = xb ? lpos : pc;
+                            w *= geom == DD_GEOM_ARC
+                                     ? fan_fbp_weight<DD_GEOM_ARC>(vwp->srcx, vwp->srcy, cx, cy, g.iso_source)
+                                     : fan_fbp_weight<DD_GEOM_FLAT>(vwp->srcx, vwp->srcy, cx, cy, g.iso_source);
+                        }
                         acc[m].add(w, pix + (j + i) * P, pitch * P);
                     };
                     if constexpr (!WIDE) {

@@ -170,6 +170,23 @@ def test_weighted_transpose(oracle_mod, geom, W, H, D, cell, B):
     assert np.any(ref) and rel_l2(run2d(geom, "bproj_tw", x, ang, opt), ref) <= 1e-5
 
 
+# Lines that leave 8 slices no room beside that table: groups of 8 weigh each
+# overlap, the slices left over (none to 7) take the table's weights.
+@pytest.mark.parametrize("W,H,D,B", [(950, 4, 200, 8), (4, 950, 420, 16), (1000, 5, 650, 9), (930, 3, 900, 11), (900, 7, 1000, 15)])
+@pytest.mark.parametrize("geom", ["flat", "arc"])
+def test_weighted_transpose_groups_of_eight(oracle_mod, geom, W, H, D, B):
+    pix = 0.7 * 1000.0 / max(W, H)
+    det = 1200.0 / D * pix * {"flat": 1085.6 / 595.0, "arc": 1.0 / 595.0}[geom]
+    opt = [W, H, D, pix, 0.9 * pix, det, 595.0, 1085.6, 0.1, -0.2, 0.1 * det]
+    ang = (np.arange(5) * 2 * np.pi / 5 + 0.1).astype(np.float32)
+    x = np.random.default_rng(D).random((B, H, W), dtype=np.float32)
+    ref = oracle_mod.run2d(geom, "bproj_tw", x, ang, opt, nthreads=8)
+    out = run2d(geom, "bproj_tw", x, ang, opt)
+    assert np.any(ref) and rel_l2(out, ref) <= 1e-5
+    for b in (0, 7, B - 1):
+        assert rel_l2(run2d(geom, "bproj_tw", x[b:b + 1], ang, opt)[0], out[b]) <= 2e-6   # the same terms, their rounding aside
+
+
 # 2-D forward, bins of more than four pixels: 1 to 32 lanes a bin and up to 4
 # passes of 256 lanes; each slice as it is alone, whatever the group it is in.
 @pytest.mark.parametrize("W,H,D,cell", [(150, 97, 3, 45.0), (150, 97, 8, 20.0), (260, 130, 16, 17.0), (200, 150, 32, 7.0), (200, 97, 40, 5.2),
